@@ -10,6 +10,7 @@ Data is synthetic: N(0, 1) tokens, softmax routing weights, N(0, 0.02) layer wei
     prepare / run   inputs and kept state of a case / one pass
     work            bytes and operations that one pass cannot do without
     tolerance       how far the outputs of another correct implementation may be off
+    exact           the computed outputs in 64 bits, without this library's code
 """
 import math
 
@@ -303,3 +304,65 @@ def tolerance(case):
         return {'rel': 1e-3, 'max': 0.03}
     # Permuting the reduction dimensions gives up to 9.7e-4 / 2.3e-2 (token gradient, weight gradient of the bf16 backward pass)
     return {'rel': 4e-3, 'max': 0.1}
+
+
+# ----------------------------------------------------------------------------------------------------------------- exact
+def _exact_moe(x, idx, w, w13, w2, grad=None):
+    """The SwiGLU expert layer and its gradients in 64 bits, one expert at a time."""
+    I = w2.shape[2]
+    out, dx, dw = (torch.zeros(t.shape, dtype=torch.float64, device='cuda') for t in (x, x, w))
+    dw13, dw2 = [], []
+    for e in range(w2.shape[0]):
+        t, k = (idx == e).nonzero(as_tuple=True)
+        a13, a2, xe, we = w13[e].double(), w2[e].double(), x[t].double(), w[t, k].double().unsqueeze(1)
+        h = xe @ a13.t()
+        gate, up = h[:, :I], h[:, I:]
+        sig = torch.sigmoid(gate)
+        act = gate * sig * up
+        y = act @ a2.t()
+        out.index_add_(0, t, we * y)
+        if grad is None:
+            continue
+        g = grad[t].double()
+        dw[t, k] = (g * y).sum(1)
+        d_act = (we * g) @ a2
+        dh = torch.cat([d_act * up * sig * (1 + gate * (1 - sig)), d_act * gate * sig], dim=1)
+        dx.index_add_(0, t, dh @ a13)
+        dw2.append((we * g).t() @ act)
+        dw13.append(dh.t() @ xe)
+    return out if grad is None else dict(out=out, dx=dx, dw=dw, dw13=torch.stack(dw13), dw2=torch.stack(dw2))
+
+
+def exact(case, seed):
+    """The computed outputs of ``run`` from the same inputs in 64 bits; ``None`` where an output is a copy or a cast."""
+    c = case
+    torch.manual_seed(seed)
+    gen = torch.Generator(device='cuda').manual_seed(seed)
+    if c['kind'] == 'gemm':
+        s = _prepare_gemm(c, gen)
+        return s['a'].double() @ s['b'].double().t()
+    T, H, K, E = c['tokens'], c['hidden'], c['topk'], c['experts']
+    if c['kind'] == 'ep':
+        if not c['expand']:
+            return None
+        idx, w = _routing(gen, T, E, K, c['masked'], c['zipf'])
+        _bf16(gen, T, H)
+        y = _bf16(gen, T * K + E * 127, H)
+        out, row0 = torch.zeros(T, H, dtype=torch.float64, device='cuda'), 0
+        for e in range(E):
+            t, k = (idx == e).nonzero(as_tuple=True)            # rows of an expert: in token order, segments 128-aligned
+            out.index_add_(0, t, w[t, k].double().unsqueeze(1) * y[row0:row0 + t.numel()].double())
+            row0 += (t.numel() + 127) // 128 * 128
+        return dict(recv=None, counts=None, out=out)
+    if c['kind'] == 'll':
+        idx, w = _routing(gen, T, E, K)
+        return dict(count=None, out=_bf16(gen, T, H).double() * w.double().sum(1, keepdim=True))
+    I = c['inter']
+    if c['kind'] == 'll_moe':
+        idx, w = _routing(gen, T, E, K)
+        w13, w2 = _bf16(gen, E, 2 * I, H, std=0.02), _bf16(gen, E, H, I, std=0.02)
+        return dict(count=None, out=_exact_moe(_bf16(gen, T, H), idx, w, w13, w2))
+    w13, w2 = _bf16(gen, E, 2 * I, H, std=0.02), _bf16(gen, E, H, I, std=0.02)
+    idx, w = _routing(gen, T, E, K)
+    x = _bf16(gen, T, H)
+    return _exact_moe(x, idx, w, w13, w2, None if c['mode'] == 'infer' else _bf16(gen, T, H))
