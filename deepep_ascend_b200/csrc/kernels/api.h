@@ -315,6 +315,17 @@ struct SwigluQuantArgs {
     int rows, inter;
 };
 
+// w [groups, n, k] (bf16 or fp32, contiguous, k % 8 == 0) -> e4m3 [groups, n, k] with one fp32 scale per 128 x 128 block,
+// sf [groups, ceil(n / 128), ceil(k / 128)]
+struct WeightQuantArgs {
+    const void* w;
+    int w_is_f32;
+    void* q;
+    float* sf;
+    int64_t groups;
+    int n, k;
+};
+
 // Element-wise kernels of the MoE backward pass.  Each also writes the TRANSPOSE of its result ([channels, rows]),
 // which is the K-major operand layout the weight-gradient GEMM needs (K = rows), so no separate transpose pass runs.
 // `valid` (one byte per row, 0 = alignment padding row) zeroes the results of padding rows.  rows % 64 == 0.
@@ -399,6 +410,7 @@ cudaError_t launch_local_expand_plan(const LocalExpandPlanArgs& args, cudaStream
 cudaError_t launch_local_expand_copy(const LocalExpandCopyArgs& args, cudaStream_t stream);
 cudaError_t launch_local_reduce(const LocalReduceArgs& args, cudaStream_t stream);
 cudaError_t launch_expert_segments(const ExpertSegmentsArgs& args, cudaStream_t stream);
+cudaError_t launch_weight_quant(const WeightQuantArgs& args, cudaStream_t stream);
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& args, cudaStream_t stream);
 cudaError_t launch_moe_bwd(const MoeBwdArgs& args, cudaStream_t stream);
 int moe_bwd_prep_col_blocks(int cols);   // PREP writes row_dot as [col_blocks, rows] partial sums

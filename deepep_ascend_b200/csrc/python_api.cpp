@@ -338,6 +338,26 @@ at::Tensor local_reduce(const at::Tensor& pos, const at::Tensor& y, const std::o
     return res;
 }
 
+// Weights [G, N, K] (bf16 or fp32, contiguous, K % 8 == 0, 16-byte aligned) -> (e4m3 [G, N, K], fp32 scales of the 128 x 128 blocks)
+std::vector<at::Tensor> quantize_weight_blocks(const at::Tensor& w) {
+    TORCH_CHECK(w.is_cuda() && w.dim() == 3 && w.is_contiguous() && (w.scalar_type() == at::kBFloat16 || w.scalar_type() == at::kFloat),
+                "w must be contiguous bf16 or fp32 [G, N, K]");
+    const int64_t G = w.size(0), N = w.size(1), K = w.size(2);
+    TORCH_CHECK(K % 8 == 0 && N < (1ll << 31) && K < (1ll << 31), "K must be a multiple of 8");
+    at::Tensor q = at::empty({G, N, K}, w.options().dtype(at::kFloat8_e4m3fn));
+    at::Tensor sf = at::empty({G, (N + 127) / 128, (K + 127) / 128}, w.options().dtype(at::kFloat));
+    WeightQuantArgs a{};
+    a.w = w.data_ptr();
+    a.w_is_f32 = w.scalar_type() == at::kFloat;
+    a.q = q.data_ptr();
+    a.sf = sf.data_ptr<float>();
+    a.groups = G;
+    a.n = static_cast<int>(N);
+    a.k = static_cast<int>(K);
+    cuda_check(ep::launch_weight_quant(a, at::cuda::getCurrentCUDAStream()), "weight cast launch");
+    return {q, sf};
+}
+
 // Weight gradients of a grouped layer: out[e] = a_t[:, k0:k1] @ b_t[:, k0:k1]^T with (k0, k1) = k_off[e], k_off[e + 1]
 // (a_t [M, K_total], b_t [N, K_total] bf16, K = rows of the expert segment; k_off int32 [G + 1], multiples of 64).
 at::Tensor gemm_kgrouped(const at::Tensor& a_t, const at::Tensor& b_t, const at::Tensor& k_off, int64_t num_sms) {
@@ -677,6 +697,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("w") = py::none());
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("expert_segments", &expert_segments, py::arg("psum_ends"), py::arg("num_rows"), py::arg("alignment") = 128);
+    m.def("quantize_weight_blocks", &quantize_weight_blocks);
     m.def("swiglu_quant", &swiglu_quant, py::arg("h"), py::arg("keep_bf16") = false);
     m.def("gemm_kgrouped", &gemm_kgrouped, py::arg("a_t"), py::arg("b_t"), py::arg("k_off"), py::arg("num_sms") = 0);
     m.def("moe_bwd_prep", &moe_bwd_prep);

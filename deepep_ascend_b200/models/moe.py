@@ -216,8 +216,8 @@ class FusedMoE(nn.Module):
 
     def fp8_weights(self):
         if self._fp8 is None or self._fp8[0] != self._versions():
-            q13, s13 = G.quantize_weight_blocks(self.w13.detach().float())
-            q2, s2 = G.quantize_weight_blocks(self.w2.detach().float())
+            q13, s13 = G.quantize_weight_blocks(self.w13.detach())
+            q2, s2 = G.quantize_weight_blocks(self.w2.detach())
             self._fp8 = (self._versions(), (q13, s13, q2, s2))
         return self._fp8[1]
 

@@ -31,9 +31,27 @@ def grouped_gemm_nt(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, 
     return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer))
 
 
+def _plain_cuda(t: torch.Tensor) -> bool:
+    """A tensor that a kernel of this library may read in place of a differentiable / traceable PyTorch statement: on the current
+    GPU, not traced or wrapped by a function transform, and with no gradient or tangent to carry on."""
+    return (t.is_cuda and type(t) in (torch.Tensor, torch.nn.Parameter) and t.device.index == torch.cuda.current_device() and
+            not (t.requires_grad and torch.is_grad_enabled()) and torch.autograd.forward_ad._current_level < 0 and
+            not torch.compiler.is_compiling() and not torch._C._functorch.is_functorch_wrapped_tensor(t))
+
+
 def quantize_weight_blocks(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """``w [G, N, K]`` -> (e4m3 ``[G, N, K]``, fp32 scales ``[G, ceil(N/128), ceil(K/128)]``), one scale per
-    128 x 128 block (the weight format of DeepSeek-V3 style FP8 training)."""
+    128 x 128 block (the weight format of DeepSeek-V3 style FP8 training).  One kernel for contiguous bf16 / fp32 weights on a
+    GPU whose rows are whole 16-byte pieces; anything else takes the PyTorch statement below, which gives the same bits."""
+    if (_plain_cuda(w) and w.dtype in (torch.bfloat16, torch.float32) and w.dim() == 3 and w.is_contiguous() and w.shape[2] % 8 == 0 and
+            w.data_ptr() % 16 == 0):
+        q, sf = _native.load().quantize_weight_blocks(w)
+        return q, sf
+    return quantize_weight_blocks_ref(w)
+
+
+def quantize_weight_blocks_ref(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """The same cast stated with plain PyTorch operations (any device; what the kernel is tested against)."""
     G, N, K = w.shape
     nb, kb = (N + 127) // 128, (K + 127) // 128
     wp = torch.zeros(G, nb * 128, kb * 128, device=w.device, dtype=torch.float32)

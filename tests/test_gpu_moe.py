@@ -332,3 +332,26 @@ def test_fused_moe_on_a_buffer_without_expand_regions():
         assert calc_diff(layer.w13.grad.float(), w13.grad) < 3e-3 and calc_diff(w.grad, wr.grad) < 3e-3
     finally:
         buf.destroy()
+
+
+@pytest.mark.parametrize('G,N,K', [(1, 128, 128), (3, 8, 8), (2, 129, 136), (2, 384, 2056), (1, 127, 7168)])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+def test_weight_block_cast_matches_pytorch(G, N, K, dtype):
+    """The one-pass cast has the bits of the PyTorch statement: ragged edge blocks, an all-zero block (clamped amax), a block
+    with an infinity, one with a NaN, and subnormal values."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(N + K)
+    w = (torch.randn(G, N, K, device='cuda') * 0.02).to(dtype)
+    w[0, :128, :128] = 0
+    w[-1, -1, -1] = 1e-39
+    cases = [w]
+    for special in (float('inf'), float('nan'), -float('inf')):
+        v = w.clone()
+        v[0, N // 2, K // 2] = special
+        cases.append(v)
+    for v in cases:
+        q, sf = ops.quantize_weight_blocks(v)
+        q_ref, sf_ref = ops.quantize_weight_blocks_ref(v.float())
+        assert q.shape == q_ref.shape and sf.shape == sf_ref.shape
+        assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8))
+        assert torch.equal(sf.view(torch.int32), sf_ref.view(torch.int32))
