@@ -296,6 +296,9 @@ struct GemmArgs {
     // k0 = k_group_off[e], k1 = k_group_off[e + 1] (device array of num_groups + 1 multiples of 64); C is
     // [num_groups * M, N]; an empty range gives zeros.  bf16 only; null when unused.
     const int32_t* k_group_off;
+    // bf16 operands stored MN-major (K rows of contiguous elements), read through the tensor core's transposing descriptors:
+    // 0 none; 1 B is [num_groups][K, N] (row stride ldb); 2 (with k_group_off) A is [K, M] and B is [K, N]
+    int mn_operands;
 };
 enum { EP_GEMM_FUSE_NONE = 0, EP_GEMM_FUSE_ALL_GATHER = 1, EP_GEMM_FUSE_REDUCE_SCATTER = 2 };
 
@@ -326,10 +329,12 @@ struct WeightQuantArgs {
     int n, k;
 };
 
-// Element-wise kernels of the MoE backward pass.  Each also writes the TRANSPOSE of its result ([channels, rows]),
-// which is the K-major operand layout the weight-gradient GEMM needs (K = rows), so no separate transpose pass runs.
-// `valid` (one byte per row, 0 = alignment padding row) zeroes the results of padding rows.  rows % 64 == 0.
-enum { EP_MOE_BWD_PREP = 0, EP_MOE_BWD_SWIGLU = 1, EP_MOE_BWD_DEQUANT_T = 2 };
+// Element-wise kernels of the MoE backward pass.  `valid` (one byte per row, 0 = alignment padding row) zeroes the results of
+// padding rows.  PREP, SWIGLU and DEQUANT_T also write the TRANSPOSE of their result ([channels, rows]: the K-major operand of
+// `gemm_kgrouped`) and need rows % 64 == 0.  The *_ROWS operations write row-major results only (the operands of
+// `gemm_kgrouped_tn`), any number of rows, cols % 8 == 0 (DEQUANT_ROWS: % 16).
+enum { EP_MOE_BWD_PREP = 0, EP_MOE_BWD_SWIGLU = 1, EP_MOE_BWD_DEQUANT_T = 2, EP_MOE_BWD_SWIGLU_ROWS = 3, EP_MOE_BWD_DEQUANT_ROWS = 4,
+       EP_MOE_BWD_WEIGHT_ROWS = 5 };
 struct MoeBwdArgs {
     int op;
     int rows, cols;               // PREP / DEQUANT_T: cols = hidden; SWIGLU: cols = intermediate size I
@@ -343,13 +348,19 @@ struct MoeBwdArgs {
     //       optional row_dot[b * rows + row] = sum over the 64 columns of block b of d_act * activation (before w)
     // DEQUANT_T: y = q [rows, H] e4m3, w = scales (row, 128-block) at w[row * sf_stride_row + blk * sf_stride_col]
     //       -> out_t = (q * scale)^T [H, rows] bf16
+    // SWIGLU_ROWS: g, y, w as SWIGLU (w required) -> out = d_h [rows, 2I], out2 = silu(gate) * up [rows, I],
+    //       row_dot[row] = sum of d_act * activation
+    // DEQUANT_ROWS: y, w as DEQUANT_T, optional row_w -> out = q * (scale * row_w[row]) [rows, H] bf16
+    // WEIGHT_ROWS: g [rows, H], row_w -> out = g * row_w[row]
     const void* g;
     const void* y;
     const float* w;
+    const float* row_w;
     int64_t sf_stride_row, sf_stride_col;
     void* out;
     void* out_t;
     void* out2_t;
+    void* out2;
     float* row_dot;
 };
 

@@ -12,6 +12,10 @@
 // 128-channel block is accumulated into its own TMEM buffer and promoted into fp32 registers with its scale by
 // EIGHT epilogue warps (two per TMEM lane quadrant, 64 columns each, both tcgen05.ld of a block in flight before one
 // wait); four TMEM buffers let the MMAs run up to three blocks ahead of the promotion.
+// MN-major bf16 operands (`mn_operands`): the backward pass of a layer reads weights, activations and gradients row-major as the
+// forward pass left them (64 x 64 TMA boxes, transposing descriptors), at the rate of the K-major kernel: 2.3 ms for the two data
+// gradients and 2.6 ms for the two weight gradients of 34816 rows x (7168, 2 x 2048) bf16.  Transposed copies of the weights
+// cost 5.6 ms per training step, those of the activations 0.3 ms.
 // Grouped (MoE) use: `tile_group[m_tile]` selects the expert whose weights multiply that 128-row tile.
 // Every pipeline wait is bounded; on expiry the kernel raises `*error`, leaves its loops and frees its TMEM.
 #include <cuda.h>
@@ -168,7 +172,9 @@ struct PipeState {
     }
 };
 
-template <bool kFp8, int kBlockN>
+// kMnOperands: how many operands are MN-major (bf16 only).  0: A [M, K], B [N, K].  1: B is [K, N] (data gradients read the forward
+// weights as they are).  2: A is [K, M] too (weight gradients read row-major activations and gradients as they are).
+template <bool kFp8, int kBlockN, int kMnOperands>
 __global__ void __launch_bounds__(gemm_threads(kFp8, kBlockN), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -186,7 +192,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kBlockK = kFp8 ? 128 : 64;          // elements per 128-byte row
     constexpr int kUmmaK = kFp8 ? 32 : 16;            // elements per tcgen05.mma (32 bytes of K)
-    constexpr uint32_t kIdesc = umma::make_instr_desc(kBlockM, kBlockN, kFp8 ? umma::kFormatE4M3 : umma::kFormatBF16);
+    static_assert(kMnOperands == 0 || (!kFp8 && kBlockN % 64 == 0), "MN-major operands: bf16, whole 64-element chunks");
+    constexpr uint32_t kIdesc =
+        umma::make_instr_desc(kBlockM, kBlockN, kFp8 ? umma::kFormatE4M3 : umma::kFormatBF16, kMnOperands >= 2, kMnOperands >= 1);
     const int num_m = (g.M + kBlockM - 1) / kBlockM, num_n = (g.N + kBlockN - 1) / kBlockN;
     const int num_k = (g.K + kBlockK - 1) / kBlockK;
     const int num_tiles = num_m * num_n * (g.k_group_off != nullptr ? g.num_groups : 1);
@@ -266,8 +274,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         ok = wait_bar(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
                         if (!ok) break;
                         ptx::mbar_arrive_expect_tx(&sm->full[p.stage], kTileBytes + kTileBytesB);
-                        umma::tma_load_2d(s_a + p.stage * kTileBytes, &map_a, kb * kBlockK, m_blk * kBlockM, &sm->full[p.stage]);
-                        umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, grp * g.N + n_blk * kBlockN, &sm->full[p.stage]);
+                        if constexpr (kMnOperands >= 2) {
+#pragma unroll
+                            for (int i = 0; i < kBlockM / 64; ++i)
+                                umma::tma_load_3d(s_a + p.stage * kTileBytes + i * umma::kMnChunkBytes, &map_a, m_blk * kBlockM + i * 64, kb * kBlockK, 0,
+                                                  &sm->full[p.stage]);
+                        } else {
+                            umma::tma_load_2d(s_a + p.stage * kTileBytes, &map_a, kb * kBlockK, m_blk * kBlockM, &sm->full[p.stage]);
+                        }
+                        if constexpr (kMnOperands >= 1) {
+#pragma unroll
+                            for (int i = 0; i < kBlockN / 64; ++i)
+                                umma::tma_load_3d(s_b + p.stage * kTileBytesB + i * umma::kMnChunkBytes, &map_b, n_blk * kBlockN + i * 64, kb * kBlockK, grp,
+                                                  &sm->full[p.stage]);
+                        } else {
+                            umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, grp * g.N + n_blk * kBlockN, &sm->full[p.stage]);
+                        }
                         p.advance();
                     }
                 }
@@ -295,13 +317,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         ok = wait_bar(&sm->full[p.stage], p.phase, sm, g, 4);
                         if (!ok) break;
                         umma::fence_after_thread_sync();
-                        const uint64_t desc_a = umma::make_smem_desc_sw128(s_a + p.stage * kTileBytes);
-                        const uint64_t desc_b = umma::make_smem_desc_sw128(s_b + p.stage * kTileBytesB);
+                        const uint64_t desc_a = kMnOperands >= 2 ? umma::make_smem_desc_mn_sw128(s_a + p.stage * kTileBytes)
+                                                                 : umma::make_smem_desc_sw128(s_a + p.stage * kTileBytes);
+                        const uint64_t desc_b = kMnOperands >= 1 ? umma::make_smem_desc_mn_sw128(s_b + p.stage * kTileBytesB)
+                                                                 : umma::make_smem_desc_sw128(s_b + p.stage * kTileBytesB);
+                        // 16 (bf16) / 32 (e4m3) elements of K: 32 bytes along a K-major row, 16 K rows of 128 bytes otherwise
+                        constexpr int kStepA = kMnOperands >= 2 ? kUmmaK * 128 : 32, kStepB = kMnOperands >= 1 ? kUmmaK * 128 : 32;
 #pragma unroll
                         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
                             const uint32_t accumulate = kFp8 ? (k != 0) : (kb != tw.kb0 || k != 0);
-                            umma::mma_ss<kFp8>(tmem_base + acc * kBlockN, umma::advance_desc_k(desc_a, k * 32), umma::advance_desc_k(desc_b, k * 32),
-                                               kIdesc, accumulate);
+                            umma::mma_ss<kFp8>(tmem_base + acc * kBlockN, umma::advance_desc_k(desc_a, k * kStepA),
+                                               umma::advance_desc_k(desc_b, k * kStepB), kIdesc, accumulate);
                         }
                         umma::mma_commit(&sm->empty[p.stage]);       // the stage may be refilled once these MMAs are done
                         p.advance();
@@ -653,6 +679,19 @@ bool make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// MN-major operand [groups, K, mn] bf16 with contiguous mn: box = 64 elements of mn x 64 K rows of one group, 128B swizzle.  The
+// group is a dimension of its own so that K rows past the end of one group read as zero and not as the next group's.
+bool make_mn_operand_map(CUtensorMap* map, const void* base, int64_t groups, int64_t k, int64_t mn, int64_t ld_elems) {
+    EncodeTiledFn encode = get_encode_fn();
+    if (encode == nullptr) return false;
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(mn), static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(groups)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld_elems * 2), static_cast<cuuint64_t>(ld_elems * k * 2)};
+    const cuuint32_t box[3] = {64, 64, 1};
+    const cuuint32_t elem_strides[3] = {1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace
 
 cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
@@ -661,13 +700,14 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     if ((g.lda * elem) % 16 != 0 || (g.ldb * elem) % 16 != 0 || g.ldc % 8 != 0 || g.N % 8 != 0) return cudaErrorInvalidValue;
     if (reinterpret_cast<uintptr_t>(g.a) % 16 != 0 || reinterpret_cast<uintptr_t>(g.b) % 16 != 0 || reinterpret_cast<uintptr_t>(g.c) % 16 != 0)
         return cudaErrorInvalidValue;
+    // MN-major operands come in whole 64-element chunks, so they have no 224-column variant.
     // 128 x 256 output tiles (fewer A re-reads, longer MMAs); the reduce-scatter epilogue (which stages 128-column rows)
     // and narrow outputs use 128 x 128 tiles.  The bf16 kernel also has 128 x 224 tiles and takes them when they need less
     // tensor-core time: fewer idle CTAs in the last wave (8192 x 7168: 1792 tiles of 256 columns are 12.1 waves of 148
     // CTAs, paid as 13; 2048 tiles of 224 columns are 13.8 waves of 7/8 the length), or no half-empty last column tile
     // (N = 896 = 4 x 224).
     int block_n = (g.fuse != EP_GEMM_FUSE_REDUCE_SCATTER && g.N >= 256) ? 256 : 128;
-    if (block_n == 256 && !g.is_fp8) {
+    if (block_n == 256 && !g.is_fp8 && g.mn_operands == 0) {
         const int64_t num_m_tiles = (g.M + kBlockM - 1) / kBlockM, groups = g.k_group_off != nullptr ? g.num_groups : 1;
         const int64_t workers = std::max(1, (num_sms < 1 ? 1 : num_sms) - (g.fuse == EP_GEMM_FUSE_ALL_GATHER ? g.num_copy_ctas : 0));
         auto cost = [&](int bn) {
@@ -676,14 +716,22 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         };
         if (cost(224) < cost(256)) block_n = 224;
     }
+    if (g.mn_operands < 0 || g.mn_operands > 2 || (g.mn_operands != 0 && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE))) return cudaErrorInvalidValue;
+    if ((g.mn_operands == 2) != (g.k_group_off != nullptr && g.mn_operands != 0)) return cudaErrorInvalidValue;
     CUtensorMap map_a, map_b;
-    if (!make_operand_map(&map_a, g.a, g.M, g.K, g.lda, g.is_fp8, 128) ||
-        !make_operand_map(&map_b, g.b, static_cast<int64_t>(g.k_group_off != nullptr ? 1 : g.num_groups) * g.N, g.K, g.ldb, g.is_fp8, block_n))
-        return cudaErrorInvalidValue;
-    const void* fn = g.is_fp8 ? (block_n == 256 ? (const void*)gemm_kernel<true, 256> : (const void*)gemm_kernel<true, 128>)
-                              : (block_n == 256   ? (const void*)gemm_kernel<false, 256>
-                                 : block_n == 224 ? (const void*)gemm_kernel<false, 224>
-                                                  : (const void*)gemm_kernel<false, 128>);
+    const int64_t b_groups = g.k_group_off != nullptr ? 1 : g.num_groups;
+    const bool maps_ok = (g.mn_operands >= 2 ? make_mn_operand_map(&map_a, g.a, 1, g.K, g.M, g.lda)
+                                             : make_operand_map(&map_a, g.a, g.M, g.K, g.lda, g.is_fp8, 128)) &&
+                         (g.mn_operands >= 1 ? make_mn_operand_map(&map_b, g.b, b_groups, g.K, g.N, g.ldb)
+                                             : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, block_n));
+    if (!maps_ok) return cudaErrorInvalidValue;
+    const void* fn;
+    if (g.mn_operands == 2) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 2> : (const void*)gemm_kernel<false, 128, 2>;
+    else if (g.mn_operands == 1) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 1> : (const void*)gemm_kernel<false, 128, 1>;
+    else if (g.is_fp8) fn = block_n == 256 ? (const void*)gemm_kernel<true, 256, 0> : (const void*)gemm_kernel<true, 128, 0>;
+    else fn = block_n == 256   ? (const void*)gemm_kernel<false, 256, 0>
+              : block_n == 224 ? (const void*)gemm_kernel<false, 224, 0>
+                               : (const void*)gemm_kernel<false, 128, 0>;
     const int kGemmSmemBytes = gemm_smem_bytes(block_n, g.is_fp8 != 0);
     cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
     if (err != cudaSuccess) return err;

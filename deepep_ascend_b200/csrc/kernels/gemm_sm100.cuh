@@ -3,7 +3,7 @@
 //   * shared-memory matrix descriptors for K-major operands written by TMA with the 128-byte swizzle,
 //   * the 32-bit instruction descriptor of tcgen05.mma (kind::f16 and kind::f8f6f4, fp32 accumulate),
 //   * TMEM allocation, tcgen05.mma / commit / ld / fences,
-//   * 2-D tiled TMA loads (never multicast).
+//   * 2-D and 3-D tiled TMA loads (never multicast).
 #pragma once
 #include <cuda.h>
 #include <stdint.h>
@@ -27,14 +27,29 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(const void* smem_tile) 
     desc |= 2ull << 61;
     return desc;
 }
+// MN-major operand (K rows of contiguous M or N elements), 128B swizzle: the tile lies in shared memory as chunks of 64 bf16
+// (128 bytes) along M / N, each chunk kMnChunkBytes = 64 K rows x 128 bytes, exactly what one 64 x 64 TMA box writes.
+//   leading byte offset = distance of two chunks along M / N      stride byte offset = 1024: eight K rows to the next eight
+// One MMA takes 16 K rows = 2048 bytes of every chunk.
+constexpr int kMnChunkBytes = 64 * 128;
+__device__ __forceinline__ uint64_t make_smem_desc_mn_sw128(const void* smem_tile) {
+    const uint64_t addr = ptx::smem_u32(smem_tile);
+    uint64_t desc = 0;
+    desc |= (addr & 0x3ffffull) >> 4;
+    desc |= static_cast<uint64_t>(kMnChunkBytes >> 4) << 16;
+    desc |= (1024ull >> 4) << 32;
+    desc |= 1ull << 46;
+    desc |= 2ull << 61;
+    return desc;
+}
 // advance a K-major SW128 descriptor by `bytes` along K inside the 128-byte swizzle row (bytes < 128)
 __device__ __forceinline__ uint64_t advance_desc_k(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
 
-// 32-bit instruction descriptor: D fp32, A/B K-major, dense.
+// 32-bit instruction descriptor: D fp32, dense.
 //   bits [4,6) D format: 1 = F32     bits [7,10) A format     bits [10,13) B format   (kind::f16: 0 F16, 1 BF16;
-//   kind::f8f6f4: 0 E4M3, 1 E5M2)    bits [17,23) N >> 3      bits [24,29) M >> 4
-__host__ __device__ constexpr uint32_t make_instr_desc(int m, int n, int ab_format) {
-    return (1u << 4) | (static_cast<uint32_t>(ab_format) << 7) | (static_cast<uint32_t>(ab_format) << 10) |
+//   kind::f8f6f4: 0 E4M3, 1 E5M2)    bit 15 / 16 A / B is MN-major    bits [17,23) N >> 3      bits [24,29) M >> 4
+__host__ __device__ constexpr uint32_t make_instr_desc(int m, int n, int ab_format, bool a_mn_major = false, bool b_mn_major = false) {
+    return (1u << 4) | (a_mn_major ? 1u << 15 : 0u) | (b_mn_major ? 1u << 16 : 0u) | (static_cast<uint32_t>(ab_format) << 7) | (static_cast<uint32_t>(ab_format) << 10) |
            (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 constexpr int kFormatBF16 = 1;   // kind::f16
@@ -116,6 +131,13 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
             ptx::smem_u32(smem_dst)),
         "l"(map), "r"(ptx::smem_u32(bar)), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+            ptx::smem_u32(smem_dst)),
+        "l"(map), "r"(ptx::smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {

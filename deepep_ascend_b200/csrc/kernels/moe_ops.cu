@@ -384,6 +384,111 @@ __global__ void __launch_bounds__(kTileThreads) moe_bwd_dequant_t_kernel(const M
     flush_transposed(tile, a.out_t, a.rows, col0, row0);
 }
 
+// Row-major results only, for weight-gradient GEMMs that read MN-major operands (`gemm_kgrouped_tn`): one warp per row, no shared
+// memory, every byte read and written once, so the kernels are bound by HBM (0.15 ms each for 34816 rows of 7168 / 2 x 2048).
+constexpr int kRowWarps = 8;
+__global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_swiglu_rows_kernel(const MoeBwdArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (row >= a.rows) return;
+    const int I = a.cols;
+    const uint8_t* db = reinterpret_cast<const uint8_t*>(a.g) + static_cast<int64_t>(row) * I * 2;
+    const uint8_t* hb = reinterpret_cast<const uint8_t*>(a.y) + static_cast<int64_t>(row) * I * 4;
+    uint8_t* ob = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(row) * I * 4;
+    uint8_t* ab = reinterpret_cast<uint8_t*>(a.out2) + static_cast<int64_t>(row) * I * 2;
+    if (a.valid[row] == 0) {
+        const int4 zero = make_int4(0, 0, 0, 0);
+        for (int col = lane * 8; col < I; col += 256) {
+            *reinterpret_cast<int4*>(ob + col * 2) = zero;
+            *reinterpret_cast<int4*>(ob + (I + col) * 2) = zero;
+            *reinterpret_cast<int4*>(ab + col * 2) = zero;
+        }
+        if (lane == 0) a.row_dot[row] = 0.f;
+        return;
+    }
+    const float wr = __ldg(a.w + row);
+    float dot = 0.f;
+#pragma unroll 2
+    for (int col = lane * 8; col < I; col += 256) {
+        float d[8], gate[8], up[8], dg[8], du[8], act[8];
+        unpack8(ptx::ld_nc_v4(db + col * 2), d);
+        unpack8(ptx::ld_nc_v4(hb + col * 2), gate);
+        unpack8(ptx::ld_nc_v4(hb + (I + col) * 2), up);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float sig = 1.f / (1.f + __expf(-gate[j]));
+            act[j] = round_bf16(gate[j] * sig * up[j]);
+            dot = fmaf(d[j], act[j], dot);              // d loss / d weight of the row
+            const float dj = d[j] * wr;
+            du[j] = dj * gate[j] * sig;
+            dg[j] = dj * up[j] * sig * (1.f + gate[j] * (1.f - sig));
+        }
+        *reinterpret_cast<int4*>(ob + col * 2) = pack8(dg);
+        *reinterpret_cast<int4*>(ob + (I + col) * 2) = pack8(du);
+        *reinterpret_cast<int4*>(ab + col * 2) = pack8(act);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    if (lane == 0) a.row_dot[row] = dot;
+}
+
+// 16 channels per lane: one 16-byte load, two 16-byte stores (cols % 16 == 0)
+__global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_dequant_rows_kernel(const MoeBwdArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (row >= a.rows) return;
+    const int H = a.cols;
+    const uint8_t* qb = reinterpret_cast<const uint8_t*>(a.y) + static_cast<int64_t>(row) * H;
+    uint8_t* ob = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(row) * H * 2;
+    const bool ok = a.valid[row] != 0;
+    const float rw = a.row_w != nullptr ? __ldg(a.row_w + row) : 1.f;
+#pragma unroll 4
+    for (int col = lane * 16; col < H; col += 512) {
+        int4 out[2] = {make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0)};
+        if (ok) {
+            const int4 raw = ptx::ld_nc_v4(qb + col);
+            const float sf = __ldg(a.w + row * a.sf_stride_row + (col / 128) * a.sf_stride_col) * rw;
+            const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                float f[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[v * 4 + j], __NV_E4M3);
+                    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+                    f[2 * j] = x.x * sf;
+                    f[2 * j + 1] = x.y * sf;
+                }
+                out[v] = pack8(f);
+            }
+        }
+        *reinterpret_cast<int4*>(ob + col * 2) = out[0];
+        *reinterpret_cast<int4*>(ob + col * 2 + 16) = out[1];
+    }
+}
+
+// rows times their weights
+__global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_weight_rows_kernel(const MoeBwdArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (row >= a.rows) return;
+    const uint8_t* gb = reinterpret_cast<const uint8_t*>(a.g) + static_cast<int64_t>(row) * a.cols * 2;
+    uint8_t* ob = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(row) * a.cols * 2;
+    const bool ok = a.valid[row] != 0;
+    const float rw = __ldg(a.row_w + row);
+#pragma unroll 4
+    for (int col = lane * 8; col < a.cols; col += 256) {
+        int4 out = make_int4(0, 0, 0, 0);
+        if (ok) {
+            float f[8];
+            unpack8(ptx::ld_nc_v4(gb + col * 2), f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] *= rw;
+            out = pack8(f);
+        }
+        *reinterpret_cast<int4*>(ob + col * 2) = out;
+    }
+}
 
 // Expand-layout bookkeeping of a grouped GEMM in one launch: from the inclusive segment ends (segment e starts at
 // align(end[e - 1], alignment) and holds end[e] - start rows) -> the weights group of every 128-row tile (-1: no token
@@ -604,6 +709,14 @@ int moe_bwd_prep_col_blocks(int cols) { return (cols + kPrepCols - 1) / kPrepCol
 
 cudaError_t launch_moe_bwd(const MoeBwdArgs& a, cudaStream_t stream) {
     if (a.rows == 0) return cudaSuccess;
+    if (a.op == EP_MOE_BWD_SWIGLU_ROWS || a.op == EP_MOE_BWD_DEQUANT_ROWS || a.op == EP_MOE_BWD_WEIGHT_ROWS) {
+        const int blocks = (a.rows + kRowWarps - 1) / kRowWarps;
+        if (a.cols % (a.op == EP_MOE_BWD_DEQUANT_ROWS ? 16 : 8) != 0) return cudaErrorInvalidValue;
+        if (a.op == EP_MOE_BWD_SWIGLU_ROWS) moe_bwd_swiglu_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
+        else if (a.op == EP_MOE_BWD_DEQUANT_ROWS) moe_bwd_dequant_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
+        else moe_bwd_weight_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
+        return cudaGetLastError();
+    }
     if (a.rows % kTile != 0 || a.cols % kTile != 0) return cudaErrorInvalidValue;
     if (a.op == EP_MOE_BWD_PREP) moe_bwd_prep_kernel<<<dim3(a.rows / kTile, (a.cols + kPrepCols - 1) / kPrepCols), kTileThreads, 0, stream>>>(a);
     else if (a.op == EP_MOE_BWD_SWIGLU) moe_bwd_swiglu_kernel<<<dim3(a.rows / kTile, a.cols / kTile), kTileThreads, 0, stream>>>(a);

@@ -338,6 +338,145 @@ at::Tensor local_reduce(const at::Tensor& pos, const at::Tensor& y, const std::o
     return res;
 }
 
+const uint8_t* valid_ptr(const at::Tensor& valid, int64_t rows) {
+    TORCH_CHECK(valid.is_cuda() && valid.is_contiguous() && valid.numel() == rows && (valid.scalar_type() == at::kBool || valid.scalar_type() == at::kByte),
+                "valid must be a bool / uint8 tensor with one entry per row");
+    return reinterpret_cast<const uint8_t*>(valid.data_ptr());
+}
+
+const float* row_weight_ptr(const at::Tensor& w, int64_t rows) {
+    TORCH_CHECK(w.is_cuda() && w.is_contiguous() && w.scalar_type() == at::kFloat && w.numel() == rows, "row weights must be fp32 [rows]");
+    return w.data_ptr<float>();
+}
+
+// grouped data gradient: every 128-row tile t of a [M, K] is multiplied by b[tile_group[t]] [K, N] (bf16, both as stored)
+at::Tensor grouped_gemm_nn(const at::Tensor& a, const at::Tensor& b, const at::Tensor& tile_group, const std::optional<at::Tensor>& out,
+                           int64_t num_sms, ElasticBufferCore* report_to) {
+    TORCH_CHECK(a.is_cuda() && a.dim() == 2 && a.stride(1) == 1 && a.scalar_type() == at::kBFloat16, "A must be bf16 [M, K] with contiguous rows");
+    TORCH_CHECK(b.is_cuda() && b.dim() == 3 && b.is_contiguous() && b.scalar_type() == at::kBFloat16 && b.size(1) == a.size(1),
+                "B must be contiguous bf16 [G, K, N]");
+    const int64_t M = a.size(0), K = a.size(1), G = b.size(0), N = b.size(2);
+    at::Tensor c = out.has_value() ? *out : at::empty({M, N}, a.options());
+    TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kBFloat16 && c.dim() == 2 && c.size(0) == M && c.size(1) == N && c.stride(1) == 1, "bad output");
+    TORCH_CHECK(tile_group.is_cuda() && tile_group.scalar_type() == at::kInt && tile_group.is_contiguous() && tile_group.numel() >= (M + 127) / 128,
+                "bad tile_group");
+    GemmArgs g{};
+    g.a = a.data_ptr();
+    g.b = b.data_ptr();
+    g.c = c.data_ptr();
+    g.M = static_cast<int>(M);
+    g.N = static_cast<int>(N);
+    g.K = static_cast<int>(K);
+    g.num_groups = static_cast<int>(G);
+    g.lda = a.stride(0);
+    g.ldb = N;
+    g.ldc = c.stride(0);
+    g.tile_group = tile_group.data_ptr<int32_t>();
+    g.mn_operands = 1;
+    g.error = gemm_error_flag(a.get_device()).data_ptr<int>();
+    if (report_to != nullptr) {
+        report_to->check_status();
+        const RankCtx c0 = report_to->ctx();
+        g.status = c0.status;
+        g.status_rank = c0.rank;
+        g.timeout_ns = c0.timeout_ns;
+    }
+    const int sms = num_sms > 0 ? static_cast<int>(num_sms) : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    cuda_check(ep::launch_gemm(g, sms, at::cuda::getCurrentCUDAStream()), "grouped data-gradient GEMM launch");
+    return c;
+}
+
+// out[e] = a[k0:k1]^T @ b[k0:k1] with (k0, k1) = k_off[e], k_off[e + 1]: the K-grouped product on row-major operands
+// (a [K_total, M], b [K_total, N] bf16; k_off int32 [G + 1], multiples of 64)
+at::Tensor gemm_kgrouped_tn(const at::Tensor& a, const at::Tensor& b, const at::Tensor& k_off, int64_t num_sms) {
+    TORCH_CHECK(a.is_cuda() && a.dim() == 2 && a.stride(1) == 1 && a.scalar_type() == at::kBFloat16, "a must be bf16 [K, M] with contiguous rows");
+    TORCH_CHECK(b.is_cuda() && b.dim() == 2 && b.stride(1) == 1 && b.scalar_type() == at::kBFloat16 && b.size(0) == a.size(0),
+                "b must be bf16 [K, N] with contiguous rows");
+    TORCH_CHECK(k_off.is_cuda() && k_off.scalar_type() == at::kInt && k_off.is_contiguous() && k_off.numel() >= 2, "k_off must be int32 [G + 1]");
+    const int64_t M = a.size(1), N = b.size(1), K = a.size(0), G = k_off.numel() - 1;
+    if (K == 0) return at::zeros({G, M, N}, a.options());
+    at::Tensor c = at::empty({G, M, N}, a.options());
+    GemmArgs g{};
+    g.a = a.data_ptr();
+    g.b = b.data_ptr();
+    g.c = c.data_ptr();
+    g.M = static_cast<int>(M);
+    g.N = static_cast<int>(N);
+    g.K = static_cast<int>(K);
+    g.num_groups = static_cast<int>(G);
+    g.lda = a.stride(0);
+    g.ldb = b.stride(0);
+    g.ldc = N;
+    g.k_group_off = k_off.data_ptr<int32_t>();
+    g.mn_operands = 2;
+    g.error = gemm_error_flag(a.get_device()).data_ptr<int>();
+    const int sms = num_sms > 0 ? static_cast<int>(num_sms) : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    cuda_check(ep::launch_gemm(g, sms, at::cuda::getCurrentCUDAStream()), "K-grouped GEMM launch");
+    return c;
+}
+
+// Backward of SwiGLU with row-major results: (d_h [rows, 2I], activation [rows, I], d loss / d row_weight [rows])
+std::vector<at::Tensor> swiglu_bwd_rows(const at::Tensor& d_act, const at::Tensor& h, const at::Tensor& valid, const at::Tensor& row_weight) {
+    TORCH_CHECK(d_act.is_cuda() && d_act.dim() == 2 && d_act.is_contiguous() && d_act.scalar_type() == at::kBFloat16, "d_act must be contiguous bf16 [rows, I]");
+    const int64_t rows = d_act.size(0), I = d_act.size(1);
+    TORCH_CHECK(h.is_cuda() && h.is_contiguous() && h.scalar_type() == at::kBFloat16 && h.dim() == 2 && h.size(0) == rows && h.size(1) == 2 * I,
+                "h must be bf16 [rows, 2I]");
+    at::Tensor out = at::empty({rows, 2 * I}, h.options()), act = at::empty({rows, I}, h.options());
+    at::Tensor dot = at::empty({rows}, h.options().dtype(at::kFloat));
+    MoeBwdArgs a{};
+    a.op = EP_MOE_BWD_SWIGLU_ROWS;
+    a.rows = static_cast<int>(rows);
+    a.cols = static_cast<int>(I);
+    a.valid = valid_ptr(valid, rows);
+    a.g = d_act.data_ptr();
+    a.y = h.data_ptr();
+    a.w = row_weight_ptr(row_weight, rows);
+    a.out = out.data_ptr();
+    a.out2 = act.data_ptr();
+    a.row_dot = dot.data_ptr<float>();
+    cuda_check(ep::launch_moe_bwd(a, at::cuda::getCurrentCUDAStream()), "SwiGLU backward launch");
+    return {out, act, dot};
+}
+
+// g * w[:, None] in bf16 [rows, H]; padding rows give zeros
+at::Tensor weighted_rows(const at::Tensor& g_rows, const at::Tensor& w, const at::Tensor& valid) {
+    TORCH_CHECK(g_rows.is_cuda() && g_rows.dim() == 2 && g_rows.is_contiguous() && g_rows.scalar_type() == at::kBFloat16, "g must be contiguous bf16 [rows, H]");
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(g_rows.data_ptr()) % 16 == 0, "g must be 16-byte aligned");
+    at::Tensor out = at::empty_like(g_rows);
+    MoeBwdArgs a{};
+    a.op = EP_MOE_BWD_WEIGHT_ROWS;
+    a.rows = static_cast<int>(g_rows.size(0));
+    a.cols = static_cast<int>(g_rows.size(1));
+    a.valid = valid_ptr(valid, g_rows.size(0));
+    a.g = g_rows.data_ptr();
+    a.row_w = row_weight_ptr(w, g_rows.size(0));
+    a.out = out.data_ptr();
+    cuda_check(ep::launch_moe_bwd(a, at::cuda::getCurrentCUDAStream()), "row weighting launch");
+    return out;
+}
+
+// (q e4m3 [rows, H], scales per (row, 128 channels), any strides) -> bf16 q * scale (* row_weight) [rows, H]; padding rows give zeros
+at::Tensor dequant_rows(const at::Tensor& q, const at::Tensor& sf, const at::Tensor& valid, const std::optional<at::Tensor>& row_weight) {
+    TORCH_CHECK(q.is_cuda() && q.dim() == 2 && q.is_contiguous() && q.scalar_type() == at::kFloat8_e4m3fn, "q must be contiguous e4m3 [rows, H]");
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(q.data_ptr()) % 16 == 0, "q must be 16-byte aligned");
+    const int64_t rows = q.size(0), H = q.size(1);
+    TORCH_CHECK(sf.is_cuda() && sf.scalar_type() == at::kFloat && sf.dim() == 2 && sf.size(0) >= rows && sf.size(1) == (H + 127) / 128, "bad scales");
+    at::Tensor out = at::empty({rows, H}, q.options().dtype(at::kBFloat16));
+    MoeBwdArgs a{};
+    a.op = EP_MOE_BWD_DEQUANT_ROWS;
+    a.rows = static_cast<int>(rows);
+    a.cols = static_cast<int>(H);
+    a.valid = valid_ptr(valid, rows);
+    a.y = q.data_ptr();
+    a.w = sf.data_ptr<float>();
+    a.sf_stride_row = sf.stride(0);
+    a.sf_stride_col = sf.stride(1);
+    if (row_weight.has_value()) a.row_w = row_weight_ptr(*row_weight, rows);
+    a.out = out.data_ptr();
+    cuda_check(ep::launch_moe_bwd(a, at::cuda::getCurrentCUDAStream()), "dequantisation launch");
+    return out;
+}
+
 // Weights [G, N, K] (bf16 or fp32, contiguous, K % 8 == 0, 16-byte aligned) -> (e4m3 [G, N, K], fp32 scales of the 128 x 128 blocks)
 std::vector<at::Tensor> quantize_weight_blocks(const at::Tensor& w) {
     TORCH_CHECK(w.is_cuda() && w.dim() == 3 && w.is_contiguous() && (w.scalar_type() == at::kBFloat16 || w.scalar_type() == at::kFloat),
@@ -383,12 +522,6 @@ at::Tensor gemm_kgrouped(const at::Tensor& a_t, const at::Tensor& b_t, const at:
     const int sms = num_sms > 0 ? static_cast<int>(num_sms) : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     cuda_check(ep::launch_gemm(g, sms, at::cuda::getCurrentCUDAStream()), "K-grouped tcgen05 GEMM launch");
     return c;
-}
-
-const uint8_t* valid_ptr(const at::Tensor& valid, int64_t rows) {
-    TORCH_CHECK(valid.is_cuda() && valid.is_contiguous() && valid.numel() == rows && (valid.scalar_type() == at::kBool || valid.scalar_type() == at::kByte),
-                "valid must be a bool / uint8 tensor with one entry per row");
-    return reinterpret_cast<const uint8_t*>(valid.data_ptr());
 }
 
 // Backward of the weighted combine at the expert rows: (g * w [rows, H], its transpose [H, rows], sum(g * y) per row)
@@ -700,6 +833,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("quantize_weight_blocks", &quantize_weight_blocks);
     m.def("swiglu_quant", &swiglu_quant, py::arg("h"), py::arg("keep_bf16") = false);
     m.def("gemm_kgrouped", &gemm_kgrouped, py::arg("a_t"), py::arg("b_t"), py::arg("k_off"), py::arg("num_sms") = 0);
+    m.def("grouped_gemm_nn", &grouped_gemm_nn, py::arg("a"), py::arg("b"), py::arg("tile_group"), py::arg("out") = py::none(), py::arg("num_sms") = 0,
+          py::arg("report_to") = nullptr);
+    m.def("gemm_kgrouped_tn", &gemm_kgrouped_tn, py::arg("a"), py::arg("b"), py::arg("k_off"), py::arg("num_sms") = 0);
+    m.def("swiglu_bwd_rows", &swiglu_bwd_rows);
+    m.def("weighted_rows", &weighted_rows);
+    m.def("dequant_rows", &dequant_rows, py::arg("q"), py::arg("sf"), py::arg("valid"), py::arg("row_weight") = py::none());
     m.def("moe_bwd_prep", &moe_bwd_prep);
     m.def("swiglu_bwd", &swiglu_bwd, py::arg("d_act"), py::arg("h"), py::arg("valid"), py::arg("row_weight") = py::none());
     m.def("weighted_transpose", &weighted_transpose);

@@ -104,7 +104,7 @@ class _MoEFunction(torch.autograd.Function):
     def backward(ctx, d_out):
         layer, bounds = ctx.layer, ctx.bounds
         buf: ElasticBuffer = layer.buffer
-        w2_t, w13_t = (None, None) if layer.fp8_backward else layer.transposed_weights()
+        w2, w13 = (None, None) if layer.fp8_backward else (layer.w2.detach().contiguous(), layer.w13.detach().contiguous())
         d_out = d_out.contiguous()
         dxs, dws, d_w2, d_w13 = [], [], None, None
         for c, handle in enumerate(ctx.handles):
@@ -128,32 +128,32 @@ class _MoEFunction(torch.autograd.Function):
                 if local:
                     g_q, g_sf = G.local_expand_copy(pos, g_q, rows, sf=g_sf)
                 d_act_u = G.grouped_gemm_nt(g_q, q2_t, tile_group, sfa=g_sf, sfb=s2_t, buffer=buf)             # [rows, I]
-                dh, dh_t, act_t, d_w_rows = G.swiglu_bwd(d_act_u, h, valid_row, row_weight=rw)
+                dh, act, d_w_rows = G.swiglu_bwd_rows(d_act_u, h, valid_row, rw)
                 dh_q, dh_sf = G.per_token_cast_to_fp8(dh)
                 d_recv = None if local else buf.get_combine_buffer(handle)
                 d_recv = G.grouped_gemm_nt(dh_q, q13_t, tile_group, out=d_recv, sfa=dh_sf, sfb=s13_t, buffer=buf)
                 dx, d_topk_w = send_home(d_recv, d_w_rows)
-                # (g * w)^T for the weight gradient: the routing weight rides on the scales of the dequantisation
-                dy_t = G.dequant_transpose(g_q, g_sf * rw.unsqueeze(1), valid_row)
+                # g * w for the weight gradient: the routing weight rides on the scales of the dequantisation
+                dy = G.dequant_rows(g_q, g_sf, valid_row, row_weight=rw)
             else:
                 # backward of the weighted combine: every expert row receives its token's gradient g (cached dispatch)
                 g_rows, _, _, _, _ = buf.dispatch(d_out[bounds[c]:bounds[c + 1]], handle=handle, fused_fp8_cast=False, num_sms=layer.num_sms)
                 if local:
                     g_rows = G.local_expand_copy(pos, g_rows, rows)[0]
                 # down projection on the UNWEIGHTED gradient: d loss / d weight of a row is <g W2, activation> (= <g, y>, so the
-                # expert outputs need not be kept), and the weight is applied inside the SwiGLU backward kernel.  Padding rows of
-                # g_rows hold stale data; every consumer masks them.
-                d_act_u = G.grouped_gemm_nt(g_rows, w2_t, tile_group, buffer=buf)                    # [rows, I]
-                dh, dh_t, act_t, d_w_rows = G.swiglu_bwd(d_act_u, h, valid_row, row_weight=rw)
+                # expert outputs need not be kept), and the weight is applied inside the SwiGLU backward kernel.  Both data
+                # gradients read the forward weights as they are stored.  Padding rows of g_rows hold stale data; every consumer
+                # masks them.
+                d_act_u = G.grouped_gemm_nn(g_rows, w2, tile_group, buffer=buf)                      # [rows, I]
+                dh, act, d_w_rows = G.swiglu_bwd_rows(d_act_u, h, valid_row, rw)
                 # up projection: the gradient rows go into the combine region and travel home (backward of dispatch)
                 d_recv = None if local else buf.get_combine_buffer(handle)
-                d_recv = G.grouped_gemm_nt(dh, w13_t, tile_group, out=d_recv, buffer=buf)
+                d_recv = G.grouped_gemm_nn(dh, w13, tile_group, out=d_recv, buffer=buf)
                 dx, d_topk_w = send_home(d_recv, d_w_rows)
-                dy_t = G.weighted_transpose(g_rows, rw, valid_row)                                  # (g * w)^T [H, rows]
+                dy = G.weighted_rows(g_rows, rw, valid_row)                                         # g * w [rows, H]
             # weight gradients: one K-grouped GEMM per weight tensor, reduction over the rows of every expert segment
-            x_t = G.dequant_transpose(rx, rsf, valid_row)
-            g2 = G.gemm_kgrouped(dy_t, act_t, seg_off)                                          # [El, H, I]
-            g13 = G.gemm_kgrouped(dh_t, x_t, seg_off)                                           # [El, 2I, H]
+            g2 = G.gemm_kgrouped_tn(dy, act, seg_off)                                           # [El, H, I]
+            g13 = G.gemm_kgrouped_tn(dh, G.dequant_rows(rx, rsf, valid_row), seg_off)           # [El, 2I, H]
             d_w2 = g2 if d_w2 is None else d_w2 + g2
             d_w13 = g13 if d_w13 is None else d_w13 + g13
             dxs.append(dx)

@@ -162,6 +162,37 @@ def gemm_kgrouped(a_t: torch.Tensor, b_t: torch.Tensor, k_off: torch.Tensor, num
     return _native.load().gemm_kgrouped(a_t, b_t, k_off, num_sms)
 
 
+def grouped_gemm_nn(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, out: Optional[torch.Tensor] = None, num_sms: int = 0,
+                    buffer=None) -> torch.Tensor:
+    """Data gradient of a grouped layer on the forward weights as they are stored: every 128-row tile ``t`` of ``a [M, K]`` is
+    multiplied by ``b[tile_group[t]]`` with ``b [G, K, N]`` (``-1`` skips the tile) -> bf16 ``[M, N]``.  The tensor core reads the
+    N-contiguous operand through a transposing descriptor, so no transposed copy of the weights exists.  ``buffer``: see
+    :func:`gemm_nt`."""
+    return _native.load().grouped_gemm_nn(a, b, tile_group, out, num_sms, _core_of(buffer))
+
+
+def gemm_kgrouped_tn(a: torch.Tensor, b: torch.Tensor, k_off: torch.Tensor, num_sms: int = 0) -> torch.Tensor:
+    """:func:`gemm_kgrouped` on row-major operands: ``out[e] = a[k0:k1]^T @ b[k0:k1]`` with ``a [rows, M]``, ``b [rows, N]`` bf16.
+    Every row of a segment enters the sum, so alignment rows must hold zeros in both (zero times a stale NaN is a NaN)."""
+    return _native.load().gemm_kgrouped_tn(a, b, k_off, num_sms)
+
+
+def swiglu_bwd_rows(d_act: torch.Tensor, h: torch.Tensor, valid_row: torch.Tensor, row_weight: torch.Tensor):
+    """:func:`swiglu_bwd` with ``row_weight`` and row-major results -> ``(d_h [rows, 2I], activation [rows, I],
+    d loss / d row_weight [rows])``; padding rows give zeros."""
+    return _native.load().swiglu_bwd_rows(d_act, h, valid_row, row_weight)
+
+
+def weighted_rows(g_rows: torch.Tensor, w: torch.Tensor, valid_row: torch.Tensor) -> torch.Tensor:
+    """``g * w[:, None]`` as bf16 ``[rows, H]``; padding rows give zeros whatever they hold."""
+    return _native.load().weighted_rows(g_rows, w, valid_row)
+
+
+def dequant_rows(q: torch.Tensor, sf: torch.Tensor, valid_row: torch.Tensor, row_weight: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """e4m3 rows with 1 x 128 scales -> bf16 ``q * (scale * row_weight) [rows, H]``; padding rows give zeros."""
+    return _native.load().dequant_rows(q, sf, valid_row, row_weight)
+
+
 def segment_offsets(psum_expert_ends: torch.Tensor, alignment: int = BLOCK_M) -> torch.Tensor:
     """Expand-layout segment boundaries as ``int32 [G + 1]``: segment ``e`` covers rows ``[off[e], off[e + 1])``
     including its alignment padding.  Stays on the device."""

@@ -91,3 +91,50 @@ def test_k_grouped_gemm(M, N, segs):
         if n == 0:
             assert out[e].abs().max().item() == 0
         k0 += n
+
+
+@pytest.mark.parametrize('M,N,K,G', [(128, 128, 64, 1), (256, 256, 128, 2), (300, 520, 72, 3), (640, 136, 200, 4), (1000, 1032, 1096, 2)])
+def test_grouped_gemm_reads_mn_major_weights(M, N, K, G):
+    """a [M, K] @ b[group] [K, N] without a transposed copy: edge tiles in M, N and K, skipped tiles.  A K tail must not pick up the
+    next group's rows: the last group is followed by nothing, the others by NaN-free but different weights."""
+    from deepep_ascend_b200.ops import gemm as ops
+    C = _C()
+    g = torch.Generator(device='cuda').manual_seed(M + N + K)
+    a = torch.randn(M, K, device='cuda', generator=g).bfloat16()
+    b = torch.randn(G, K, N, device='cuda', generator=g).bfloat16()
+    tiles = (M + 127) // 128
+    tile_group = torch.tensor([t % (G + 1) - 1 for t in range(tiles)], dtype=torch.int32, device='cuda')
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device='cuda')
+    ops.grouped_gemm_nn(a, b, tile_group, out=out)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0
+    for t in range(tiles):
+        rows, grp = slice(t * 128, min(M, (t + 1) * 128)), int(tile_group[t])
+        if grp < 0:
+            assert bool((out[rows] == 7.0).all())
+            continue
+        ref = a[rows].double() @ b[grp].double()
+        # fp32 sums rounded once to bf16: half an ulp (2^-9) of the value plus K fp32 roundings of the summed magnitudes
+        bound = ref.abs() * 2.0 ** -8 + (a[rows].double().abs() @ b[grp].double().abs()) * K * 2.0 ** -24 + 1e-6
+        assert bool(((out[rows].double() - ref).abs() <= bound).all()), t
+
+
+@pytest.mark.parametrize('M,N,segs', [(128, 128, [64, 0, 192]), (384, 520, [128, 256, 0, 0, 640]), (136, 264, [64]), (2048, 7168, [1152, 1024, 0, 1280])])
+def test_k_grouped_gemm_on_row_major_operands(M, N, segs):
+    """out[e] = a[seg_e]^T @ b[seg_e]; empty segments give zeros; strided rows."""
+    from deepep_ascend_b200.ops import gemm as ops
+    C = _C()
+    g = torch.Generator(device='cuda').manual_seed(M + N)
+    K = sum(segs)
+    a = torch.randn(K, M + 8, device='cuda', generator=g).bfloat16()[:, :M]
+    b = torch.randn(K, N, device='cuda', generator=g).bfloat16()
+    off = torch.tensor([0] + list(torch.tensor(segs).cumsum(0)), dtype=torch.int32, device='cuda')
+    out = ops.gemm_kgrouped_tn(a, b, off)
+    torch.cuda.synchronize()
+    assert C.gemm_error(0) == 0 and out.shape == (len(segs), M, N)
+    k0 = 0
+    for e, n in enumerate(segs):
+        ref = a[k0:k0 + n].double().t() @ b[k0:k0 + n].double()
+        bound = ref.abs() * 2.0 ** -8 + (a[k0:k0 + n].double().abs().t() @ b[k0:k0 + n].double().abs()) * max(n, 1) * 2.0 ** -24 + 1e-6
+        assert bool(((out[e].double() - ref).abs() <= (bound if n else 0)).all()), e
+        k0 += n

@@ -355,3 +355,41 @@ def test_weight_block_cast_matches_pytorch(G, N, K, dtype):
         assert q.shape == q_ref.shape and sf.shape == sf_ref.shape
         assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8))
         assert torch.equal(sf.view(torch.int32), sf_ref.view(torch.int32))
+
+
+@pytest.mark.parametrize('rows,I,H', [(1, 128, 128), (67, 136, 144), (256, 2048, 7168)])
+def test_row_major_backward_kernels(rows, I, H):
+    """The row-major SwiGLU gradient and dequantisation against the transposing kernels' PyTorch statement: ragged rows, masked rows
+    with NaN payloads give exact zeros."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows)
+    valid = torch.rand(rows, device='cuda') > 0.2
+    vm = valid.unsqueeze(1)
+    d_act, h = torch.randn(rows, I, device='cuda').bfloat16(), torch.randn(rows, 2 * I, device='cuda').bfloat16()
+    w = torch.rand(rows, device='cuda')
+    d_act[~valid], h[~valid] = float('nan'), float('nan')
+    dh, act, dot = ops.swiglu_bwd_rows(d_act, h, valid, w)
+    gate, up, d = h[:, :I].double(), h[:, I:].double(), d_act.double()
+    sig = torch.sigmoid(gate)
+    wd = w.double().unsqueeze(1)
+    ref_dh = torch.where(vm, torch.cat([wd * d * up * sig * (1 + gate * (1 - sig)), wd * d * gate * sig], dim=1), 0.0)
+    ref_act = torch.where(vm, gate * sig * up, 0.0)
+    # one rounding to bf16 (2^-9 of the value) and the fp32 expression around __expf (a few 2^-22 relative)
+    torch.testing.assert_close(dh.double(), ref_dh, rtol=2.0 ** -8, atol=1e-5)
+    torch.testing.assert_close(act.double(), ref_act, rtol=2.0 ** -8, atol=1e-5)
+    act16 = (gate * sig * up).float().bfloat16().double()
+    ref_dot = torch.where(valid, (d * act16).sum(1), 0.0)
+    scale = torch.where(valid, (d * act16).abs().sum(1), 0.0)
+    assert bool(((dot.double() - ref_dot).abs() <= scale * 2.0 ** -8 + 1e-6).all())
+    x = torch.randn(rows, H, device='cuda').bfloat16()
+    q, sf = ops.per_token_cast_to_fp8(x)
+    sf[~valid] = float('nan')
+    out = ops.dequant_rows(q, sf, valid)
+    ref = (q.float().view(rows, -1) * sf.repeat_interleave(128, dim=1)[:, :H]).bfloat16()
+    assert torch.equal(out, torch.where(vm, ref, torch.zeros_like(ref)))
+    out = ops.dequant_rows(q, sf, valid, row_weight=w)
+    ref = (q.float().view(rows, -1) * (sf * w.unsqueeze(1)).repeat_interleave(128, dim=1)[:, :H]).bfloat16()
+    assert torch.equal(out, torch.where(vm, ref, torch.zeros_like(ref)))
+    x[~valid] = float('nan')
+    ref = (x.float() * w.unsqueeze(1)).bfloat16()
+    assert torch.equal(ops.weighted_rows(x, w, valid), torch.where(vm, ref, torch.zeros_like(ref)))
