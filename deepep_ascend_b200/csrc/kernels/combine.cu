@@ -3,11 +3,15 @@
 // peer mappings, no multicast) and reduces them in fp32 registers, so the reduction is fused into the gather
 // and no intermediate slab is written or re-read.
 //
-// Work item = (token, column chunk of 32 lanes x 16 B x kUnroll).  Items are claimed dynamically by the warps of all
-// CTAs from one counter, a whole token's chunks per claim at first and single chunks near the end, so that no warp is
-// left with a long tail.  Each warp owns a ring of chunk buffers with one mbarrier each: while it reduces one chunk,
-// the loads of the following ones are in flight.  The accumulation order is fixed (bias0 + bias1 first, then the plan
-// entries in top-k lane order), so results are bitwise reproducible.
+// A row is pulled in column chunks of 32 lanes x 16 B x kUnroll; units of work are claimed dynamically by the warps of all CTAs,
+// whole tokens first and single chunks at the end (see the body).  Each warp owns a ring of chunk buffers with one mbarrier
+// each: while it reduces one chunk, the loads of the following ones are in flight.  The accumulation order is fixed (bias0 +
+// bias1 first, then the plan entries in top-k lane order), so results are bitwise reproducible.
+//
+// What bounds it: a warp's own chain per chunk (wait, read, convert, store, refill), so SM count and warps matter until HBM or the
+// link does.  With divisions, queue and claim work per chunk taken off that chain, the claims and plan entries requested ahead,
+// and 16 instead of 12 warps, 8192 rows x 7168 (235 MB moved, one rank) take 378 / 104 / 56 / 47 us on 8 / 32 / 64 / 148 SMs
+// (before: 717 / 190 / 101 / 53); 24 warps with 2 KB chunks are slower (403 / 111 / 63 / 47).
 //
 // There is no grid-wide barrier and no exit barrier.  Entry: CTA 0 signals every peer, every CTA watches the peers'
 // signals itself (all ranks' input rows are in place once all ranks have entered the call).  Exit: the caller
@@ -17,23 +21,25 @@
 // Parity: does the work of combine_impl + combine_reduce_epilogue_impl
 // (deep_ep/include/deep_ep/impls/combine.cuh:15-243, combine_reduce_epilogue.cuh:12-143) plus the weighted
 // reduction of the legacy low-latency combine (csrc/kernels/legacy/internode_ll.cu:1033-1136).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ep {
 
 namespace {
 
-constexpr int kCombineMaxWarps = 12;
+constexpr int kCombineMaxWarps = 16;
 constexpr int kCombineMaxRing = 32;              // chunk buffers (and mbarriers) per warp
 constexpr int kCombineSmemBudget = 208 * 1024;
-constexpr int kCombineQueue = 64;                // claimed-token queue per warp (producer -> consumer)
+constexpr int kCombineQueue = 32;                // queue of started units per warp (producer -> consumer)
 
 template <int kUnroll>
 struct CombineCfg {
     static constexpr int kChunkBytes = 32 * 16 * kUnroll;
 };
 
-// Shared-memory plan: [peer table | mbarriers W x ring | chunk buffers W x ring]
+// Shared-memory plan: [peer table | mbarriers W x ring | unit queues W | chunk buffers W x ring]
 struct CombineSmemPlan {
     int num_warps, ring, off_bar, off_queue, off_data, total;
 };
@@ -42,7 +48,7 @@ __host__ __device__ inline CombineSmemPlan combine_smem_plan(int chunk_bytes, in
     p.num_warps = num_warps;
     p.off_bar = 128;
     p.off_queue = 128 + num_warps * kCombineMaxRing * 8;
-    p.off_data = p.off_queue + num_warps * kCombineQueue * 8;   // claimed ranges: first item and length
+    p.off_data = p.off_queue + num_warps * kCombineQueue * 16;   // int4 per unit: token, first chunk, end chunk, source lanes
     p.off_data = (p.off_data + 1023) / 1024 * 1024;
     int ring = (kCombineSmemBudget - p.off_data) / (num_warps * chunk_bytes);
     p.ring = ring > kCombineMaxRing ? kCombineMaxRing : ring;
@@ -50,18 +56,8 @@ __host__ __device__ inline CombineSmemPlan combine_smem_plan(int chunk_bytes, in
     return p;
 }
 
-// Cursor over the flattened sequence of (work item, source) pairs of one warp.  Items are numbered token * num_chunks +
-// chunk; a cursor walks a claimed range [item, range_end).  Lane k holds plan[t][k] of the cursor's token; `pending`
-// has one bit per source that is still to be visited, lowest lane first.
-struct PullCursor {
-    int item, range_end;   // current item and end of the claimed range (item == range_end: range used up)
-    int token;             // token whose plan is loaded, -1 for none
-    int plan_k;
-    uint32_t sources;      // lanes of the token's plan that hold a row
-    uint32_t pending;      // sources of the current chunk not visited yet
-};
-
-template <int kUnroll>
+// kFull: the row is a whole number of chunks, so no lane of a chunk is idle
+template <int kUnroll, bool kFull>
 __device__ __forceinline__ void combine_body(const CombineArgs& a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kChunk = CombineCfg<kUnroll>::kChunkBytes;
@@ -78,8 +74,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a) {
     uint8_t** s_peer = reinterpret_cast<uint8_t**>(smem);
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + sp.off_bar) + warp * kCombineMaxRing;
     uint8_t* s_data = smem + sp.off_data + static_cast<size_t>(warp) * ring * kChunk;
-    int* s_queue = reinterpret_cast<int*>(smem + sp.off_queue) + warp * 2 * kCombineQueue;
-    int* s_qlen = s_queue + kCombineQueue;
+    int4* s_queue = reinterpret_cast<int4*>(smem + sp.off_queue) + warp * kCombineQueue;
     // every CTA reads the entry-barrier sequence before it arrives anywhere; the last CTA to finish writes the new one
     const uint64_t entry_seq = *reinterpret_cast<volatile uint64_t*>(&ws->comb_seq) + 1;
 
@@ -110,207 +105,185 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a) {
     }
     stamp(1);
 
-    // Items are claimed from a counter shared by all CTAs of this rank (SMs that get a smaller share of the NVLink
-    // bandwidth claim fewer), which is zero at entry: the last CTA of every call clears it.  The producer cursor
-    // claims; the claimed ranges travel through a small per-warp queue to the consumer cursor, which follows in the
-    // same order.
-    const int total_items = T * num_chunks;
-    const int tail_zone = 2 * static_cast<int>(gridDim.x) * num_warps * num_chunks;
-    uint32_t claimed = 0, started = 0;     // ranges claimed by the producer / started by the consumer
-    int last_base = 0;
-    auto claim_range = [&](int& amount) -> int {   // -> first item of the range; base and length also go into the queue
-        amount = last_base + tail_zone < total_items ? num_chunks : 1;
-        int base = 0;
-        if (lane == 0) {
-            base = static_cast<int>(atomicAdd(&ws->dyn_counter[EP_CH_COMBINE], static_cast<uint32_t>(amount)));
-            s_queue[claimed % kCombineQueue] = base;
-            s_qlen[claimed % kCombineQueue] = amount;
-        }
-        __syncwarp();
-        ++claimed;
-        base = __shfl_sync(0xffffffffu, base, 0);
-        last_base = base;
-        return base;
-    };
-    auto load_token = [&](PullCursor& c) {
-        // (re)load the plan of the cursor's current item if it belongs to another token
-        const int tkn = c.item < total_items ? c.item / num_chunks : -1;
-        if (tkn != c.token) {
-            c.token = tkn;
-            c.plan_k = -1;
-            c.sources = 0;
-            if (tkn >= 0) {
-                c.plan_k = lane < K ? __ldg(a.plan + static_cast<int64_t>(tkn) * K + lane) : -1;
-                c.sources = __ballot_sync(0xffffffffu, c.plan_k >= 0);
-            }
-        }
-        c.pending = c.sources;
-    };
-    auto set_range = [&](PullCursor& c, int base, int len) {
-        c.item = base;
-        c.range_end = min(total_items, base + len);
-        if (c.item >= c.range_end) c.item = c.range_end = total_items;   // nothing left anywhere
-        load_token(c);
-    };
-    // producer: move to its next range (claims one); returns false when the queue is too full to claim right now
-    auto producer_next_range = [&](PullCursor& c) -> bool {
-        if (claimed - started >= static_cast<uint32_t>(kCombineQueue - 8)) return false;
-        if (c.item >= total_items) return true;   // exhausted: stay there
-        int len;
-        const int base = claim_range(len);
-        set_range(c, base, len);
-        return true;
-    };
-
+    // Units of work: the first `whole` tokens are one unit each, every later token is num_chunks units of one chunk (about one
+    // token per warp, so that no warp is left with a long tail).  Every warp's first unit is fixed; later ones are claimed from a
+    // counter shared by all CTAs of this rank (SMs that get a smaller share of the NVLink bandwidth claim fewer), which is zero
+    // at entry: the last CTA of every call clears it.  The producer side of a warp keeps two claims ahead: while the loads of one
+    // unit are issued, the plan entries of the next are on their way and the atomic of the one after has been sent, so neither
+    // latency is paid per token.  Started units travel through a small queue to the consumer side, which follows in order.
     if (alive) {
-        PullCursor prod{0, 0, -1, -1, 0, 0}, cons{0, 0, -1, -1, 0, 0};
-        {
-            int len;
-            const int base = claim_range(len);
-            set_range(prod, base, len);
-        }
-        uint32_t issued = 0, consumed = 0;   // loads issued / consumed by this warp; buffer = counter % ring
+        const int total_warps = static_cast<int>(gridDim.x) * num_warps;
+        const int whole = max(0, T - total_warps);
+        const int num_units = whole + (T - whole) * num_chunks;
+        auto unit_token = [&](int u) { return u < whole ? u : whole + (u - whole) / num_chunks; };
+        auto claim = [&]() -> int {      // lane 0 holds the result
+            return lane == 0 ? total_warps + static_cast<int>(atomicAdd(&ws->dyn_counter[EP_CH_COMBINE], 1u)) : 0;
+        };
+        auto load_plan = [&](int u) -> int {
+            return u < num_units && lane < K ? __ldg(a.plan + static_cast<int64_t>(unit_token(u)) * K + lane) : -1;
+        };
+        // producer state: unit whose loads are being issued / the next one / the claim after that
+        int p_chunk = 0, p_end = 0, p_plan = -1, p_slot = 0;
+        uint32_t p_sources = 0, p_pending = 0;
+        int n_unit = warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+        int n_plan = load_plan(n_unit);
+        int n_claim = n_unit < num_units ? claim() : 0;
+        uint32_t pushed = 0, popped = 0;
+        int in_flight = 0;
 
-        // issue loads in sequence order until the ring is full or the warp's work is exhausted
+        // issue loads in sequence order until the ring is full or the work is exhausted
         auto issue_ahead = [&]() {
-            while (issued - consumed < static_cast<uint32_t>(ring) && prod.item < total_items) {
-                if (prod.pending == 0) {
-                    if (prod.item + 1 >= prod.range_end) {
-                        prod.item = prod.range_end;
-                        if (!producer_next_range(prod)) {
-                            prod.item = prod.range_end - 1;   // retry the claim on the next call
-                            break;
-                        }
+            while (in_flight < ring) {
+                if (p_pending == 0) {
+                    if (p_sources != 0 && p_chunk + 1 < p_end) {
+                        ++p_chunk;
+                        p_pending = p_sources;
                     } else {
-                        ++prod.item;
-                        load_token(prod);
+                        if (n_unit >= num_units || pushed - popped >= kCombineQueue) break;
+                        const int tkn = unit_token(n_unit);
+                        p_chunk = n_unit < whole ? 0 : (n_unit - whole) - (tkn - whole) * num_chunks;
+                        p_end = n_unit < whole ? num_chunks : p_chunk + 1;
+                        p_plan = n_plan;
+                        p_sources = p_pending = __ballot_sync(0xffffffffu, p_plan >= 0);
+                        if (lane == 0) s_queue[pushed % kCombineQueue] = make_int4(tkn, p_chunk, p_end, static_cast<int>(p_sources));
+                        ++pushed;
+                        n_unit = __shfl_sync(0xffffffffu, n_claim, 0);
+                        n_plan = load_plan(n_unit);
+                        if (n_unit < num_units) n_claim = claim();
                     }
                     continue;
                 }
-                const int k = __ffs(prod.pending) - 1;
-                prod.pending &= prod.pending - 1;
-                const int p = __shfl_sync(0xffffffffu, prod.plan_k, k);
+                const int k = __ffs(p_pending) - 1;
+                p_pending &= p_pending - 1;
+                const int p = __shfl_sync(0xffffffffu, p_plan, k);
                 if (lane == 0) {
-                    const int c = prod.item % num_chunks;
-                    const int bytes = min(kChunk, row_bytes - c * kChunk);
-                    const int b = issued % ring;
-                    const uint8_t* src = s_peer[p >> 24] + a.off_x + static_cast<int64_t>(p & 0xffffff) * row_bytes +
-                                         static_cast<int64_t>(c) * kChunk;
-                    ptx::mbar_arrive_expect_tx(&s_bar[b], bytes);
-                    ptx::bulk_load(s_data + b * kChunk, src, bytes, &s_bar[b]);
+                    const int bytes = kFull ? kChunk : min(kChunk, row_bytes - p_chunk * kChunk);
+                    const uint8_t* src = s_peer[p >> 24] + a.off_x + static_cast<int64_t>(p & 0xffffff) * row_bytes + p_chunk * kChunk;
+                    ptx::mbar_arrive_expect_tx(&s_bar[p_slot], bytes);
+                    ptx::bulk_load(s_data + p_slot * kChunk, src, bytes, &s_bar[p_slot]);
                 }
-                ++issued;
+                p_slot = p_slot + 1 == ring ? 0 : p_slot + 1;
+                ++in_flight;
             }
+            __syncwarp();     // queue entries are visible to all lanes
         };
 
-        // consumer: pop the next claimed range (making the producer claim one if it has not run ahead)
-        auto consumer_next_range = [&](PullCursor& c) {
-            if (started == claimed) {
-                // the producer has used up all its claims too: it sits at the end of its current range
-                int len;
-                const int base = claim_range(len);
-                set_range(prod, base, len);
-            }
-            const int base = s_queue[started % kCombineQueue], len = s_qlen[started % kCombineQueue];
-            ++started;
-            set_range(c, base, len);
-        };
-        consumer_next_range(cons);
-        for (; cons.item < total_items && alive;) {
-            const int t = cons.token, c = cons.item % num_chunks;
-            const int bytes = min(kChunk, row_bytes - c * kChunk);
-            const int col0 = c * kChunk;   // byte offset inside the row
-            issue_ahead();
-
-            float acc[kUnroll * 8];
-#pragma unroll
-            for (int i = 0; i < kUnroll * 8; ++i) acc[i] = 0.f;
-            // bias0 + bias1 in fp32 first
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const uint8_t* bias = reinterpret_cast<const uint8_t*>(b == 0 ? a.bias0 : a.bias1);
-                if (bias == nullptr) continue;
-#pragma unroll
-                for (int u = 0; u < kUnroll; ++u) {
-                    const int off = (u * 32 + lane) * 16;
-                    if (off < bytes) {
-                        const int4 raw = ptx::ld_nc_v4(bias + static_cast<int64_t>(t) * row_bytes + col0 + off);
-                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(h[j]);
-                            acc[u * 8 + 2 * j] += f.x;
-                            acc[u * 8 + 2 * j + 1] += f.y;
-                        }
-                    }
-                }
-            }
-            // weights that travel back with the rows (dispatch backward): one small peer load per lane
-            if (c == 0 && a.out_w != nullptr && lane < K) {
-                const int ls = a.lane_src[static_cast<int64_t>(t) * K + lane];
-                float w = 0.f;
-                if (ls >= 0) {
-                    const float* wp = reinterpret_cast<const float*>(s_peer[ls >> 24] + a.off_w);
-                    const int64_t row = ls & 0xffffff;
-                    w = *reinterpret_cast<const volatile float*>(a.w_cols == 1 ? wp + row : wp + row * a.w_cols + lane);
-                }
-                a.out_w[static_cast<int64_t>(t) * K + lane] = w;
-            }
+        int c_slot = 0;
+        uint32_t c_parity = 0;
+        issue_ahead();
+        while (popped != pushed && alive) {
+            const int4 unit = s_queue[popped % kCombineQueue];
+            __syncwarp();
+            ++popped;
+            const int t = unit.x;
             float mul_k = 1.f;
             if (a.mul_weights != nullptr && lane < K) mul_k = __ldg(a.mul_weights + static_cast<int64_t>(t) * K + lane);
-
-            // sources in top-k lane order; each one sits in the next ring buffer
-            uint32_t srcs = cons.pending;
-            while (srcs != 0 && alive) {
-                const int k = __ffs(srcs) - 1;
-                srcs &= srcs - 1;
-                const int b = consumed % ring;
-                alive = mbar_wait_bounded(ctx, ws, &s_bar[b], (consumed / ring) & 1, EP_PH_COMBINE_LOAD);
-                if (!alive) break;
-                const float w = __shfl_sync(0xffffffffu, mul_k, k);
-                const uint8_t* buf = s_data + b * kChunk;
+            // weights that travel back with the rows (dispatch backward): one small peer load per lane, stored after the chunk
+            const bool with_w = unit.y == 0 && a.out_w != nullptr && lane < K;
+            const int w_src = with_w ? __ldg(a.lane_src + static_cast<int64_t>(t) * K + lane) : -1;
+            for (int c = unit.y; c < unit.z && alive; ++c) {
+                const int col0 = c * kChunk;   // byte offset inside the row
+                const int bytes = kFull ? kChunk : min(kChunk, row_bytes - col0);
+                float acc[kUnroll * 8];
+                bool first = true;             // nothing accumulated yet
+                if (a.bias0 != nullptr || a.bias1 != nullptr) {
+                    // bias0 + bias1 in fp32 first
+                    first = false;
 #pragma unroll
-                for (int u = 0; u < kUnroll; ++u) {
-                    const int off = (u * 32 + lane) * 16;
-                    if (off < bytes) {
-                        const int4 raw = *reinterpret_cast<const int4*>(buf + off);
-                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+                    for (int i = 0; i < kUnroll * 8; ++i) acc[i] = 0.f;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(h[j]);
-                            acc[u * 8 + 2 * j] = fmaf(w, f.x, acc[u * 8 + 2 * j]);
-                            acc[u * 8 + 2 * j + 1] = fmaf(w, f.y, acc[u * 8 + 2 * j + 1]);
+                    for (int b = 0; b < 2; ++b) {
+                        const uint8_t* bias = reinterpret_cast<const uint8_t*>(b == 0 ? a.bias0 : a.bias1);
+                        if (bias == nullptr) continue;
+#pragma unroll
+                        for (int u = 0; u < kUnroll; ++u) {
+                            const int off = (u * 32 + lane) * 16;
+                            if (kFull || off < bytes) {
+                                const int4 raw = ptx::ld_nc_v4(bias + static_cast<int64_t>(t) * row_bytes + col0 + off);
+                                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float2 f = __bfloat1622float2(h[j]);
+                                    acc[u * 8 + 2 * j] += f.x;
+                                    acc[u * 8 + 2 * j + 1] += f.y;
+                                }
+                            }
                         }
                     }
                 }
-                // the buffer may be refilled once every lane has read it
-                ptx::fence_proxy_async_smem();
-                __syncwarp();
-                ++consumed;
-                issue_ahead();
-            }
-            if (!alive) break;
-            uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(t) * row_bytes + col0;
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int off = (u * 32 + lane) * 16;
-                if (off < bytes) {
-                    int4 raw;
-                    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(acc[u * 8 + 2 * j], acc[u * 8 + 2 * j + 1]);
-                    ptx::st_na_v4(out + off, raw);
+                float w_val = 0.f;
+                if (c == 0 && with_w && w_src >= 0) {
+                    const float* wp = reinterpret_cast<const float*>(s_peer[w_src >> 24] + a.off_w);
+                    const int64_t row = w_src & 0xffffff;
+                    w_val = *reinterpret_cast<const volatile float*>(a.w_cols == 1 ? wp + row : wp + row * a.w_cols + lane);
                 }
+
+                // sources in top-k lane order; each one sits in the next ring buffer
+                uint32_t srcs = static_cast<uint32_t>(unit.w);
+                while (srcs != 0) {
+                    const int k = __ffs(srcs) - 1;
+                    srcs &= srcs - 1;
+                    alive = mbar_wait_bounded(ctx, ws, &s_bar[c_slot], c_parity, EP_PH_COMBINE_LOAD);
+                    if (!alive) break;
+                    const float w = __shfl_sync(0xffffffffu, mul_k, k);
+                    const uint8_t* buf = s_data + c_slot * kChunk;
+                    auto add = [&](auto is_first) {
+#pragma unroll
+                        for (int u = 0; u < kUnroll; ++u) {
+                            const int off = (u * 32 + lane) * 16;
+                            const int4 raw = kFull || off < bytes ? *reinterpret_cast<const int4*>(buf + off) : make_int4(0, 0, 0, 0);
+                            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __bfloat1622float2(h[j]);
+                                acc[u * 8 + 2 * j] = fmaf(w, f.x, decltype(is_first)::value ? 0.f : acc[u * 8 + 2 * j]);
+                                acc[u * 8 + 2 * j + 1] = fmaf(w, f.y, decltype(is_first)::value ? 0.f : acc[u * 8 + 2 * j + 1]);
+                            }
+                        }
+                    };
+                    if (first) add(std::true_type{});
+                    else add(std::false_type{});
+                    first = false;
+                    // the buffer may be refilled once every lane has read it
+                    ptx::fence_proxy_async_smem();
+                    __syncwarp();
+                    --in_flight;
+                    if (++c_slot == ring) {
+                        c_slot = 0;
+                        c_parity ^= 1;
+                    }
+                    issue_ahead();
+                }
+                if (!alive) break;
+                if (first) {
+#pragma unroll
+                    for (int i = 0; i < kUnroll * 8; ++i) acc[i] = 0.f;      // a token without any row
+                }
+                uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(t) * row_bytes + col0;
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    const int off = (u * 32 + lane) * 16;
+                    if (kFull || off < bytes) {
+                        int4 raw;
+                        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(acc[u * 8 + 2 * j], acc[u * 8 + 2 * j + 1]);
+                        ptx::st_na_v4(out + off, raw);
+                    }
+                }
+                if (c == 0 && with_w) a.out_w[static_cast<int64_t>(t) * K + lane] = w_val;
             }
-            if (cons.item + 1 >= cons.range_end) consumer_next_range(cons);
-            else {
-                ++cons.item;
-                load_token(cons);
-            }
+            issue_ahead();
         }
         // loads still in flight belong to nobody once the loop was left early: give them time to land so that no
         // copy arrives in shared memory after the CTA has exited
-        for (; consumed < issued; ++consumed) mbar_drain(&s_bar[consumed % ring], (consumed / ring) & 1, 1000ull * 1000 * 1000);
+        for (; in_flight > 0; --in_flight) {
+            mbar_drain(&s_bar[c_slot], c_parity, 1000ull * 1000 * 1000);
+            if (++c_slot == ring) {
+                c_slot = 0;
+                c_parity ^= 1;
+            }
+        }
     }
 
     stamp(2);
@@ -324,13 +297,17 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a) {
     }
 }
 
-template <int kUnroll>
+template <int kUnroll, bool kFull>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32, 1) combine_kernel(const __grid_constant__ CombineArgs args) {
-    combine_body<kUnroll>(args);
+    combine_body<kUnroll, kFull>(args);
 }
-template <int kUnroll>
+template <int kUnroll, bool kFull>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32, 1) combine_kernel_multi(const CombineArgs* args) {
-    combine_body<kUnroll>(args[blockIdx.y]);
+    combine_body<kUnroll, kFull>(args[blockIdx.y]);
+}
+template <int kUnroll, bool kFull>
+const void* combine_fn(int n) {
+    return n == 1 ? (const void*)combine_kernel<kUnroll, kFull> : (const void*)combine_kernel_multi<kUnroll, kFull>;
 }
 
 // column chunk = 512 B x unroll: larger chunks amortise the per-chunk bookkeeping: 3584 B when the row divides evenly
@@ -357,13 +334,11 @@ cudaError_t launch_combine(const CombineArgs* args, int n, int num_sms, cudaStre
     const LaunchShape shape = combine_launch_shape(a0, num_sms);
     if (shape.smem_bytes > 227 * 1024) return cudaErrorInvalidValue;
     const int unroll = pick_unroll(a0);
-    const void* fn;
-    if (n == 1)
-        fn = unroll == 7 ? (const void*)combine_kernel<7> : unroll == 4 ? (const void*)combine_kernel<4>
-             : unroll == 2 ? (const void*)combine_kernel<2> : (const void*)combine_kernel<1>;
-    else
-        fn = unroll == 7 ? (const void*)combine_kernel_multi<7> : unroll == 4 ? (const void*)combine_kernel_multi<4>
-             : unroll == 2 ? (const void*)combine_kernel_multi<2> : (const void*)combine_kernel_multi<1>;
+    const bool full = a0.hidden * 2 % (512 * unroll) == 0;
+    const void* fn = unroll == 7   ? combine_fn<7, true>(n)
+                     : unroll == 4 ? (full ? combine_fn<4, true>(n) : combine_fn<4, false>(n))
+                     : unroll == 2 ? combine_fn<2, true>(n)
+                                   : (full ? combine_fn<1, true>(n) : combine_fn<1, false>(n));
     cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, shape.smem_bytes);
     if (err != cudaSuccess) return err;
     dim3 grid(shape.num_ctas, n, 1), block(shape.num_warps * 32, 1, 1);

@@ -145,3 +145,30 @@ def test_no_cpu_sync_and_col_major_sf():
             assert torch.equal(sf[:n].cpu(), expect[r]['sf'])
     finally:
         world.destroy()
+
+
+@pytest.mark.parametrize('H', [64, 512, 1088, 1536, 7168])
+@pytest.mark.parametrize('T', [1, 5, 37, 161])
+def test_combine_units_of_work(T, H):
+    """Few SMs and every chunk width: fewer tokens than warps (chunks only), a few whole tokens before the chunks, many; rows that
+    are not whole chunks; tokens without any row; two ranks, so that tokens have zero, one or two sources."""
+    from deepep_ascend_b200.backends.emulated import EmulatedWorld
+    from deepep_ascend_b200.utils import refs
+    R, E, K = 2, 8, 3
+    world = EmulatedWorld(R, num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_experts=E)
+    try:
+        xs, idxs, ws = _make_inputs(R, T, H, E, K, seed=T + H, drop=0.5)
+        outs = world.dispatch(xs, idxs, ws, E, num_sms=2)
+        expect = refs.dispatch_all(xs, None, idxs, ws, E, T, False, 1)
+        ys = [torch.randn(o[3].num_rows, H).bfloat16().cuda() for o in outs]
+        for sms in (1, 2):
+            res = world.combine(ys, [o[3] for o in outs], topk_weights=[o[2] for o in outs], num_sms=sms)
+            torch.cuda.synchronize()
+            want = refs.combine_all(ys, [e['layout'] for e in expect], H)
+            for r in range(R):
+                world.buffers[r].check_status()
+                assert torch.equal(res[r][0].cpu().view(torch.int16), want[r].view(torch.int16))
+                valid = (idxs[r] >= 0).cpu()
+                assert torch.equal(res[r][1].cpu()[valid], ws[r].cpu()[valid])
+    finally:
+        world.destroy()
