@@ -207,38 +207,47 @@ __device__ __forceinline__ void scales_from_amax(float* sf, int num_groups) {
     for (int g = ptx::lane_id(); g < num_groups; g += 32) sf[g] = __fdiv_rn(sf[g], 448.f);
 }
 
+// Instruction count is what bounds the cast (a batch is a chain of ALU work on data that is already there), so
+//   * the amax is taken on packed bf16 pairs (the largest of bf16 magnitudes is one of them: no rounding), and two steps share one
+//     register through the four shuffles of their reduction;
+//   * lane j of a half-warp computes the scale of step j, once per batch, instead of all lanes computing all of them;
+//   * products are formed two at a time (mul.rn.f32x2: the same two roundings).
+// 8192 tokens x 7168 on one rank, whole dispatch kernel: 689 -> 505 us on 8 SMs, 190 -> 144 on 32, 106 -> 84 on 64, 69 -> 63 on 148.
 __device__ __forceinline__ void cast_batch(const RowBatch& b, uint8_t* out, float* sf, int H, int batch) {
     const int lane = ptx::lane_id();
+    constexpr int kPairs = (kCastSteps + 1) / 2;
+    __nv_bfloat162 amax[kPairs];            // (step 2p, step 2p + 1)
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        __nv_bfloat162 m[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = 2 * p + q < kCastSteps ? 2 * p + q : 2 * p;
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&b.v[i]);
+            m[q] = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+        }
+        amax[p] = __hmax2(__lows2bfloat162(m[0], m[1]), __highs2bfloat162(m[0], m[1]));
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) amax[p] = __hmax2(amax[p], __shfl_xor_sync(0xffffffffu, amax[p], o));
+    // lane j of the half-warp: step j
+    const int j = lane & 15;
+    __nv_bfloat162 mine = amax[0];
+#pragma unroll
+    for (int p = 1; p < kPairs; ++p)
+        if ((j >> 1) == p) mine = amax[p];
+    const float my_amax = fmaxf((j & 1) ? __high2float(mine) : __low2float(mine), 1e-4f);
+    // 448 * (1 / amax), each step correctly rounded: bit-identical to the PyTorch expression `448.0 / amax`
+    const float my_scale = __fmul_rn(448.f, __frcp_rn(my_amax));
+    const int group = (batch * kCastSteps + j) * 2 + (lane >> 4);
+    if (j < kCastSteps && group * 128 < H) sf[group] = my_amax;      // divided by 448 once per row, see scales_from_amax
 #pragma unroll
     for (int i = 0; i < kCastSteps; ++i) {
         const int elem = ((batch * kCastSteps + i) * 32 + lane) * 8;
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&b.v[i]);
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(h[j]);
-            v[2 * j] = f.x;
-            v[2 * j + 1] = f.y;
-        }
-        float amax = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
-        amax = fmaxf(ptx::warp_max_16(amax), 1e-4f);
-        // 448 * (1 / amax), each step correctly rounded: bit-identical to the PyTorch expression `448.0 / amax`
-        const float scale = __fmul_rn(448.f, __frcp_rn(amax));
-        if (elem < H) {
-            uint32_t packed[2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] * scale, v[4 * j + 1] * scale),
-                                                              __NV_SATFINITE, __NV_E4M3);
-                const uint32_t hi = __nv_cvt_float2_to_fp8x2(
-                    make_float2(v[4 * j + 2] * scale, v[4 * j + 3] * scale), __NV_SATFINITE, __NV_E4M3);
-                packed[j] = lo | (hi << 16);
-            }
-            *reinterpret_cast<uint2*>(out + elem) = make_uint2(packed[0], packed[1]);
-            if ((lane & 15) == 0) sf[elem / 128] = amax;      // divided by 448 once per row, see scales_from_amax
-        }
+        const float scale = __shfl_sync(0xffffffffu, my_scale, (lane & 16) + i);
+        if (elem < H) *reinterpret_cast<uint2*>(out + elem) = ptx::cast8_e4m3(b.v[i], scale);
     }
 }
 

@@ -135,6 +135,25 @@ __device__ __forceinline__ void st_na_v4(void* p, const int4& v) {
                  : "memory");
 }
 
+// ---------------------------------------------------------------- casts
+// Eight bf16 values times `scale` (fp32, round to nearest), cast to e4m3 (saturating).
+__device__ __forceinline__ uint2 cast8_e4m3(const int4& raw, float scale) {
+    uint64_t scale2;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(scale2) : "f"(scale));
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
+    uint32_t half[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        uint64_t x2;
+        float lo, hi;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x2) : "r"(w[j] << 16), "r"(w[j] & 0xffff0000u));
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(x2) : "l"(x2), "l"(scale2));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x2));
+        half[j] = __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
+    }
+    return make_uint2(half[0] | (half[1] << 16), half[2] | (half[3] << 16));
+}
+
 // ---------------------------------------------------------------- warp helpers
 __device__ __forceinline__ float warp_max_16(float v) {   // max over each aligned group of 16 lanes
 #pragma unroll
