@@ -35,12 +35,14 @@ constexpr int kBlockM = 128, kTileBytes = 128 * 128;   // A tile: 128 rows x 128
 constexpr int kMaxStages = 7;
 constexpr int kEpiRowBytes = 128 * 2 + 16;              // one staged bf16 output row (128 columns), padded against bank conflicts
 constexpr int kEpiStageBytes = 4 * 32 * kEpiRowBytes;   // four epilogue warps x 32 rows
+constexpr int kOutStageBytes = 32 * 128;                // per epilogue warp: 32 output rows x 64 bf16 columns on their way out
 // shared memory: [A stages | B stages | barriers (1 KB) | epilogue staging]
 __host__ __device__ constexpr int stage_bytes(int block_n) { return kTileBytes + block_n * 128; }
 // e4m3 tiles carry half the math per byte of bf16 tiles, so that kernel keeps as many bytes in flight as fit (7 stages)
 __host__ __device__ constexpr int num_stages(int block_n, bool fp8) { return block_n == 256 ? 4 : (fp8 ? 7 : 5); }
 __host__ __device__ constexpr int gemm_smem_bytes(int block_n, bool fp8) {
-    return num_stages(block_n, fp8) * stage_bytes(block_n) + 1024 + (block_n == 128 && !fp8 ? kEpiStageBytes : 0);
+    return num_stages(block_n, fp8) * stage_bytes(block_n) + 1024 +
+           (block_n == 256 ? (fp8 ? 8 : 4) * kOutStageBytes : (block_n == 128 && !fp8 ? kEpiStageBytes : 0));
 }
 constexpr int kMaxCopyWarps = 6;
 // copy warps of a copier CTA (all-gather fusion): each owns two 16 KB staging buffers in the shared memory that the tensor-core
@@ -160,6 +162,31 @@ __device__ __forceinline__ TileWork tile_work(const GemmArgs& g, int tile, int n
     return w;
 }
 
+// 32 rows x 64 columns of the output, one row per lane (packed bf16 pairs), leave as whole 128-byte lines: through shared memory
+// (16-byte pieces, xor-swizzled: no bank conflicts) so that eight lanes write one row together.  Stored straight from the
+// registers, every instruction touches 32 rows with 16 bytes each, and the 64 KB of a 128 x 256 tile take 4.8 us; this way
+// 0.6 us.  That time is exposed in the e4m3 kernel (its epilogue warps promote) and in bf16 products with few K blocks: 32 experts x
+// 1024 rows, e4m3 K = 7168 / N = 4096: 1.00 -> 0.96 ms, K = 2048 / N = 7168: 0.66 -> 0.55 ms; bf16 K = 2048: 0.76 -> 0.70 ms.
+__device__ __forceinline__ void store_rows_64(uint8_t* stage, const uint32_t (&w)[32], uint8_t* c, int64_t ldc, int row0, int rows, int col0, int cols) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+        *reinterpret_cast<int4*>(stage + lane * 128 + ((v ^ (lane & 7)) * 16)) = make_int4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+    __syncwarp();
+    const int v = lane & 7, col = col0 + v * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3);
+        const int4 out = *reinterpret_cast<const int4*>(stage + r * 128 + ((v ^ (r & 7)) * 16));
+        if (row0 + r < rows && col + 8 <= cols) *reinterpret_cast<int4*>(c + (static_cast<int64_t>(row0 + r) * ldc + col) * 2) = out;
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 template <int kStages>
 struct PipeState {
     int stage = 0;
@@ -200,7 +227,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int num_tiles = num_m * num_n * (g.k_group_off != nullptr ? g.num_groups : 1);
     const int gemm_ctas = static_cast<int>(gridDim.x) - g.num_copy_ctas;
     const bool is_copier = static_cast<int>(blockIdx.x) >= gemm_ctas;
-    uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;   // present only in the 128-column variant
+    uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;   // output staging: 256- and bf16 128-column variants
     Workspace* ws = g.fuse != EP_GEMM_FUSE_NONE ? local_ws(g.ctx) : nullptr;
     const uint64_t epoch = ws != nullptr ? ws->epoch[EP_CH_GEMM] + 1 : 0;
     const int tiles_per_shard = g.fuse != EP_GEMM_FUSE_NONE ? num_m / g.ctx.num_ranks : num_m;
@@ -382,23 +409,39 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     ptx::bulk_wait_read<0>();     // the staging rows were the source of the previous tile's stores
                     __syncwarp();
                 }
+                if (kBlockN % 128 == 0 && !to_peer) {
 #pragma unroll
-                for (int c = 0; c < kBlockN / 32; ++c) {
-                    uint32_t r[32];
-                    umma::tmem_ld_32x32(tmem_base + lane_addr + acc * kBlockN + c * 32, r);
-                    umma::tmem_ld_wait();
-                    if (row < g.M) {
+                    for (int c = 0; c < kBlockN / 64; ++c) {
+                        uint32_t r0[32], r1[32], w[32];
+                        umma::tmem_ld_32x32(tmem_base + lane_addr + acc * kBlockN + c * 64, r0);
+                        umma::tmem_ld_32x32(tmem_base + lane_addr + acc * kBlockN + c * 64 + 32, r1);
+                        umma::tmem_ld_wait();
 #pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            const int col = n0 + c * 32 + v * 8;
-                            if (col + 8 <= g.N) {
-                                int4 out;
-                                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
+                        for (int j = 0; j < 16; ++j) {
+                            w[j] = pack_bf16(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1]));
+                            w[16 + j] = pack_bf16(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1]));
+                        }
+                        store_rows_64(s_epi + quad * kOutStageBytes, w, cb + tw.c_row0 * g.ldc * 2, g.ldc, m_blk * kBlockM + quad * 32, g.M, n0 + c * 64, g.N);
+                    }
+                } else {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    h[j] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * j]), __uint_as_float(r[v * 8 + 2 * j + 1]));
-                                if (to_peer) *reinterpret_cast<int4*>(my_stage + (c * 32 + v * 8) * 2) = out;
-                                else *reinterpret_cast<int4*>(cb + ((tw.c_row0 + row) * g.ldc + col) * 2) = out;
+                    for (int c = 0; c < kBlockN / 32; ++c) {
+                        uint32_t r[32];
+                        umma::tmem_ld_32x32(tmem_base + lane_addr + acc * kBlockN + c * 32, r);
+                        umma::tmem_ld_wait();
+                        if (row < g.M) {
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) {
+                                const int col = n0 + c * 32 + v * 8;
+                                if (col + 8 <= g.N) {
+                                    int4 out;
+                                    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j)
+                                        h[j] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * j]), __uint_as_float(r[v * 8 + 2 * j + 1]));
+                                    if (to_peer) *reinterpret_cast<int4*>(my_stage + (c * 32 + v * 8) * 2) = out;
+                                    else *reinterpret_cast<int4*>(cb + ((tw.c_row0 + row) * g.ldc + col) * 2) = out;
+                                }
                             }
                         }
                     }
@@ -423,41 +466,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     acc_phase ^= 1;
                 }
             } else {
-                // this warp promotes one half of the tile's columns for its 32 rows
-                constexpr int kCols = kBlockN / 2;
-                const int col_half = (warp - kEpiWarp0) >> 2;
-                uint64_t sum2[kCols / 2];   // fp32 pairs (columns 2i, 2i + 1)
+                if constexpr (kWide) {
+                    // this warp promotes 128 of the 256 columns for its 32 rows; little is kept alive across the K blocks (128 sums and 64
+                    // loaded values per thread leave about 40 registers)
+                    constexpr int kCols = 128;
+                    const int col_half = (warp - kEpiWarp0) >> 2;
+                    uint64_t sum2[kCols / 2];   // fp32 pairs (columns 2i, 2i + 1)
 #pragma unroll
-                for (int i = 0; i < kCols / 2; ++i) sum2[i] = 0ull;
-                const int num_kb_sf = (g.K + 127) / 128, num_nb_sf = (g.N + 127) / 128;
-                // the B scale block of this warp's columns (a half tile never straddles two 128-column blocks)
-                const int nb_sf = min((n0 + col_half * kCols) / 128, num_nb_sf - 1);
-                const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + nb_sf) * num_kb_sf;
-                float scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row) : 0.f) * __ldg(sfb);
-                for (int kb = 0; kb < num_k && ok; ++kb) {
-                    const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale_next), __float_as_uint(scale_next));
-                    if (kb + 1 < num_k)
-                        scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row + (kb + 1) * g.sfa_stride_kb) : 0.f) * __ldg(sfb + kb + 1);
-                    ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    umma::fence_after_thread_sync();
-                    const uint32_t taddr = tmem_base + lane_addr + acc * kBlockN + col_half * kCols;
-                    if (kCols == 64) {
-                        uint32_t r0[32], r1[32];
-                        umma::tmem_ld_32x32(taddr, r0);
-                        umma::tmem_ld_32x32(taddr + 32, r1);
-                        umma::tmem_ld_wait();
-                        // the values are in registers: hand the buffer back before the arithmetic
-                        umma::fence_before_thread_sync();
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(&sm->tmem_empty[acc]);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            umma::fma_f32x2(sum2[i], umma::pack_f32x2(r0[2 * i], r0[2 * i + 1]), scale2);
-                            umma::fma_f32x2(sum2[16 + i], umma::pack_f32x2(r1[2 * i], r1[2 * i + 1]), scale2);
+                    for (int i = 0; i < kCols / 2; ++i) sum2[i] = 0ull;
+                    const int num_kb_sf = (g.K + 127) / 128, num_nb_sf = (g.N + 127) / 128;
+                    const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + min(n0 / 128 + col_half, num_nb_sf - 1)) * num_kb_sf;
+                    const float* sfa = g.sfa + min(row, g.M - 1) * g.sfa_stride_row;     // rows past the end are not stored
+                    const uint32_t taddr0 = tmem_base + lane_addr + col_half * kCols;
+                    // The scales of the next block are requested a whole block ahead and multiplied only when they are used: a product formed
+                    // at the load waits for it, and with 230 KB of shared memory taken, L1 keeps few of the scale lines.
+                    float sa = __ldg(sfa), sb = __ldg(sfb);
+#pragma unroll 1
+                    for (int kb = 0; kb < num_k; ++kb) {
+                        const float scale = sa * sb;
+                        const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale), __float_as_uint(scale));
+                        if (kb + 1 < num_k) {
+                            sfa += g.sfa_stride_kb;
+                            sa = __ldg(sfa);
+                            sb = __ldg(++sfb);
                         }
-                    } else {
+                        ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        umma::fence_after_thread_sync();
+                        const uint32_t taddr = taddr0 + acc * kBlockN;
                         // 128 columns in two steps of two loads each (64 loaded values live at a time)
 #pragma unroll
                         for (int c = 0; c < kCols / 64; ++c) {
@@ -476,26 +513,80 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 umma::fma_f32x2(sum2[c * 32 + 16 + i], umma::pack_f32x2(r1[2 * i], r1[2 * i + 1]), scale2);
                             }
                         }
+                        if (++acc == kAccBufs) {
+                            acc = 0;
+                            acc_phase ^= 1;
+                        }
                     }
-                    if (++acc == kAccBufs) {
-                        acc = 0;
-                        acc_phase ^= 1;
-                    }
-                }
-                if (ok && row < g.M) {
+                    if (ok) {
+                        const TileWork out = tile_work(g, tile, num_m, num_n, num_k, group_m, kBlockK);
 #pragma unroll
-                    for (int v = 0; v < kCols / 8; ++v) {
-                        const int col = n0 + col_half * kCols + v * 8;
-                        if (col + 8 <= g.N) {
-                            int4 out;
-                            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
+                        for (int c = 0; c < kCols / 64; ++c) {
+                            uint32_t w[32];
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
+                            for (int j = 0; j < 32; ++j) {
                                 float lo, hi;
-                                umma::unpack_f32x2(sum2[v * 4 + j], lo, hi);
-                                h[j] = __floats2bfloat162_rn(lo, hi);
+                                umma::unpack_f32x2(sum2[c * 32 + j], lo, hi);
+                                w[j] = pack_bf16(lo, hi);
                             }
-                            *reinterpret_cast<int4*>(cb + (static_cast<int64_t>(row) * g.ldc + col) * 2) = out;
+                            store_rows_64(s_epi + (warp - kEpiWarp0) * kOutStageBytes, w, cb, g.ldc, out.m * kBlockM + quad * 32, g.M,
+                                          out.n * kBlockN + col_half * kCols + c * 64, g.N);
+                        }
+                    }
+                } else {
+                    // this warp promotes one half of the tile's columns for its 32 rows
+                    constexpr int kCols = kBlockN / 2;
+                    const int col_half = (warp - kEpiWarp0) >> 2;
+                    uint64_t sum2[kCols / 2];   // fp32 pairs (columns 2i, 2i + 1)
+#pragma unroll
+                    for (int i = 0; i < kCols / 2; ++i) sum2[i] = 0ull;
+                    const int num_kb_sf = (g.K + 127) / 128, num_nb_sf = (g.N + 127) / 128;
+                    // the B scale block of this warp's columns (a half tile never straddles two 128-column blocks)
+                    const int nb_sf = min((n0 + col_half * kCols) / 128, num_nb_sf - 1);
+                    const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + nb_sf) * num_kb_sf;
+                    float scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row) : 0.f) * __ldg(sfb);
+                    for (int kb = 0; kb < num_k && ok; ++kb) {
+                        const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale_next), __float_as_uint(scale_next));
+                        if (kb + 1 < num_k)
+                            scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row + (kb + 1) * g.sfa_stride_kb) : 0.f) * __ldg(sfb + kb + 1);
+                        ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        umma::fence_after_thread_sync();
+                        const uint32_t taddr = tmem_base + lane_addr + acc * kBlockN + col_half * kCols;
+                        uint32_t r0[32], r1[32];
+                        umma::tmem_ld_32x32(taddr, r0);
+                        umma::tmem_ld_32x32(taddr + 32, r1);
+                        umma::tmem_ld_wait();
+                        // the values are in registers: hand the buffer back before the arithmetic
+                        umma::fence_before_thread_sync();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(&sm->tmem_empty[acc]);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            umma::fma_f32x2(sum2[i], umma::pack_f32x2(r0[2 * i], r0[2 * i + 1]), scale2);
+                            umma::fma_f32x2(sum2[16 + i], umma::pack_f32x2(r1[2 * i], r1[2 * i + 1]), scale2);
+                        }
+                        if (++acc == kAccBufs) {
+                            acc = 0;
+                            acc_phase ^= 1;
+                        }
+                    }
+                    if (ok && row < g.M) {
+#pragma unroll
+                        for (int v = 0; v < kCols / 8; ++v) {
+                            const int col = n0 + col_half * kCols + v * 8;
+                            if (col + 8 <= g.N) {
+                                int4 out;
+                                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    float lo, hi;
+                                    umma::unpack_f32x2(sum2[v * 4 + j], lo, hi);
+                                    h[j] = __floats2bfloat162_rn(lo, hi);
+                                }
+                                *reinterpret_cast<int4*>(cb + (static_cast<int64_t>(row) * g.ldc + col) * 2) = out;
+                            }
                         }
                     }
                 }

@@ -138,3 +138,34 @@ def test_k_grouped_gemm_on_row_major_operands(M, N, segs):
         bound = ref.abs() * 2.0 ** -8 + (a[k0:k0 + n].double().abs().t() @ b[k0:k0 + n].double().abs()) * max(n, 1) * 2.0 ** -24 + 1e-6
         assert bool(((out[e].double() - ref).abs() <= (bound if n else 0)).all()), e
         k0 += n
+
+
+@pytest.mark.parametrize('M,N,K,num_sms', [(128, 256, 128, 0), (300, 264, 256, 0), (513, 520, 1152, 2), (200, 1032, 384, 1)])
+@pytest.mark.parametrize('fp8', [False, True])
+def test_output_rows_leave_through_shared_memory(M, N, K, num_sms, fp8):
+    """Ragged last rows and columns of 256-column tiles, several tiles per CTA, an output with a row pitch whose padding must not be
+    touched."""
+    from deepep_ascend_b200.ops import gemm as ops
+    from deepep_ascend_b200.utils.math import per_token_cast_to_fp8
+    gen = torch.Generator(device='cuda').manual_seed(M + N)
+    a = torch.randn(M, K, device='cuda', generator=gen).bfloat16()
+    w = torch.randn(1, N, K, device='cuda', generator=gen).bfloat16()
+    tile_group = torch.zeros((M + 127) // 128, dtype=torch.int32, device='cuda')
+    full = torch.full((M + 1, N + 24), 7.0, dtype=torch.bfloat16, device='cuda')
+    out = full[:M, :N]
+    if fp8:
+        q, sf = per_token_cast_to_fp8(a)
+        qw, sw = ops.quantize_weight_blocks(w)
+        ops.grouped_gemm_nt(q, qw, tile_group, out=out, sfa=sf, sfb=sw, num_sms=num_sms)
+        a = q.double() * sf.double().repeat_interleave(128, 1)[:, :K]
+        w = qw.double() * sw.double().repeat_interleave(128, 1)[:, :N].repeat_interleave(128, 2)[:, :, :K]
+    else:
+        ops.grouped_gemm_nt(a, w, tile_group, out=out, num_sms=num_sms)
+    torch.cuda.synchronize()
+    assert _C().gemm_error(0) == 0
+    a, b_t = a.double(), w[0].double().t()
+    ref = a @ b_t
+    # fp32 sums (and, for e4m3, one fp32 product with the scales per 128 channels) rounded once to bf16
+    bound = ref.abs() * 2.0 ** -8 + (a.abs() @ b_t.abs()) * K * 2.0 ** -24 + 1e-6
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    assert bool((full[M:] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
