@@ -640,11 +640,13 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
         }
     }
     if (a.sf_src != nullptr) {
-        for (int c = lane; c < a.sf_cols; c += 32) {
-            const float f = __ldg(a.sf_src + static_cast<int64_t>(row) * a.sf_stride_row + c * a.sf_stride_col);
+        // every lane takes part in the shuffles, also where the last columns leave some without work
+        for (int c0 = 0; c0 < a.sf_cols; c0 += 32) {
+            const int c = c0 + lane;
+            const float f = c < a.sf_cols ? __ldg(a.sf_src + static_cast<int64_t>(row) * a.sf_stride_row + c * a.sf_stride_col) : 0.f;
             for (uint32_t m = dests; m != 0; m &= m - 1) {
                 const int64_t to = __shfl_sync(0xffffffffu, my_pos, __ffs(m) - 1);
-                a.sf_dst[to * a.sf_cols + c] = f;
+                if (c < a.sf_cols) a.sf_dst[to * a.sf_cols + c] = f;
             }
         }
     }

@@ -393,3 +393,17 @@ def test_row_major_backward_kernels(rows, I, H):
     x[~valid] = float('nan')
     ref = (x.float() * w.unsqueeze(1)).bfloat16()
     assert torch.equal(ops.weighted_rows(x, w, valid), torch.where(vm, ref, torch.zeros_like(ref)))
+
+
+@pytest.mark.parametrize('K', [1, 6, 8, 16])
+def test_expand_copy_of_few_scale_columns(K):
+    """Scale rows whose last 32-column step has fewer columns than there are top-k lanes (hidden 512 .. 5120)."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(K)
+    for G in (1, 4, 5, 31, 32, 33, 39, 40):
+        rows = 50
+        pos = torch.randperm(rows * K, device='cuda').to(torch.int32).view(rows, K)
+        x, sf = torch.randn(rows, 64, device='cuda').bfloat16(), torch.randn(rows, G, device='cuda')
+        out, sf_out = ops.local_expand_copy(pos, x, rows * K, sf=sf)
+        for k in range(K):
+            assert torch.equal(sf_out[pos[:, k].long()], sf) and torch.equal(out[pos[:, k].long()], x)
