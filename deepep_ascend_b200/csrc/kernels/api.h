@@ -316,6 +316,7 @@ struct SwigluQuantArgs {
     int64_t sf_stride_row, sf_stride_col;
     void* act_bf16;         // optional [rows, inter] bf16 copy of the activation (kept for the backward pass), or null
     int rows, inter;
+    int col_chunk;          // columns per warp, a multiple of 256 (set by the launcher)
 };
 
 // w [groups, n, k] (bf16 or fp32, contiguous, k % 8 == 0) -> e4m3 [groups, n, k] with one fp32 scale per 128 x 128 block,

@@ -10,7 +10,12 @@ namespace ep {
 
 namespace {
 
-// one warp per row; each step covers 256 channels (two 128-channel scale groups).  The loads of two steps are issued
+// A row-per-warp kernel with fewer CTAs than this splits its rows over several warps by columns (grid.y).  With 512 CTAs a split
+// gains nothing (SwiGLU of 4096 rows: 11.2 us whole, 10.7 us split in two).
+constexpr int kWantedCtas = 2 * 148;
+inline int column_splits(int ctas, int steps) { return max(1, min(steps, (kWantedCtas + ctas - 1) / max(ctas, 1))); }
+
+// one warp per row (or per part of a row); each step covers 256 channels (two 128-channel scale groups).  The loads of two steps are issued
 // before the arithmetic of the first, the sigmoid uses the fast reciprocal (the activation is rounded to bf16 right
 // after), and the correctly rounded amax / 448 of a group is computed once per 16 steps by the lane that kept that amax
 // (all lanes divide at once) instead of by two lanes in every step.
@@ -32,11 +37,12 @@ __global__ void swiglu_quant_kernel(const SwigluQuantArgs a) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= a.rows) return;
-    const int I = a.inter;
-    const uint8_t* gate = reinterpret_cast<const uint8_t*>(a.h) + static_cast<int64_t>(row) * a.ldh * 2;
-    const uint8_t* up = gate + static_cast<int64_t>(I) * 2;
-    uint8_t* q = reinterpret_cast<uint8_t*>(a.q) + static_cast<int64_t>(row) * I;
-    float* sf_row = a.sf + static_cast<int64_t>(row) * a.sf_stride_row;
+    // this warp's columns: [first, first + I) of the row
+    const int first = blockIdx.y * a.col_chunk, I = min(a.inter - first, a.col_chunk);
+    const uint8_t* gate = reinterpret_cast<const uint8_t*>(a.h) + (static_cast<int64_t>(row) * a.ldh + first) * 2;
+    const uint8_t* up = gate + static_cast<int64_t>(a.inter) * 2;
+    uint8_t* q = reinterpret_cast<uint8_t*>(a.q) + static_cast<int64_t>(row) * a.inter + first;
+    float* sf_row = a.sf + static_cast<int64_t>(row) * a.sf_stride_row + (first / 128) * a.sf_stride_col;
     const int iters = (I + 255) / 256, num_groups = (I + 127) / 128;
     float kept = 0.f;                 // amax of the group this lane will divide: step (lane & 15) of the current 16, half lane >> 4
     auto flush_scales = [&](int first_step) {
@@ -65,7 +71,7 @@ __global__ void swiglu_quant_kernel(const SwigluQuantArgs a) {
                 v[2 * j + 1] = r.y;
             }
             if (in_range && a.act_bf16 != nullptr)
-                *reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.act_bf16) + (static_cast<int64_t>(row) * I + elem) * 2) = act_raw;
+                *reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.act_bf16) + (static_cast<int64_t>(row) * a.inter + first + elem) * 2) = act_raw;
         }
         float amax = 0.f;
 #pragma unroll
@@ -522,7 +528,8 @@ __global__ void __launch_bounds__(kSegThreads) expert_segments_kernel(const Expe
 // (kPlanWarps warps per CTA).  COUNT: every warp counts its pairs per expert.  ASSIGN: a warp's first number for expert e
 // is the segment start plus the counts of all warps before it, and inside its share the warp numbers the pairs in
 // order (match_any groups the lanes of a step by expert), so the rows of an expert segment are ordered by received
-// row: the same result on every run.
+// row: the same result on every run.  Both are bound by latency, so a CTA takes 1024 pairs (one batch of four per lane) and the
+// sums over lower CTAs are shared out over its warps: 32768 pairs take 4 + 4 us (4096 pairs per CTA and serial sums: 10 + 14 us).
 constexpr int kPlanWarps = 8;
 __device__ __forceinline__ int plan_id(const LocalExpandPlanArgs& a, int i, int total) {   // rows * K < 2^31
     if (i >= total) return -1;
@@ -567,20 +574,30 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_count_kernel(con
     }
 }
 __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_assign_kernel(const LocalExpandPlanArgs a) {
-    extern __shared__ int s_plan[];                    // [kPlanWarps][El] next number of every expert for each warp
+    extern __shared__ int s_plan[];                    // [kPlanWarps][El] next number of every expert for each warp, [kPlanWarps][El] partial sums
     const int El = a.num_local_experts, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int me = blockIdx.x * kPlanWarps + warp, num_warps = gridDim.x * kPlanWarps;
     int* next = s_plan + warp * El;
+    int* part = s_plan + kPlanWarps * El;
+    // counts of the CTAs below this one, shared out over the warps (CTA 0 has none below it: it sums all CTAs for seg_end)
+    const int ctas = blockIdx.x == 0 ? gridDim.x : blockIdx.x;
     for (int e = lane; e < El; e += 32) {
-        int before = e == 0 ? 0 : __ldg(a.seg_end_aligned + e - 1), all = before;
-        for (int b = 0; b < static_cast<int>(gridDim.x); ++b) {
-            const int c = __ldg(a.cta_counts + static_cast<int64_t>(b) * El + e);
-            before += b < static_cast<int>(blockIdx.x) ? c : 0;
-            all += c;
+        int sum = 0;
+#pragma unroll 4
+        for (int b = warp; b < ctas; b += kPlanWarps) sum += __ldg(a.cta_counts + static_cast<int64_t>(b) * El + e);
+        part[warp * El + e] = sum;
+    }
+    __syncthreads();
+    for (int e = lane; e < El; e += 32) {
+        const int start = e == 0 ? 0 : __ldg(a.seg_end_aligned + e - 1);
+        int below = 0, own = 0;
+#pragma unroll
+        for (int w = 0; w < kPlanWarps; ++w) {
+            below += part[w * El + e];
+            if (w < warp) own += __ldg(a.warp_counts + static_cast<int64_t>(blockIdx.x * kPlanWarps + w) * El + e);
         }
-        for (int w = 0; w < warp; ++w) before += __ldg(a.warp_counts + static_cast<int64_t>(blockIdx.x * kPlanWarps + w) * El + e);
-        next[e] = before;
-        if (me == 0) a.seg_end[e] = all;
+        if (me == 0) a.seg_end[e] = start + below;
+        next[e] = start + (blockIdx.x == 0 ? 0 : below) + own;
     }
     __syncwarp();
     int lo, hi;
@@ -603,13 +620,15 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_assign_kernel(co
                 }
                 base = __shfl_sync(peers, base, leader);
                 a.pos[first + j * 32 + lane] = base + __popc(peers & ptx::lanemask_lt());
+            } else if (first + j * 32 + lane < hi) {
+                a.pos[first + j * 32 + lane] = -1;
             }
             __syncwarp();
         }
     }
 }
 
-// COPY: one warp per received row; every 512-byte piece is read once and written to each expert row of the row.
+// COPY: one warp per received row (or part of it); every 512-byte piece is read once and written to each expert row of the row.
 constexpr int kExpandWarps = 8, kMaxExpandTopk = 32;
 __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(const LocalExpandCopyArgs a) {
     const int lane = threadIdx.x & 31;
@@ -618,11 +637,11 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
     const int my_pos = lane < a.num_topk ? __ldg(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
     uint32_t dests = __ballot_sync(0xffffffffu, my_pos >= 0);
     if (dests == 0) return;
-    if (a.w_src != nullptr && my_pos >= 0) a.w_dst[my_pos] = __ldg(a.w_src + static_cast<int64_t>(row) * a.w_pitch + lane);
+    if (a.w_src != nullptr && my_pos >= 0 && blockIdx.y == 0) a.w_dst[my_pos] = __ldg(a.w_src + static_cast<int64_t>(row) * a.w_pitch + lane);
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src) + static_cast<int64_t>(row) * a.src_pitch;
     uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst);
     const int pieces = a.row_bytes / 16;
-    for (int p0 = 0; p0 < pieces; p0 += 128) {
+    for (int p0 = blockIdx.y * 128; p0 < pieces; p0 += 128 * gridDim.y) {
         int4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -639,7 +658,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
             }
         }
     }
-    if (a.sf_src != nullptr) {
+    if (a.sf_src != nullptr && blockIdx.y == 0) {
         // every lane takes part in the shuffles, also where the last columns leave some without work
         for (int c0 = 0; c0 < a.sf_cols; c0 += 32) {
             const int c = c0 + lane;
@@ -652,7 +671,11 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
     }
 }
 
-// REDUCE: one warp per received row; fp32 sum of its expert rows (in top-k order), optionally weighted, rounded once to bf16.
+// REDUCE: one warp per received row (or part of it); fp32 sum of its expert rows (in top-k order), optionally weighted, rounded once to bf16.
+// kAhead: source rows whose loads are in flight together (their products are always added in top-k order).  Two, with the rows split
+// by columns, when there are so few rows that latency counts (8 x 7168 channels each: 64 rows 62 -> 12 us, 512 rows 65 -> 20 us);
+// one, with whole rows, otherwise: it leaves registers for more warps (4096 rows, 530 MB: 96 us against 109 us).
+template <int kAhead>
 __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const LocalReduceArgs a) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kExpandWarps + (threadIdx.x >> 5);
@@ -664,23 +687,21 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const L
     uint8_t* out = reinterpret_cast<uint8_t*>(a.dst) + static_cast<int64_t>(row) * a.cols * 2;
     const int pieces = a.cols / 8;            // 16-byte pieces of 8 bf16
     constexpr int kPer = 4;                   // pieces per lane and step: the loads of a step are issued together
-    for (int p0 = 0; p0 < pieces; p0 += 32 * kPer) {
+    const int part = kAhead == 2 ? blockIdx.y : 0, parts = kAhead == 2 ? gridDim.y : 1;     // columns of a split row
+    for (int p0 = part * 32 * kPer; p0 < pieces; p0 += 32 * kPer * parts) {
         float acc[kPer][8];
 #pragma unroll
         for (int j = 0; j < kPer; ++j)
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-        for (uint32_t m = srcs; m != 0; m &= m - 1) {
-            const int k = __ffs(m) - 1;
-            const int64_t from = __shfl_sync(0xffffffffu, my_pos, k);
-            const float w = __shfl_sync(0xffffffffu, my_w, k);
-            const uint8_t* in = src + from * a.cols * 2;
-            int4 v[kPer];
+        auto load = [&](int4 (&v)[kPer], int64_t from) {
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const int p = p0 + j * 32 + lane;
-                v[j] = p < pieces ? ptx::ld_nc_v4(in + p * 16) : make_int4(0, 0, 0, 0);
+                v[j] = p < pieces ? ptx::ld_nc_v4(src + from * a.cols * 2 + p * 16) : make_int4(0, 0, 0, 0);
             }
+        };
+        auto add = [&](const int4 (&v)[kPer], float w) {
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
@@ -690,6 +711,26 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const L
                     acc[j][2 * i] = fmaf(w, f.x, acc[j][2 * i]);
                     acc[j][2 * i + 1] = fmaf(w, f.y, acc[j][2 * i + 1]);
                 }
+            }
+        };
+        if constexpr (kAhead == 1) {
+            for (uint32_t m = srcs; m != 0; m &= m - 1) {
+                const int k = __ffs(m) - 1;
+                int4 v[kPer];
+                load(v, __shfl_sync(0xffffffffu, my_pos, k));
+                add(v, __shfl_sync(0xffffffffu, my_w, k));
+            }
+        } else {
+            for (uint32_t m = srcs; m != 0; m &= m - 1) {
+                const int k0 = __ffs(m) - 1;
+                int4 v0[kPer], v1[kPer];
+                load(v0, __shfl_sync(0xffffffffu, my_pos, k0));
+                m &= m - 1;
+                const int k1 = __ffs(m) - 1;              // -1: no second row
+                if (k1 >= 0) load(v1, __shfl_sync(0xffffffffu, my_pos, k1));
+                add(v0, __shfl_sync(0xffffffffu, my_w, k0));
+                if (k1 < 0) break;
+                add(v1, __shfl_sync(0xffffffffu, my_w, k1));
             }
         }
 #pragma unroll
@@ -731,8 +772,12 @@ cudaError_t launch_local_expand_plan(const LocalExpandPlanArgs& a, cudaStream_t 
     if (a.num_local_experts < 1 || a.num_topk < 1 || a.num_topk > kMaxExpandTopk || a.num_rows < 0) return cudaErrorInvalidValue;
     if (a.num_ctas < 1 || a.num_local_experts > 1024 || a.warp_counts == nullptr || a.cta_counts == nullptr) return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(kPlanWarps) * a.num_local_experts * sizeof(int);
+    if (2 * smem > 48 * 1024) {
+        const cudaError_t err = cudaFuncSetAttribute(local_expand_assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(2 * smem));
+        if (err != cudaSuccess) return err;
+    }
     local_expand_count_kernel<<<a.num_ctas, kPlanWarps * 32, smem, stream>>>(a);
-    local_expand_assign_kernel<<<a.num_ctas, kPlanWarps * 32, smem, stream>>>(a);
+    local_expand_assign_kernel<<<a.num_ctas, kPlanWarps * 32, 2 * smem, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -741,7 +786,8 @@ cudaError_t launch_local_expand_copy(const LocalExpandCopyArgs& a, cudaStream_t 
     if (a.num_topk < 1 || a.num_topk > kMaxExpandTopk || a.row_bytes % 16 != 0 || a.src_pitch % 16 != 0 ||
         reinterpret_cast<uintptr_t>(a.src) % 16 != 0 || reinterpret_cast<uintptr_t>(a.dst) % 16 != 0)
         return cudaErrorInvalidValue;
-    local_expand_copy_kernel<<<(a.num_rows + kExpandWarps - 1) / kExpandWarps, kExpandWarps * 32, 0, stream>>>(a);
+    const int ctas = (a.num_rows + kExpandWarps - 1) / kExpandWarps;
+    local_expand_copy_kernel<<<dim3(ctas, column_splits(ctas, (a.row_bytes + 2047) / 2048)), kExpandWarps * 32, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -750,7 +796,10 @@ cudaError_t launch_local_reduce(const LocalReduceArgs& a, cudaStream_t stream) {
     if (a.num_topk < 1 || a.num_topk > kMaxExpandTopk || a.cols % 8 != 0 || reinterpret_cast<uintptr_t>(a.src) % 16 != 0 ||
         reinterpret_cast<uintptr_t>(a.dst) % 16 != 0)
         return cudaErrorInvalidValue;
-    local_reduce_kernel<<<(a.num_rows + kExpandWarps - 1) / kExpandWarps, kExpandWarps * 32, 0, stream>>>(a);
+    const int ctas = (a.num_rows + kExpandWarps - 1) / kExpandWarps;
+    const dim3 grid(ctas, column_splits(ctas, (a.cols + 1023) / 1024));
+    if (ctas < kWantedCtas) local_reduce_kernel<2><<<grid, kExpandWarps * 32, 0, stream>>>(a);
+    else local_reduce_kernel<1><<<grid, kExpandWarps * 32, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -773,8 +822,11 @@ cudaError_t launch_weight_quant(const WeightQuantArgs& a, cudaStream_t stream) {
 
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& a, cudaStream_t stream) {
     if (a.rows == 0) return cudaSuccess;
-    const int warps = 8;
-    swiglu_quant_kernel<<<(a.rows + warps - 1) / warps, warps * 32, 0, stream>>>(a);
+    const int warps = 8, ctas = (a.rows + warps - 1) / warps, steps = (a.inter + 255) / 256;
+    SwigluQuantArgs args = a;
+    const int per = (steps + column_splits(ctas, steps) - 1) / column_splits(ctas, steps);
+    args.col_chunk = per * 256;
+    swiglu_quant_kernel<<<dim3(ctas, (steps + per - 1) / per), warps * 32, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

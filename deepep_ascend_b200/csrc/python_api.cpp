@@ -253,7 +253,7 @@ std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::
     const int64_t rows = recv_idx.size(0), K = recv_idx.size(1), El = seg_end_aligned.numel();
     TORCH_CHECK(rows * K < (int64_t(1) << 31), "too many (row, k) pairs");
     const auto i32 = seg_end_aligned.options();
-    at::Tensor pos = at::full({rows, K}, -1, i32);
+    at::Tensor pos = at::empty({rows, K}, i32);          // every pair is written
     at::Tensor seg_end = at::empty({El}, i32);
     LocalExpandPlanArgs a{};
     a.recv_idx = recv_idx.data_ptr();
@@ -265,8 +265,8 @@ std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::
     a.seg_end_aligned = seg_end_aligned.data_ptr<int32_t>();
     a.pos = pos.data_ptr<int32_t>();
     a.seg_end = seg_end.data_ptr<int32_t>();
-    // one CTA per ~4096 pairs, at most one per SM: every warp sums the counts of all warps before it
-    a.num_ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(148, (rows * K + 4095) / 4096)));
+    // one CTA per 1024 pairs, at most one per SM
+    a.num_ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(148, (rows * K + 1023) / 1024)));
     at::Tensor scratch = at::empty({a.num_ctas * 9, El}, i32);
     a.warp_counts = scratch.data_ptr<int32_t>();
     a.cta_counts = a.warp_counts + static_cast<int64_t>(a.num_ctas) * 8 * El;

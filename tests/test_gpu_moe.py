@@ -407,3 +407,40 @@ def test_expand_copy_of_few_scale_columns(K):
         out, sf_out = ops.local_expand_copy(pos, x, rows * K, sf=sf)
         for k in range(K):
             assert torch.equal(sf_out[pos[:, k].long()], sf) and torch.equal(out[pos[:, k].long()], x)
+
+
+@pytest.mark.parametrize('rows', [1, 9, 64])
+@pytest.mark.parametrize('H,I', [(64, 16), (1032, 272), (7168, 2048)])
+def test_few_rows_are_split_by_columns(rows, H, I):
+    """With few rows the element-wise kernels give several warps one row: the bits are those of the unsplit kernel, which the same
+    rows take inside a tall tensor."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows + H)
+    K, tall = 8, 8 * 600
+    h = torch.randn(tall, 2 * I, device='cuda').bfloat16()
+    q, sf, act = ops.swiglu_quant(h, keep_bf16=True)
+    q1, sf1, act1 = ops.swiglu_quant(h[:rows].contiguous(), keep_bf16=True)
+    assert torch.equal(q1.view(torch.uint8), q[:rows].view(torch.uint8)) and torch.equal(sf1, sf[:rows]) and torch.equal(act1, act[:rows])
+    pos = torch.randperm(tall * K, device='cuda').to(torch.int32).view(tall, K)[:, :K].contiguous()
+    pos[torch.rand(tall, K, device='cuda') < 0.3] = -1
+    y = torch.randn(tall * K, H, device='cuda').bfloat16()
+    w = torch.rand(tall * K, device='cuda')
+    assert torch.equal(ops.local_reduce(pos[:rows].contiguous(), y, w=w), ops.local_reduce(pos, y, w=w)[:rows])
+    x, xs, xw = torch.randn(rows, H, device='cuda').bfloat16(), torch.randn(rows, (H + 127) // 128, device='cuda'), torch.rand(rows, K, device='cuda')
+    out, s_out, w_out = ops.local_expand_copy(pos[:rows].contiguous(), x, tall * K, sf=xs, w=xw)
+    r, k = torch.nonzero(pos[:rows] >= 0, as_tuple=True)
+    at = pos[r, k].long()
+    assert torch.equal(out[at], x[r]) and torch.equal(s_out[at], xs[r]) and torch.equal(w_out[at], xw[r, k])
+
+
+@pytest.mark.parametrize('rows,K,El', [(0, 4, 8), (1, 1, 1), (511, 2, 3), (513, 16, 40), (20000, 8, 256), (300, 8, 1024)])
+def test_expand_plan_over_many_ctas(rows, K, El):
+    """Pairs over 1 to 148 CTAs, more experts than fit the default shared memory, ids outside the local range."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows + El)
+    idx = torch.randint(-1, El + 1, (rows, K), device='cuda')
+    counts = torch.bincount(idx[(idx >= 0) & (idx < El)].flatten(), minlength=El)
+    psum = ((counts + 127) // 128 * 128).cumsum(0).to(torch.int32)
+    pos, seg_end = ops.local_expand_plan(idx, psum)
+    want_pos, want_end = ops.local_expand_plan_ref(idx.cpu(), psum.cpu())
+    assert torch.equal(pos.cpu(), want_pos) and torch.equal(seg_end.cpu(), want_end)
