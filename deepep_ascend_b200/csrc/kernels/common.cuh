@@ -137,9 +137,8 @@ __device__ __forceinline__ bool arrive_is_last(uint32_t* counter) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        const bool last = atomicAdd(counter, 1u) == gridDim.x - 1;
-        if (last) atomicExch(counter, 0u);
-        __threadfence();
+        const bool last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;      // the last arrival wraps the counter to zero
+        if (last) __threadfence();                                                // only that CTA reads what the others wrote
         s_last = last ? 1 : 0;
     }
     __syncthreads();

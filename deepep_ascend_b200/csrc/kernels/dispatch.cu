@@ -309,6 +309,12 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
         if (a.prof != nullptr && cta == 0 && tid == 0) a.prof[i] = globaltimer_ns();
     };
     stamp(0);
+    // With few tokens the row of this warp's first token (see scatter) starts on its way while the counts are exchanged: 61 tokens
+    // 30 -> 25 us.  With many, the rows would only hold up the routing ids that are counted first (8192 tokens: + 2 us).
+    if (lane == 0 && warp * num_ctas + cta < T && T <= 4 * num_ctas * num_warps) {
+        const int in_row = a.hidden * (a.x_is_fp8 ? 1 : 2);
+        ptx::bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(a.x) + static_cast<int64_t>(warp * num_ctas + cta) * in_row, in_row);
+    }
     const bool bookkeeper = cta == num_ctas - 1;   // writes what this rank receives (handle tensors, host counters); its tokens are claimed last
     const bool need_experts = a.do_expand || bookkeeper;
 
@@ -495,24 +501,33 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
 
     // -------------------------------------------------------------------- 3b. zero padding of the expand layout
     if (alive && a.do_expand && a.do_zero_padding && a.expert_alignment > 1) {
-        // rows between the end of a local expert's segment and its aligned end are written by nobody: zero them here
-        // (payload and scales), one expert per warp
+        // rows between the end of a local expert's segment and its aligned end are written by nobody: zero them here (payload
+        // and scales), single rows dealt out over all warps of the rank (an expert per warp left whole segments to single warps:
+        // 64 experts with up to 127 rows of 8 KB each held the kernel up by 80 us)
         const uint32_t A = a.expert_alignment;
         const int out_row = (kQuant || a.x_is_fp8) ? a.hidden : a.hidden * 2;
         const bool has_sf = kQuant || a.sf != nullptr;
         uint8_t* base = s_peer[me];
-        for (int j = cta * num_warps + warp; j < El; j += num_ctas * num_warps) {
-            uint32_t end;
-            if (a.cached) end = static_cast<uint32_t>(__ldcg(a.psum_expert + j));
-            else end = s_start[me * El + j] + s_tot[me * El + j];
-            uint32_t aligned_end = (end + A - 1) / A * A;
-            if (aligned_end > static_cast<uint32_t>(a.recv_capacity_rows)) aligned_end = a.recv_capacity_rows;
-            for (uint32_t row = end; row < aligned_end; ++row) {
-                uint8_t* dst = base + a.off_recv_x + static_cast<int64_t>(row) * out_row;
-                for (int off = lane * 16; off < out_row; off += 32 * 16) ptx::st_na_v4(dst + off, make_int4(0, 0, 0, 0));
-                if (has_sf) {
-                    float* sfp = reinterpret_cast<float*>(base + a.off_recv_sf);
-                    for (int g = lane; g < G; g += 32) sfp[static_cast<int64_t>(row) * a.sf_stride_row + g * a.sf_stride_col] = 0.f;
+        const uint32_t total_warps = num_ctas * num_warps, gw = warp * num_ctas + cta;
+        for (int j0 = 0; j0 < El; j0 += 32) {
+            const int j = j0 + lane;
+            uint32_t first = 0, end = 0;      // this warp's rows of expert j: first, first + total_warps, ... below `end`
+            if (j < El) {
+                const uint32_t seg = a.cached ? static_cast<uint32_t>(__ldcg(a.psum_expert + j)) : s_start[me * El + j] + s_tot[me * El + j];
+                end = min((seg + A - 1) / A * A, static_cast<uint32_t>(a.recv_capacity_rows));
+                // the deal goes on from expert to expert, about A / 2 rows each
+                first = seg + (gw + total_warps - (static_cast<uint32_t>(j) * (A / 2 + 1)) % total_warps) % total_warps;
+            }
+            for (uint32_t m = __ballot_sync(0xffffffffu, first < end); m != 0; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const uint32_t row_end = __shfl_sync(0xffffffffu, end, src);
+                for (uint32_t row = __shfl_sync(0xffffffffu, first, src); row < row_end; row += total_warps) {
+                    uint8_t* dst = base + a.off_recv_x + static_cast<int64_t>(row) * out_row;
+                    for (int off = lane * 16; off < out_row; off += 32 * 16) ptx::st_na_v4(dst + off, make_int4(0, 0, 0, 0));
+                    if (has_sf) {
+                        float* sfp = reinterpret_cast<float*>(base + a.off_recv_sf);
+                        for (int g = lane; g < G; g += 32) sfp[static_cast<int64_t>(row) * a.sf_stride_row + g * a.sf_stride_col] = 0.f;
+                    }
                 }
             }
         }
@@ -531,27 +546,23 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
         const int S_side = sp.n_side;
         const int num_batches = ((a.hidden + 255) / 256 + kCastSteps - 1) / kCastSteps;
         const uint32_t lt = ptx::lanemask_lt();
-        // Tokens are claimed dynamically from a counter shared by all CTAs of this rank: SMs that get a smaller share of
-        // the NVLink bandwidth simply claim fewer tokens.  Two tokens per claim, one near the end so that no warp is
-        // left with a long tail.  The counter is zero at entry: the last CTA of every call clears it.
-        const int tail_zone = 4 * num_ctas * num_warps;
-        int last_base = 0;
-        auto claim = [&](int& amount) -> int {
-            amount = last_base + tail_zone < T ? 2 : 1;
-            int b = 0;
-            if (lane == 0) b = static_cast<int>(atomicAdd(&ws->dyn_counter[EP_CH_DISPATCH], static_cast<uint32_t>(amount)));
-            b = __shfl_sync(0xffffffffu, b, 0);
-            last_base = b;
-            return b;
+        // The first token of every warp is fixed (with few tokens its row was requested into L2 at kernel entry); later ones are claimed from a
+        // counter shared by all CTAs of this rank: SMs that get a smaller share of the NVLink bandwidth simply claim fewer
+        // tokens.  Two tokens per claim, one near the end so that no warp is left with a long tail; a claim is sent one range
+        // ahead and its answer read when it is needed.  The counter is zero at entry: the last CTA of every call clears it.
+        const int total_warps = num_ctas * num_warps, tail_zone = 4 * total_warps;
+        int chunk_base = warp * num_ctas + cta, chunk_n = 1, in_chunk = 0;
+        int next_n = 1, next_claim = 0;               // lane 0 of next_claim holds the answer
+        auto claim = [&]() {
+            next_n = chunk_base + tail_zone < T ? 2 : 1;
+            if (lane == 0) next_claim = total_warps + static_cast<int>(atomicAdd(&ws->dyn_counter[EP_CH_DISPATCH], static_cast<uint32_t>(next_n)));
         };
-        int chunk_n = 0, next_n = 0;
-        int chunk_base = claim(chunk_n), next_base = claim(next_n), in_chunk = 0;
+        if (chunk_base < T) claim();
         auto next_token = [&]() -> int {
             if (in_chunk == chunk_n) {
-                chunk_base = next_base;
+                chunk_base = chunk_base < T ? __shfl_sync(0xffffffffu, next_claim, 0) : T;
                 chunk_n = next_n;
-                if (chunk_base < T) next_base = claim(next_n);
-                else next_base = T, next_n = 1;
+                if (chunk_base < T) claim();
                 in_chunk = 0;
             }
             const int t = chunk_base + in_chunk++;
@@ -720,7 +731,8 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     // ------------------------------------------------------------------------ 5. finish
     ptx::bulk_commit();
     ptx::bulk_wait<0>();
-    __threadfence_system();
+    // with side records all stores to peers are bulk stores of the first K lanes; other lanes have nothing to make visible
+    if (!a.side_packed || lane < K) __threadfence_system();
     stamp(4);
     // Every CTA arrives once its own stores are complete; only the last one stays: it tells every peer "all rows of my
     // dispatch number `epoch` have arrived", waits for the same word from every peer (the kernel must not end before

@@ -197,7 +197,8 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
         ptx::bulk_commit();
         stamp(1);
         ptx::bulk_wait<0>();
-        __threadfence_system();
+        // only threads that have stored to a peer have something to make visible
+        if (n > 0 && warp < K && lane == 0) __threadfence_system();
         stamp(2);
         // No grid barrier: the last CTA of this rank to finish its sends publishes how many messages every expert got
         // from this rank (a tagged zero means "none"); the others go straight on to the receive phase.
@@ -407,7 +408,8 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
         ptx::bulk_commit();
         stamp(1);
         ptx::bulk_wait<0>();
-        __threadfence_system();
+        // only lanes that have stored to a peer have something to make visible
+        if (n_loaded > 0 && lane == 0) __threadfence_system();
         stamp(2);
         // the last CTA of this rank to finish its stores raises this rank's flag at every peer (no grid barrier)
         if (arrive_is_last(&ws->arrive[EP_CH_LL_COMBINE][0]) && !is_aborted(ws)) {

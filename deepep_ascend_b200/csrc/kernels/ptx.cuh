@@ -76,6 +76,10 @@ __device__ __forceinline__ void bulk_store(void* gmem_dst, const void* smem_src,
                  "r"(smem_u32(smem_src)), "r"(bytes)
                  : "memory");
 }
+// global rows into L2 (16-byte aligned address and size)
+__device__ __forceinline__ void bulk_prefetch_l2(const void* gmem, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int kPending>
 __device__ __forceinline__ void bulk_wait_read() {   // sources may be overwritten afterwards
