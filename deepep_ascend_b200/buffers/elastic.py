@@ -29,6 +29,7 @@ from ..utils.comm import all_gather_object
 from ..utils.event import EventHandle, EventOverlap
 from ..utils.math import align
 from ..utils.semantic import value_or
+from ..utils.streams import current_stream, on_stream
 
 topk_idx_t = torch.int64 if int(os.environ.get('EP_NUM_TOPK_IDX_BITS', '64')) == 64 else torch.int32
 
@@ -362,13 +363,13 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         if self.is_cpu:
             dist.barrier(group=self.group)
             return
-        stream = self.comm_stream if use_comm_stream else torch.cuda.current_stream()
+        stream = self.comm_stream if use_comm_stream else current_stream()
         if use_comm_stream:
-            stream.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(stream):
+            stream.wait_stream(current_stream())
+        with on_stream(stream):
             self.core.barrier()
         if use_comm_stream:
-            torch.cuda.current_stream().wait_stream(stream)
+            current_stream().wait_stream(stream)
         if with_cpu_sync:
             stream.synchronize()
             self.core.check_status()
@@ -390,7 +391,7 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         if previous_event is not None and not allocate_on_comm_stream:
             raise ValueError('`previous_event` requires `allocate_on_comm_stream=True`')
         self._stream_prologue(previous_event, None)
-        with torch.cuda.stream(self.comm_stream):
+        with on_stream(self.comm_stream):
             idx = topk_idx.contiguous()
             per_rank, per_expert, in_rank = self._C.get_dispatch_layout(idx, num_experts, self.num_ranks)
         event = self._stream_epilogue(async_finish, (per_rank, per_expert, in_rank), (idx, topk_idx))
@@ -478,23 +479,23 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
 
         K = (handle.topk_idx if topk_idx is None else topk_idx).shape[1]
         num_sms = self.get_theoretical_num_sms(num_experts, K) if num_sms == 0 else num_sms
-        alloc_stream = self.comm_stream if allocate_on_comm_stream else torch.cuda.current_stream()
+        cur = current_stream()
+        prepare = (x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts, num_max_tokens_per_rank, expert_alignment,
+                   num_sms, handle, do_handle_copy, do_cpu_sync, do_expand, use_tma_aligned_col_major_sf, fused_fp8_cast, do_zero_padding)
         if allocate_on_comm_stream:
-            self._stream_prologue(previous_event, previous_event_before_epilogue)
-        with torch.cuda.stream(alloc_stream):
-            st = self._prepare_dispatch(x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts,
-                                        num_max_tokens_per_rank, expert_alignment, num_sms, handle, do_handle_copy,
-                                        do_cpu_sync, do_expand, use_tma_aligned_col_major_sf, fused_fp8_cast,
-                                        do_zero_padding)
-        if not allocate_on_comm_stream:
-            # input copies made while preparing ran on the caller's stream: wait for them too
-            self._stream_prologue(previous_event, previous_event_before_epilogue)
-        with torch.cuda.stream(self.comm_stream):
+            self._stream_prologue(previous_event, previous_event_before_epilogue, self.comm_stream, cur)
+            with on_stream(self.comm_stream):
+                st = self._prepare_dispatch(*prepare)
+        else:
+            # input copies made while preparing run on the caller's stream: wait for them too
+            st = self._prepare_dispatch(*prepare)
+            self._stream_prologue(previous_event, previous_event_before_epilogue, self.comm_stream, cur)
+        with on_stream(self.comm_stream):
             self._timed('dispatch', lambda: self.core.dispatch(st.call, num_sms))
             out = self._finish_dispatch(st)
         inputs = (st.call.x, st.call.sf, st.call.topk_idx, st.call.topk_weights, st.call.stats, st.call.lane_src,
                   st.call.plan, st.call.psum_rank, st.call.psum_expert, st.call.recv_per_expert, x, topk_idx, topk_weights)
-        event = self._stream_epilogue(async_with_compute_stream, out, inputs)
+        event = self._stream_epilogue(async_with_compute_stream, out, inputs, self.comm_stream, cur)
         return (*out, event)
 
     def _next_recv_slot(self) -> int:
@@ -520,7 +521,6 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         assert H <= self.hidden or self.hidden == 0, 'hidden exceeds what the buffer was sized for'
         assert not do_expand or self.enable_expand, 'construct the buffer with enable_expand=True for the expand layout'
         dev = x_in.device
-        i32 = dict(dtype=torch.int32, device=dev)
         call = C.DispatchCall()
         call.x = x_in.contiguous()
         if sf_in is not None:
@@ -536,11 +536,7 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
             call.psum_expert = handle.psum_num_recv_tokens_per_expert
             call.recv_per_expert = handle.num_unaligned_recv_tokens_per_expert
         else:
-            call.lane_src = torch.empty((T, K), **i32)
-            call.plan = torch.empty((T, K), **i32)
-            call.psum_rank = torch.empty((R,), **i32)
-            call.psum_expert = torch.empty((El,), **i32)
-            call.recv_per_expert = torch.empty((El,), **i32)
+            call.allocate_handle(T, K, R, El, dev)
         call.num_experts = num_experts
         call.expert_alignment = alignment
         call.num_max_tokens = num_max_tokens
@@ -599,7 +595,8 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         elif st.do_cpu_sync:
             counts = core.wait_recv_counts(El)
             num_recv, num_expanded = counts[0], counts[1]
-            per_expert_list = [align(c, st.alignment) for c in counts[2:]]
+            A = st.alignment
+            per_expert_list = counts[2:] if A == 1 else [(c + A - 1) // A * A for c in counts[2:]]
         else:
             num_recv = min(cap, R * st.call.num_max_tokens)
             num_expanded = cap if st.do_expand else 0
@@ -685,20 +682,21 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
             return self._cpu.combine(self, x, handle, topk_weights, bias0, bias1, weighted)
         num_sms = value_or(num_sms or None, handle.num_sms)
         stream = self.combine_stream
-        alloc_stream = stream if allocate_on_comm_stream else torch.cuda.current_stream()
+        cur = current_stream()
         if allocate_on_comm_stream:
-            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
-        with torch.cuda.stream(alloc_stream):
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream, cur)
+            with on_stream(stream):
+                call, out, out_w, staged = self._prepare_combine(x, handle, topk_weights, bias0, bias1, weighted, out)
+        else:
             call, out, out_w, staged = self._prepare_combine(x, handle, topk_weights, bias0, bias1, weighted, out)
-        if not allocate_on_comm_stream:
-            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
-        with torch.cuda.stream(stream):
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream, cur)
+        with on_stream(stream):
             for dst, src in staged:      # plain tensors go through the symmetric buffer
                 dst.copy_(src)
             self._timed('combine', lambda: self.core.combine(call, num_sms), stream)
         inputs = (x, topk_weights, bias0, bias1, call.bias0, call.bias1, call.mul_weights, handle.plan,
                   handle.dst_buffer_slot_idx)
-        event = self._stream_epilogue(async_with_compute_stream, (out, out_w), inputs, stream)
+        event = self._stream_epilogue(async_with_compute_stream, (out, out_w), inputs, stream, cur)
         return out, out_w, event
 
     def _prepare_combine(self, x, handle: EPHandle, topk_weights, bias0, bias1, weighted, out=None):
@@ -743,53 +741,54 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         return call, out, out_w, staged
 
     # ------------------------------------------------------------------------------------------ streams
-    def _stream_prologue(self, previous_event: Optional[EventHandle], before_epilogue: Optional[EventHandle], stream=None) -> None:
+    def _stream_prologue(self, previous_event: Optional[EventHandle], before_epilogue: Optional[EventHandle], stream=None,
+                         cur=None) -> None:
         """The communication stream waits for ``previous_event`` or for the current stream's work so far, and for
         ``before_epilogue`` (see :meth:`dispatch`)."""
         stream = self.comm_stream if stream is None else stream
         if previous_event is not None and previous_event.event is not None:
             stream.wait_event(previous_event.event)
         else:
-            stream.wait_stream(torch.cuda.current_stream())
+            stream.wait_stream(current_stream() if cur is None else cur)
         if before_epilogue is not None and before_epilogue.event is not None:
             stream.wait_event(before_epilogue.event)
 
-    def _stream_epilogue(self, async_with_compute_stream: bool, outputs, inputs=(), stream=None) -> EventOverlap:
+    def _stream_epilogue(self, async_with_compute_stream: bool, outputs, inputs=(), stream=None, cur=None) -> EventOverlap:
         """Either hand back an event on the communication stream (async) or make the current stream wait.
 
         In the async case the caching allocator must not hand a block to someone else while the other stream still
         uses it: every tensor involved (inputs read by the kernel, handle tensors, outputs; the handle is walked
         too) is recorded on both streams, or, with ``EP_AVOID_RECORD_STREAM=1``, kept alive by the returned event
         instead (csrc/elastic/buffer.hpp:558-586, 1151-1164 of the reference)."""
-        flat: List[torch.Tensor] = []
-
-        def walk(o):
-            if isinstance(o, torch.Tensor):
-                flat.append(o)
-            elif isinstance(o, (tuple, list)):
-                for i in o:
-                    walk(i)
-            elif isinstance(o, EPHandle):
-                for v in vars(o).values():
-                    if isinstance(v, torch.Tensor):
-                        flat.append(v)
-        walk(outputs)
-        walk(inputs)
         stream = self.comm_stream if stream is None else stream
+        cur = current_stream() if cur is None else cur
         if async_with_compute_stream:
+            flat: List[torch.Tensor] = []
+
+            def walk(o):
+                if isinstance(o, torch.Tensor):
+                    flat.append(o)
+                elif isinstance(o, (tuple, list)):
+                    for i in o:
+                        walk(i)
+                elif isinstance(o, EPHandle):
+                    for v in vars(o).values():
+                        if isinstance(v, torch.Tensor):
+                            flat.append(v)
+            walk(outputs)
+            walk(inputs)
             if os.environ.get('EP_AVOID_RECORD_STREAM', '0') != '1':
-                cur = torch.cuda.current_stream()
                 for t in flat:
                     if t.is_cuda:
                         t.record_stream(cur)
                         t.record_stream(stream)
             return EventOverlap(EventHandle(stream, tuple(flat)))
-        torch.cuda.current_stream().wait_stream(stream)
+        cur.wait_stream(stream)
         return EventOverlap(None)
 
     def capture(self) -> EventHandle:
         """An event on the current stream, usable as ``previous_event``."""
-        return EventHandle(torch.cuda.current_stream() if not self.is_cpu else None)
+        return EventHandle(current_stream() if not self.is_cpu else None)
 
     # ------------------------------------------------------------------------------------------ kernel timing
     def enable_kernel_timing(self, enabled: bool = True) -> None:

@@ -13,12 +13,14 @@ import torch
 
 from ..utils.event import EventHandle, EventOverlap
 from ..utils.math import align
+from ..utils.streams import current_stream, on_stream
 
 
 class LowLatencyMixin:
     """Mixed into ``ElasticBuffer``; uses ``self.core``, ``self.reserve`` and the rank attributes."""
 
     _ll = None
+    _ll_device_sms = None
 
     @staticmethod
     def get_low_latency_size_hint(num_max_dispatch_tokens_per_rank: int, hidden: int, num_ranks: int, num_experts: int,
@@ -51,7 +53,9 @@ class LowLatencyMixin:
     def _ll_num_sms(self, num_sms: int) -> int:
         if num_sms:
             return num_sms
-        return min(torch.cuda.get_device_properties('cuda').multi_processor_count, 148) if self._virtual is None else 8
+        if self._ll_device_sms is None:
+            self._ll_device_sms = min(torch.cuda.get_device_properties('cuda').multi_processor_count, 148)
+        return self._ll_device_sms if self._virtual is None else 8
 
     # ------------------------------------------------------------------------------------------ dispatch
     def _ll_prepare_dispatch(self, x, topk_idx, M, E, cumulative_stats, wait_stats, use_fp8, round_scale, use_ue8m0, phases):
@@ -109,11 +113,12 @@ class LowLatencyMixin:
                                                        use_ue8m0)
         C = self._C
         num_sms = self._ll_num_sms(num_sms)
-        stream = torch.cuda.current_stream() if return_recv_hook else self.comm_stream
+        cur = current_stream()
+        stream = cur if return_recv_hook else self.comm_stream
         if not return_recv_hook:
-            stream.wait_stream(torch.cuda.current_stream())
+            stream.wait_stream(cur)
         phases = 1 if return_recv_hook else 3
-        with torch.cuda.stream(stream):
+        with on_stream(stream):
             call, sf_view = self._ll_prepare_dispatch(x, topk_idx, M, E, cumulative_local_expert_recv_stats,
                                                       dispatch_wait_recv_cost_stats, use_fp8, round_scale, use_ue8m0, phases)
             C.ll_dispatch_group([self.core], [call], num_sms)
@@ -127,7 +132,7 @@ class LowLatencyMixin:
         elif async_finish:
             event = EventOverlap(EventHandle(stream, (call.packed_x,)))
         else:
-            torch.cuda.current_stream().wait_stream(stream)
+            cur.wait_stream(stream)
         return recv_x, call.packed_count, handle, event, hook
 
     # ------------------------------------------------------------------------------------------ combine
@@ -170,10 +175,11 @@ class LowLatencyMixin:
             return self._cpu_coll.low_latency_combine(x, topk_idx, topk_weights, handle, use_logfmt, out)
         C = self._C
         num_sms = self._ll_num_sms(num_sms)
-        stream = torch.cuda.current_stream() if return_recv_hook else self.comm_stream
+        cur = current_stream()
+        stream = cur if return_recv_hook else self.comm_stream
         if not return_recv_hook:
-            stream.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(stream):
+            stream.wait_stream(cur)
+        with on_stream(stream):
             call = self._ll_prepare_combine(x, topk_idx, topk_weights, handle, out, combine_wait_recv_cost_stats,
                                             1 if return_recv_hook else 3, use_logfmt)
             C.ll_combine_group([self.core], [call], num_sms)
@@ -185,7 +191,7 @@ class LowLatencyMixin:
         elif async_finish:
             event = EventOverlap(EventHandle(stream, (call.out,)))
         else:
-            torch.cuda.current_stream().wait_stream(stream)
+            cur.wait_stream(stream)
         return call.out, event, hook
 
     def get_next_low_latency_combine_buffer(self, handle: tuple) -> torch.Tensor:

@@ -677,6 +677,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("psum_rank", &DispatchCall::psum_rank)
         .def_readwrite("psum_expert", &DispatchCall::psum_expert)
         .def_readwrite("recv_per_expert", &DispatchCall::recv_per_expert)
+        .def("allocate_handle",
+             [](DispatchCall& c, int64_t T, int64_t K, int64_t R, int64_t El, const at::Device& device) {
+                 // the int32 tensors that a fresh dispatch writes and its handle keeps
+                 const auto i32 = at::TensorOptions().dtype(at::kInt).device(device);
+                 c.lane_src = at::empty({T, K}, i32);
+                 c.plan = at::empty({T, K}, i32);
+                 c.psum_rank = at::empty({R}, i32);
+                 c.psum_expert = at::empty({El}, i32);
+                 c.recv_per_expert = at::empty({El}, i32);
+             })
         .def_readwrite("num_experts", &DispatchCall::num_experts)
         .def_readwrite("expert_alignment", &DispatchCall::expert_alignment)
         .def_readwrite("num_max_tokens", &DispatchCall::num_max_tokens)

@@ -4,6 +4,8 @@ from typing import Any, Callable, Optional, Tuple
 
 import torch
 
+from .streams import current_stream
+
 
 class EventHandle:
     """A CUDA event recorded on the stream that ran a communication kernel, plus the tensors that must
@@ -12,13 +14,13 @@ class EventHandle:
     def __init__(self, stream: Optional['torch.cuda.Stream'] = None, keep_alive: Tuple[Any, ...] = ()):
         self.event = None
         self.keep_alive = keep_alive
-        if torch.cuda.is_available() and (stream is not None or torch.cuda.is_initialized()):
+        if stream is not None or torch.cuda.is_initialized():
             self.event = torch.cuda.Event()
-            self.event.record(stream if stream is not None else torch.cuda.current_stream())
+            self.event.record(stream if stream is not None else current_stream())
 
     def current_stream_wait(self) -> None:
         if self.event is not None:
-            torch.cuda.current_stream().wait_event(self.event)
+            current_stream().wait_event(self.event)
 
     def synchronize(self) -> None:
         if self.event is not None:
