@@ -666,7 +666,7 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         multiplied by the token's own ``topk_weights[t, k]`` (fused weighted reduce).  ``topk_weights`` given
         here are carried back to the home rank unchanged (``[rows, K]`` non-expand, ``[rows]`` expand) and
         returned as ``combined_topk_weights [T, K]``.  A plain ``x`` is first copied into the buffer's input region
-        (one local pass over the rows); a tensor obtained from :meth:`get_combine_buffer` is read in place.
+        (one local pass over the rows) when there are peers to pull it; a tensor obtained from :meth:`get_combine_buffer` is read in place.
         Stream arguments behave as in :meth:`dispatch` (the kernel runs on ``self.combine_stream``).  ``out`` (contiguous
         bf16 ``[T, H]``) receives the result in place of a new tensor.
         Returns ``(combined_x, combined_topk_weights, event)``.
@@ -707,12 +707,19 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         region = self._combine_slot_counter & 1
         self._combine_slot_counter += 1
         off_x, off_w = self.regions.combine_x(region), self.regions.combine_w(region)
-        staging = self.core.view(off_x, [rows, H], [H, 1], torch.bfloat16)
-        staged = []
-        if x.data_ptr() != staging.data_ptr():
-            staged.append((staging, x[:rows]))
+        staged, local_x = [], None
+        if (self.num_ranks == 1 and x.is_contiguous() and x.data_ptr() % 16 == 0 and x.device == handle.plan.device and
+                (out is None or out.untyped_storage().data_ptr() != x.untyped_storage().data_ptr())):
+            # Nobody else pulls: the kernel reads the rows where they are (the region or any other tensor), which saves the copy of a
+            # plain tensor: 72 MB take 29 us.  An output that shares memory with the input still needs it.
+            local_x = x
+        else:
+            staging = self.core.view(off_x, [rows, H], [H, 1], torch.bfloat16)
+            if x.data_ptr() != staging.data_ptr():
+                staged.append((staging, x[:rows]))
         call = C.CombineCall()
         call.off_x = off_x
+        call.local_x = local_x
         call.plan = handle.plan
         call.lane_src = handle.dst_buffer_slot_idx
         call.hidden = H

@@ -714,6 +714,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::class_<CombineCall>(m, "CombineCall")
         .def(py::init<>())
         .def_readwrite("off_x", &CombineCall::off_x)
+        .def_readwrite("local_x", &CombineCall::local_x)
         .def_readwrite("off_w", &CombineCall::off_w)
         .def_readwrite("w_cols", &CombineCall::w_cols)
         .def_readwrite("plan", &CombineCall::plan)

@@ -57,6 +57,7 @@ struct CombineCall {
     at::Tensor plan, lane_src;     // [T, K] int32
     OptTensor mul_weights;         // [T, K] fp32
     OptTensor bias0, bias1;        // [T, H] bf16
+    OptTensor local_x;             // one rank: contiguous bf16 rows that are read where they are, in place of the region at off_x
     at::Tensor out;                // [T, H] bf16
     OptTensor out_w;               // [T, K] fp32
     int64_t hidden = 0;
@@ -494,6 +495,15 @@ private:
             TORCH_CHECK(c.mul_weights->scalar_type() == at::kFloat && c.mul_weights->is_contiguous() &&
                             c.mul_weights->numel() == T * K, "mul_weights must be contiguous fp32 [T, K]");
         a.off_x = c.off_x;
+        if (c.local_x.has_value()) {
+            const at::Tensor& x = *c.local_x;
+            TORCH_CHECK(a.ctx.num_ranks == 1, "peers cannot reach a plain tensor");
+            TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(1) == H &&
+                            reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0,
+                        "local_x must be contiguous 16-byte aligned bf16 [rows, H]");
+            // the kernel adds the offset to the buffer's base address (modulo 2^64)
+            a.off_x = reinterpret_cast<uint64_t>(x.data_ptr()) - reinterpret_cast<uint64_t>(a.ctx.peer_base[a.ctx.rank]);
+        }
         a.off_w = c.off_w;
         a.w_cols = static_cast<int>(c.w_cols);
         a.plan = c.plan.data_ptr<int32_t>();

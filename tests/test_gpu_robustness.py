@@ -399,3 +399,44 @@ def test_buffers_allocated_with_cuda_virtual_memory():
         finally:
             world.destroy()
     assert results['ipc'] == results['vmm'] and len(results['vmm']) == 1
+
+
+@pytest.mark.parametrize('kind', ['plain', 'taller', 'strided', 'misaligned', 'region', 'into_input', 'no_rows'])
+def test_combine_input_of_one_rank_wherever_it_lies(kind):
+    """One rank reads a plain tensor in place; inputs that the kernel cannot read there (pitch, alignment, an output over the input)
+    are staged as before.  All give the same rows."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 37, 528, 8, 2
+    torch.manual_seed(5)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    try:
+        idx = torch.randint(0, E, (T, K), device='cuda')
+        idx[3] = -1
+        if kind == 'no_rows':
+            idx[:] = -1
+        x = torch.randn(T, H, device='cuda').bfloat16()
+        _, _, _, h, _ = buf.dispatch(x, idx, num_experts=E)
+        y = torch.randn(h.num_rows, H, device='cuda').bfloat16()
+        want = torch.zeros(T, H, device='cuda', dtype=torch.bfloat16)
+        rows = torch.nonzero((idx >= 0).any(1)).flatten()
+        want[rows] = y                                   # rows arrive in token order
+        out = None
+        if kind == 'taller':
+            y = torch.cat([y, torch.full((5, H), float('nan'), device='cuda').bfloat16()])
+        elif kind == 'strided':
+            y = torch.cat([y, y], dim=1)[:, :H]
+        elif kind == 'misaligned':
+            y = torch.cat([torch.zeros(1, device='cuda').bfloat16(), y.flatten()])[1:].view(-1, H)
+        elif kind == 'region':
+            buf.get_combine_buffer(h).copy_(y)
+            y = buf.get_combine_buffer(h)
+        elif kind == 'into_input':
+            big = torch.zeros(T, H, device='cuda', dtype=torch.bfloat16)
+            big[:len(rows)] = y
+            y = out = big
+        got, _, _ = buf.combine(y, h, out=out)
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert torch.equal(got, want)
+    finally:
+        buf.destroy()
