@@ -136,10 +136,12 @@ __device__ __forceinline__ TileCoord tile_coord(int tile, int num_m, int num_n, 
 // What one tile index means: output tile (m, n), weights group of B, K blocks [kb0, kb1), first output row of its group.
 struct TileWork {
     int m, n, grp, kb0, kb1;
+    int half;          // -1: the whole tile; 0 / 1: its first / second 128 columns (see the kernel)
     int64_t c_row0;
 };
 __device__ __forceinline__ TileWork tile_work(const GemmArgs& g, int tile, int num_m, int num_n, int num_k, int group_m, int block_k) {
     TileWork w;
+    w.half = -1;
     int e = 0;
     if (g.k_group_off != nullptr) {
         e = tile / (num_m * num_n);
@@ -222,17 +224,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     static_assert(kMnOperands == 0 || (!kFp8 && kBlockN % 64 == 0), "MN-major operands: bf16, whole 64-element chunks");
     constexpr uint32_t kIdesc =
         umma::make_instr_desc(kBlockM, kBlockN, kFp8 ? umma::kFormatE4M3 : umma::kFormatBF16, kMnOperands >= 2, kMnOperands >= 1);
+    constexpr uint32_t kIdescHalf = umma::make_instr_desc(kBlockM, 128, umma::kFormatE4M3);
     const int num_m = (g.M + kBlockM - 1) / kBlockM, num_n = (g.N + kBlockN - 1) / kBlockN;
     const int num_k = (g.K + kBlockK - 1) / kBlockK;
     const int num_tiles = num_m * num_n * (g.k_group_off != nullptr ? g.num_groups : 1);
     const int gemm_ctas = static_cast<int>(gridDim.x) - g.num_copy_ctas;
     const bool is_copier = static_cast<int>(blockIdx.x) >= gemm_ctas;
+    // The last wave of the wide e4m3 kernel: if it would leave at least half of the CTAs idle, its tiles are cut into halves of 128
+    // columns.  This is for products that are bound by reading the weights (one M tile per expert), where the CTAs of a
+    // thin last wave cannot pull the bandwidth that is free.
+    const int rem = num_tiles % gemm_ctas;
+    const bool cut_last = kWide && 2 * rem <= gemm_ctas;
+    const int whole_items = cut_last ? num_tiles - rem : num_tiles, num_items = cut_last ? num_tiles + rem : num_tiles;
     uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;   // output staging: 256- and bf16 128-column variants
     Workspace* ws = g.fuse != EP_GEMM_FUSE_NONE ? local_ws(g.ctx) : nullptr;
     const uint64_t epoch = ws != nullptr ? ws->epoch[EP_CH_GEMM] + 1 : 0;
     const int tiles_per_shard = g.fuse != EP_GEMM_FUSE_NONE ? num_m / g.ctx.num_ranks : num_m;
     // all-gather fusion wants the M tiles in arrival order, so its groups never span two shards
     const int group_m = g.fuse == EP_GEMM_FUSE_ALL_GATHER ? min(8, tiles_per_shard) : 16;
+
+    auto item_work = [&](int item) {
+        if (!kWide || item < whole_items) return tile_work(g, item, num_m, num_n, num_k, group_m, kBlockK);
+        TileWork w = tile_work(g, whole_items + (item - whole_items) / 2, num_m, num_n, num_k, group_m, kBlockK);
+        w.half = (item - whole_items) & 1;
+        return w;
+    };
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
@@ -266,8 +282,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             if (lane == 0) {
                 PipeState<kStages> p;
                 bool ok = true;
-                for (int tile = blockIdx.x; !is_copier && tile < num_tiles && ok; tile += gemm_ctas) {
-                    const TileWork tw = tile_work(g, tile, num_m, num_n, num_k, group_m, kBlockK);
+                for (int tile = blockIdx.x; !is_copier && tile < num_items && ok; tile += gemm_ctas) {
+                    const TileWork tw = item_work(tile);
                     const int m_blk = tw.m, n_blk = tw.n, grp = tw.grp;
                     if (grp < 0 || tw.kb1 <= tw.kb0) continue;
                     if (g.fuse == EP_GEMM_FUSE_ALL_GATHER && m_blk / tiles_per_shard != g.ctx.rank) {
@@ -300,7 +316,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
                         ok = wait_bar(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
                         if (!ok) break;
-                        ptx::mbar_arrive_expect_tx(&sm->full[p.stage], kTileBytes + kTileBytesB);
+                        ptx::mbar_arrive_expect_tx(&sm->full[p.stage], kTileBytes + (tw.half >= 0 ? kTileBytesB / 2 : kTileBytesB));
                         if constexpr (kMnOperands >= 2) {
 #pragma unroll
                             for (int i = 0; i < kBlockM / 64; ++i)
@@ -314,6 +330,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             for (int i = 0; i < kBlockN / 64; ++i)
                                 umma::tma_load_3d(s_b + p.stage * kTileBytesB + i * umma::kMnChunkBytes, &map_b, n_blk * kBlockN + i * 64, kb * kBlockK, grp,
                                                   &sm->full[p.stage]);
+                        } else if constexpr (kWide) {
+                            // boxes of 128 rows: both halves of the tile, or one
+                            const int b_row = grp * g.N + n_blk * kBlockN + (tw.half > 0 ? 128 : 0);
+                            umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, b_row, &sm->full[p.stage]);
+                            if (tw.half < 0)
+                                umma::tma_load_2d(s_b + p.stage * kTileBytesB + kTileBytesB / 2, &map_b, kb * kBlockK, b_row + 128, &sm->full[p.stage]);
                         } else {
                             umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, grp * g.N + n_blk * kBlockN, &sm->full[p.stage]);
                         }
@@ -328,8 +350,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 int acc = 0;
                 uint32_t acc_phase = 0;
                 bool ok = true;
-                for (int tile = blockIdx.x; !is_copier && tile < num_tiles && ok; tile += gemm_ctas) {
-                    const TileWork tw = tile_work(g, tile, num_m, num_n, num_k, group_m, kBlockK);
+                for (int tile = blockIdx.x; !is_copier && tile < num_items && ok; tile += gemm_ctas) {
+                    const TileWork tw = item_work(tile);
                     if (tw.grp < 0 || tw.kb1 <= tw.kb0) continue;
                     if (!kFp8) {
                         ok = wait_bar(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
@@ -354,7 +376,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
                             const uint32_t accumulate = kFp8 ? (k != 0) : (kb != tw.kb0 || k != 0);
                             umma::mma_ss<kFp8>(tmem_base + acc * kBlockN, umma::advance_desc_k(desc_a, k * kStepA),
-                                               umma::advance_desc_k(desc_b, k * kStepB), kIdesc, accumulate);
+                                               umma::advance_desc_k(desc_b, k * kStepB), kWide && tw.half >= 0 ? kIdescHalf : kIdesc, accumulate);
                         }
                         umma::mma_commit(&sm->empty[p.stage]);       // the stage may be refilled once these MMAs are done
                         p.advance();
@@ -384,8 +406,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         uint32_t acc_phase = 0;
         bool ok = true;
         uint8_t* cb = reinterpret_cast<uint8_t*>(g.c);
-        for (int tile = blockIdx.x; !is_copier && tile < num_tiles && ok; tile += gemm_ctas) {
-            const TileWork tw = tile_work(g, tile, num_m, num_n, num_k, group_m, kBlockK);
+        for (int tile = blockIdx.x; !is_copier && tile < num_items && ok; tile += gemm_ctas) {
+            const TileWork tw = item_work(tile);
             const int m_blk = tw.m, n_blk = tw.n, grp = tw.grp;
             if (grp < 0) continue;
             const int row = m_blk * kBlockM + quad * 32 + lane;
@@ -471,11 +493,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     // loaded values per thread leave about 40 registers)
                     constexpr int kCols = 128;
                     const int col_half = (warp - kEpiWarp0) >> 2;
+                    if (tw.half >= 0 && col_half == 1) {
+                        // half a tile: the first four warps have all of its columns, these only take part in the hand-over
+                        for (int kb = 0; kb < num_k; ++kb) {
+                            ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                            ok = __all_sync(0xffffffffu, ok);
+                            if (!ok) break;
+                            if (lane == 0) ptx::mbar_arrive(&sm->tmem_empty[acc]);
+                            if (++acc == kAccBufs) {
+                                acc = 0;
+                                acc_phase ^= 1;
+                            }
+                        }
+                        continue;
+                    }
                     uint64_t sum2[kCols / 2];   // fp32 pairs (columns 2i, 2i + 1)
 #pragma unroll
                     for (int i = 0; i < kCols / 2; ++i) sum2[i] = 0ull;
                     const int num_kb_sf = (g.K + 127) / 128, num_nb_sf = (g.N + 127) / 128;
-                    const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + min(n0 / 128 + col_half, num_nb_sf - 1)) * num_kb_sf;
+                    const int nb_sf = min(n0 / 128 + (tw.half > 0 ? 1 : col_half), num_nb_sf - 1);
+                    const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + nb_sf) * num_kb_sf;
                     const float* sfa = g.sfa + min(row, g.M - 1) * g.sfa_stride_row;     // rows past the end are not stored
                     const uint32_t taddr0 = tmem_base + lane_addr + col_half * kCols;
                     // The scales of the next block are requested a whole block ahead and multiplied only when they are used: a product formed
@@ -519,7 +556,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         }
                     }
                     if (ok) {
-                        const TileWork out = tile_work(g, tile, num_m, num_n, num_k, group_m, kBlockK);
+                        const TileWork out = item_work(tile);
 #pragma unroll
                         for (int c = 0; c < kCols / 64; ++c) {
                             uint32_t w[32];
@@ -530,7 +567,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 w[j] = pack_bf16(lo, hi);
                             }
                             store_rows_64(s_epi + (warp - kEpiWarp0) * kOutStageBytes, w, cb, g.ldc, out.m * kBlockM + quad * 32, g.M,
-                                          out.n * kBlockN + col_half * kCols + c * 64, g.N);
+                                          out.n * kBlockN + (out.half > 0 ? 1 : col_half) * kCols + c * 64, g.N);
                         }
                     }
                 } else {
@@ -814,7 +851,7 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     const bool maps_ok = (g.mn_operands >= 2 ? make_mn_operand_map(&map_a, g.a, 1, g.K, g.M, g.lda)
                                              : make_operand_map(&map_a, g.a, g.M, g.K, g.lda, g.is_fp8, 128)) &&
                          (g.mn_operands >= 1 ? make_mn_operand_map(&map_b, g.b, b_groups, g.K, g.N, g.ldb)
-                                             : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, block_n));
+                                             : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, g.is_fp8 ? 128 : block_n));
     if (!maps_ok) return cudaErrorInvalidValue;
     const void* fn;
     if (g.mn_operands == 2) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 2> : (const void*)gemm_kernel<false, 128, 2>;
@@ -839,7 +876,8 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         if (g.M / kBlockM >= EP_MAX_TILE_FLAGS - 1) return cudaErrorInvalidValue;
         return cudaLaunchCooperativeKernel(fn, dim3(ctas, 1, 1), dim3(kGemmThreads, 1, 1), params, kGemmSmemBytes, stream);
     }
-    if (ctas > num_tiles) ctas = num_tiles;
+    // whole tiles, or halves where all of them fit into one wave (the kernel cuts its last wave by the same rule)
+    if (ctas > num_tiles) ctas = g.is_fp8 && block_n == 256 && 2 * num_tiles <= ctas ? 2 * num_tiles : num_tiles;
     return cudaLaunchKernel(fn, dim3(ctas, 1, 1), dim3(gemm_threads(g.is_fp8 != 0, block_n), 1, 1), params, kGemmSmemBytes, stream);
 }
 
