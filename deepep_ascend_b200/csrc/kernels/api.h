@@ -274,6 +274,8 @@ struct GemmArgs {
     int64_t sfa_stride_row, sfa_stride_kb;
     const float* sfb;                 // fp8: [num_groups, ceil(N/128), ceil(K/128)] contiguous
     const int32_t* tile_group;        // [ceil(M/128)] or null (single group 0)
+    const int32_t* tile_rows;         // optional [ceil(M/128)]: leading rows of every tile that count; the others need not be read and
+                                      // their results are not needed (used by the wide e4m3 kernel, ignored elsewhere)
     int* error;                       // device int set to non-zero if a pipeline wait ran out
     uint64_t* status;                 // status block of a communication buffer that should hear about such a failure, or null
     int status_rank;
@@ -316,6 +318,7 @@ struct SwigluQuantArgs {
     int64_t sf_stride_row, sf_stride_col;
     void* act_bf16;         // optional [rows, inter] bf16 copy of the activation (kept for the backward pass), or null
     int rows, inter;
+    const uint8_t* valid;   // optional [rows]: rows with 0 are skipped (their results keep what the memory held)
     int col_chunk;          // columns per warp, a multiple of 256 (set by the launcher)
 };
 
@@ -373,6 +376,7 @@ struct ExpertSegmentsArgs {
     int32_t* tile_group;          // [ceil(num_rows / 128)] or null
     uint8_t* valid_row;           // [num_rows] or null
     int32_t* seg_off;             // [num_groups + 1] or null
+    int32_t* tile_rows;           // [ceil(num_rows / 128)] token rows of every tile, or null
 };
 
 // Local expansion of a (token, rank) layout into the (token, expert) layout of a grouped GEMM, and its inverse.  A

@@ -205,7 +205,8 @@ struct PipeState {
 // weights as they are).  2: A is [K, M] too (weight gradients read row-major activations and gradients as they are).
 template <bool kFp8, int kBlockN, int kMnOperands>
 __global__ void __launch_bounds__(gemm_threads(kFp8, kBlockN), 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs g) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a32,
+            const GemmArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kStages = num_stages(kBlockN, kFp8);
     constexpr int kTileBytesB = kBlockN * 128;
@@ -313,14 +314,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         }
                         if (!ok) break;
                     }
+                    // A thin tile (few tokens of an expert) is loaded in boxes of 32 rows: the SM's loads in flight are what bounds a
+                    // product that streams the weights, and a full box takes a third of them.  The other rows of the stage keep
+                    // what they held; their products are not stored.
+                    const int a_boxes = kWide && g.tile_rows != nullptr ? min(4, max(1, (__ldg(g.tile_rows + m_blk) + 31) / 32)) : 4;
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
                         ok = wait_bar(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
                         if (!ok) break;
-                        ptx::mbar_arrive_expect_tx(&sm->full[p.stage], kTileBytes + (tw.half >= 0 ? kTileBytesB / 2 : kTileBytesB));
+                        ptx::mbar_arrive_expect_tx(&sm->full[p.stage], a_boxes * (kTileBytes / 4) + (tw.half >= 0 ? kTileBytesB / 2 : kTileBytesB));
                         if constexpr (kMnOperands >= 2) {
 #pragma unroll
                             for (int i = 0; i < kBlockM / 64; ++i)
                                 umma::tma_load_3d(s_a + p.stage * kTileBytes + i * umma::kMnChunkBytes, &map_a, m_blk * kBlockM + i * 64, kb * kBlockK, 0,
+                                                  &sm->full[p.stage]);
+                        } else if (kWide && a_boxes < 4) {
+                            for (int i = 0; i < a_boxes; ++i)
+                                umma::tma_load_2d(s_a + p.stage * kTileBytes + i * (kTileBytes / 4), &map_a32, kb * kBlockK, m_blk * kBlockM + i * 32,
                                                   &sm->full[p.stage]);
                         } else {
                             umma::tma_load_2d(s_a + p.stage * kTileBytes, &map_a, kb * kBlockK, m_blk * kBlockM, &sm->full[p.stage]);
@@ -557,6 +566,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     }
                     if (ok) {
                         const TileWork out = item_work(tile);
+                        const int rows_end = g.tile_rows != nullptr ? min(g.M, out.m * kBlockM + __ldg(g.tile_rows + out.m)) : g.M;
 #pragma unroll
                         for (int c = 0; c < kCols / 64; ++c) {
                             uint32_t w[32];
@@ -566,7 +576,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 umma::unpack_f32x2(sum2[c * 32 + j], lo, hi);
                                 w[j] = pack_bf16(lo, hi);
                             }
-                            store_rows_64(s_epi + (warp - kEpiWarp0) * kOutStageBytes, w, cb, g.ldc, out.m * kBlockM + quad * 32, g.M,
+                            store_rows_64(s_epi + (warp - kEpiWarp0) * kOutStageBytes, w, cb, g.ldc, out.m * kBlockM + quad * 32, rows_end,
                                           out.n * kBlockN + (out.half > 0 ? 1 : col_half) * kCols + c * 64, g.N);
                         }
                     }
@@ -846,13 +856,15 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     }
     if (g.mn_operands < 0 || g.mn_operands > 2 || (g.mn_operands != 0 && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE))) return cudaErrorInvalidValue;
     if ((g.mn_operands == 2) != (g.k_group_off != nullptr && g.mn_operands != 0)) return cudaErrorInvalidValue;
-    CUtensorMap map_a, map_b;
+    CUtensorMap map_a, map_b, map_a32;
     const int64_t b_groups = g.k_group_off != nullptr ? 1 : g.num_groups;
     const bool maps_ok = (g.mn_operands >= 2 ? make_mn_operand_map(&map_a, g.a, 1, g.K, g.M, g.lda)
                                              : make_operand_map(&map_a, g.a, g.M, g.K, g.lda, g.is_fp8, 128)) &&
                          (g.mn_operands >= 1 ? make_mn_operand_map(&map_b, g.b, b_groups, g.K, g.N, g.ldb)
                                              : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, g.is_fp8 ? 128 : block_n));
     if (!maps_ok) return cudaErrorInvalidValue;
+    map_a32 = map_a;
+    if (g.is_fp8 && g.tile_rows != nullptr && !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32)) return cudaErrorInvalidValue;
     const void* fn;
     if (g.mn_operands == 2) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 2> : (const void*)gemm_kernel<false, 128, 2>;
     else if (g.mn_operands == 1) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 1> : (const void*)gemm_kernel<false, 128, 1>;
@@ -866,7 +878,7 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     if (g.k_group_off != nullptr && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE || g.tile_group != nullptr || g.num_groups < 1)) return cudaErrorInvalidValue;
     const int num_tiles = ((g.M + kBlockM - 1) / kBlockM) * ((g.N + block_n - 1) / block_n) * (g.k_group_off != nullptr ? g.num_groups : 1);
     int ctas = num_sms < 1 ? 1 : num_sms;
-    void* params[] = {&map_a, &map_b, const_cast<GemmArgs*>(&g)};
+    void* params[] = {&map_a, &map_b, &map_a32, const_cast<GemmArgs*>(&g)};
     if (g.fuse != EP_GEMM_FUSE_NONE) {
         // the CTAs of a fused launch wait on one another (grid barrier, copier -> producer flags): cooperative launch
         const int R = g.ctx.num_ranks;

@@ -36,7 +36,7 @@ __device__ __forceinline__ SwigluStep swiglu_load(const uint8_t* gate, const uin
 __global__ void swiglu_quant_kernel(const SwigluQuantArgs a) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= a.rows) return;
+    if (row >= a.rows || (a.valid != nullptr && a.valid[row] == 0)) return;
     // this warp's columns: [first, first + I) of the row
     const int first = blockIdx.y * a.col_chunk, I = min(a.inter - first, a.col_chunk);
     const uint8_t* gate = reinterpret_cast<const uint8_t*>(a.h) + (static_cast<int64_t>(row) * a.ldh + first) * 2;
@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(kSegThreads) expert_segments_kernel(const Expe
         const bool in_segment = lo < a.num_groups && row < __ldg(a.psum_ends + lo);
         if (row < a.num_rows && a.valid_row != nullptr) a.valid_row[row] = in_segment ? 1 : 0;
         if ((row & 127) == 0 && a.tile_group != nullptr) a.tile_group[row >> 7] = in_segment ? lo : -1;
+        if ((row & 127) == 0 && a.tile_rows != nullptr) a.tile_rows[row >> 7] = in_segment ? min(128, __ldg(a.psum_ends + lo) - row) : 0;
     }
 }
 

@@ -71,7 +71,7 @@ at::Tensor& gemm_error_flag(int device) {
 at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional<at::Tensor>& sfa, const std::optional<at::Tensor>& sfb,
                    const std::optional<at::Tensor>& tile_group, const std::optional<at::Tensor>& out, int64_t num_sms,
                    const std::optional<at::Tensor>& a_ready_flags, int64_t a_ready_value, const std::optional<at::Tensor>& a_flag_of_tile,
-                   ElasticBufferCore* report_to) {
+                   ElasticBufferCore* report_to, const std::optional<at::Tensor>& tile_rows) {
     TORCH_CHECK(a.is_cuda() && a.dim() == 2 && a.stride(1) == 1, "A must be [M, K] with contiguous rows");
     TORCH_CHECK(b.is_cuda() && (b.dim() == 2 || b.dim() == 3) && b.is_contiguous(), "B must be contiguous [N, K] or [G, N, K]");
     const bool fp8 = a.scalar_type() == at::kFloat8_e4m3fn;
@@ -107,6 +107,11 @@ at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional
         g.tile_group = tile_group->data_ptr<int32_t>();
     } else {
         TORCH_CHECK(G == 1, "several weight groups need tile_group");
+    }
+    if (tile_rows.has_value()) {
+        TORCH_CHECK(tile_rows->is_cuda() && tile_rows->scalar_type() == at::kInt && tile_rows->is_contiguous() && tile_rows->numel() >= (M + 127) / 128,
+                    "bad tile_rows");
+        g.tile_rows = tile_rows->data_ptr<int32_t>();
     }
     if (a_ready_flags.has_value()) {
         TORCH_CHECK(a_ready_flags->scalar_type() == at::kLong, "flags must be int64");
@@ -198,8 +203,15 @@ at::Tensor gemm_rs(ElasticBufferCore& core, const at::Tensor& a, const at::Tenso
     return out;
 }
 
-// h [rows, 2I] bf16 (gate | up) -> (e4m3 [rows, I], fp32 scales [rows, I/128], optional bf16 activation)
-std::vector<at::Tensor> swiglu_quant(const at::Tensor& h, bool keep_bf16) {
+const uint8_t* valid_ptr(const at::Tensor& valid, int64_t rows) {
+    TORCH_CHECK(valid.is_cuda() && valid.is_contiguous() && valid.numel() == rows && (valid.scalar_type() == at::kBool || valid.scalar_type() == at::kByte),
+                "valid must be a bool / uint8 tensor with one entry per row");
+    return reinterpret_cast<const uint8_t*>(valid.data_ptr());
+}
+
+// h [rows, 2I] bf16 (gate | up) -> (e4m3 [rows, I], fp32 scales [rows, I/128], optional bf16 activation).  With `valid`
+// (one bool per row) the rows marked false are skipped.
+std::vector<at::Tensor> swiglu_quant(const at::Tensor& h, bool keep_bf16, const std::optional<at::Tensor>& valid) {
     TORCH_CHECK(h.is_cuda() && h.dim() == 2 && h.stride(1) == 1 && h.scalar_type() == at::kBFloat16 && h.size(1) % 32 == 0,
                 "h must be bf16 [rows, 2 * I] with contiguous rows and I a multiple of 16");
     const int64_t rows = h.size(0), I = h.size(1) / 2;
@@ -216,12 +228,14 @@ std::vector<at::Tensor> swiglu_quant(const at::Tensor& h, bool keep_bf16) {
     a.act_bf16 = keep_bf16 ? act.data_ptr() : nullptr;
     a.rows = static_cast<int>(rows);
     a.inter = static_cast<int>(I);
+    if (valid.has_value()) a.valid = valid_ptr(*valid, rows);
     cuda_check(ep::launch_swiglu_quant(a, at::cuda::getCurrentCUDAStream()), "swiglu launch");
     if (keep_bf16) return {q, sf, act};
     return {q, sf};
 }
 
-// Expand-layout bookkeeping in one launch -> (tile_group int32 [ceil(rows / 128)], valid_row bool [rows], seg_off int32 [G + 1]).
+// Expand-layout bookkeeping in one launch -> (tile_group int32 [ceil(rows / 128)], valid_row bool [rows], seg_off int32 [G + 1],
+// tile_rows int32 [ceil(rows / 128)]).
 std::vector<at::Tensor> expert_segments(const at::Tensor& psum_ends, int64_t num_rows, int64_t alignment) {
     TORCH_CHECK(psum_ends.is_cuda() && psum_ends.is_contiguous() && psum_ends.scalar_type() == at::kInt && psum_ends.dim() == 1,
                 "psum_ends must be a contiguous int32 vector on the device");
@@ -238,8 +252,10 @@ std::vector<at::Tensor> expert_segments(const at::Tensor& psum_ends, int64_t num
     a.tile_group = tile_group.data_ptr<int32_t>();
     a.valid_row = reinterpret_cast<uint8_t*>(valid.data_ptr());
     a.seg_off = seg_off.data_ptr<int32_t>();
+    at::Tensor tile_rows = at::empty_like(tile_group);
+    a.tile_rows = tile_rows.data_ptr<int32_t>();
     cuda_check(ep::launch_expert_segments(a, at::cuda::getCurrentCUDAStream()), "expert_segments launch");
-    return {tile_group, valid, seg_off};
+    return {tile_group, valid, seg_off, tile_rows};
 }
 
 // Numbers the (row, k) pairs of a non-expand dispatch inside their experts' 128-aligned segments
@@ -336,12 +352,6 @@ at::Tensor local_reduce(const at::Tensor& pos, const at::Tensor& y, const std::o
     a.dst = res.data_ptr();
     cuda_check(ep::launch_local_reduce(a, at::cuda::getCurrentCUDAStream()), "local_reduce launch");
     return res;
-}
-
-const uint8_t* valid_ptr(const at::Tensor& valid, int64_t rows) {
-    TORCH_CHECK(valid.is_cuda() && valid.is_contiguous() && valid.numel() == rows && (valid.scalar_type() == at::kBool || valid.scalar_type() == at::kByte),
-                "valid must be a bool / uint8 tensor with one entry per row");
-    return reinterpret_cast<const uint8_t*>(valid.data_ptr());
 }
 
 const float* row_weight_ptr(const at::Tensor& w, int64_t rows) {
@@ -833,7 +843,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.attr("CH_ENGRAM") = static_cast<int>(EP_CH_ENGRAM);
     m.def("gemm_nt", &gemm_nt, py::arg("a"), py::arg("b"), py::arg("sfa") = py::none(), py::arg("sfb") = py::none(),
           py::arg("tile_group") = py::none(), py::arg("out") = py::none(), py::arg("num_sms") = 0, py::arg("a_ready_flags") = py::none(),
-          py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr);
+          py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr, py::arg("tile_rows") = py::none());
     m.def("ag_gemm", &ag_gemm);
     m.def("gemm_rs", &gemm_rs);
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));
@@ -842,7 +852,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("expert_segments", &expert_segments, py::arg("psum_ends"), py::arg("num_rows"), py::arg("alignment") = 128);
     m.def("quantize_weight_blocks", &quantize_weight_blocks);
-    m.def("swiglu_quant", &swiglu_quant, py::arg("h"), py::arg("keep_bf16") = false);
+    m.def("swiglu_quant", &swiglu_quant, py::arg("h"), py::arg("keep_bf16") = false, py::arg("valid") = py::none());
     m.def("gemm_kgrouped", &gemm_kgrouped, py::arg("a_t"), py::arg("b_t"), py::arg("k_off"), py::arg("num_sms") = 0);
     m.def("grouped_gemm_nn", &grouped_gemm_nn, py::arg("a"), py::arg("b"), py::arg("tile_group"), py::arg("out") = py::none(), py::arg("num_sms") = 0,
           py::arg("report_to") = nullptr);

@@ -24,11 +24,13 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
 
 
 def grouped_gemm_nt(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, out: Optional[torch.Tensor] = None,
-                    sfa: Optional[torch.Tensor] = None, sfb: Optional[torch.Tensor] = None, num_sms: int = 0, buffer=None) -> torch.Tensor:
+                    sfa: Optional[torch.Tensor] = None, sfb: Optional[torch.Tensor] = None, num_sms: int = 0, buffer=None,
+                    tile_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Every 128-row tile ``t`` of ``a`` is multiplied by ``b[tile_group[t]]`` (``-1`` skips the tile).  bf16 operands,
     or e4m3 operands with ``sfa [M, K/128]`` and ``sfb [G, N/128, K/128]`` fp32 block scales.  ``buffer``: see
-    :func:`gemm_nt`."""
-    return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer))
+    :func:`gemm_nt`.  ``tile_rows`` int32 (of :func:`expert_tiles`): how many leading rows of every tile count; the kernel may leave
+    the others unread and their results unwritten, which it does for e4m3 with ``N >= 256``."""
+    return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer), tile_rows)
 
 
 def _plain_cuda(t: torch.Tensor) -> bool:
@@ -71,7 +73,18 @@ def expert_segments(psum_expert_ends: torch.Tensor, num_rows: int, alignment: in
     if not psum_expert_ends.is_cuda:
         return expert_segments_ref(psum_expert_ends, num_rows, alignment)
     ends = psum_expert_ends if psum_expert_ends.dtype == torch.int32 else psum_expert_ends.to(torch.int32)
-    return tuple(_native.load().expert_segments(ends.contiguous(), num_rows, alignment))
+    return tuple(_native.load().expert_segments(ends.contiguous(), num_rows, alignment)[:3])
+
+
+def expert_tiles(psum_expert_ends: torch.Tensor, num_rows: int, alignment: int = BLOCK_M):
+    """:func:`expert_segments` with a fourth tensor, ``tile_rows int32 [ceil(num_rows / 128)]``: the token rows of every tile."""
+    if not psum_expert_ends.is_cuda:
+        tile_group, valid_row, seg_off = expert_segments_ref(psum_expert_ends, num_rows, alignment)
+        padded = torch.zeros(tile_group.numel() * BLOCK_M, dtype=torch.bool)
+        padded[:num_rows] = valid_row
+        return tile_group, valid_row, seg_off, padded.view(-1, BLOCK_M).sum(1).to(torch.int32)
+    assert alignment % BLOCK_M == 0, 'expert segments must start on a tile boundary'
+    return tuple(_native.load().expert_segments(psum_expert_ends.to(torch.int32).contiguous(), num_rows, alignment))
 
 
 def expert_tile_groups(psum_expert_ends: torch.Tensor, num_rows: int, alignment: int = BLOCK_M) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -149,9 +162,10 @@ def per_token_cast_to_fp8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     return q, sf
 
 
-def swiglu_quant(h: torch.Tensor, keep_bf16: bool = False):
-    """``h [rows, 2I]`` bf16 (gate | up) -> ``(e4m3 [rows, I], scales [rows, I/128][, bf16 activation])``."""
-    return _native.load().swiglu_quant(h, keep_bf16)
+def swiglu_quant(h: torch.Tensor, keep_bf16: bool = False, valid_row: Optional[torch.Tensor] = None):
+    """``h [rows, 2I]`` bf16 (gate | up) -> ``(e4m3 [rows, I], scales [rows, I/128][, bf16 activation])``.  Rows marked false in
+    ``valid_row`` are skipped: nothing of them is read, and their results are not written."""
+    return _native.load().swiglu_quant(h, keep_bf16, valid_row)
 
 
 def gemm_kgrouped(a_t: torch.Tensor, b_t: torch.Tensor, k_off: torch.Tensor, num_sms: int = 0) -> torch.Tensor:

@@ -444,3 +444,35 @@ def test_expand_plan_over_many_ctas(rows, K, El):
     pos, seg_end = ops.local_expand_plan(idx, psum)
     want_pos, want_end = ops.local_expand_plan_ref(idx.cpu(), psum.cpu())
     assert torch.equal(pos.cpu(), want_pos) and torch.equal(seg_end.cpu(), want_end)
+
+
+@pytest.mark.parametrize('counts', [[1, 31, 32, 33], [64, 0, 65, 96, 97], [127, 128, 129, 300, 0]])
+def test_thin_tiles_are_read_and_stored_by_rows(counts):
+    """Tiles with few token rows: results of those rows are those of the whole-tile product, other rows of the output and of the
+    activation keep what they held."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(len(counts))
+    E, N, K = len(counts), 264, 384
+    cnt = torch.tensor(counts)
+    aligned = (cnt + 127) // 128 * 128
+    ends = (aligned.cumsum(0) - aligned + cnt).to(torch.int32)
+    rows = int(aligned.sum())
+    tile_group, valid, seg_off, tile_rows = ops.expert_tiles(ends.cuda(), rows)
+    for got, want in zip((tile_group, valid, seg_off, tile_rows), ops.expert_tiles(ends, rows)):
+        assert torch.equal(got.cpu(), want)
+    x = torch.randn(rows, K, device='cuda').bfloat16()
+    q, sf = ops.per_token_cast_to_fp8(x)
+    w, sw = ops.quantize_weight_blocks(torch.randn(E, N, K, device='cuda').bfloat16())
+    want = ops.grouped_gemm_nt(q, w, tile_group, sfa=sf, sfb=sw)
+    # rows without a token hold NaN in both operands' buffers
+    q.view(torch.uint8)[~valid] = 0x7f
+    sf[~valid] = float('nan')
+    out = torch.full((rows, N), 7.0, dtype=torch.bfloat16, device='cuda')
+    for num_sms in (0, 1, 3):
+        ops.grouped_gemm_nt(q, w, tile_group, out=out, sfa=sf, sfb=sw, num_sms=num_sms, tile_rows=tile_rows)
+        assert torch.equal(out[valid], want[valid]) and bool((out[~valid] == 7.0).all())
+    h = torch.randn(rows, 512, device='cuda').bfloat16()
+    a, s = ops.swiglu_quant(h)
+    h[~valid] = float('nan')
+    a1, s1 = ops.swiglu_quant(h, valid_row=valid)
+    assert torch.equal(a1.view(torch.uint8)[valid], a.view(torch.uint8)[valid]) and torch.equal(s1[valid], s[valid])
