@@ -423,6 +423,9 @@ struct LocalReduceArgs {
 
 namespace ep {
 cudaError_t launch_local_expand_plan(const LocalExpandPlanArgs& args, cudaStream_t stream);
+int local_expand_pairs_per_cta();      // (row, k) pairs that one CTA of the plan takes
+// plan and segments (seg.psum_ends = a.seg_end); one launch when the plan has one CTA
+cudaError_t launch_local_expand_layout(const LocalExpandPlanArgs& args, const ExpertSegmentsArgs& seg, cudaStream_t stream);
 cudaError_t launch_local_expand_copy(const LocalExpandCopyArgs& args, cudaStream_t stream);
 cudaError_t launch_local_reduce(const LocalReduceArgs& args, cudaStream_t stream);
 cudaError_t launch_expert_segments(const ExpertSegmentsArgs& args, cudaStream_t stream);

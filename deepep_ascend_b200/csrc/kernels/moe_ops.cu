@@ -500,11 +500,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_weight_rows_kernel(con
 // align(end[e - 1], alignment) and holds end[e] - start rows) -> the weights group of every 128-row tile (-1: no token
 // in the tile), one validity byte per row (0: alignment padding) and the aligned segment boundaries [G + 1].
 constexpr int kSegThreads = 256;
-__global__ void __launch_bounds__(kSegThreads) expert_segments_kernel(const ExpertSegmentsArgs a) {
-    extern __shared__ int s_seg[];                    // aligned ends [G]
-    for (int e = threadIdx.x; e < a.num_groups; e += kSegThreads)
-        s_seg[e] = (__ldg(a.psum_ends + e) + a.alignment - 1) / a.alignment * a.alignment;
-    __syncthreads();
+// s_seg: aligned ends of all segments; `ends`: their unaligned ends (shared or global memory); threads / CTAs of the grid share the rows
+__device__ __forceinline__ void write_segments(const ExpertSegmentsArgs& a, const int* s_seg, const int* ends) {
     if (blockIdx.x == 0 && a.seg_off != nullptr) {
         for (int e = threadIdx.x; e <= a.num_groups; e += kSegThreads) a.seg_off[e] = e == 0 ? 0 : s_seg[e - 1];
     }
@@ -517,11 +514,19 @@ __global__ void __launch_bounds__(kSegThreads) expert_segments_kernel(const Expe
             if (s_seg[mid] > row) hi = mid;
             else lo = mid + 1;
         }
-        const bool in_segment = lo < a.num_groups && row < __ldg(a.psum_ends + lo);
+        const int end = lo < a.num_groups ? ends[lo] : 0;
+        const bool in_segment = row < end;
         if (row < a.num_rows && a.valid_row != nullptr) a.valid_row[row] = in_segment ? 1 : 0;
         if ((row & 127) == 0 && a.tile_group != nullptr) a.tile_group[row >> 7] = in_segment ? lo : -1;
-        if ((row & 127) == 0 && a.tile_rows != nullptr) a.tile_rows[row >> 7] = in_segment ? min(128, __ldg(a.psum_ends + lo) - row) : 0;
+        if ((row & 127) == 0 && a.tile_rows != nullptr) a.tile_rows[row >> 7] = in_segment ? min(128, end - row) : 0;
     }
+}
+__global__ void __launch_bounds__(kSegThreads) expert_segments_kernel(const ExpertSegmentsArgs a) {
+    extern __shared__ int s_seg[];                    // aligned ends [G]
+    for (int e = threadIdx.x; e < a.num_groups; e += kSegThreads)
+        s_seg[e] = (__ldg(a.psum_ends + e) + a.alignment - 1) / a.alignment * a.alignment;
+    __syncthreads();
+    write_segments(a, s_seg, a.psum_ends);
 }
 
 // ------------------------------------------------------------------------------------------------ local expansion
@@ -547,6 +552,46 @@ __device__ __forceinline__ void plan_share(const LocalExpandPlanArgs& a, int w, 
     lo = min(w * share, total);
     hi = min(lo + share, total);
 }
+constexpr int kPlanBatch = 4, kPlanPairsPerCta = kPlanWarps * 32 * kPlanBatch;
+// this warp's counts per expert of the pairs [lo, hi), added to `mine`
+__device__ __forceinline__ void plan_count(const LocalExpandPlanArgs& a, int lo, int hi, int* mine) {
+    const int lane = threadIdx.x & 31;
+    for (int first = lo; first < hi; first += 32 * kPlanBatch) {
+        int id[kPlanBatch];
+#pragma unroll
+        for (int j = 0; j < kPlanBatch; ++j) id[j] = plan_id(a, first + j * 32 + lane, hi);
+#pragma unroll
+        for (int j = 0; j < kPlanBatch; ++j)
+            if (id[j] >= 0) atomicAdd(mine + id[j], 1);
+    }
+}
+// numbers the pairs [lo, hi) from next[expert] on
+__device__ __forceinline__ void plan_assign(const LocalExpandPlanArgs& a, int lo, int hi, int* next) {
+    const int lane = threadIdx.x & 31;
+    for (int first = lo; first < hi; first += 32 * kPlanBatch) {
+        int id[kPlanBatch];
+#pragma unroll
+        for (int j = 0; j < kPlanBatch; ++j) id[j] = plan_id(a, first + j * 32 + lane, hi);
+#pragma unroll
+        for (int j = 0; j < kPlanBatch; ++j) {
+            // lanes with the same expert: the lowest takes the numbers for all of them
+            const uint32_t peers = __match_any_sync(0xffffffffu, id[j]);
+            if (id[j] >= 0) {
+                const int leader = __ffs(peers) - 1;
+                int base = 0;
+                if (lane == leader) {
+                    base = next[id[j]];
+                    next[id[j]] = base + __popc(peers);
+                }
+                base = __shfl_sync(peers, base, leader);
+                a.pos[first + j * 32 + lane] = base + __popc(peers & ptx::lanemask_lt());
+            } else if (first + j * 32 + lane < hi) {
+                a.pos[first + j * 32 + lane] = -1;
+            }
+            __syncwarp();
+        }
+    }
+}
 __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_count_kernel(const LocalExpandPlanArgs a) {
     extern __shared__ int s_plan[];                    // [kPlanWarps][El]
     const int El = a.num_local_experts, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -555,15 +600,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_count_kernel(con
     __syncwarp();
     int lo, hi;
     plan_share(a, blockIdx.x * kPlanWarps + warp, gridDim.x * kPlanWarps, lo, hi);
-    constexpr int kBatch = 4;
-    for (int first = lo; first < hi; first += 32 * kBatch) {
-        int id[kBatch];
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) id[j] = plan_id(a, first + j * 32 + lane, hi);
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j)
-            if (id[j] >= 0) atomicAdd(mine + id[j], 1);
-    }
+    plan_count(a, lo, hi, mine);
     __syncthreads();
     // per-warp counts and, for the prefix over CTAs, their sum
     int* out = a.warp_counts + static_cast<int64_t>(blockIdx.x * kPlanWarps + warp) * El;
@@ -603,30 +640,36 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_assign_kernel(co
     __syncwarp();
     int lo, hi;
     plan_share(a, me, num_warps, lo, hi);
-    constexpr int kBatch = 4;
-    for (int first = lo; first < hi; first += 32 * kBatch) {
-        int id[kBatch];
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) id[j] = plan_id(a, first + j * 32 + lane, hi);
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            // lanes with the same expert: the lowest takes the numbers for all of them
-            const uint32_t peers = __match_any_sync(0xffffffffu, id[j]);
-            if (id[j] >= 0) {
-                const int leader = __ffs(peers) - 1;
-                int base = 0;
-                if (lane == leader) {
-                    base = next[id[j]];
-                    next[id[j]] = base + __popc(peers);
-                }
-                base = __shfl_sync(peers, base, leader);
-                a.pos[first + j * 32 + lane] = base + __popc(peers & ptx::lanemask_lt());
-            } else if (first + j * 32 + lane < hi) {
-                a.pos[first + j * 32 + lane] = -1;
-            }
-            __syncwarp();
+    plan_assign(a, lo, hi, next);
+}
+// Few pairs (one CTA's worth): plan and segments in ONE launch.  A layer on a short prompt waits for the launches of these small
+// kernels rather than for the kernels (64 tokens: three launches less to queue between the dispatch and the first GEMM).
+__global__ void __launch_bounds__(kPlanWarps * 32) local_expand_layout_kernel(const LocalExpandPlanArgs a, const ExpertSegmentsArgs seg) {
+    extern __shared__ int s_plan[];                    // [kPlanWarps][El] counts, then next numbers; [El] segment ends; [El] aligned ends
+    static_assert(kPlanWarps * 32 == kSegThreads, "write_segments counts on the block size");
+    const int El = a.num_local_experts, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* mine = s_plan + warp * El;
+    int* s_end = s_plan + kPlanWarps * El;
+    int* s_seg = s_end + El;
+    for (int e = lane; e < El; e += 32) mine[e] = 0;
+    __syncwarp();
+    int lo, hi;
+    plan_share(a, warp, kPlanWarps, lo, hi);
+    plan_count(a, lo, hi, mine);
+    __syncthreads();
+    for (int e = threadIdx.x; e < El; e += kPlanWarps * 32) {
+        int next = e == 0 ? 0 : __ldg(a.seg_end_aligned + e - 1);
+        for (int w = 0; w < kPlanWarps; ++w) {
+            const int n = s_plan[w * El + e];
+            s_plan[w * El + e] = next;
+            next += n;
         }
+        a.seg_end[e] = s_end[e] = next;
+        s_seg[e] = (next + seg.alignment - 1) / seg.alignment * seg.alignment;
     }
+    __syncthreads();
+    plan_assign(a, lo, hi, mine);
+    write_segments(seg, s_seg, s_end);
 }
 
 // COPY: one warp per received row (or part of it); every 512-byte piece is read once and written to each expert row of the row.
@@ -779,6 +822,20 @@ cudaError_t launch_local_expand_plan(const LocalExpandPlanArgs& a, cudaStream_t 
     }
     local_expand_count_kernel<<<a.num_ctas, kPlanWarps * 32, smem, stream>>>(a);
     local_expand_assign_kernel<<<a.num_ctas, kPlanWarps * 32, 2 * smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+int local_expand_pairs_per_cta() { return kPlanPairsPerCta; }
+
+cudaError_t launch_local_expand_layout(const LocalExpandPlanArgs& a, const ExpertSegmentsArgs& seg, cudaStream_t stream) {
+    if (a.num_ctas > 1 || a.num_local_experts > 512) {
+        const cudaError_t err = launch_local_expand_plan(a, stream);
+        return err != cudaSuccess ? err : launch_expert_segments(seg, stream);
+    }
+    if (a.num_local_experts < 1 || a.num_topk < 1 || a.num_topk > kMaxExpandTopk || a.num_rows < 0) return cudaErrorInvalidValue;
+    if (seg.num_groups != a.num_local_experts || seg.alignment < 128 || seg.alignment % 128 != 0 || seg.num_rows < 0) return cudaErrorInvalidValue;
+    const size_t smem = static_cast<size_t>(kPlanWarps + 2) * a.num_local_experts * sizeof(int);       // at most 20 KB
+    local_expand_layout_kernel<<<1, kPlanWarps * 32, smem, stream>>>(a, seg);
     return cudaGetLastError();
 }
 

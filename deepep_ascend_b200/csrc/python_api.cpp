@@ -258,9 +258,11 @@ std::vector<at::Tensor> expert_segments(const at::Tensor& psum_ends, int64_t num
     return {tile_group, valid, seg_off, tile_rows};
 }
 
-// Numbers the (row, k) pairs of a non-expand dispatch inside their experts' 128-aligned segments
-// -> (pos int32 [rows, K] (-1: no local expert), seg_end int32 [El]: end of the token rows of every segment).
-std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::Tensor& seg_end_aligned) {
+struct ExpandPlan {
+    LocalExpandPlanArgs args{};
+    at::Tensor pos, seg_end, scratch;
+};
+ExpandPlan make_expand_plan(const at::Tensor& recv_idx, const at::Tensor& seg_end_aligned) {
     TORCH_CHECK(recv_idx.is_cuda() && recv_idx.dim() == 2 && recv_idx.stride(1) == 1 &&
                     (recv_idx.scalar_type() == at::kLong || recv_idx.scalar_type() == at::kInt),
                 "recv_idx must be int64 / int32 [rows, K] with contiguous rows");
@@ -269,9 +271,10 @@ std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::
     const int64_t rows = recv_idx.size(0), K = recv_idx.size(1), El = seg_end_aligned.numel();
     TORCH_CHECK(rows * K < (int64_t(1) << 31), "too many (row, k) pairs");
     const auto i32 = seg_end_aligned.options();
-    at::Tensor pos = at::empty({rows, K}, i32);          // every pair is written
-    at::Tensor seg_end = at::empty({El}, i32);
-    LocalExpandPlanArgs a{};
+    ExpandPlan p;
+    p.pos = at::empty({rows, K}, i32);          // every pair is written
+    p.seg_end = at::empty({El}, i32);
+    LocalExpandPlanArgs& a = p.args;
     a.recv_idx = recv_idx.data_ptr();
     a.idx_is_64 = recv_idx.scalar_type() == at::kLong;
     a.idx_pitch = recv_idx.stride(0);
@@ -279,15 +282,43 @@ std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::
     a.num_topk = static_cast<int>(K);
     a.num_local_experts = static_cast<int>(El);
     a.seg_end_aligned = seg_end_aligned.data_ptr<int32_t>();
-    a.pos = pos.data_ptr<int32_t>();
-    a.seg_end = seg_end.data_ptr<int32_t>();
-    // one CTA per 1024 pairs, at most one per SM
-    a.num_ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(148, (rows * K + 1023) / 1024)));
-    at::Tensor scratch = at::empty({a.num_ctas * 9, El}, i32);
-    a.warp_counts = scratch.data_ptr<int32_t>();
+    a.pos = p.pos.data_ptr<int32_t>();
+    a.seg_end = p.seg_end.data_ptr<int32_t>();
+    // one CTA per batch of pairs, at most one per SM
+    const int64_t per_cta = ep::local_expand_pairs_per_cta();
+    a.num_ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(148, (rows * K + per_cta - 1) / per_cta)));
+    p.scratch = at::empty({a.num_ctas * 9, El}, i32);
+    a.warp_counts = p.scratch.data_ptr<int32_t>();
     a.cta_counts = a.warp_counts + static_cast<int64_t>(a.num_ctas) * 8 * El;
-    cuda_check(ep::launch_local_expand_plan(a, at::cuda::getCurrentCUDAStream()), "local_expand_plan launch");
-    return {pos, seg_end};
+    return p;
+}
+
+// Numbers the (row, k) pairs of a non-expand dispatch inside their experts' 128-aligned segments
+// -> (pos int32 [rows, K] (-1: no local expert), seg_end int32 [El]: end of the token rows of every segment).
+std::vector<at::Tensor> local_expand_plan(const at::Tensor& recv_idx, const at::Tensor& seg_end_aligned) {
+    const ExpandPlan p = make_expand_plan(recv_idx, seg_end_aligned);
+    cuda_check(ep::launch_local_expand_plan(p.args, at::cuda::getCurrentCUDAStream()), "local_expand_plan launch");
+    return {p.pos, p.seg_end};
+}
+
+// local_expand_plan and expert_segments of its segments -> (pos, seg_end, tile_group, valid_row, seg_off, tile_rows)
+std::vector<at::Tensor> local_expand_layout(const at::Tensor& recv_idx, const at::Tensor& seg_end_aligned, int64_t num_rows) {
+    TORCH_CHECK(num_rows >= 0 && num_rows < (int64_t(1) << 31), "bad num_rows");
+    const ExpandPlan p = make_expand_plan(recv_idx, seg_end_aligned);
+    const auto i32 = seg_end_aligned.options();
+    at::Tensor tile_group = at::empty({(num_rows + 127) / 128}, i32), tile_rows = at::empty_like(tile_group);
+    at::Tensor valid = at::empty({num_rows}, i32.dtype(at::kBool)), seg_off = at::empty({p.seg_end.numel() + 1}, i32);
+    ExpertSegmentsArgs seg{};
+    seg.psum_ends = p.seg_end.data_ptr<int32_t>();
+    seg.num_groups = p.args.num_local_experts;
+    seg.num_rows = static_cast<int>(num_rows);
+    seg.alignment = 128;
+    seg.tile_group = tile_group.data_ptr<int32_t>();
+    seg.valid_row = reinterpret_cast<uint8_t*>(valid.data_ptr());
+    seg.seg_off = seg_off.data_ptr<int32_t>();
+    seg.tile_rows = tile_rows.data_ptr<int32_t>();
+    cuda_check(ep::launch_local_expand_layout(p.args, seg, at::cuda::getCurrentCUDAStream()), "local_expand_layout launch");
+    return {p.pos, p.seg_end, tile_group, valid, seg_off, tile_rows};
 }
 
 // Copies every received row (and its scales / weights) to its expert rows -> (rows_out [num_out, width], sf_out or none, w_out or none).
@@ -847,6 +878,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("ag_gemm", &ag_gemm);
     m.def("gemm_rs", &gemm_rs);
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));
+    m.def("local_expand_layout", &local_expand_layout);
     m.def("local_expand_copy", &local_expand_copy, py::arg("pos"), py::arg("x"), py::arg("num_out"), py::arg("sf") = py::none(),
           py::arg("w") = py::none());
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());

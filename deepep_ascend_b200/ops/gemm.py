@@ -143,6 +143,15 @@ def local_expand_plan_ref(recv_idx: torch.Tensor, psum_aligned: torch.Tensor) ->
     return pos.reshape(idx.shape).to(torch.int32), (starts + counts).to(torch.int32)
 
 
+def local_expand_layout(recv_idx: torch.Tensor, psum_aligned: torch.Tensor, num_rows: int):
+    """:func:`local_expand_plan` and :func:`expert_tiles` of its segments -> ``(pos, seg_end, tile_group, valid_row, seg_off,
+    tile_rows)``; one launch when there are at most 1024 (row, k) pairs."""
+    if not recv_idx.is_cuda:
+        pos, seg_end = local_expand_plan_ref(recv_idx, psum_aligned)
+        return (pos, seg_end, *expert_tiles(seg_end, num_rows))
+    return tuple(_native.load().local_expand_layout(recv_idx, psum_aligned.contiguous(), num_rows))
+
+
 def local_expand_copy(pos: torch.Tensor, x: torch.Tensor, num_out: int, sf: Optional[torch.Tensor] = None,
                       w: Optional[torch.Tensor] = None):
     """Writes every received row of ``x`` (and its scales ``sf [rows, G]`` / weights ``w [rows, K]``) to its expert rows ->

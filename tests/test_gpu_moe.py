@@ -433,7 +433,7 @@ def test_few_rows_are_split_by_columns(rows, H, I):
     assert torch.equal(out[at], x[r]) and torch.equal(s_out[at], xs[r]) and torch.equal(w_out[at], xw[r, k])
 
 
-@pytest.mark.parametrize('rows,K,El', [(0, 4, 8), (1, 1, 1), (511, 2, 3), (513, 16, 40), (20000, 8, 256), (300, 8, 1024)])
+@pytest.mark.parametrize('rows,K,El', [(0, 4, 8), (1, 1, 1), (511, 2, 3), (128, 8, 32), (128, 8, 512), (129, 8, 32), (64, 8, 513), (513, 16, 40), (20000, 8, 256), (300, 8, 1024)])
 def test_expand_plan_over_many_ctas(rows, K, El):
     """Pairs over 1 to 148 CTAs, more experts than fit the default shared memory, ids outside the local range."""
     from deepep_ascend_b200.ops import gemm as ops
@@ -444,6 +444,9 @@ def test_expand_plan_over_many_ctas(rows, K, El):
     pos, seg_end = ops.local_expand_plan(idx, psum)
     want_pos, want_end = ops.local_expand_plan_ref(idx.cpu(), psum.cpu())
     assert torch.equal(pos.cpu(), want_pos) and torch.equal(seg_end.cpu(), want_end)
+    # plan and segments together: one launch up to 1024 pairs and 512 experts, three otherwise
+    for got, want in zip(ops.local_expand_layout(idx, psum, int(psum[-1])), ops.local_expand_layout(idx.cpu(), psum.cpu(), int(psum[-1]))):
+        assert torch.equal(got.cpu(), want)
 
 
 @pytest.mark.parametrize('counts', [[1, 31, 32, 33], [64, 0, 65, 96, 97], [127, 128, 129, 300, 0]])
