@@ -13,6 +13,8 @@
 //                    CTAs: every row is bulk-copied into the slot [source token][top-k lane] of the token's home
 //                    rank; the last CTA to finish raises one epoch-tagged flag per rank pair.
 //            RECV  - wait for all ranks' flags, then out[t] = sum_k w[t,k] * slot[t,k] in fp32 -> bf16.
+// With one rank (both halves in one launch) nothing has to travel: dispatch stores a message's payload, scales and source straight at
+// the packed position, which is the claimed slot, and combine leaves row numbers in the slots and reduces the rows where they lie.
 // No CTA waits for another CTA of its own rank (no grid barrier): phases end with an arrival counter whose last
 // arriver does the publishing.
 // SEND and RECV can be launched separately (phases argument) so that no SM is held while data is in flight.
@@ -115,6 +117,22 @@ __device__ __forceinline__ bool shrink_wait(const RankCtx& ctx, Workspace* ws, c
     return true;
 }
 
+// the G scales of one packed row (local expert j, row `at` of `rows` per expert), stored by one warp; get(group) -> fp32 scale
+template <typename Get>
+__device__ __forceinline__ void ll_store_scales(const LLDispatchArgs& a, int j, int G, int64_t rows, int64_t at, Get get) {
+    const int lane = threadIdx.x & 31;
+    if (a.use_ue8m0) {
+        // four exponents per int32, groups along the slow axis: [E_local, ceil(G/4), R*M]
+        uint8_t* dst = reinterpret_cast<uint8_t*>(a.packed_sf);
+        const int64_t G4 = (G + 3) / 4;
+        for (int gi = lane; gi < G; gi += 32)
+            dst[((static_cast<int64_t>(j) * G4 + gi / 4) * rows + at) * 4 + (gi & 3)] = static_cast<uint8_t>(__float_as_uint(get(gi)) >> 23);
+    } else {
+        float* dst = reinterpret_cast<float*>(a.packed_sf);
+        for (int gi = lane; gi < G; gi += 32) dst[(static_cast<int64_t>(j) * G + gi) * rows + at] = get(gi);
+    }
+}
+
 __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const RankCtx& ctx = a.ctx;
@@ -176,7 +194,26 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
             }
             ptx::fence_proxy_async_smem();
             __syncthreads();
-            if (warp < K && lane == 0) {
+            if (a.direct_rows && warp < K) {
+                // one rank: the claimed slot IS the packed position, so payload, scales and source go there at once
+                const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
+                if (e >= 0 && e < E && !rank_masked(a.mask, 0)) {
+                    uint32_t slot = 0;
+                    if (lane == 0) slot = atomicAdd(&slot_counter[e], 1u);
+                    slot = __shfl_sync(0xffffffffu, slot, 0);
+                    if (slot < static_cast<uint32_t>(M)) {
+                        const int64_t pos = static_cast<int64_t>(e) * M + slot;
+                        if (lane == 0) {
+                            ptx::bulk_store(reinterpret_cast<uint8_t*>(a.packed_x) + pos * payload, msg + 16, payload);
+                            a.packed_src_info[pos] = (warp << 20) | t;
+                        }
+                        if (a.use_fp8) ll_store_scales(a, e, G, M, slot, [&](int gi) { return reinterpret_cast<const float*>(msg + 16 + H)[gi]; });
+                    } else if (lane == 0) {
+                        report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
+                    }
+                }
+                ptx::bulk_commit();
+            } else if (!a.direct_rows && warp < K && lane == 0) {
                 const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
                 if (e >= 0 && e < E && !rank_masked(a.mask, e / El)) {
                     const uint32_t slot = atomicAdd(&slot_counter[e], 1u);
@@ -263,7 +300,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
                 }
             }
             const uint32_t pieces = (payload + 2047) / 2048;
-            const uint32_t items = s_pref[P] * pieces;
+            const uint32_t items = a.direct_rows ? 0u : s_pref[P] * pieces;
             for (uint32_t u = blockIdx.x * kLLWarps + warp; u < items; u += gridDim.x * kLLWarps) {
                 const uint32_t g = u / pieces, c = u - g * pieces;
                 const int p = find_segment(s_pref, P, g);
@@ -288,18 +325,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
                 }
                 if (a.use_fp8 && c == pieces - 1) {
                     const float* sf = reinterpret_cast<const float*>(m + 16 + H);
-                    if (a.use_ue8m0) {
-                        // four exponents per int32, groups along the slow axis: [E_local, ceil(G/4), R*M]
-                        uint8_t* dst = reinterpret_cast<uint8_t*>(a.packed_sf);
-                        const int64_t G4 = (G + 3) / 4;
-                        for (int gi = lane; gi < G; gi += 32)
-                            dst[((static_cast<int64_t>(j) * G4 + gi / 4) * rows_per_expert + begin + i) * 4 + (gi & 3)] =
-                                static_cast<uint8_t>(__float_as_uint(__ldcg(sf + gi)) >> 23);
-                    } else {
-                        float* dst = reinterpret_cast<float*>(a.packed_sf);
-                        for (int gi = lane; gi < G; gi += 32)
-                            dst[(static_cast<int64_t>(j) * G + gi) * rows_per_expert + begin + i] = __ldcg(sf + gi);
-                    }
+                    ll_store_scales(a, j, G, rows_per_expert, begin + i, [&](int gi) { return __ldcg(sf + gi); });
                 }
             }
         }
@@ -374,10 +400,22 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
             }
             return pos;
         };
+        bool indexed = false;
+        if (a.direct_rows) {
+            // one rank: the slot of a (token, lane) gets the row's number instead of the row, one thread each
+            for (uint32_t r = blockIdx.x * blockDim.x + tid; r < total && alive; r += gridDim.x * blockDim.x) {
+                const int p = find_segment(s_pref, P, r);
+                const int64_t at = static_cast<int64_t>(p) * M + s_begin[p] + (r - s_pref[p]);
+                const int info = a.src_info[at];
+                *reinterpret_cast<int*>(s_peer[me] + a.off_slab[set] + (static_cast<int64_t>(info & 0xfffff) * K + (info >> 20)) * row_bytes) = static_cast<int>(at);
+                indexed = true;
+            }
+        }
         uint32_t g = blockIdx.x * send_warps + warp;
         int64_t pos = 0;
-        if (warp < send_warps && g < total && alive) pos = issue_load(g, 0);
-        for (; warp < send_warps && g < total && alive; g += g_stride) {
+        const bool stage_rows = warp < send_warps && !a.direct_rows;
+        if (stage_rows && g < total && alive) pos = issue_load(g, 0);
+        for (; stage_rows && g < total && alive; g += g_stride) {
             const int s = next_src;
             const int info = a.src_info[pos];
             const int t = info & 0xfffff, k = info >> 20;
@@ -409,7 +447,7 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
         stamp(1);
         ptx::bulk_wait<0>();
         // only lanes that have stored to a peer have something to make visible
-        if (n_loaded > 0 && lane == 0) __threadfence_system();
+        if ((n_loaded > 0 && lane == 0) || indexed) __threadfence_system();
         stamp(2);
         // the last CTA of this rank to finish its stores raises this rank's flag at every peer (no grid barrier)
         if (arrive_is_last(&ws->arrive[EP_CH_LL_COMBINE][0]) && !is_aborted(ws)) {
@@ -523,10 +561,20 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
                 }
                 const uint32_t srcs = __ballot_sync(0xffffffffu, e_k >= 0 && e_k < E);
                 const uint8_t* rows = slab + static_cast<int64_t>(t) * K * row_bytes + off;
+                // direct rows: the slots hold row numbers (of this call; anything else is kept inside x)
+                int my_row = 0;
+                if (a.direct_rows && lane < K && ((srcs >> lane) & 1u)) {
+                    my_row = __ldcg(reinterpret_cast<const int*>(slab + (static_cast<int64_t>(t) * K + lane) * row_bytes));
+                    if (static_cast<uint32_t>(my_row) >= static_cast<uint32_t>(E) * M) my_row = 0;
+                }
                 int4 raw[EP_MAX_TOPK];
 #pragma unroll
                 for (int k = 0; k < EP_MAX_TOPK; ++k)
-                    if (k < K && ((srcs >> k) & 1u) && in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(rows + static_cast<int64_t>(k) * row_bytes));
+                    if (k < K && ((srcs >> k) & 1u)) {
+                        const int64_t at = __shfl_sync(0xffffffffu, my_row, k);
+                        const uint8_t* src = a.direct_rows ? reinterpret_cast<const uint8_t*>(a.x) + at * row_bytes + off : rows + static_cast<int64_t>(k) * row_bytes;
+                        if (in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(src));
+                    }
                 float acc[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -603,6 +651,11 @@ cudaError_t launch_ll(const void* single, const void* multi, const Args* args, i
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* args, int n, int num_sms, cudaStream_t stream) {
     const int smem = 2 * args[0].msg_bytes;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
+    if (n == 1) {
+        LLDispatchArgs one = args[0];
+        one.direct_rows = one.ctx.num_ranks == 1 && one.phases == (EP_LL_SEND | EP_LL_RECV);
+        return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, &one, n, num_sms, smem, stream);
+    }
     return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, args, n, num_sms, smem, stream);
 }
 
@@ -610,6 +663,15 @@ cudaError_t launch_ll_combine(const LLCombineArgs* args, int n, int num_sms, cud
     const int smem = 1024 + ll_combine_send_warps(args[0].hidden) * (2 * args[0].hidden * 2 + ll_combine_hdr_bytes(args[0].hidden));
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
     if (args[0].use_logfmt && args[0].hidden % 128 != 0) return cudaErrorInvalidValue;
+    if (n == 1) {
+        // Rows are reduced where they lie if nobody else needs them (one rank), no one may change them in between (both phases in one
+        // launch), they are not re-coded, and the output does not overlap them.
+        LLCombineArgs one = args[0];
+        const uint64_t row = static_cast<uint64_t>(one.hidden) * 2, x0 = reinterpret_cast<uint64_t>(one.x), o0 = reinterpret_cast<uint64_t>(one.out);
+        const uint64_t x1 = x0 + row * one.num_experts * one.num_max_tokens, o1 = o0 + row * one.num_tokens;
+        one.direct_rows = one.ctx.num_ranks == 1 && one.phases == (EP_LL_SEND | EP_LL_RECV) && !one.use_logfmt && (x1 <= o0 || o1 <= x0) && x0 % 16 == 0;
+        return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, &one, n, num_sms, smem, stream);
+    }
     return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, args, n, num_sms, smem, stream);
 }
 

@@ -123,3 +123,33 @@ def test_low_latency_combine_logfmt(R, T, H, E, K, split):
                 torch.testing.assert_close(got[1, :128], (-1.5 * wsum[1]).expand(128).bfloat16().float(), atol=0, rtol=1e-2)
     finally:
         world.destroy()
+
+
+@pytest.mark.parametrize('T,H,E,K', [(1, 128, 4, 1), (33, 2048, 32, 4), (128, 7168, 64, 8)])
+@pytest.mark.parametrize('mode', ['bf16', 'fp8', 'ue8m0'])
+@pytest.mark.parametrize('split', [False, True])
+def test_one_rank_moves_rows_once(T, H, E, K, mode, split):
+    """One rank: both halves in one launch place and reduce the rows directly, the split halves go through the slabs; same contract,
+    and an output over the expert rows still reads all of them first."""
+    test_low_latency_roundtrip(1, T, H, E, K, mode, split)
+    from deepep_ascend_b200 import ElasticBuffer
+    M = T + 3
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=M, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(M, H, 1, E, K) + (1 << 20))
+    try:
+        xs, idxs, ws = _inputs(1, T, H, E, K, seed=9)
+        recv, _, handle, _, hook = buf.low_latency_dispatch(xs[0], idxs[0], M, E, use_fp8=False, return_recv_hook=split)
+        if split:
+            hook()
+        want, _, hook = buf.low_latency_combine(recv, idxs[0], ws[0], handle, return_recv_hook=split)
+        if split:
+            hook()
+        over = recv.view(-1, H)[:T]
+        got, _, hook = buf.low_latency_combine(recv, idxs[0], ws[0], handle, out=over, return_recv_hook=split)
+        if split:
+            hook()
+        torch.cuda.synchronize()
+        buf.check_status()
+        assert torch.equal(got, want)
+    finally:
+        buf.destroy()
