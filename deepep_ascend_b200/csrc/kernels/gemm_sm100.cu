@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_sm100.cuh"
@@ -205,8 +206,8 @@ struct PipeState {
 // weights as they are).  2: A is [K, M] too (weight gradients read row-major activations and gradients as they are).
 template <bool kFp8, int kBlockN, int kMnOperands>
 __global__ void __launch_bounds__(gemm_threads(kFp8, kBlockN), 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a32,
-            const GemmArgs g) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+            const __grid_constant__ std::conditional_t<kFp8 && kBlockN == 256, CUtensorMap, int> map_a32, const GemmArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kStages = num_stages(kBlockN, kFp8);
     constexpr int kTileBytesB = kBlockN * 128;
@@ -237,7 +238,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int rem = num_tiles % gemm_ctas;
     const bool cut_last = kWide && 2 * rem <= gemm_ctas;
     const int whole_items = cut_last ? num_tiles - rem : num_tiles, num_items = cut_last ? num_tiles + rem : num_tiles;
-    uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;   // output staging: 256- and bf16 128-column variants
+    // output staging: of the 256-column variants, and of the reduce-scatter in the bf16 128-column one (narrow products, mostly of one
+    // wave: 64 x 128 x 128 takes 5.0 us with direct stores, 5.3 us staged)
+    uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;
     Workspace* ws = g.fuse != EP_GEMM_FUSE_NONE ? local_ws(g.ctx) : nullptr;
     const uint64_t epoch = ws != nullptr ? ws->epoch[EP_CH_GEMM] + 1 : 0;
     const int tiles_per_shard = g.fuse != EP_GEMM_FUSE_NONE ? num_m / g.ctx.num_ranks : num_m;
@@ -327,12 +330,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             for (int i = 0; i < kBlockM / 64; ++i)
                                 umma::tma_load_3d(s_a + p.stage * kTileBytes + i * umma::kMnChunkBytes, &map_a, m_blk * kBlockM + i * 64, kb * kBlockK, 0,
                                                   &sm->full[p.stage]);
-                        } else if (kWide && a_boxes < 4) {
-                            for (int i = 0; i < a_boxes; ++i)
-                                umma::tma_load_2d(s_a + p.stage * kTileBytes + i * (kTileBytes / 4), &map_a32, kb * kBlockK, m_blk * kBlockM + i * 32,
-                                                  &sm->full[p.stage]);
                         } else {
-                            umma::tma_load_2d(s_a + p.stage * kTileBytes, &map_a, kb * kBlockK, m_blk * kBlockM, &sm->full[p.stage]);
+                            if (a_boxes == 4) umma::tma_load_2d(s_a + p.stage * kTileBytes, &map_a, kb * kBlockK, m_blk * kBlockM, &sm->full[p.stage]);
+                            if constexpr (kWide) {
+                                for (int i = 0; i < (a_boxes & 3); ++i)
+                                    umma::tma_load_2d(s_a + p.stage * kTileBytes + i * (kTileBytes / 4), &map_a32, kb * kBlockK, m_blk * kBlockM + i * 32,
+                                                      &sm->full[p.stage]);
+                            }
                         }
                         if constexpr (kMnOperands >= 1) {
 #pragma unroll
@@ -440,7 +444,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     ptx::bulk_wait_read<0>();     // the staging rows were the source of the previous tile's stores
                     __syncwarp();
                 }
-                if (kBlockN % 128 == 0 && !to_peer) {
+                if (kBlockN == 256) {
 #pragma unroll
                     for (int c = 0; c < kBlockN / 64; ++c) {
                         uint32_t r0[32], r1[32], w[32];
