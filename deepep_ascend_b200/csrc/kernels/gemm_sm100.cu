@@ -86,22 +86,37 @@ __device__ __forceinline__ uint64_t wait_limit_ns(const GemmArgs& g) { return g.
 // a communication buffer, record the failure there too, so that the buffer's check_status() reports it and poisons the
 // buffer like any other failed device wait.  `code`: 1 = empty stage, 2 = free accumulator, 3 = rows-ready flag,
 // 4 = full stage, 5 = finished accumulator, 7 = all-gather copy.
-__device__ __noinline__ void gemm_fail(const GemmArgs& g, GemmSmem* sm, int code) {
-    sm->failed = code;
-    if (g.error != nullptr && atomicCAS(g.error, 0, code) == 0 && g.status != nullptr) {
-        volatile uint64_t* st = g.status;
+__device__ __forceinline__ void gemm_fail_values(int* error, uint64_t* status, int status_rank, int* failed, int code) {
+    *failed = code;
+    if (error != nullptr && atomicCAS(error, 0, code) == 0 && status != nullptr) {
+        volatile uint64_t* st = status;
         st[EP_STATUS_PHASE] = EP_PH_GEMM_PIPE;
         st[EP_STATUS_PEER] = static_cast<uint64_t>(-1ll);
         st[EP_STATUS_EXPECTED] = static_cast<uint64_t>(code);
         st[EP_STATUS_OBSERVED] = blockIdx.x;
-        st[EP_STATUS_RANK] = static_cast<uint64_t>(g.status_rank);
+        st[EP_STATUS_RANK] = static_cast<uint64_t>(status_rank);
         __threadfence_system();
         st[EP_STATUS_CODE] = EP_ERR_TIMEOUT;
         __threadfence_system();
     }
 }
+// Two ways to the same report.  By value: the arguments stay in the kernel's parameter bank.  By reference: the compiler keeps a copy of
+// all arguments in local memory, made by every thread at kernel entry, which only the wide e4m3 kernel is better off with (its
+// promotion loop spills without it: 0.98 -> 1.18 ms).
+__device__ __noinline__ void gemm_fail_by_value(int* error, uint64_t* status, int status_rank, int* failed, int code) {
+    gemm_fail_values(error, status, status_rank, failed, code);
+}
+__device__ __noinline__ void gemm_fail_by_reference(const GemmArgs& g, int* failed, int code) {
+    gemm_fail_values(g.error, g.status, g.status_rank, failed, code);
+}
+template <bool kByReference>
+__device__ __forceinline__ void gemm_fail(const GemmArgs& g, GemmSmem* sm, int code) {
+    if constexpr (kByReference) gemm_fail_by_reference(g, &sm->failed, code);
+    else gemm_fail_by_value(g.error, g.status, g.status_rank, &sm->failed, code);
+}
 
 // bounded mbarrier wait; returns false (and raises the failure flags) when the limit runs out
+template <bool kByReference>
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, GemmSmem* sm, const GemmArgs& g, int code) {
     if (ptx::mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = gemm_timer();
@@ -110,7 +125,7 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, GemmSme
         if ((++spins & 63u) == 0u) {
             if (*reinterpret_cast<volatile int*>(&sm->failed)) return false;
             if (gemm_timer() - t0 > wait_limit_ns(g)) {
-                gemm_fail(g, sm, code);
+                gemm_fail<kByReference>(g, sm, code);
                 return false;
             }
         }
@@ -296,7 +311,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         const uint64_t t0 = gemm_timer();
                         while (ptx::ld_acquire_sys(flag) < epoch) {
                             if (gemm_timer() - t0 > wait_limit_ns(g) || *reinterpret_cast<volatile int*>(&sm->failed)) {
-                                gemm_fail(g, sm, 3);
+                                gemm_fail<kWide>(g, sm, 3);
                                 ok = false;
                                 break;
                             }
@@ -310,7 +325,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         const uint64_t t0 = gemm_timer();
                         while (ptx::ld_acquire_sys(flag) < g.a_ready_value) {
                             if (gemm_timer() - t0 > wait_limit_ns(g) || *reinterpret_cast<volatile int*>(&sm->failed)) {
-                                gemm_fail(g, sm, 3);
+                                gemm_fail<kWide>(g, sm, 3);
                                 ok = false;
                                 break;
                             }
@@ -322,7 +337,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     // what they held; their products are not stored.
                     const int a_boxes = kWide && g.tile_rows != nullptr ? min(4, max(1, (__ldg(g.tile_rows + m_blk) + 31) / 32)) : 4;
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
-                        ok = wait_bar(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
+                        ok = wait_bar<kWide>(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
                         if (!ok) break;
                         ptx::mbar_arrive_expect_tx(&sm->full[p.stage], a_boxes * (kTileBytes / 4) + (tw.half >= 0 ? kTileBytesB / 2 : kTileBytesB));
                         if constexpr (kMnOperands >= 2) {
@@ -367,16 +382,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     const TileWork tw = item_work(tile);
                     if (tw.grp < 0 || tw.kb1 <= tw.kb0) continue;
                     if (!kFp8) {
-                        ok = wait_bar(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
+                        ok = wait_bar<kWide>(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
                         if (!ok) break;
                         umma::fence_after_thread_sync();
                     }
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
                         if (kFp8) {
-                            ok = wait_bar(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
+                            ok = wait_bar<kWide>(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
                             if (!ok) break;
                         }
-                        ok = wait_bar(&sm->full[p.stage], p.phase, sm, g, 4);
+                        ok = wait_bar<kWide>(&sm->full[p.stage], p.phase, sm, g, 4);
                         if (!ok) break;
                         umma::fence_after_thread_sync();
                         const uint64_t desc_a = kMnOperands >= 2 ? umma::make_smem_desc_mn_sw128(s_a + p.stage * kTileBytes)
@@ -434,7 +449,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             }
             const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
             if (!kFp8) {
-                ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 umma::fence_after_thread_sync();
@@ -509,7 +524,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     if (tw.half >= 0 && col_half == 1) {
                         // half a tile: the first four warps have all of its columns, these only take part in the hand-over
                         for (int kb = 0; kb < num_k; ++kb) {
-                            ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                            ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                             ok = __all_sync(0xffffffffu, ok);
                             if (!ok) break;
                             if (lane == 0) ptx::mbar_arrive(&sm->tmem_empty[acc]);
@@ -540,7 +555,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             sa = __ldg(sfa);
                             sb = __ldg(++sfb);
                         }
-                        ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                        ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                         umma::fence_after_thread_sync();
@@ -600,7 +615,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale_next), __float_as_uint(scale_next));
                         if (kb + 1 < num_k)
                             scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row + (kb + 1) * g.sfa_stride_kb) : 0.f) * __ldg(sfb + kb + 1);
-                        ok = wait_bar(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                        ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                         umma::fence_after_thread_sync();
