@@ -33,12 +33,19 @@ def grouped_gemm_nt(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, 
     return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer), tile_rows)
 
 
+def _plain(t: torch.Tensor) -> bool:
+    """A tensor whose PyTorch statement nobody watches, so that a kernel of this library may take its place: no subclass, not wrapped
+    by a function transform, no gradient or tangent to carry on, and nothing that records or intercepts operations is active.
+    A native call would be invisible to those: ``torch.jit.trace`` and ``make_fx`` (a dispatch mode; fake tensors are another) would
+    record the allocation of its results and not the launch that fills them."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and not (t.requires_grad and torch.is_grad_enabled()) and
+            torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and
+            torch._C._len_torch_dispatch_stack() == 0 and not torch._C._functorch.is_functorch_wrapped_tensor(t))
+
+
 def _plain_cuda(t: torch.Tensor) -> bool:
-    """A tensor that a kernel of this library may read in place of a differentiable / traceable PyTorch statement: on the current
-    GPU, not traced or wrapped by a function transform, and with no gradient or tangent to carry on."""
-    return (t.is_cuda and type(t) in (torch.Tensor, torch.nn.Parameter) and t.device.index == torch.cuda.current_device() and
-            not (t.requires_grad and torch.is_grad_enabled()) and torch.autograd.forward_ad._current_level < 0 and
-            not torch.compiler.is_compiling() and not torch._C._functorch.is_functorch_wrapped_tensor(t))
+    """:func:`_plain`, on the current GPU."""
+    return t.is_cuda and t.device.index == torch.cuda.current_device() and _plain(t)
 
 
 def quantize_weight_blocks(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
