@@ -879,7 +879,7 @@ cudaError_t launch_weight_quant(const WeightQuantArgs& a, cudaStream_t stream) {
 }
 
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& a, cudaStream_t stream) {
-    if (a.rows == 0) return cudaSuccess;
+    if (a.rows == 0 || a.inter == 0) return cudaSuccess;
     const int warps = 8, ctas = (a.rows + warps - 1) / warps, steps = (a.inter + 255) / 256;
     SwigluQuantArgs args = a;
     const int per = (steps + column_splits(ctas, steps) - 1) / column_splits(ctas, steps);

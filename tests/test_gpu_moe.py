@@ -479,3 +479,15 @@ def test_thin_tiles_are_read_and_stored_by_rows(counts):
     h[~valid] = float('nan')
     a1, s1 = ops.swiglu_quant(h, valid_row=valid)
     assert torch.equal(a1.view(torch.uint8)[valid], a.view(torch.uint8)[valid]) and torch.equal(s1[valid], s[valid])
+
+
+@pytest.mark.parametrize('rows,I', [(0, 128), (4, 0), (0, 0)])
+@pytest.mark.parametrize('masked', [False, True])
+def test_swiglu_of_nothing(rows, I, masked):
+    """No rows or no channels: empty results and no launch."""
+    from deepep_ascend_b200.ops import gemm as ops
+    h = torch.empty(rows, 2 * I, dtype=torch.bfloat16, device='cuda')
+    valid = torch.ones(rows, dtype=torch.bool, device='cuda') if masked else None
+    q, sf, act = ops.swiglu_quant(h, keep_bf16=True, valid_row=valid)
+    torch.cuda.synchronize()
+    assert q.shape == act.shape == (rows, I) and sf.shape == (rows, (I + 127) // 128)
