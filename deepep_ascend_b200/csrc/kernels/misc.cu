@@ -274,6 +274,8 @@ cudaError_t launch_quant(const QuantArgs& a, cudaStream_t stream) {
     const int warps = 8;
     const int blocks = (a.num_tokens + warps - 1) / warps;
     if (blocks == 0) return cudaSuccess;
+    // the kernel reads 16 and writes 8 bytes at a time
+    if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0 || reinterpret_cast<uintptr_t>(a.q) % 8 != 0) return cudaErrorInvalidValue;
     quant_kernel<<<blocks, warps * 32, 0, stream>>>(a);
     return cudaGetLastError();
 }

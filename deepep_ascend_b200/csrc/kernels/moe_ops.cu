@@ -15,6 +15,9 @@ namespace {
 constexpr int kWantedCtas = 2 * 148;
 inline int column_splits(int ctas, int steps) { return max(1, min(steps, (kWantedCtas + ctas - 1) / max(ctas, 1))); }
 
+// Operands of 16-byte (8-byte) accesses; a kernel that is given others takes a misaligned access, so its launcher refuses them
+inline bool aligned(const void* p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
 // one warp per row (or per part of a row); each step covers 256 channels (two 128-channel scale groups).  The loads of two steps are issued
 // before the arithmetic of the first, the sigmoid uses the fast reciprocal (the activation is rounded to bf16 right
 // after), and the correctly rounded amax / 448 of a group is computed once per 16 steps by the lane that kept that amax
@@ -796,6 +799,7 @@ int moe_bwd_prep_col_blocks(int cols) { return (cols + kPrepCols - 1) / kPrepCol
 
 cudaError_t launch_moe_bwd(const MoeBwdArgs& a, cudaStream_t stream) {
     if (a.rows == 0) return cudaSuccess;
+    if (!aligned(a.g, 16) || !aligned(a.y, a.op == EP_MOE_BWD_DEQUANT_T ? 8 : 16) || !aligned(a.out, 16) || !aligned(a.out2, 16)) return cudaErrorInvalidValue;
     if (a.op == EP_MOE_BWD_SWIGLU_ROWS || a.op == EP_MOE_BWD_DEQUANT_ROWS || a.op == EP_MOE_BWD_WEIGHT_ROWS) {
         const int blocks = (a.rows + kRowWarps - 1) / kRowWarps;
         if (a.cols % (a.op == EP_MOE_BWD_DEQUANT_ROWS ? 16 : 8) != 0) return cudaErrorInvalidValue;
@@ -880,6 +884,7 @@ cudaError_t launch_weight_quant(const WeightQuantArgs& a, cudaStream_t stream) {
 
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& a, cudaStream_t stream) {
     if (a.rows == 0 || a.inter == 0) return cudaSuccess;
+    if (!aligned(a.h, 16) || (a.rows > 1 && a.ldh % 8 != 0) || !aligned(a.q, 8) || !aligned(a.act_bf16, 16)) return cudaErrorInvalidValue;
     const int warps = 8, ctas = (a.rows + warps - 1) / warps, steps = (a.inter + 255) / 256;
     SwigluQuantArgs args = a;
     const int per = (steps + column_splits(ctas, steps) - 1) / column_splits(ctas, steps);

@@ -462,6 +462,8 @@ std::vector<at::Tensor> swiglu_bwd_rows(const at::Tensor& d_act, const at::Tenso
     const int64_t rows = d_act.size(0), I = d_act.size(1);
     TORCH_CHECK(h.is_cuda() && h.is_contiguous() && h.scalar_type() == at::kBFloat16 && h.dim() == 2 && h.size(0) == rows && h.size(1) == 2 * I,
                 "h must be bf16 [rows, 2I]");
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(d_act.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(h.data_ptr()) % 16 == 0,
+                "d_act and h must be 16-byte aligned");
     at::Tensor out = at::empty({rows, 2 * I}, h.options()), act = at::empty({rows, I}, h.options());
     at::Tensor dot = at::empty({rows}, h.options().dtype(at::kFloat));
     MoeBwdArgs a{};

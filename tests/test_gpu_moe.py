@@ -491,3 +491,44 @@ def test_swiglu_of_nothing(rows, I, masked):
     q, sf, act = ops.swiglu_quant(h, keep_bf16=True, valid_row=valid)
     torch.cuda.synchronize()
     assert q.shape == act.shape == (rows, I) and sf.shape == (rows, (I + 127) // 128)
+
+
+def _off_by_one(t):
+    """The same values at a storage offset of one element."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat.view(torch.uint8)[t.element_size():].copy_(t.contiguous().view(-1).view(torch.uint8))
+    return flat[1:].view(t.shape)
+
+
+@pytest.mark.parametrize('name', ['swiglu_bwd_rows d_act', 'swiglu_bwd_rows h', 'weighted_rows', 'dequant_rows', 'swiglu_bwd d_act', 'swiglu_bwd h',
+                                  'moe_bwd_prep g', 'moe_bwd_prep y', 'weighted_transpose', 'dequant_transpose', 'swiglu_quant',
+                                  'swiglu_quant pitch', 'per_token_cast_to_fp8'])
+def test_operands_off_their_alignment_are_refused(name):
+    """Contiguous tensors that start (or whose rows start) between the kernel's vectors: an error on the host, no launch."""
+    from deepep_ascend_b200.ops import gemm as ops
+    rows, I, off = 64, 128, _off_by_one
+    d, h, w = (torch.randn(rows, n, device='cuda').bfloat16() for n in (I, 2 * I, I))
+    q, sf = ops.per_token_cast_to_fp8(d)
+    rw, valid = torch.rand(rows, device='cuda'), torch.ones(rows, dtype=torch.bool, device='cuda')
+    pitched = torch.randn(rows, 2 * I + 1, device='cuda').bfloat16()[:, :2 * I]
+    call = {
+        'swiglu_bwd_rows d_act': lambda: ops.swiglu_bwd_rows(off(d), h, valid, rw),
+        'swiglu_bwd_rows h': lambda: ops.swiglu_bwd_rows(d, off(h), valid, rw),
+        'weighted_rows': lambda: ops.weighted_rows(off(d), rw, valid),
+        'dequant_rows': lambda: ops.dequant_rows(off(q), sf, valid),
+        'swiglu_bwd d_act': lambda: ops.swiglu_bwd(off(d), h, valid),
+        'swiglu_bwd h': lambda: ops.swiglu_bwd(d, off(h), valid),
+        'moe_bwd_prep g': lambda: ops.moe_bwd_prep(off(d), w, rw, valid),
+        'moe_bwd_prep y': lambda: ops.moe_bwd_prep(d, off(w), rw, valid),
+        'weighted_transpose': lambda: ops.weighted_transpose(off(d), rw, valid),
+        'dequant_transpose': lambda: ops.dequant_transpose(off(q), sf, valid),
+        'swiglu_quant': lambda: ops.swiglu_quant(off(h)),
+        'swiglu_quant pitch': lambda: ops.swiglu_quant(pitched),
+        'per_token_cast_to_fp8': lambda: ops.per_token_cast_to_fp8(off(d)),
+    }[name]
+    with pytest.raises(RuntimeError):
+        call()
+    torch.cuda.synchronize()
+    # a single row has no pitch
+    got, want = ops.swiglu_quant(pitched[:1]), ops.swiglu_quant(pitched[:1].clone())
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, want))
