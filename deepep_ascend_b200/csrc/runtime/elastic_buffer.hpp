@@ -26,6 +26,9 @@ namespace ep_host {
 
 using OptTensor = std::optional<at::Tensor>;
 
+// the kernels read and write rows 16 bytes at a time and with bulk copies: anything else is a fault on the device
+inline bool vector_aligned(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
 struct DispatchCall {
     at::Tensor x;                  // [T, H] bf16 or float8_e4m3fn
     OptTensor sf;                  // [T, H/128] fp32 when x is fp8
@@ -369,7 +372,7 @@ private:
         const int64_t T = c.x.size(0), H = c.x.size(1);
         TORCH_CHECK(T <= c.num_max_tokens, "num_tokens exceeds num_max_tokens_per_rank");
         TORCH_CHECK((H * c.x.element_size()) % 16 == 0 && H % 16 == 0, "hidden bytes must be a multiple of 16");
-        TORCH_CHECK(reinterpret_cast<uintptr_t>(c.x.data_ptr()) % 16 == 0, "x must be 16-byte aligned");
+        TORCH_CHECK(vector_aligned(c.x), "x must be 16-byte aligned");
         TORCH_CHECK(!(c.quantize && fp8), "fused quantization takes bf16 input");
         const int64_t G = (H + 127) / 128;
         if (fp8) {
@@ -478,10 +481,13 @@ private:
         TORCH_CHECK(K >= 1 && K <= EP_MAX_TOPK && H > 0 && (H * 2) % 16 == 0, "bad combine shape");
         TORCH_CHECK(c.out.scalar_type() == at::kBFloat16 && c.out.is_contiguous() && c.out.size(0) == T && c.out.size(1) == H,
                     "out must be contiguous bf16 [T, H]");
+        TORCH_CHECK(vector_aligned(c.out), "out must be 16-byte aligned");
         for (const OptTensor* b : {&c.bias0, &c.bias1})
-            if (b->has_value())
+            if (b->has_value()) {
                 TORCH_CHECK((*b)->scalar_type() == at::kBFloat16 && (*b)->is_contiguous() && (*b)->sizes() == c.out.sizes(),
                             "bias must be contiguous bf16 [T, H]");
+                TORCH_CHECK(vector_aligned(**b), "bias must be 16-byte aligned");
+            }
         TORCH_CHECK(c.off_x >= static_cast<int64_t>(EP_WORKSPACE_BYTES) && c.off_x % 16 == 0 && c.off_x < mem_->bytes(),
                     "combine input offset outside the symmetric buffer");
         if (c.out_w.has_value()) {
@@ -498,8 +504,7 @@ private:
         if (c.local_x.has_value()) {
             const at::Tensor& x = *c.local_x;
             TORCH_CHECK(a.ctx.num_ranks == 1, "peers cannot reach a plain tensor");
-            TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(1) == H &&
-                            reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0,
+            TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 2 && x.size(1) == H && vector_aligned(x),
                         "local_x must be contiguous 16-byte aligned bf16 [rows, H]");
             // the kernel adds the offset to the buffer's base address (modulo 2^64)
             a.off_x = reinterpret_cast<uint64_t>(x.data_ptr()) - reinterpret_cast<uint64_t>(a.ctx.peer_base[a.ctx.rank]);

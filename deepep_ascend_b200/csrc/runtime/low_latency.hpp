@@ -49,6 +49,7 @@ inline LLDispatchArgs make_ll_dispatch_args(ElasticBufferCore& core, const LLDis
     const int R = a.ctx.num_ranks;
     TORCH_CHECK(c.x.is_cuda() && c.x.is_contiguous() && c.x.dim() == 2 && c.x.scalar_type() == at::kBFloat16,
                 "x must be contiguous bf16 [T, H]");
+    TORCH_CHECK(vector_aligned(c.x), "x must be 16-byte aligned");
     const int64_t T = c.x.size(0), H = c.x.size(1), K = c.topk_idx.size(1);
     TORCH_CHECK(H % 16 == 0 && T <= c.num_max_tokens && c.num_max_tokens < (1 << 20), "bad low-latency shape");
     TORCH_CHECK(c.topk_idx.is_contiguous() && c.topk_idx.size(0) == T && K <= EP_MAX_TOPK && K <= 16 &&
@@ -118,6 +119,7 @@ inline LLCombineArgs make_ll_combine_args(ElasticBufferCore& core, const LLCombi
                 "handle tensors have the wrong size");
     TORCH_CHECK(c.out.is_contiguous() && c.out.scalar_type() == at::kBFloat16 && c.out.size(0) == T && c.out.size(1) == H,
                 "out must be contiguous bf16 [T, H]");
+    TORCH_CHECK(vector_aligned(c.x) && vector_aligned(c.out), "x and out must be 16-byte aligned");
     const int64_t slab = c.num_max_tokens * K * H * 2;
     for (int64_t off : {c.off_slab0, c.off_slab1})
         TORCH_CHECK(off >= static_cast<int64_t>(EP_WORKSPACE_BYTES) && off % 16 == 0 && off + slab <= core.num_bytes(),

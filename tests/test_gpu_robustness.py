@@ -7,6 +7,7 @@ the others' waits carry a 0.2 s limit after which the kernels return normally.
 Reference tests of the same kind: tests/legacy/test_low_latency.py:14-36, 283-307; tests/elastic/test_ep.py:598-615, 771-781;
 tests/elastic/test_agrs.py:20-54, 112-139.
 """
+import math
 import random
 
 import pytest
@@ -438,5 +439,35 @@ def test_combine_input_of_one_rank_wherever_it_lies(kind):
         torch.cuda.synchronize()
         buf.check_status()
         assert torch.equal(got, want)
+    finally:
+        buf.destroy()
+
+
+@pytest.mark.parametrize('operand', ['dispatch x', 'combine out', 'combine bias', 'low-latency x', 'low-latency rows', 'low-latency out'])
+def test_misaligned_operands_of_an_exchange_are_refused(operand):
+    """Rows move in 16-byte pieces and bulk copies: a contiguous tensor that starts between them is an error on the host."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 5, 512, 8, 2
+
+    def off(*shape):
+        return torch.zeros(math.prod(shape) + 1, dtype=torch.bfloat16, device='cuda')[1:].view(shape)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+    try:
+        x, idx, w = torch.randn(T, H, device='cuda').bfloat16(), torch.randint(0, E, (T, K), device='cuda'), torch.rand(T, K, device='cuda')
+        _, _, _, h, _ = buf.dispatch(x, idx, num_experts=E)
+        rows, _, ll, _, _ = buf.low_latency_dispatch(x, idx, T, E, use_fp8=False)
+        call = {
+            'dispatch x': lambda: buf.dispatch(off(T, H), idx, num_experts=E),
+            'combine out': lambda: buf.combine(x[:h.num_rows], h, out=off(T, H)),
+            'combine bias': lambda: buf.combine(x[:h.num_rows], h, bias=off(T, H)),
+            'low-latency x': lambda: buf.low_latency_dispatch(off(T, H), idx, T, E, use_fp8=False),
+            'low-latency rows': lambda: buf.low_latency_combine(off(E, T, H), idx, w, ll),
+            'low-latency out': lambda: buf.low_latency_combine(rows, idx, w, ll, out=off(T, H)),
+        }[operand]
+        with pytest.raises(RuntimeError, match='16-byte aligned'):
+            call()
+        torch.cuda.synchronize()
+        assert buf.core.read_status()[0] == 0
     finally:
         buf.destroy()
