@@ -711,7 +711,9 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         if (self.num_ranks == 1 and x.is_contiguous() and x.data_ptr() % 16 == 0 and x.device == handle.plan.device and
                 (out is None or out.data_ptr() >= x.data_ptr() + x.nbytes or x.data_ptr() >= out.data_ptr() + out.nbytes)):
             # Nobody else pulls: the kernel reads the rows where they are (the region or any other tensor), which saves the copy of a
-            # plain tensor: 72 MB take 29 us.  An output that overlaps the input still needs it.
+            # plain tensor: 72 MB take 29 us.  An output that overlaps the input still needs it.  Rows that would not fit the buffer
+            # of several ranks are refused here too.
+            self.core.check_view(off_x, rows * H * 2)
             local_x = x
         else:
             staging = self.core.view(off_x, [rows, H], [H, 1], torch.bfloat16)

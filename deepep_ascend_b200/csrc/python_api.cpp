@@ -796,6 +796,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("generation", &ElasticBufferCore::generation)
         .def("set_gpu_timeout", &ElasticBufferCore::set_gpu_timeout)
         .def("view", &ElasticBufferCore::view)
+        .def("check_view", &ElasticBufferCore::check_view)
         .def("read_status", &ElasticBufferCore::read_status)
         .def("check_status", &ElasticBufferCore::check_status)
         .def("wait_recv_counts", &ElasticBufferCore::wait_recv_counts)

@@ -102,6 +102,11 @@ public:
     uint64_t generation() const { return coord_.generation(); }
     void set_gpu_timeout(double secs) { gpu_timeout_ns_ = static_cast<uint64_t>(secs * 1e9); }
 
+    // throws unless [offset, offset + bytes) lies in the data area
+    void check_view(int64_t offset, int64_t bytes) const {
+        TORCH_CHECK(offset >= static_cast<int64_t>(EP_WORKSPACE_BYTES) && offset + bytes <= mem_->bytes(),
+                    "view [", offset, ", ", offset + bytes, ") is outside the data area of the symmetric buffer");
+    }
     // a tensor that aliases [offset, offset + bytes) of the local symmetric buffer
     at::Tensor view(int64_t offset, std::vector<int64_t> sizes, std::vector<int64_t> strides, at::ScalarType dtype) const {
         int64_t max_index = 0;
@@ -109,9 +114,7 @@ public:
             if (sizes[i] == 0) { max_index = -1; break; }
             max_index += (sizes[i] - 1) * strides[i];
         }
-        const int64_t end = offset + (max_index + 1) * static_cast<int64_t>(c10::elementSize(dtype));
-        TORCH_CHECK(offset >= static_cast<int64_t>(EP_WORKSPACE_BYTES) && end <= mem_->bytes(),
-                    "view [", offset, ", ", end, ") is outside the data area of the symmetric buffer");
+        check_view(offset, (max_index + 1) * static_cast<int64_t>(c10::elementSize(dtype)));
         auto opts = at::TensorOptions().dtype(dtype).device(at::kCUDA, mem_->device());
         return at::from_blob(mem_->local() + offset, sizes, strides, [](void*) {}, opts);
     }

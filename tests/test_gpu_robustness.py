@@ -471,3 +471,39 @@ def test_misaligned_operands_of_an_exchange_are_refused(operand):
         assert buf.core.read_status()[0] == 0
     finally:
         buf.destroy()
+
+
+@pytest.mark.parametrize('R', [1, 2])
+def test_combine_input_that_does_not_fit_the_buffer_is_refused(R):
+    """Rows wider than the buffer holds are refused by one rank, which would read them where they are, as by several; the refusal
+    comes before anything is launched, so the buffer goes on."""
+    from deepep_ascend_b200 import ElasticBuffer
+    from deepep_ascend_b200.backends.emulated import EmulatedWorld
+    T, H, E, K = 64, 256, 8, 2
+    idxs, ws = _routing(R, T, E, K, 3, drop=0.0)
+    idxs, ws = [i.cuda() for i in idxs], [w.cuda() for w in ws]
+    xs = [torch.randn(T, H, device='cuda').bfloat16() for _ in range(R)]
+    if R == 1:
+        buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+        outs = [buf.dispatch(xs[0], idxs[0], ws[0], num_experts=E)]
+        bufs, destroy = [buf], buf.destroy
+        run = lambda ys: [buf.combine(ys[0], outs[0][3])]    # noqa: E731
+    else:
+        world = EmulatedWorld(R, num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_experts=E)
+        outs = world.dispatch(xs, idxs, ws, E)
+        bufs, destroy = world.buffers, world.destroy
+        run = lambda ys: world.combine(ys, [o[3] for o in outs])    # noqa: E731
+    try:
+        wide = bufs[0].num_bytes // (2 * T) // 16 * 16
+        ys = [torch.zeros(o[3].num_rows, wide, dtype=torch.bfloat16, device='cuda') for o in outs]
+        for _ in range(2):       # both input regions
+            with pytest.raises(RuntimeError, match='outside the data area'):
+                run(ys)
+        got = run([o[0][:o[3].num_rows].clone() for o in outs])
+        torch.cuda.synchronize()
+        for b in bufs:
+            b.check_status()
+        if R == 1:
+            assert torch.equal(got[0][0], xs[0])
+    finally:
+        destroy()
