@@ -17,6 +17,13 @@ from ..buffers.elastic import ElasticBuffer
 from ..ops import gemm as G
 
 
+def _tma_readable(w: torch.Tensor) -> torch.Tensor:
+    """The weights as the data-gradient GEMMs load them: contiguous and starting on 16 bytes.  Parameters that are views of a flat
+    buffer may start anywhere; those are copied."""
+    w = w.detach().contiguous()
+    return w if w.data_ptr() % 16 == 0 else w.clone()
+
+
 class _MoEFunction(torch.autograd.Function):
     """Forward and backward of the layer.  The token batch is cut into ``layer.num_chunks`` pieces that run as a software
     pipeline: while the tensor cores work on the experts of chunk c, the communication stream combines chunk c - 1 and
@@ -103,7 +110,7 @@ class _MoEFunction(torch.autograd.Function):
     def backward(ctx, d_out):
         layer, bounds = ctx.layer, ctx.bounds
         buf: ElasticBuffer = layer.buffer
-        w2, w13 = (None, None) if layer.fp8_backward else (layer.w2.detach().contiguous(), layer.w13.detach().contiguous())
+        w2, w13 = (None, None) if layer.fp8_backward else (_tma_readable(layer.w2), _tma_readable(layer.w13))
         d_out = d_out.contiguous()
         dxs, dws, d_w2, d_w13 = [], [], None, None
         for c, handle in enumerate(ctx.handles):

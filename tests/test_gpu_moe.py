@@ -532,3 +532,36 @@ def test_operands_off_their_alignment_are_refused(name):
     # a single row has no pitch
     got, want = ops.swiglu_quant(pitched[:1]), ops.swiglu_quant(pitched[:1].clone())
     assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize('fp8_backward', [False, True])
+@pytest.mark.parametrize('layout', ['odd offset', 'transposed storage'])
+def test_layer_on_weights_that_are_views(layout, fp8_backward):
+    """Weights inside a flat buffer (starting between two 16-byte pieces) or stored with other strides: forward and every gradient
+    have the bits of the layer on ordinary weights."""
+    from deepep_ascend_b200 import ElasticBuffer
+    from deepep_ascend_b200.models.moe import FusedMoE
+    T, H, I, E, K = 200, 256, 128, 4, 2
+    torch.manual_seed(4)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    try:
+        layer = FusedMoE(buf, E, H, I, init_std=0.05, num_sms=16, fp8_backward=fp8_backward)
+        x, g = torch.randn(T, H, device='cuda').bfloat16().requires_grad_(True), torch.randn(T, H, device='cuda').bfloat16()
+        w, idx = torch.softmax(torch.randn(T, E, device='cuda'), dim=-1).topk(K, dim=-1)
+        w = w.clone().requires_grad_(True)
+
+        def step():
+            out = layer(x, idx, w)
+            return (out.detach().clone(), *torch.autograd.grad(out, [x, w, layer.w13, layer.w2], g))
+        want = step()
+        for name in ('w13', 'w2'):
+            p = getattr(layer, name)
+            p.data = _off_by_one(p.data) if layout == 'odd offset' else p.data.transpose(1, 2).contiguous().transpose(1, 2)
+            assert p.data_ptr() % 16 != 0 or not p.is_contiguous()
+        got = step()
+        torch.cuda.synchronize()
+        buf.check_status()
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+    finally:
+        buf.destroy()
