@@ -264,20 +264,21 @@ def main():
                                    fused_fp8_cast=True, num_sms=64)
         d_only()
         (rx, rsf), _, rw, hd, _ = st['o']
-        tile_group, valid_row = G.expert_tile_groups(hd.psum_num_recv_tokens_per_expert, hd.num_rows)
+        tile_group, valid_row, seg_off, tile_rows = G.expert_tiles(hd.psum_num_recv_tokens_per_expert, hd.num_rows)
         q13, s13, q2, s2 = layer.fp8_weights()
         t_disp = np.median(timeit(d_only, buf, iters=bi, warm=bw))
         hbuf = {}
 
         def g1():
-            hbuf['h'] = G.grouped_gemm_nt(rx, q13, tile_group, sfa=rsf, sfb=s13)
+            hbuf['h'] = G.grouped_gemm_nt(rx, q13, tile_group, sfa=rsf, sfb=s13, tile_rows=tile_rows)
         t_g1 = np.median(timeit(g1, None, iters=bi, warm=bw))
 
         def sw():
-            hbuf['a'] = G.swiglu_quant(hbuf['h'])
+            hbuf['a'] = G.swiglu_quant(hbuf['h'], valid_row=valid_row)
         t_sw = np.median(timeit(sw, None, iters=bi, warm=bw))
         ybuf = buf.get_combine_buffer(hd)
-        t_g2 = np.median(timeit(lambda: G.grouped_gemm_nt(hbuf['a'][0], q2, tile_group, out=ybuf, sfa=hbuf['a'][1], sfb=s2), None, iters=bi, warm=bw))
+        t_g2 = np.median(timeit(lambda: G.grouped_gemm_nt(hbuf['a'][0], q2, tile_group, out=ybuf, sfa=hbuf['a'][1], sfb=s2, tile_rows=tile_rows),
+                                None, iters=bi, warm=bw))
         t_comb = np.median(timeit(lambda: buf.combine(ybuf, hd, weighted=True, num_sms=64), buf, iters=bi, warm=bw))
         emit(bench='fused_moe_forward_breakdown_ms', rows=hd.num_rows, dispatch_expand_fp8=float(t_disp), gemm1_fp8=float(t_g1),
              swiglu_cast=float(t_sw), gemm2_fp8=float(t_g2), combine_weighted=float(t_comb),
@@ -290,43 +291,42 @@ def main():
         t_dl = np.median(timeit(d_loc, buf, iters=bi, warm=bw))
         (rx_r, rsf_r), ridx, rw_r, hl, _ = st['l']
         rows_l = sum(hl.num_recv_tokens_per_expert_list)
-        t_plan = np.median(timeit(lambda: G.local_expand_plan(ridx, hl.psum_num_recv_tokens_per_expert), None, iters=bi, warm=bw))
-        pos, seg_end = G.local_expand_plan(ridx, hl.psum_num_recv_tokens_per_expert)
+        t_plan = np.median(timeit(lambda: G.local_expand_layout(ridx, hl.psum_num_recv_tokens_per_expert, rows_l), None, iters=bi, warm=bw))
+        pos = G.local_expand_layout(ridx, hl.psum_num_recv_tokens_per_expert, rows_l)[0]
         t_copy = np.median(timeit(lambda: G.local_expand_copy(pos, rx_r, rows_l, sf=rsf_r, w=rw_r), None, iters=bi, warm=bw))
         w_e = G.local_expand_copy(pos, rx_r, rows_l, sf=rsf_r, w=rw_r)[2]
         y_exp = torch.randn(rows_l, H, device='cuda').bfloat16()
         t_red = np.median(timeit(lambda: G.local_reduce(pos, y_exp, w=w_e, out=buf.get_combine_buffer(hl)), None, iters=bi, warm=bw))
         t_cl = np.median(timeit(lambda: buf.combine(buf.get_combine_buffer(hl), hl, num_sms=64), buf, iters=bi, warm=bw))
         emit(bench='fused_moe_local_expand_breakdown_ms', received_rows=hl.num_rows, expert_rows=rows_l, dispatch_fp8=float(t_dl),
-             plan=float(t_plan), expand_copy=float(t_copy), local_reduce=float(t_red), combine=float(t_cl))
+             layout=float(t_plan), expand_copy=float(t_copy), local_reduce=float(t_red), combine=float(t_cl))
         del y_exp, w_e
         # backward pieces, timed one by one on this rank's rows
         g_rows = torch.randn(hd.num_rows, H, device='cuda').bfloat16()
         rwc = rw.contiguous()
-        seg_off = G.segment_offsets(hd.psum_num_recv_tokens_per_expert)
-        w2_t, w13_t = layer.transposed_weights()
+        w2, w13 = layer.w2.detach(), layer.w13.detach()
         bb = {}
 
-        def prep():
-            bb['dy_t'] = G.weighted_transpose(g_rows, rwc, valid_row)
-        t_prep = np.median(timeit(prep, None, iters=bi, warm=bw))
-
         def dgrad2():
-            bb['d_act'] = G.grouped_gemm_nt(g_rows, w2_t, tile_group)
+            bb['d_act'] = G.grouped_gemm_nn(g_rows, w2, tile_group)
         t_dg2 = np.median(timeit(dgrad2, None, iters=bi, warm=bw))
 
         def swb():
-            bb['dh'], bb['dh_t'], bb['act_t'], bb['dot'] = G.swiglu_bwd(bb['d_act'], hbuf['h'], valid_row, row_weight=rwc)
+            bb['dh'], bb['act'], bb['dot'] = G.swiglu_bwd_rows(bb['d_act'], hbuf['h'], valid_row, rwc)
         t_swb = np.median(timeit(swb, None, iters=bi, warm=bw))
-        t_dg1 = np.median(timeit(lambda: G.grouped_gemm_nt(bb['dh'], w13_t, tile_group, out=ybuf), None, iters=bi, warm=bw))
+        t_dg1 = np.median(timeit(lambda: G.grouped_gemm_nn(bb['dh'], w13, tile_group, out=ybuf), None, iters=bi, warm=bw))
 
-        def xt():
-            bb['x_t'] = G.dequant_transpose(rx, rsf, valid_row)
-        t_xt = np.median(timeit(xt, None, iters=bi, warm=bw))
-        t_wg2 = np.median(timeit(lambda: G.gemm_kgrouped(bb['dy_t'], bb['act_t'], seg_off), None, iters=bi, warm=bw))
-        t_wg1 = np.median(timeit(lambda: G.gemm_kgrouped(bb['dh_t'], bb['x_t'], seg_off), None, iters=bi, warm=bw))
-        emit(bench='fused_moe_backward_breakdown_ms', rows=hd.num_rows, weighted_transpose=float(t_prep), dgrad_down_bf16=float(t_dg2),
-             swiglu_bwd=float(t_swb), dgrad_up_bf16=float(t_dg1), dequant_transpose=float(t_xt), wgrad_down=float(t_wg2),
+        def dy():
+            bb['dy'] = G.weighted_rows(g_rows, rwc, valid_row)
+        t_dy = np.median(timeit(dy, None, iters=bi, warm=bw))
+
+        def dx():
+            bb['x'] = G.dequant_rows(rx, rsf, valid_row)
+        t_dx = np.median(timeit(dx, None, iters=bi, warm=bw))
+        t_wg2 = np.median(timeit(lambda: G.gemm_kgrouped_tn(bb['dy'], bb['act'], seg_off), None, iters=bi, warm=bw))
+        t_wg1 = np.median(timeit(lambda: G.gemm_kgrouped_tn(bb['dh'], bb['x'], seg_off), None, iters=bi, warm=bw))
+        emit(bench='fused_moe_backward_breakdown_ms', rows=hd.num_rows, dgrad_down_bf16=float(t_dg2), swiglu_bwd_rows=float(t_swb),
+             dgrad_up_bf16=float(t_dg1), weighted_rows=float(t_dy), dequant_rows=float(t_dx), wgrad_down=float(t_wg2),
              wgrad_up=float(t_wg1), dgrad_down_tflops=2 * hd.num_rows * H * I / t_dg2 / 1e9,
              dgrad_up_tflops=2 * hd.num_rows * H * 2 * I / t_dg1 / 1e9, wgrad_down_tflops=2 * hd.num_rows * H * I / t_wg2 / 1e9,
              wgrad_up_tflops=2 * hd.num_rows * H * 2 * I / t_wg1 / 1e9)

@@ -206,7 +206,6 @@ class FusedMoE(nn.Module):
         self.w2 = nn.Parameter((torch.randn(el, hidden, intermediate, device=device) * init_std).bfloat16())
         self._fp8 = None
         self._fp8_t = None
-        self._t = None
 
     def sm_split(self, pipelined: bool):
         """(SMs of the communication kernels, SMs of the GEMMs; 0 = all).  In the pipelined schedule the two run at the same
@@ -236,11 +235,6 @@ class FusedMoE(nn.Module):
             self._fp8_t = (self._versions(), (t(q2.view(torch.uint8)).view(torch.float8_e4m3fn), t(s2),
                                               t(q13.view(torch.uint8)).view(torch.float8_e4m3fn), t(s13)))
         return self._fp8_t[1]
-
-    def transposed_weights(self):
-        if self._t is None or self._t[0] != self._versions():
-            self._t = (self._versions(), (self.w2.detach().transpose(1, 2).contiguous(), self.w13.detach().transpose(1, 2).contiguous()))
-        return self._t[1]
 
     def forward(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor) -> torch.Tensor:
         return _MoEFunction.apply(x, topk_weights, self.w13, self.w2, self, topk_idx)
