@@ -1,6 +1,6 @@
 // Persistent tcgen05 GEMM for sm_100a: C[M, N] (bf16) = A[M, K] * B[g][N, K]^T.
 //
-//   warp 0   : TMA producer - 2-D tiled loads of 128 x 128-byte A and B tiles (128B swizzle) into a ring of
+//   warp 0   : TMA producer - tiled loads of A (128 rows) and B (kBlockN rows) x 128 bytes (128B swizzle) into a ring of
 //              shared-memory stages, completion counted on mbarriers; optionally waits for an "A rows are ready"
 //              flag per M tile (all-gather fused into the loads)
 //   warp 1   : MMA issuer   - one elected thread issues tcgen05.mma (kind::f16 for bf16, kind::f8f6f4 for e4m3)
@@ -10,8 +10,8 @@
 // bf16 operands: one accumulator per output tile, two TMEM buffers so the epilogue of tile i overlaps the MMAs of
 // tile i+1.  e4m3 operands with fp32 block scales (A: per row x 128 channels, B: per 128 x 128 block): every
 // 128-channel block is accumulated into its own TMEM buffer and promoted into fp32 registers with its scale by
-// EIGHT epilogue warps (two per TMEM lane quadrant, 64 columns each, both tcgen05.ld of a block in flight before one
-// wait); four TMEM buffers let the MMAs run up to three blocks ahead of the promotion.
+// EIGHT epilogue warps, two per TMEM lane quadrant: 64 columns each of 128-column tiles, with four TMEM buffers, so that the MMAs
+// run up to three blocks ahead of the promotion; 128 columns each of 256-column tiles, with two.
 // MN-major bf16 operands (`mn_operands`): the backward pass of a layer reads weights, activations and gradients row-major as the
 // forward pass left them (64 x 64 TMA boxes, transposing descriptors), at the rate of the K-major kernel: 2.3 ms for the two data
 // gradients and 2.6 ms for the two weight gradients of 34816 rows x (7168, 2 x 2048) bf16.  Transposed copies of the weights
@@ -823,7 +823,7 @@ EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-// K-major [rows, K] operand, box = box_rows (128 or 256) rows x 128 bytes, 128B swizzle, out-of-range elements read as zero
+// K-major [rows, K] operand, box = box_rows (32, 128, 224 or 256) rows x 128 bytes, 128B swizzle, out-of-range elements read as zero
 bool make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k, int64_t ld_elems, bool fp8, int box_rows) {
     EncodeTiledFn encode = get_encode_fn();
     if (encode == nullptr) return false;
@@ -883,7 +883,8 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
                                              : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, g.is_fp8 ? 128 : block_n));
     if (!maps_ok) return cudaErrorInvalidValue;
     map_a32 = map_a;
-    if (g.is_fp8 && g.tile_rows != nullptr && !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32)) return cudaErrorInvalidValue;
+    // boxes of 32 rows for thin tiles: only the wide e4m3 kernel reads them
+    if (g.is_fp8 && block_n == 256 && g.tile_rows != nullptr && !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32)) return cudaErrorInvalidValue;
     const void* fn;
     if (g.mn_operands == 2) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 2> : (const void*)gemm_kernel<false, 128, 2>;
     else if (g.mn_operands == 1) fn = block_n == 256 ? (const void*)gemm_kernel<false, 256, 1> : (const void*)gemm_kernel<false, 128, 1>;
