@@ -315,7 +315,9 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
         const int in_row = a.hidden * (a.x_is_fp8 ? 1 : 2);
         ptx::bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(a.x) + static_cast<int64_t>(warp * num_ctas + cta) * in_row, in_row);
     }
-    const bool bookkeeper = cta == num_ctas - 1;   // writes what this rank receives (handle tensors, host counters); its tokens are claimed last
+    // The bookkeeper writes what this rank receives (handle tensors, host counters) before it sends anything.  The first token of each
+    // of its warps is fixed like everybody's and waits for that; of the claimed tokens it gets fewer.
+    const bool bookkeeper = cta == num_ctas - 1;
     const bool need_experts = a.do_expand || bookkeeper;
 
     if (!a.cached) {

@@ -1,7 +1,8 @@
 // Element-wise pieces of the MoE expert FFN that sit between the two grouped GEMMs: SwiGLU fused with the
 // e4m3 (1x128 scales) cast of the second GEMM's input, so the activation is written once in FP8 instead of being
-// written in bf16 and re-read by a separate quantisation kernel; and the element-wise kernels of the backward pass,
-// which also emit the transposed operands of the weight-gradient GEMMs.
+// written in bf16 and re-read by a separate quantisation kernel; the cast of the weights, the expansion of received rows to
+// expert rows and its inverse; and the element-wise kernels of the backward pass.  The layer's backward pass uses the row-major
+// ones; those that also write transposed results serve callers of the K-major weight-gradient product (`gemm_kgrouped`).
 #include <cuda_fp8.h>
 
 #include "common.cuh"

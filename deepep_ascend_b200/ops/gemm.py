@@ -188,7 +188,9 @@ def gemm_kgrouped(a_t: torch.Tensor, b_t: torch.Tensor, k_off: torch.Tensor, num
     """Weight gradients of a grouped layer in one launch: ``out[e] = a_t[:, k0:k1] @ b_t[:, k0:k1]^T`` with
     ``(k0, k1) = (k_off[e], k_off[e + 1])``; ``a_t [M, rows]``, ``b_t [N, rows]`` bf16 (the transposed activations and
     gradients, so that the reduction dimension = rows of the expert segment is contiguous), ``k_off`` int32
-    ``[G + 1]`` multiples of 64 on the device.  -> bf16 ``[G, M, N]``; an expert without rows gets zeros."""
+    ``[G + 1]`` multiples of 64 on the device.  -> bf16 ``[G, M, N]``; an expert without rows gets zeros.  For callers that hold
+    transposed operands (:func:`moe_bwd_prep`, :func:`swiglu_bwd`, :func:`weighted_transpose` and :func:`dequant_transpose` write them);
+    ``FusedMoE`` uses :func:`gemm_kgrouped_tn` on row-major ones."""
     return _native.load().gemm_kgrouped(a_t, b_t, k_off, num_sms)
 
 
