@@ -147,11 +147,11 @@ def test_no_cpu_sync_and_col_major_sf():
         world.destroy()
 
 
-@pytest.mark.parametrize('H', [64, 512, 1088, 1536, 7168])
+@pytest.mark.parametrize('H', [64, 256, 512, 1024, 1088, 1536, 7168])
 @pytest.mark.parametrize('T', [1, 5, 37, 161])
 def test_combine_units_of_work(T, H):
-    """Few SMs and every chunk width: fewer tokens than warps (chunks only), a few whole tokens before the chunks, many; rows that
-    are not whole chunks; tokens without any row; two ranks, so that tokens have zero, one or two sources."""
+    """Few SMs and every chunk width, with whole chunks and without where both exist: fewer tokens than warps (chunks only), a few
+    whole tokens before the chunks, many; rows that are not whole chunks; tokens without any row; two ranks, so that tokens have zero, one or two sources."""
     from deepep_ascend_b200.backends.emulated import EmulatedWorld
     from deepep_ascend_b200.utils import refs
     R, E, K = 2, 8, 3
