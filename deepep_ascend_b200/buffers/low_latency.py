@@ -104,7 +104,9 @@ class LowLatencyMixin:
 
         ``recv_x [E_local, ranks * max_tokens, H]`` (e4m3 with ``use_fp8`` else bf16), ``recv_scales
         [E_local, ranks * max_tokens, H / 128]`` fp32 (or ``H / 512`` int32 of packed UE8M0) column-major in the
-        last two dims, ``recv_count [E_local]``; only the first ``recv_count[e]`` rows of expert ``e`` are valid.
+        last two dims, ``recv_count [E_local]``; only the first ``recv_count[e]`` rows of expert ``e`` are valid.  Pass that on:
+        ``ops.gemm.grouped_gemm_nt(tile_rows=...)`` loads and stores only the rows of a tile that count (with one 128-row tile per
+        expert the argument is ``recv_count`` itself), ``ops.gemm.swiglu_quant(valid_row=...)`` skips the others.
         ``handle = (src_info, layout_range, max_tokens, hidden, num_experts)``.
         """
         M, E = num_max_dispatch_tokens_per_rank, num_experts
