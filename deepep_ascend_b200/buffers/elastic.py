@@ -725,6 +725,7 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         call.plan = handle.plan
         call.lane_src = handle.dst_buffer_slot_idx
         call.hidden = H
+        call.expanded = handle.do_expand
         if self.profile is not None:
             call.prof = self.profile['combine']
         T, K = handle.plan.shape

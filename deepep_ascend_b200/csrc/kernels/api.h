@@ -130,6 +130,7 @@ struct CombineArgs {
     void* out;                     // [T, H] bf16
     float* out_w;                  // [T, K] or null
     int num_tokens, hidden, num_topk;
+    int one_row;                   // no token has more than one row (one rank, non-expand layout)
     uint64_t* prof;                // optional [8] phase timestamps (ns) written by CTA 0, or null
 };
 

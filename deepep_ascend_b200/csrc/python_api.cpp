@@ -759,6 +759,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("off_x", &CombineCall::off_x)
         .def_readwrite("local_x", &CombineCall::local_x)
         .def_readwrite("off_w", &CombineCall::off_w)
+        .def_readwrite("expanded", &CombineCall::expanded)
         .def_readwrite("w_cols", &CombineCall::w_cols)
         .def_readwrite("plan", &CombineCall::plan)
         .def_readwrite("lane_src", &CombineCall::lane_src)

@@ -64,6 +64,7 @@ struct CombineCall {
     at::Tensor out;                // [T, H] bf16
     OptTensor out_w;               // [T, K] fp32
     int64_t hidden = 0;
+    bool expanded = true;          // the plan may name several rows of one rank for a token (expand layout)
     OptTensor prof;                // int64 [8]: phase timestamps of CTA 0 (profiling)
 };
 
@@ -504,6 +505,7 @@ private:
             TORCH_CHECK(c.mul_weights->scalar_type() == at::kFloat && c.mul_weights->is_contiguous() &&
                             c.mul_weights->numel() == T * K, "mul_weights must be contiguous fp32 [T, K]");
         a.off_x = c.off_x;
+        a.one_row = a.ctx.num_ranks == 1 && !c.expanded;
         if (c.local_x.has_value()) {
             const at::Tensor& x = *c.local_x;
             TORCH_CHECK(a.ctx.num_ranks == 1, "peers cannot reach a plain tensor");
