@@ -171,7 +171,7 @@ cudaError_t launch_wait_flag_test(const RankCtx* ctxs, int n, uint64_t expected,
 cudaError_t launch_layout(const LayoutArgs& args, cudaStream_t stream);
 cudaError_t launch_quant(const QuantArgs& args, cudaStream_t stream);
 
-LaunchShape dispatch_launch_shape(const DispatchArgs& a, int num_sms);
+LaunchShape dispatch_launch_shape(const DispatchArgs& a, int num_sms, bool local);
 LaunchShape combine_launch_shape(const CombineArgs& a, int num_sms);
 
 }  // namespace ep

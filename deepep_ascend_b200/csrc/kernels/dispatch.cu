@@ -29,6 +29,7 @@ namespace ep {
 namespace {
 
 constexpr int kDispatchMaxWarps = 12;
+constexpr int kLocalWarps = 20, kLocalUnitBytes = 4096;      // one rank
 constexpr int kDispatchMaxStages = 4;
 constexpr int kDispatchSmemBudget = 222 * 1024;
 
@@ -51,7 +52,8 @@ struct DispatchSmemPlan {
 
 __host__ __device__ inline int align_int(int x, int a) { return (x + a - 1) / a * a; }
 
-__host__ __device__ inline DispatchSmemPlan make_smem_plan(const DispatchArgs& a, int num_warps, int num_stages) {
+// local (one rank): rows go straight from registers to their place, so nothing is staged
+__host__ __device__ inline DispatchSmemPlan make_smem_plan(const DispatchArgs& a, int num_warps, int num_stages, bool local) {
     DispatchSmemPlan p;
     const int E = a.num_experts, R = a.ctx.num_ranks;
     const int G = (a.hidden + 127) / 128;
@@ -69,8 +71,8 @@ __host__ __device__ inline DispatchSmemPlan make_smem_plan(const DispatchArgs& a
     p.off_wc_rank = off;    off += align_int(num_warps * R * 4, 16);
     p.off_wc_expert = off;  off += align_int((a.do_expand ? num_warps : 1) * E * 4, 16);
     p.off_bar = off;        off += align_int(num_warps * 3 * 8, 16);   // keeps everything behind it 16-byte aligned (bulk copy sources)
-    p.off_sf = off;         off += num_warps * p.n_side * p.sf_floats * 4;
-    p.off_tail = off;       off += a.side_packed ? num_warps * p.n_side * p.max_dst * a.tail_bytes : 0;
+    p.off_sf = off;         off += local ? 0 : num_warps * p.n_side * p.sf_floats * 4;
+    p.off_tail = off;       off += a.side_packed && !local ? num_warps * p.n_side * p.max_dst * a.tail_bytes : 0;
     off = align_int(off, 128);
     p.off_stage = off;
     const int in_row = a.hidden * (a.x_is_fp8 ? 1 : 2);
@@ -88,7 +90,7 @@ __host__ __device__ inline DispatchSmemPlan make_smem_plan(const DispatchArgs& a
         p.n_out = 0;
     }
     p.warp_stage_bytes = p.n_in * p.in_bytes + p.n_out * p.out_bytes;
-    p.total = off + num_warps * p.warp_stage_bytes;
+    p.total = off + num_warps * (local ? (a.quantize ? 2 * kLocalUnitBytes : 0) : p.warp_stage_bytes);
     return p;
 }
 
@@ -102,17 +104,23 @@ struct Slice {
     int begin, end;
 };
 
-// Contiguous token slice of (cta, warp); warp slices are multiples of the tokens handled per layout step.
-__device__ __forceinline__ Slice warp_slice(int T, int K, int num_warps, int warp) {
-    const int chunk = (T + gridDim.x - 1) / gridDim.x;
-    const int cta_begin = min(T, static_cast<int>(blockIdx.x) * chunk);
-    const int cta_end = min(T, cta_begin + chunk);
+// Contiguous token slice of a CTA.  kLocal (one rank): the CTA also sends its slice, so the slices are as even as they can be;
+// otherwise any warp may send a token, and all slices but the last have the same length so that a token's owner is known.
+template <bool kLocal>
+__device__ __forceinline__ Slice cta_slice(int T) {
+    const int cta = static_cast<int>(blockIdx.x), ctas = static_cast<int>(gridDim.x);
+    if (kLocal) return {static_cast<int>(static_cast<int64_t>(T) * cta / ctas), static_cast<int>(static_cast<int64_t>(T) * (cta + 1) / ctas)};
+    const int chunk = (T + ctas - 1) / ctas, begin = min(T, cta * chunk);
+    return {begin, min(T, begin + chunk)};
+}
+// Contiguous part of it per warp: a multiple of the tokens handled per layout step.
+__device__ __forceinline__ Slice warp_slice(Slice cta, int K, int num_warps, int warp) {
     const int tps = 32 / K;
-    int sub = (chunk + num_warps - 1) / num_warps;
+    int sub = (cta.end - cta.begin + num_warps - 1) / num_warps;
     sub = (sub + tps - 1) / tps * tps;
     Slice s;
-    s.begin = min(cta_end, cta_begin + warp * sub);
-    s.end = min(cta_end, s.begin + sub);
+    s.begin = min(cta.end, cta.begin + warp * sub);
+    s.end = min(cta.end, s.begin + sub);
     return s;
 }
 
@@ -180,26 +188,46 @@ __device__ __forceinline__ void layout_pass(const DispatchArgs& a, Slice sl, uin
 
 __device__ __forceinline__ uint32_t count_of(uint64_t word) { return static_cast<uint32_t>(word & 0xffffffffull); }
 
-// Fused cast: a row is processed in register batches of kCastSteps x 256 channels.  All 16-byte loads of a batch
-// are issued back to back straight from global memory, the next batch is requested before the current one is
-// converted, and the unrolled conversions of a batch are independent of one another, so neither the memory
-// latency nor the shuffle / reciprocal latency chains of one 128-channel group are exposed.
-// q = x * (448 / max(amax, 1e-4)) rounded to nearest even, scale = max(amax, 1e-4) / 448.
-// The correctly rounded division amax / 448 costs ~20 instructions that only two lanes of a step would use, so the steps
+// Fused cast: a row is processed in register batches of two blocks of 1024 channels.  All 16-byte loads of a batch are issued back
+// to back straight from global memory and the next batch is requested before the current one is converted, so the memory latency
+// is not exposed.  q = x * (448 / max(amax, 1e-4)) rounded to nearest even, scale = max(amax, 1e-4) / 448.
+// The correctly rounded division amax / 448 costs ~20 instructions that only eight lanes of a block would use, so the blocks
 // leave the clamped amax in the staging row and scales_from_amax divides all groups of the row at once, one group per lane.
-constexpr int kCastSteps = 7;
+constexpr int kCastChannels = 1024, kCastBlocks = 2;      // per block, blocks per batch
+static_assert(kLocalUnitBytes == kCastChannels * kCastBlocks * 2, "a unit of one rank is a batch of the cast");
 
 struct RowBatch {
-    int4 v[kCastSteps];
+    int4 v[kCastBlocks][4];
 };
+// Four lanes share one of a block's eight 128-channel groups: lane (g, c) = (lane / 4, lane % 4) holds the 16-byte pieces 4 * j + c of
+// group g, j = 0..3.  Odd groups swap the pieces of a pair (j, j ^ 1), which spreads shared-memory accesses over the banks.  So piece
+// i lies at cast_lane(i & 1) + (i / 2) * 64 channels: two addresses per lane, the rest are immediate offsets.
+__device__ __forceinline__ int cast_lane(int odd) {
+    const int lane = ptx::lane_id(), g = lane >> 2, c = lane & 3;
+    return g * 128 + c * 8 + ((g ^ odd) & 1) * 32;
+}
+__device__ __forceinline__ int cast_piece(int k, int i) { return k * kCastChannels + (i >> 1) * 64; }
 
-__device__ __forceinline__ void load_batch(RowBatch& b, const uint8_t* row, int H, int batch) {
-    const int lane = ptx::lane_id();
+// the pieces of `batch` from a row of bf16 in global memory; channels beyond the row are zero
+template <typename Load>
+__device__ __forceinline__ void load_pieces(RowBatch& b, const uint8_t* row, int channels, Load load) {
+    const uint8_t* p[2] = {row + cast_lane(0) * 2, row + cast_lane(1) * 2};
+    if (channels >= kCastBlocks * kCastChannels) {
 #pragma unroll
-    for (int i = 0; i < kCastSteps; ++i) {
-        const int elem = ((batch * kCastSteps + i) * 32 + lane) * 8;
-        b.v[i] = elem < H ? ptx::ld_nc_v4(row + elem * 2) : make_int4(0, 0, 0, 0);
+        for (int k = 0; k < kCastBlocks; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) b.v[k][i] = load(p[i & 1] + cast_piece(k, i) * 2);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kCastBlocks; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                b.v[k][i] = cast_lane(i & 1) + cast_piece(k, i) < channels ? load(p[i & 1] + cast_piece(k, i) * 2) : make_int4(0, 0, 0, 0);
     }
+}
+__device__ __forceinline__ void load_batch(RowBatch& b, const uint8_t* row, int H, int batch) {
+    const int first = batch * kCastBlocks * kCastChannels;
+    load_pieces(b, row + first * 2, H - first, [](const uint8_t* p) { return ptx::ld_nc_v4(p); });
 }
 
 __device__ __forceinline__ void scales_from_amax(float* sf, int num_groups) {
@@ -207,48 +235,77 @@ __device__ __forceinline__ void scales_from_amax(float* sf, int num_groups) {
     for (int g = ptx::lane_id(); g < num_groups; g += 32) sf[g] = __fdiv_rn(sf[g], 448.f);
 }
 
-// Instruction count is what bounds the cast (a batch is a chain of ALU work on data that is already there), so
-//   * the amax is taken on packed bf16 pairs (the largest of bf16 magnitudes is one of them: no rounding), and two steps share one
-//     register through the four shuffles of their reduction;
-//   * lane j of a half-warp computes the scale of step j, once per batch, instead of all lanes computing all of them;
+// Instruction issue bounds the cast, the integer and conversion pipe (half rate) above all, so
+//   * a lane's 32 values of a block belong to one group: the amax is taken on packed bf16 pairs inside the lane (the largest of bf16
+//     magnitudes is one of them: no rounding) and needs two shuffles per block, and the scale is already where it is used;
+//   * whole blocks carry no bounds checks, and the chains of a batch's two blocks are interleaved;
 //   * products are formed two at a time (mul.rn.f32x2: the same two roundings).
-// 8192 tokens x 7168 on one rank, whole dispatch kernel: 689 -> 505 us on 8 SMs, 190 -> 144 on 32, 106 -> 84 on 64, 69 -> 63 on 148.
-__device__ __forceinline__ void cast_batch(const RowBatch& b, uint8_t* out, float* sf, int H, int batch) {
-    const int lane = ptx::lane_id();
-    constexpr int kPairs = (kCastSteps + 1) / 2;
-    __nv_bfloat162 amax[kPairs];            // (step 2p, step 2p + 1)
+// 8192 tokens x 7168 on 64 SMs: 135 instructions per 256 channels and lane -> 75 in the direct kernel of one rank; the staging kernel, whose
+// 12 warps are latency-bound next to that, gains 3 us of 92.
+template <int kBlocks>
+__device__ __forceinline__ void cast_blocks(const RowBatch& b, uint2 (&q)[kCastBlocks][4], float (&amax)[kCastBlocks]) {
+    float scale[kBlocks];
 #pragma unroll
-    for (int p = 0; p < kPairs; ++p) {
-        __nv_bfloat162 m[2];
+    for (int k = 0; k < kBlocks; ++k) {
+        uint32_t m[2];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int i = 2 * p + q < kCastSteps ? 2 * p + q : 2 * p;
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&b.v[i]);
-            m[q] = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(&b.v[k][i]);
+            const uint32_t p = ptx::max_magnitude2(ptx::max_magnitude2(w[0], w[1]), ptx::max_magnitude2(w[2], w[3]));
+            m[i & 1] = i < 2 ? p : ptx::max_magnitude2(m[i & 1], p);
         }
-        amax[p] = __hmax2(__lows2bfloat162(m[0], m[1]), __highs2bfloat162(m[0], m[1]));
+        m[0] = ptx::max_magnitude2(m[0], m[1]);
+        amax[k] = fmaxf(fabsf(__uint_as_float(m[0] << 16)), fabsf(__uint_as_float(m[0] & 0xffff0000u)));
     }
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
+    for (int o = 1; o <= 2; o <<= 1)
 #pragma unroll
-        for (int p = 0; p < kPairs; ++p) amax[p] = __hmax2(amax[p], __shfl_xor_sync(0xffffffffu, amax[p], o));
-    // lane j of the half-warp: step j
-    const int j = lane & 15;
-    __nv_bfloat162 mine = amax[0];
+        for (int k = 0; k < kBlocks; ++k) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], o));
 #pragma unroll
-    for (int p = 1; p < kPairs; ++p)
-        if ((j >> 1) == p) mine = amax[p];
-    const float my_amax = fmaxf((j & 1) ? __high2float(mine) : __low2float(mine), 1e-4f);
-    // 448 * (1 / amax), each step correctly rounded: bit-identical to the PyTorch expression `448.0 / amax`
-    const float my_scale = __fmul_rn(448.f, __frcp_rn(my_amax));
-    const int group = (batch * kCastSteps + j) * 2 + (lane >> 4);
-    if (j < kCastSteps && group * 128 < H) sf[group] = my_amax;      // divided by 448 once per row, see scales_from_amax
-#pragma unroll
-    for (int i = 0; i < kCastSteps; ++i) {
-        const int elem = ((batch * kCastSteps + i) * 32 + lane) * 8;
-        const float scale = __shfl_sync(0xffffffffu, my_scale, (lane & 16) + i);
-        if (elem < H) *reinterpret_cast<uint2*>(out + elem) = ptx::cast8_e4m3(b.v[i], scale);
+    for (int k = 0; k < kBlocks; ++k) {
+        amax[k] = fmaxf(amax[k], 1e-4f);
+        // 448 * (1 / amax), each step correctly rounded: bit-identical to the PyTorch expression `448.0 / amax`
+        scale[k] = __fmul_rn(448.f, __frcp_rn(amax[k]));
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < kBlocks; ++k) q[k][i] = ptx::cast8_e4m3(b.v[k][i], scale[k]);
+}
+// e4m3 pieces of a batch whose first channel is at `out` (in a row that goes on for `channels` from there)
+__device__ __forceinline__ void store_pieces(uint8_t* out, const uint2 (&q)[kCastBlocks][4], int channels) {
+    uint8_t* p[2] = {out + cast_lane(0), out + cast_lane(1)};
+#pragma unroll
+    for (int k = 0; k < kCastBlocks; ++k) {
+        if (channels >= (k + 1) * kCastChannels) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint2*>(p[i & 1] + cast_piece(k, i)) = q[k][i];
+        } else if (channels > k * kCastChannels) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (cast_lane(i & 1) + cast_piece(k, i) < channels) *reinterpret_cast<uint2*>(p[i & 1] + cast_piece(k, i)) = q[k][i];
+        }
+    }
+}
+// f(block, group inside the batch) by the lane that keeps a scale group of the row
+template <typename F>
+__device__ __forceinline__ void for_groups(int channels, F f) {
+    const int g = ptx::lane_id() >> 2;
+    if ((ptx::lane_id() & 3) != 0) return;
+#pragma unroll
+    for (int k = 0; k < kCastBlocks; ++k) {
+        const int group = k * (kCastChannels / 128) + g;
+        if (group * 128 < channels) f(k, group);
+    }
+}
+__device__ __forceinline__ void cast_batch(const RowBatch& b, uint8_t* out, float* sf, int H, int batch) {
+    uint2 q[kCastBlocks][4];
+    float amax[kCastBlocks];
+    const int first = batch * kCastBlocks * kCastChannels, channels = H - first;
+    if (channels <= kCastChannels) cast_blocks<1>(b, q, amax);
+    else cast_blocks<kCastBlocks>(b, q, amax);
+    store_pieces(out + first, q, channels);
+    for_groups(channels, [&](int k, int group) { sf[first / 128 + group] = amax[k]; });      // divided by 448 once per row, see scales_from_amax
 }
 
 // sources of all but the `pending` most recent bulk groups of this thread have been read
@@ -261,7 +318,170 @@ __device__ __forceinline__ void bulk_wait_read_n(int pending) {
     }
 }
 
+// ------------------------------------------------------------------------------------------------ one rank
+// With one rank every destination row lies in this GPU's own memory: the tokens of a CTA's slice go from registers straight to their
+// rows, without staging, claims or a word to anyone.  A unit of work is up to 4 KB of one token (a batch of the cast); the first parts
+// of all tokens come first, and with them the small pieces.  A warp has the plan entries and small pieces of its next unit on their
+// way; rows to be cast come through two buffers per warp that are filled two units ahead, others are requested as a whole unit.
+// An SM moves at most 97 GB/s in and out together (plain copies, any number of warps): 5003 pre-quantised tokens on 24 SMs take 58 us
+// against 74 in the staging kernel (31 at that rate), 4096 bf16 tokens on 64 SMs 40 against 53 (19).  The cast is bound by
+// instruction issue: 8192 tokens on 64 SMs 73 us against 92.  20 warps: with 24 the kernel spills (+ 8 us), 16 are slower (+ 6 us).
+// The small pieces of a token: lane k has its id and weight of top-k lane k, every lane two scales of a pre-quantised token.
+struct SidePieces {
+    int e;
+    float w, sf[2];
+};
+__device__ __forceinline__ SidePieces load_side(const DispatchArgs& a, int t) {
+    const int lane = ptx::lane_id(), K = a.num_topk, G = (a.hidden + 127) / 128;
+    SidePieces s{-1, 0.f, {0.f, 0.f}};
+    if (lane < K) {
+        s.e = load_idx(a, t, lane);
+        if (a.topk_weights != nullptr) s.w = __ldg(a.topk_weights + static_cast<int64_t>(t) * K + lane);
+    }
+    if (a.sf != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (i * 32 + lane < G) s.sf[i] = __ldg(a.sf + static_cast<int64_t>(t) * G + i * 32 + lane);
+    }
+    return s;
+}
+__device__ __forceinline__ void send_side_local(const DispatchArgs& a, int t, const SidePieces& s, int plan_k, uint32_t sends) {
+    const int lane = ptx::lane_id(), K = a.num_topk, me = a.ctx.rank, G = (a.hidden + 127) / 128;
+    const int e_k = s.e >= 0 && s.e < a.num_experts ? s.e : -1;
+    uint8_t* base = a.ctx.peer_base[me];
+    for (uint32_t m = sends; m != 0; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const int64_t row = __shfl_sync(0xffffffffu, plan_k, k) & 0xffffff;
+        int2* meta = reinterpret_cast<int2*>(base + a.off_recv_meta) + row;
+        if (a.do_expand) {
+            if (lane == k && a.topk_weights != nullptr) reinterpret_cast<float*>(base + a.off_recv_w)[row] = s.w;
+        } else {
+            uint8_t* ids = base + a.off_recv_idx + row * K * (a.idx_is_64 ? 8 : 4);
+            float* w = reinterpret_cast<float*>(base + a.off_recv_w) + row * K;
+            if (a.side_packed) {
+                ids = base + a.off_recv_tail + row * a.tail_pitch;
+                w = reinterpret_cast<float*>(ids + a.tail_off_w);
+                meta = reinterpret_cast<int2*>(ids + a.tail_off_meta);
+            }
+            if (lane < K) {
+                if (a.idx_is_64) reinterpret_cast<long long*>(ids)[lane] = e_k;
+                else reinterpret_cast<int*>(ids)[lane] = e_k;
+                if (a.topk_weights != nullptr || a.side_packed) w[lane] = s.w;
+            }
+        }
+        if (lane == 0) *meta = make_int2(me * a.num_max_tokens + t, me * K + k);
+        if (a.sf != nullptr) {
+            float* sf = reinterpret_cast<float*>(base + a.off_recv_sf) + row * a.sf_stride_row;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (i * 32 + lane < G) sf[(i * 32 + lane) * a.sf_stride_col] = s.sf[i];
+            for (int g = 64 + lane; g < G; g += 32) sf[g * a.sf_stride_col] = __ldg(a.sf + static_cast<int64_t>(t) * G + g);
+        }
+    }
+}
+
+// unit of a warp: part `part` of token `t` (an offset into the CTA's slice); all tokens' first parts come first
+struct LocalUnit {
+    int t, part;
+    __device__ __forceinline__ void advance(int by, int tokens) {
+        for (t += by; t >= tokens; t -= tokens) ++part;
+    }
+};
 template <bool kQuant>
+__device__ __forceinline__ bool scatter_local(const DispatchArgs& a, Workspace* ws, Slice slice, uint64_t* bars, uint8_t* stage) {
+    const int lane = ptx::lane_id(), warp = threadIdx.x >> 5, num_warps = blockDim.x >> 5, K = a.num_topk, H = a.hidden;
+    uint8_t* base = a.ctx.peer_base[a.ctx.rank];
+    const uint8_t* xb = reinterpret_cast<const uint8_t*>(a.x);
+    const int in_row = H * (a.x_is_fp8 ? 1 : 2), tokens = slice.end - slice.begin;
+    if (tokens == 0) return true;
+    // rows that are not cast: steps of 512 bytes, up to eight per unit, fewer where that gives more warps work
+    constexpr int kSteps = kCastBlocks * 4;
+    const int steps = (in_row + 511) / 512, wanted = kQuant ? kSteps : max(1, min(kSteps, (tokens * steps + num_warps - 1) / num_warps));
+    const int parts = (steps + wanted - 1) / wanted, unit_bytes = kQuant ? kLocalUnitBytes : (steps + parts - 1) / parts * 512;
+    LocalUnit cur{0, 0}, next, ahead;
+    cur.advance(warp, tokens);
+    next = cur;
+    next.advance(num_warps, tokens);
+    ahead = cur;
+    int issued = 0;
+    // cast: units two ahead are on their way into this warp's two staging buffers
+    auto issue = [&]() {
+        if (ahead.part >= parts) return;
+        if (lane == 0) {
+            const int off = ahead.part * kLocalUnitBytes, bytes = min(kLocalUnitBytes, in_row - off);
+            ptx::mbar_arrive_expect_tx(&bars[issued & 1], bytes);
+            ptx::bulk_load(stage + (issued & 1) * kLocalUnitBytes, xb + static_cast<int64_t>(slice.begin + ahead.t) * in_row + off, bytes, &bars[issued & 1]);
+        }
+        ++issued;
+        ahead.advance(num_warps, tokens);
+    };
+    if (kQuant) {
+        issue();
+        issue();
+    }
+    auto load_plan = [&](const LocalUnit& u) -> int {
+        return u.part < parts && lane < K ? __ldcg(a.plan + static_cast<int64_t>(slice.begin + u.t) * K + lane) : -1;
+    };
+    int next_plan = load_plan(cur);
+    SidePieces next_side{};
+    if (cur.part == 0) next_side = load_side(a, slice.begin + cur.t);
+    bool alive = true;
+    int n = 0;
+    for (; cur.part < parts && alive; cur = next, next.advance(num_warps, tokens), ++n) {
+        const int part = cur.part, t = slice.begin + cur.t;
+        int plan_k = next_plan;
+        const SidePieces side = next_side;
+        RowBatch b;
+        const int off0 = part * unit_bytes + lane * 16, end = min(in_row, (part + 1) * unit_bytes);
+        if constexpr (!kQuant) {
+            const uint8_t* src = xb + static_cast<int64_t>(t) * in_row;
+#pragma unroll
+            for (int i = 0; i < kSteps; ++i)
+                if (off0 + i * 512 < end) b.v[i / 4][i % 4] = ptx::ld_nc_v4(src + off0 + i * 512);
+        }
+        next_plan = load_plan(next);
+        if (next.part == 0) next_side = load_side(a, slice.begin + next.t);
+        if (plan_k >= 0 && (plan_k & 0xffffff) >= a.recv_capacity_rows) {
+            report_failure(a.ctx, ws, EP_ERR_BOUNDS, EP_PH_DISPATCH_LOAD, a.ctx.rank, a.recv_capacity_rows, plan_k & 0xffffff);
+            plan_k = -1;
+        }
+        const uint32_t sends = __ballot_sync(0xffffffffu, plan_k >= 0);
+        if (part == 0) send_side_local(a, t, side, plan_k, sends);
+        uint2 q[kCastBlocks][4];
+        float amax[kCastBlocks];
+        const int channels = H - part * kCastBlocks * kCastChannels;
+        if constexpr (kQuant) {
+            alive = mbar_wait_bounded(a.ctx, ws, &bars[n & 1], (n >> 1) & 1, EP_PH_DISPATCH_LOAD);
+            if (!alive) break;
+            const uint8_t* buf = stage + (n & 1) * kLocalUnitBytes;
+            load_pieces(b, buf, channels, [](const uint8_t* p) { return *reinterpret_cast<const int4*>(p); });
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            issue();          // into the buffer that was just read
+            if (channels <= kCastChannels) cast_blocks<1>(b, q, amax);
+            else cast_blocks<kCastBlocks>(b, q, amax);
+        }
+        for (uint32_t m = sends; m != 0; m &= m - 1) {
+            const int64_t row = __shfl_sync(0xffffffffu, plan_k, __ffs(m) - 1) & 0xffffff;
+            if constexpr (kQuant) {
+                const int first = part * kCastBlocks * kCastChannels;
+                float* sf = reinterpret_cast<float*>(base + a.off_recv_sf) + row * a.sf_stride_row + first / 128 * a.sf_stride_col;
+                store_pieces(base + a.off_recv_x + row * H + first, q, channels);
+                for_groups(channels, [&](int k, int group) { sf[group * a.sf_stride_col] = __fdiv_rn(amax[k], 448.f); });
+            } else {
+                uint8_t* dst = base + a.off_recv_x + row * in_row;
+#pragma unroll
+                for (int i = 0; i < kSteps; ++i)
+                    if (off0 + i * 512 < end) ptx::st_na_v4(dst + off0 + i * 512, b.v[i / 4][i % 4]);
+            }
+        }
+    }
+    // left early after a failure: loads still in flight must land before this CTA gives up its shared memory
+    for (; n < issued; ++n) mbar_drain(&bars[n & 1], (n >> 1) & 1, 1000ull * 1000 * 1000);
+    return alive;
+}
+
+template <bool kQuant, bool kLocal>
 __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const RankCtx& ctx = a.ctx;
@@ -271,7 +491,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     const int cta = blockIdx.x, num_ctas = gridDim.x;
     const int R = ctx.num_ranks, me = ctx.rank, E = a.num_experts, El = E / R, K = a.num_topk, T = a.num_tokens;
     const int G = (a.hidden + 127) / 128;
-    const DispatchSmemPlan sp = make_smem_plan(a, num_warps, a.tune_stages);
+    const DispatchSmemPlan sp = make_smem_plan(a, num_warps, a.tune_stages, kLocal);
 
     uint8_t** s_peer = reinterpret_cast<uint8_t**>(smem + sp.off_peer);
     uint32_t* s_tot = reinterpret_cast<uint32_t*>(smem + sp.off_tot);
@@ -302,7 +522,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     __syncthreads();
     ptx::fence_proxy_async_smem();
 
-    const Slice sl = warp_slice(T, K, num_warps, warp);
+    const Slice cta_tokens = cta_slice<kLocal>(T), sl = warp_slice(cta_tokens, K, num_warps, warp);
     const int own_chunk = max(1, (T + num_ctas - 1) / num_ctas);
     bool alive = !is_aborted(ws);
     auto stamp = [&](int i) {
@@ -311,9 +531,10 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     stamp(0);
     // With few tokens the row of this warp's first token (see scatter) starts on its way while the counts are exchanged: 61 tokens
     // 30 -> 25 us.  With many, the rows would only hold up the routing ids that are counted first (8192 tokens: + 2 us).
-    if (lane == 0 && warp * num_ctas + cta < T && T <= 4 * num_ctas * num_warps) {
+    const int first_token = kLocal ? cta_tokens.begin + warp : warp * num_ctas + cta;
+    if (lane == 0 && first_token < (kLocal ? cta_tokens.end : T) && T <= 4 * num_ctas * (kLocal ? kDispatchMaxWarps : num_warps)) {
         const int in_row = a.hidden * (a.x_is_fp8 ? 1 : 2);
-        ptx::bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(a.x) + static_cast<int64_t>(warp * num_ctas + cta) * in_row, in_row);
+        ptx::bulk_prefetch_l2(reinterpret_cast<const uint8_t*>(a.x) + static_cast<int64_t>(first_token) * in_row, in_row);
     }
     // The bookkeeper writes what this rank receives (handle tensors, host counters) before it sends anything.  The first token of each
     // of its warps is fixed like everybody's and waits for that; of the claimed tokens it gets fewer.
@@ -486,7 +707,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
         __threadfence();
         __syncthreads();
         if (tid == 0 && alive) ptx::st_release_gpu_u32(&ws->cta_assigned[cta], epoch32);
-    } else {
+    } else if (!kLocal) {
         // cached layout: only the entry barrier (receivers must be done with the previous contents); CTA 0 signals the
         // peers, every CTA watches the peers' arrivals itself
         int ok = alive ? 1 : 0;
@@ -536,7 +757,8 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     }
 
     // -------------------------------------------------------------------- 4. scatter
-    if (alive) {
+    if (kLocal && alive) alive = scatter_local<kQuant>(a, ws, cta_tokens, s_bar, smem + sp.off_stage + warp * 2 * kLocalUnitBytes);
+    if (!kLocal && alive) {
         const int in_row = a.hidden * (a.x_is_fp8 ? 1 : 2);
         const int out_row = kQuant ? a.hidden : in_row;
         const int idx_bytes = a.idx_is_64 ? 8 : 4;
@@ -546,7 +768,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
         const uint8_t* xb = reinterpret_cast<const uint8_t*>(a.x);
         const int S_in = kQuant ? 1 : sp.n_in;
         const int S_side = sp.n_side;
-        const int num_batches = ((a.hidden + 255) / 256 + kCastSteps - 1) / kCastSteps;
+        const int num_batches = (a.hidden + kCastBlocks * kCastChannels - 1) / (kCastBlocks * kCastChannels);
         const uint32_t lt = ptx::lanemask_lt();
         // The first token of every warp is fixed (with few tokens its row was requested into L2 at kernel entry); later ones are claimed from a
         // counter shared by all CTAs of this rank: SMs that get a smaller share of the NVLink bandwidth simply claim fewer
@@ -588,7 +810,33 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
             known_hi = min(T, known_lo + own_chunk);
             return ok != 0;
         };
+        // The small pieces of a token are requested one token ahead: row numbers, ids and weights by the lanes below K, the scales of a
+        // pre-quantised row two per lane (of a wider row the rest when they are needed).  Asked for when the token's turn came, they were a
+        // third of a warp's chain: scatter of 5003 pre-quantised tokens x 7168 on 24 SMs 43 -> 36 us.
+        struct Side {
+            int e, plan;
+            float w, sf[2];
+        };
+        auto load_side = [&](int tok) {
+            Side s{-1, -1, 0.f, {0.f, 0.f}};
+            if (lane < K) {
+                s.e = load_idx(a, tok, lane);
+                s.plan = __ldcg(a.plan + static_cast<int64_t>(tok) * K + lane);
+                if (a.topk_weights != nullptr) s.w = __ldg(a.topk_weights + static_cast<int64_t>(tok) * K + lane);
+            }
+            if (!kQuant && has_sf) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (i * 32 + lane < G) s.sf[i] = __ldg(a.sf + static_cast<int64_t>(tok) * G + i * 32 + lane);
+            }
+            return s;
+        };
         int t = next_token(), t_next = next_token();
+        Side side_next{-1, -1, 0.f, {0.f, 0.f}};
+        if (t >= 0) {
+            alive = rows_assigned(t);
+            if (alive) side_next = load_side(t);
+        }
         int loads_issued = 0, loads_waited = 0;   // bulk loads of the pass-through path (token i uses stage i % S_in)
         RowBatch cur;
         if (kQuant) {
@@ -617,22 +865,26 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
                     ++loads_issued;
                 }
             }
-            if (!rows_assigned(t)) {
-                alive = false;
-                break;
-            }
-            int e_k = -1, plan_k = -1;
-            float w_k = 0.f;
-            if (lane < K) {
-                e_k = load_idx(a, t, lane);
-                plan_k = __ldcg(a.plan + static_cast<int64_t>(t) * K + lane);
-                if (a.topk_weights != nullptr) w_k = __ldg(a.topk_weights + static_cast<int64_t>(t) * K + lane);
+            const Side side = side_next;
+            const int e_k = side.e;
+            int plan_k = side.plan;
+            const float w_k = side.w;
+            if (t_next >= 0) {
+                if (!rows_assigned(t_next)) {
+                    alive = false;
+                    break;
+                }
+                side_next = load_side(t_next);
             }
             const int side_slot = n % S_side;
             float* sf_cur = s_sf + side_slot * sp.sf_floats;
             uint8_t* tail_cur = s_tail + side_slot * sp.max_dst * a.tail_bytes;
-            if (!kQuant && has_sf)
-                for (int j = lane; j < G; j += 32) sf_cur[j] = __ldg(a.sf + static_cast<int64_t>(t) * G + j);
+            if (!kQuant && has_sf) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (i * 32 + lane < G) sf_cur[i * 32 + lane] = side.sf[i];
+                for (int j = 64 + lane; j < G; j += 32) sf_cur[j] = __ldg(a.sf + static_cast<int64_t>(t) * G + j);
+            }
             const uint8_t* src_smem;
             if (kQuant) {
                 uint8_t* o = out_stage + side_slot * sp.out_bytes;
@@ -734,7 +986,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     ptx::bulk_commit();
     ptx::bulk_wait<0>();
     // with side records all stores to peers are bulk stores of the first K lanes; other lanes have nothing to make visible
-    if (!a.side_packed || lane < K) __threadfence_system();
+    if (!kLocal && (!a.side_packed || lane < K)) __threadfence_system();
     stamp(4);
     // Every CTA arrives once its own stores are complete; only the last one stays: it tells every peer "all rows of my
     // dispatch number `epoch` have arrived", waits for the same word from every peer (the kernel must not end before
@@ -745,7 +997,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     };
     stamp_last(5);
     alive = !is_aborted(ws);
-    {
+    if (!kLocal) {
         int ok = alive ? 1 : 0;
         if (alive && tid < R) {
             ptx::st_release_sys(&reinterpret_cast<Workspace*>(s_peer[tid])->disp_done[me], epoch);
@@ -758,8 +1010,8 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
     }
     stamp_last(6);
     if (tid == 0) {
-        atomicExch(&ws->dyn_counter[EP_CH_DISPATCH], 0u);
-        if (a.cached) ws->bar_seq[EP_CH_DISPATCH] = entry_seq;
+        if (!kLocal) atomicExch(&ws->dyn_counter[EP_CH_DISPATCH], 0u);
+        if (!kLocal && a.cached) ws->bar_seq[EP_CH_DISPATCH] = entry_seq;
         ws->epoch[EP_CH_DISPATCH] = epoch;
     }
     stamp_last(7);
@@ -767,31 +1019,36 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
 
 template <bool kQuant>
 __global__ void __launch_bounds__(kDispatchMaxWarps * 32, 1) dispatch_kernel(const __grid_constant__ DispatchArgs args) {
-    dispatch_body<kQuant>(args);
+    dispatch_body<kQuant, false>(args);
+}
+template <bool kQuant>
+__global__ void __launch_bounds__(kLocalWarps * 32, 1) dispatch_local_kernel(const __grid_constant__ DispatchArgs args) {
+    dispatch_body<kQuant, true>(args);
 }
 
 // n virtual ranks on one device: blockIdx.y selects the rank
 template <bool kQuant>
 __global__ void __launch_bounds__(kDispatchMaxWarps * 32, 1) dispatch_kernel_multi(const DispatchArgs* args) {
-    dispatch_body<kQuant>(args[blockIdx.y]);
+    dispatch_body<kQuant, false>(args[blockIdx.y]);
 }
 
 }  // namespace
 
-LaunchShape dispatch_launch_shape(const DispatchArgs& a, int num_sms) {
+LaunchShape dispatch_launch_shape(const DispatchArgs& a, int num_sms, bool local) {
     LaunchShape s;
     s.num_ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
     // staging buffers per warp of the fused-cast path (two unless the caller asks for more), then as many warps (each
     // with its own staging ring) as fit in shared memory; the token-per-step layout needs at least one warp
     s.num_stages = a.tune_stages >= 2 && a.tune_stages <= kDispatchMaxStages ? a.tune_stages : 2;
-    s.num_warps = a.tune_warps >= 1 && a.tune_warps <= kDispatchMaxWarps ? a.tune_warps : kDispatchMaxWarps;
-    while (s.num_warps > 1 && make_smem_plan(a, s.num_warps, s.num_stages).total > kDispatchSmemBudget) --s.num_warps;
-    s.smem_bytes = make_smem_plan(a, s.num_warps, s.num_stages).total;
+    s.num_warps = a.tune_warps >= 1 && a.tune_warps <= kDispatchMaxWarps ? a.tune_warps : (local ? kLocalWarps : kDispatchMaxWarps);
+    while (s.num_warps > 1 && make_smem_plan(a, s.num_warps, s.num_stages, local).total > kDispatchSmemBudget) --s.num_warps;
+    s.smem_bytes = make_smem_plan(a, s.num_warps, s.num_stages, local).total;
     return s;
 }
 
 cudaError_t launch_dispatch(const DispatchArgs* args_in, int n, int num_sms, cudaStream_t stream) {
-    const LaunchShape shape = dispatch_launch_shape(args_in[0], num_sms);
+    const bool local = n == 1 && args_in[0].ctx.num_ranks == 1;
+    const LaunchShape shape = dispatch_launch_shape(args_in[0], num_sms, local);
     if (shape.smem_bytes > 227 * 1024 || n < 1 || n > EP_MAX_RANKS) return cudaErrorInvalidValue;
     // the kernel derives its shared-memory plan from the resolved shape
     DispatchArgs args[EP_MAX_RANKS];
@@ -802,7 +1059,8 @@ cudaError_t launch_dispatch(const DispatchArgs* args_in, int n, int num_sms, cud
     }
     const DispatchArgs& a0 = args[0];
     const void* fn;
-    if (n == 1) fn = a0.quantize ? (const void*)dispatch_kernel<true> : (const void*)dispatch_kernel<false>;
+    if (local) fn = a0.quantize ? (const void*)dispatch_local_kernel<true> : (const void*)dispatch_local_kernel<false>;
+    else if (n == 1) fn = a0.quantize ? (const void*)dispatch_kernel<true> : (const void*)dispatch_kernel<false>;
     else fn = a0.quantize ? (const void*)dispatch_kernel_multi<true> : (const void*)dispatch_kernel_multi<false>;
     cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, shape.smem_bytes);
     if (err != cudaSuccess) return err;

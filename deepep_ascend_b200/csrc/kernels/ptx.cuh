@@ -140,22 +140,34 @@ __device__ __forceinline__ void st_na_v4(void* p, const int4& v) {
 }
 
 // ---------------------------------------------------------------- casts
+// Four fp32 values -> e4m3 (saturating), in order.  Both conversions in one statement: they write the halves of one register.
+__device__ __forceinline__ uint32_t cvt4_e4m3(float a, float b, float c, float d) {
+    uint32_t out;
+    asm("{\n .reg .b16 lo, hi;\n cvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n mov.b32 %0, {lo, hi};\n}\n"
+        : "=r"(out)
+        : "f"(a), "f"(b), "f"(c), "f"(d));
+    return out;
+}
 // Eight bf16 values times `scale` (fp32, round to nearest), cast to e4m3 (saturating).
 __device__ __forceinline__ uint2 cast8_e4m3(const int4& raw, float scale) {
     uint64_t scale2;
     asm("mov.b64 %0, {%1, %1};" : "=l"(scale2) : "f"(scale));
     const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
-    uint32_t half[4];
+    float f[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         uint64_t x2;
-        float lo, hi;
         asm("mov.b64 %0, {%1, %2};" : "=l"(x2) : "r"(w[j] << 16), "r"(w[j] & 0xffff0000u));
         asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(x2) : "l"(x2), "l"(scale2));
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x2));
-        half[j] = __nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(f[2 * j]), "=f"(f[2 * j + 1]) : "l"(x2));
     }
-    return make_uint2(half[0] | (half[1] << 16), half[2] | (half[3] << 16));
+    return make_uint2(cvt4_e4m3(f[0], f[1], f[2], f[3]), cvt4_e4m3(f[4], f[5], f[6], f[7]));
+}
+// Larger magnitude of each bf16 pair, a NaN loses against a number; the sign of the result means nothing (drop it at the end).
+__device__ __forceinline__ uint32_t max_magnitude2(uint32_t a, uint32_t b) {
+    uint32_t out;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(b));
+    return out;
 }
 
 // ---------------------------------------------------------------- warp helpers

@@ -1,4 +1,5 @@
-"""Edges of the exchange kernels that move rows directly when there is a single rank.  Everything is compared bitwise."""
+"""Edges of the exchange kernels: the fused cast at ragged row widths on one and on two ranks, and the kernels that move rows directly when
+there is a single rank.  Everything is compared bitwise."""
 import pytest
 import torch
 
@@ -23,6 +24,47 @@ def _routing(T, E, K, seed):
     idx[torch.rand(T, K, generator=g) < 0.2] = -1
     idx[T // 3] = -1                                       # a token that goes nowhere
     return idx.cuda(), torch.rand(T, K, generator=g).cuda()
+
+
+@pytest.mark.parametrize('R', [1, 2])
+@pytest.mark.parametrize('T,H,sms', [(1, 128, 3), (3, 1024, 5), (37, 1152, 2), (64, 2048, 3), (90, 2176, 1), (41, 4096, 8), (130, 7168, 4)])
+@pytest.mark.parametrize('mode', ['cast', 'fp8_in', 'bf16'])
+@pytest.mark.parametrize('do_expand', [False, True])
+def test_dispatch_rows_at_the_edges_of_a_batch(R, T, H, sms, mode, do_expand):
+    """Rows of less than, exactly and more than one block (1024 channels) and one batch (2048) of the cast, whole and cut units of one
+    rank's rows, fewer tokens than SMs and many per SM.  The cast is that of ``per_token_cast_to_fp8`` (another kernel)."""
+    from deepep_ascend_b200.backends.emulated import EmulatedWorld
+    from deepep_ascend_b200.ops import gemm as G
+    from deepep_ascend_b200.utils import refs
+    E, K, A = 8, 3, 4 if do_expand else 1
+    world = EmulatedWorld(R, num_max_tokens_per_rank=T, hidden=H, num_topk=K, use_fp8_dispatch=mode != 'bf16', enable_expand=do_expand,
+                          num_experts=E, expert_alignment=A)
+    try:
+        xs = [_rows(T, H, 10 * T + r) for r in range(R)]
+        idxs, ws = zip(*[_routing(T, E, K, T + r) for r in range(R)])
+        cast = [G.per_token_cast_to_fp8(x) for x in xs]
+        ins = cast if mode == 'fp8_in' else xs
+        for handles in (None, 'cached'):
+            if handles is not None:
+                outs = world.dispatch(ins, [None] * R, ws, E, num_sms=sms, handles=[o[3] for o in outs])
+            else:
+                outs = world.dispatch(ins, idxs, ws, E, num_sms=sms, expert_alignment=A, do_expand=do_expand)
+            torch.cuda.synchronize()
+            expect = refs.dispatch_all([q if mode != 'bf16' else x for (q, _), x in zip(cast, xs)],
+                                       [sf for _, sf in cast] if mode != 'bf16' else None, list(idxs), list(ws), E, T, do_expand, A)
+            for r, (x, idx, w, handle) in enumerate(outs):
+                world.buffers[r].check_status()
+                e, valid = expect[r], expect[r]['valid']
+                x, sf = x if mode != 'bf16' else (x, None)
+                assert torch.equal(x.cpu().view(torch.uint8)[valid], e['x'].cpu().view(torch.uint8)[valid])
+                if sf is not None:
+                    assert torch.equal(sf.cpu()[valid], e['sf'].cpu()[valid])
+                if not do_expand:
+                    assert torch.equal(idx.cpu(), e['idx'])
+                assert torch.equal(w.cpu()[valid], e['w'][valid])
+                assert torch.equal(handle.recv_src_metadata.cpu()[valid], e['meta'][valid])
+    finally:
+        world.destroy()
 
 
 @pytest.mark.parametrize('T,H,sms', [(1, 128, 3), (5, 256, 2), (37, 1168, 1), (64, 2048, 3), (90, 4112, 7), (41, 7168, 64), (300, 7168, 4)])
