@@ -14,6 +14,7 @@ How it differs from the reference by design:
 
 The same class runs on CPU tensors with a gloo group (``backends/cpu.py``) with identical handle semantics.
 """
+import contextlib
 import itertools
 import math
 import os
@@ -112,9 +113,8 @@ class EPHandle:
 
 class _DispatchState:
     """Book-keeping between the three steps of a dispatch (prepare -> launch -> finish)."""
-    __slots__ = ('call', 'T', 'H', 'K', 'E', 'fp8_out', 'do_expand', 'alignment', 'slot_idx', 'slot', 'handle_tensors',
-                 'topk_idx', 'topk_weights', 'do_cpu_sync', 'num_sms', 'col_major_sf', 'cached_handle', 'x_dtype',
-                 'keep_alive', 'do_handle_copy', 'side')
+    __slots__ = ('call', 'T', 'H', 'K', 'E', 'fp8_out', 'do_expand', 'alignment', 'num_max_tokens', 'slot_idx', 'topk_idx', 'topk_weights',
+                 'do_cpu_sync', 'num_sms', 'cached_handle', 'do_handle_copy')
 
 
 class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
@@ -479,24 +479,25 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
 
         K = (handle.topk_idx if topk_idx is None else topk_idx).shape[1]
         num_sms = self.get_theoretical_num_sms(num_experts, K) if num_sms == 0 else num_sms
-        cur = current_stream()
+        stream = self.comm_stream
         prepare = (x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts, num_max_tokens_per_rank, expert_alignment,
                    num_sms, handle, do_handle_copy, do_cpu_sync, do_expand, use_tma_aligned_col_major_sf, fused_fp8_cast, do_zero_padding)
         if allocate_on_comm_stream:
-            self._stream_prologue(previous_event, previous_event_before_epilogue, self.comm_stream, cur)
-            with on_stream(self.comm_stream):
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
+            with on_stream(stream):
                 st = self._prepare_dispatch(*prepare)
         else:
             # input copies made while preparing run on the caller's stream: wait for them too
             st = self._prepare_dispatch(*prepare)
-            self._stream_prologue(previous_event, previous_event_before_epilogue, self.comm_stream, cur)
-        with on_stream(self.comm_stream):
-            self._timed('dispatch', lambda: self.core.dispatch(st.call, num_sms))
-            out = self._finish_dispatch(st)
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
+        self._launch('dispatch', self.core.dispatch, st.call, num_sms, stream)
+        out = self._finish_dispatch(st, stream.stream_id)
+        if not async_with_compute_stream:
+            self.core.current_waits_for_stream(stream.stream_id)
+            return (*out, EventOverlap(None))
         inputs = (st.call.x, st.call.sf, st.call.topk_idx, st.call.topk_weights, st.call.stats, st.call.lane_src,
                   st.call.plan, st.call.psum_rank, st.call.psum_expert, st.call.recv_per_expert, x, topk_idx, topk_weights)
-        event = self._stream_epilogue(async_with_compute_stream, out, inputs, self.comm_stream, cur)
-        return (*out, event)
+        return (*out, self._async_event(out, inputs, stream))
 
     def _next_recv_slot(self) -> int:
         slot = self._recv_slot_counter % self.regions.num_recv_slots
@@ -506,142 +507,58 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
     def _prepare_dispatch(self, x, topk_idx, topk_weights, stats, num_experts, num_max_tokens, alignment, num_sms, handle,
                           do_handle_copy, do_cpu_sync, do_expand, col_major_sf, fused_fp8_cast=None,
                           do_zero_padding=False) -> _DispatchState:
-        C = self._C
         x_in, sf_in = x if isinstance(x, tuple) else (x, None)
         T, H = x_in.shape
         cached = handle is not None
         idx = handle.topk_idx if cached else topk_idx
         assert idx.dtype in (torch.int64, torch.int32)
         K = idx.shape[1]
-        R, El = self.num_ranks, num_experts // self.num_ranks
         quantize = (self.use_fp8_dispatch if fused_fp8_cast is None else fused_fp8_cast) and x_in.dtype == torch.bfloat16
         assert H * (1 if quantize or x_in.dtype == torch.float8_e4m3fn else 2) <= self.regions.x_row_bytes, \
             'rows are wider than the receive regions: size the buffer with use_fp8_dispatch=False for bf16 rows'
         fp8_out = quantize or x_in.dtype == torch.float8_e4m3fn
         assert H <= self.hidden or self.hidden == 0, 'hidden exceeds what the buffer was sized for'
         assert not do_expand or self.enable_expand, 'construct the buffer with enable_expand=True for the expand layout'
-        dev = x_in.device
-        call = C.DispatchCall()
-        call.x = x_in.contiguous()
-        if sf_in is not None:
-            call.sf = sf_in.contiguous().float() if sf_in.dtype != torch.float32 else sf_in.contiguous()
-        call.topk_idx = idx.contiguous()
-        if topk_weights is not None:
-            call.topk_weights = topk_weights.contiguous()
-        if stats is not None:
-            call.stats = stats
-        if cached:
-            call.lane_src, call.plan = handle.dst_buffer_slot_idx, handle.plan
-            call.psum_rank = handle.psum_num_recv_tokens_per_scaleup_rank
-            call.psum_expert = handle.psum_num_recv_tokens_per_expert
-            call.recv_per_expert = handle.num_unaligned_recv_tokens_per_expert
-        else:
-            call.allocate_handle(T, K, R, El, dev)
-        call.num_experts = num_experts
-        call.expert_alignment = alignment
-        call.num_max_tokens = num_max_tokens
-        call.quantize = quantize
-        call.do_expand = do_expand
-        call.do_zero_padding = bool(do_zero_padding)
-        call.cached = cached
-        call.tune_warps, call.tune_stages = self._tune
         slot_idx = self._next_recv_slot()
-        slot = self.regions.slot(slot_idx)
-        cap = self.regions.capacity_rows
-        call.off_recv_x, call.off_recv_sf, call.off_recv_idx = slot.x, slot.sf, slot.idx
-        call.off_recv_w, call.off_recv_meta = slot.w, slot.meta
-        G = (H + 127) // 128
-        call.sf_stride_row, call.sf_stride_col = (1, cap) if col_major_sf else (G, 1)
-        call.recv_capacity_rows = cap
-        tail = None
-        if not do_expand and not col_major_sf and (not fp8_out or (G * 4) % 16 == 0):
-            # scales travel as one bulk store per row; expert ids (already relative to the receiver), weights and
-            # source ids as one more: the tail record {ids | weights | metadata}
-            off_w = K * idx.element_size()
-            off_meta = align(off_w + K * 4, 8)
-            tail_bytes = align(off_meta + 8, 16)
-            tail_pitch = align(tail_bytes, 128) if self._side_aligned else tail_bytes
-            sf_pitch = align(G * 4, 128) // 4 if self._side_aligned else G
-            assert tail_pitch <= self.regions.tail_bytes and sf_pitch * 4 <= self.regions.sf_row_bytes, \
-                'side records larger than the buffer was sized for'
-            call.side_packed = True
-            call.tail_bytes, call.tail_off_w, call.tail_off_meta, call.tail_pitch = tail_bytes, off_w, off_meta, tail_pitch
-            call.sf_stride_row = sf_pitch
-            call.off_recv_tail = slot.tail
-            tail = (tail_pitch, off_w, off_meta, sf_pitch)
-        if self.profile is not None:
-            call.prof = self.profile['dispatch']
-
         st = _DispatchState()
-        st.call, st.T, st.H, st.K, st.E = call, T, H, K, num_experts
-        st.fp8_out, st.do_expand, st.alignment = fp8_out, do_expand, alignment
-        st.slot_idx, st.slot = slot_idx, slot
-        st.topk_idx, st.topk_weights = idx, topk_weights
-        st.do_cpu_sync, st.num_sms, st.col_major_sf = do_cpu_sync, num_sms, col_major_sf
-        st.cached_handle = handle
-        st.x_dtype = x_in.dtype
-        st.do_handle_copy = do_handle_copy
-        st.side = tail
+        st.call = self.core.make_dispatch_call(
+            self.regions, x_in, sf_in, idx, topk_weights, stats,
+            (handle.dst_buffer_slot_idx, handle.plan, handle.psum_num_recv_tokens_per_scaleup_rank, handle.psum_num_recv_tokens_per_expert,
+             handle.num_unaligned_recv_tokens_per_expert) if cached else None,
+            None if self.profile is None else self.profile['dispatch'], num_experts, alignment, num_max_tokens, quantize, do_expand,
+            bool(do_zero_padding), col_major_sf, self._side_aligned, *self._tune, slot_idx)
+        st.T, st.H, st.K, st.E = T, H, K, num_experts
+        st.fp8_out, st.do_expand, st.alignment, st.num_max_tokens = fp8_out, do_expand, alignment, num_max_tokens
+        st.slot_idx, st.topk_weights = slot_idx, topk_weights
+        st.topk_idx = idx
+        st.do_cpu_sync, st.num_sms = do_cpu_sync, num_sms
+        st.cached_handle, st.do_handle_copy = handle, do_handle_copy
         return st
 
-    def _finish_dispatch(self, st: _DispatchState):
-        core, cap = self.core, self.regions.capacity_rows
-        R, El = self.num_ranks, st.E // self.num_ranks
-        K, H = st.K, st.H
-        per_expert_list = None
-        if st.cached_handle is not None:
-            num_recv, num_expanded = st.cached_handle.num_recv_tokens, st.cached_handle.num_expanded_tokens
-            per_expert_list = st.cached_handle.num_recv_tokens_per_expert_list
-        elif st.do_cpu_sync:
-            counts = core.wait_recv_counts(El)
-            num_recv, num_expanded = counts[0], counts[1]
-            A = st.alignment
-            per_expert_list = counts[2:] if A == 1 else [(c + A - 1) // A * A for c in counts[2:]]
-        else:
-            num_recv = min(cap, R * st.call.num_max_tokens)
-            num_expanded = cap if st.do_expand else 0
-        rows = num_expanded if st.do_expand else num_recv
-        G = (H + 127) // 128
-        x_dtype = torch.float8_e4m3fn if st.fp8_out else torch.bfloat16
-        recv_x = core.view(st.slot.x, [rows, H], [H, 1], x_dtype)
-        recv_sf = recv_w = None
-        if st.side is not None:
-            # contiguous scales; strided views over the tail records
-            tail_bytes, off_w, off_meta, sf_pitch = st.side      # tail_bytes: distance of two rows' records
-            if st.fp8_out:
-                recv_sf = core.view(st.slot.sf, [rows, G], [sf_pitch, 1], torch.float32)
-            isz = st.topk_idx.element_size()
-            recv_idx = core.view(st.slot.tail, [rows, K], [tail_bytes // isz, 1], st.topk_idx.dtype)
-            if st.topk_weights is not None:
-                recv_w = core.view(st.slot.tail + off_w, [rows, K], [tail_bytes // 4, 1], torch.float32)
-            meta = core.view(st.slot.tail + off_meta, [rows, 2], [tail_bytes // 4, 1], torch.int32)
-        else:
-            if st.fp8_out:
-                strides = [1, cap] if st.col_major_sf else [G, 1]
-                recv_sf = core.view(st.slot.sf, [rows, G], strides, torch.float32)
-            recv_idx = None if st.do_expand else core.view(st.slot.idx, [rows, K], [K, 1], st.topk_idx.dtype)
-            if st.topk_weights is not None:
-                recv_w = core.view(st.slot.w, [rows], [1], torch.float32) if st.do_expand else \
-                    core.view(st.slot.w, [rows, K], [K, 1], torch.float32)
-            meta = core.view(st.slot.meta, [rows, 2], [2, 1], torch.int32)
+    def _finish_dispatch(self, st: _DispatchState, stream_id: Optional[int] = None):
+        """The results of a launched dispatch: views of its receive slot and the handle (the copy of the ids in it is made on the stream
+        ``stream_id``, by default the current one)."""
+        handle = st.cached_handle
+        known = (-1, -1) if handle is None else (handle.num_recv_tokens, handle.num_expanded_tokens)
+        num_recv, num_expanded, per_expert_list, recv_x, recv_sf, recv_idx, recv_w, meta, idx_copy = self.core.finish_dispatch(
+            st.call, self.regions, *known, handle is None and st.do_cpu_sync, handle is None and st.do_handle_copy, stream_id)
         if not self.zero_copy:
-            recv_x = recv_x.clone()
-            recv_sf = None if recv_sf is None else recv_sf.clone()
-            recv_idx = None if recv_idx is None else recv_idx.clone()
-            recv_w = None if recv_w is None else recv_w.clone()
-            meta = meta.clone()
-        if st.cached_handle is not None:
-            handle = st.cached_handle
+            recv_x, recv_sf, recv_idx, recv_w, meta = self._copies((recv_x, recv_sf, recv_idx, recv_w, meta), stream_id)
+        if handle is not None:
             handle.recv_slot = st.slot_idx
             handle.recv_src_metadata = meta
         else:
-            idx_copy = st.topk_idx.clone() if st.do_handle_copy else st.topk_idx
-            handle = EPHandle(st.do_expand, st.E, st.alignment, st.call.num_max_tokens, st.num_sms, idx_copy, num_recv,
-                              num_expanded, per_expert_list, st.call.psum_rank, st.call.psum_expert,
-                              st.call.recv_per_expert, meta, st.call.lane_src, st.call.plan, H, st.slot_idx,
-                              st.topk_weights, stamp=self._stamp(st.T, K))
+            handle = EPHandle(st.do_expand, st.E, st.alignment, st.num_max_tokens, st.num_sms, st.topk_idx if idx_copy is None else idx_copy,
+                              num_recv, num_expanded, per_expert_list, st.call.psum_rank, st.call.psum_expert,
+                              st.call.recv_per_expert, meta, st.call.lane_src, st.call.plan, st.H, st.slot_idx,
+                              st.topk_weights, stamp=self._stamp(st.T, st.K))
         x_out = (recv_x, recv_sf) if st.fp8_out else recv_x
         return x_out, recv_idx, recv_w, handle
+
+    def _copies(self, tensors, stream_id: Optional[int]):
+        """Copies made on the communication stream (``stream_id``) or, without one, on the current stream."""
+        with on_stream(self.comm_stream) if stream_id is not None else contextlib.nullcontext():
+            return [None if t is None else t.clone() for t in tensors]
 
     # ------------------------------------------------------------------------------------------ combine
     def get_combine_buffer(self, handle: EPHandle, hidden: Optional[int] = None) -> torch.Tensor:
@@ -682,25 +599,26 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
             return self._cpu.combine(self, x, handle, topk_weights, bias0, bias1, weighted)
         num_sms = value_or(num_sms or None, handle.num_sms)
         stream = self.combine_stream
-        cur = current_stream()
         if allocate_on_comm_stream:
-            self._stream_prologue(previous_event, previous_event_before_epilogue, stream, cur)
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
             with on_stream(stream):
                 call, out, out_w, staged = self._prepare_combine(x, handle, topk_weights, bias0, bias1, weighted, out)
         else:
             call, out, out_w, staged = self._prepare_combine(x, handle, topk_weights, bias0, bias1, weighted, out)
-            self._stream_prologue(previous_event, previous_event_before_epilogue, stream, cur)
-        with on_stream(stream):
-            for dst, src in staged:      # plain tensors go through the symmetric buffer
-                dst.copy_(src)
-            self._timed('combine', lambda: self.core.combine(call, num_sms), stream)
+            self._stream_prologue(previous_event, previous_event_before_epilogue, stream)
+        if staged:
+            with on_stream(stream):
+                for dst, src in staged:      # plain tensors go through the symmetric buffer
+                    dst.copy_(src)
+        self._launch('combine', self.core.combine, call, num_sms, stream)
+        if not async_with_compute_stream:
+            self.core.current_waits_for_stream(stream.stream_id)
+            return out, out_w, EventOverlap(None)
         inputs = (x, topk_weights, bias0, bias1, call.bias0, call.bias1, call.mul_weights, handle.plan,
                   handle.dst_buffer_slot_idx)
-        event = self._stream_epilogue(async_with_compute_stream, (out, out_w), inputs, stream, cur)
-        return out, out_w, event
+        return out, out_w, self._async_event((out, out_w), inputs, stream)
 
     def _prepare_combine(self, x, handle: EPHandle, topk_weights, bias0, bias1, weighted, out=None):
-        C = self._C
         H = x.shape[1]
         rows = handle.num_rows
         assert x.dtype == torch.bfloat16 and x.shape[0] >= rows, 'combine input must be bf16 with one row per received row'
@@ -719,82 +637,70 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
             staging = self.core.view(off_x, [rows, H], [H, 1], torch.bfloat16)
             if x.data_ptr() != staging.data_ptr():
                 staged.append((staging, x[:rows]))
-        call = C.CombineCall()
-        call.off_x = off_x
-        call.local_x = local_x
-        call.plan = handle.plan
-        call.lane_src = handle.dst_buffer_slot_idx
-        call.hidden = H
-        call.expanded = handle.do_expand
-        if self.profile is not None:
-            call.prof = self.profile['combine']
         T, K = handle.plan.shape
-        if out is None:
-            out = torch.empty((T, H), dtype=torch.bfloat16, device=x.device)
-        assert out.shape == (T, H) and out.dtype == torch.bfloat16 and out.is_contiguous(), '`out` must be contiguous bf16 [T, H]'
-        call.out = out
-        out_w = None
+        if out is not None:
+            assert out.shape == (T, H) and out.dtype == torch.bfloat16 and out.is_contiguous(), '`out` must be contiguous bf16 [T, H]'
+        w_cols = 0
         if topk_weights is not None:
             w_cols = 1 if handle.do_expand else K
             wview = self.core.view(off_w, [rows, w_cols], [w_cols, 1], torch.float32)
             staged.append((wview, topk_weights[:rows].reshape(rows, w_cols)))
-            out_w = torch.empty((T, K), dtype=torch.float32, device=x.device)
-            call.off_w, call.w_cols, call.out_w = off_w, w_cols, out_w
+        mul_weights = None
         if weighted:
             assert handle.do_expand, 'the fused weighted reduce needs the expand layout (one row per expert hit)'
             assert handle.topk_weights is not None, 'dispatch must have been given topk_weights'
-            call.mul_weights = handle.topk_weights.contiguous()
-        if bias0 is not None:
-            call.bias0 = bias0.contiguous()
-        if bias1 is not None:
-            call.bias1 = bias1.contiguous()
-        return call, out, out_w, staged
+            mul_weights = handle.topk_weights
+        call = self.core.make_combine_call(off_x, local_x, handle.plan, handle.dst_buffer_slot_idx, H, handle.do_expand,
+                                           None if self.profile is None else self.profile['combine'], out, topk_weights is not None, off_w,
+                                           w_cols, mul_weights, bias0, bias1)
+        return call, call.out if out is None else out, call.out_w, staged
 
     # ------------------------------------------------------------------------------------------ streams
-    def _stream_prologue(self, previous_event: Optional[EventHandle], before_epilogue: Optional[EventHandle], stream=None,
-                         cur=None) -> None:
+    def _stream_prologue(self, previous_event: Optional[EventHandle], before_epilogue: Optional[EventHandle], stream=None) -> None:
         """The communication stream waits for ``previous_event`` or for the current stream's work so far, and for
         ``before_epilogue`` (see :meth:`dispatch`)."""
         stream = self.comm_stream if stream is None else stream
         if previous_event is not None and previous_event.event is not None:
             stream.wait_event(previous_event.event)
         else:
-            stream.wait_stream(current_stream() if cur is None else cur)
+            self.core.stream_waits_for_current(stream.stream_id)
         if before_epilogue is not None and before_epilogue.event is not None:
             stream.wait_event(before_epilogue.event)
 
-    def _stream_epilogue(self, async_with_compute_stream: bool, outputs, inputs=(), stream=None, cur=None) -> EventOverlap:
-        """Either hand back an event on the communication stream (async) or make the current stream wait.
+    def _stream_epilogue(self, async_with_compute_stream: bool, outputs, inputs=(), stream=None) -> EventOverlap:
+        """Either hand back an event on the communication stream (async) or make the current stream wait."""
+        stream = self.comm_stream if stream is None else stream
+        if async_with_compute_stream:
+            return self._async_event(outputs, inputs, stream)
+        self.core.current_waits_for_stream(stream.stream_id)
+        return EventOverlap(None)
 
-        In the async case the caching allocator must not hand a block to someone else while the other stream still
+    def _async_event(self, outputs, inputs, stream) -> EventOverlap:
+        """An event on the communication stream.  The caching allocator must not hand a block to someone else while the other stream still
         uses it: every tensor involved (inputs read by the kernel, handle tensors, outputs; the handle is walked
         too) is recorded on both streams, or, with ``EP_AVOID_RECORD_STREAM=1``, kept alive by the returned event
         instead (csrc/elastic/buffer.hpp:558-586, 1151-1164 of the reference)."""
-        stream = self.comm_stream if stream is None else stream
-        cur = current_stream() if cur is None else cur
-        if async_with_compute_stream:
-            flat: List[torch.Tensor] = []
+        cur = current_stream()
+        flat: List[torch.Tensor] = []
 
-            def walk(o):
-                if isinstance(o, torch.Tensor):
-                    flat.append(o)
-                elif isinstance(o, (tuple, list)):
-                    for i in o:
-                        walk(i)
-                elif isinstance(o, EPHandle):
-                    for v in vars(o).values():
-                        if isinstance(v, torch.Tensor):
-                            flat.append(v)
-            walk(outputs)
-            walk(inputs)
-            if os.environ.get('EP_AVOID_RECORD_STREAM', '0') != '1':
-                for t in flat:
-                    if t.is_cuda:
-                        t.record_stream(cur)
-                        t.record_stream(stream)
-            return EventOverlap(EventHandle(stream, tuple(flat)))
-        cur.wait_stream(stream)
-        return EventOverlap(None)
+        def walk(o):
+            if isinstance(o, torch.Tensor):
+                flat.append(o)
+            elif isinstance(o, (tuple, list)):
+                for i in o:
+                    walk(i)
+            elif isinstance(o, EPHandle):
+                for v in vars(o).values():
+                    if isinstance(v, torch.Tensor):
+                        flat.append(v)
+        walk(outputs)
+        walk(inputs)
+        if os.environ.get('EP_AVOID_RECORD_STREAM', '0') != '1':
+            for t in flat:
+                if t.is_cuda:
+                    t.record_stream(cur)
+                    t.record_stream(stream)
+        return EventOverlap(EventHandle(stream, tuple(flat)))
 
     def capture(self) -> EventHandle:
         """An event on the current stream, usable as ``previous_event``."""
@@ -807,14 +713,13 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         Read the pairs with :meth:`kernel_times_ms`."""
         self._kernel_timing = {'dispatch': [], 'combine': []} if enabled else None
 
-    def _timed(self, name: str, launch, stream=None) -> None:
+    def _launch(self, name: str, launch, call, num_sms: int, stream) -> None:
         if self._kernel_timing is None:
-            launch()
+            launch(call, num_sms, stream.stream_id)
             return
-        stream = self.comm_stream if stream is None else stream
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(stream)
-        launch()
+        launch(call, num_sms, stream.stream_id)
         e1.record(stream)
         self._kernel_timing[name].append((e0, e1))
 

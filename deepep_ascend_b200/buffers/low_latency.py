@@ -13,7 +13,6 @@ import torch
 
 from ..utils.event import EventHandle, EventOverlap
 from ..utils.math import align
-from ..utils.streams import current_stream, on_stream
 
 
 class LowLatencyMixin:
@@ -48,6 +47,7 @@ class LowLatencyMixin:
             'mask': torch.zeros(self.num_ranks, dtype=torch.int32, device='cuda'),
             'c_bytes': c_bytes, 'calls': 0,
         }
+        self._ll['dispatch_regions'] = (*self._ll['dispatch'], msg)
         return self._ll
 
     def _ll_num_sms(self, num_sms: int) -> int:
@@ -58,42 +58,13 @@ class LowLatencyMixin:
         return self._ll_device_sms if self._virtual is None else 8
 
     # ------------------------------------------------------------------------------------------ dispatch
-    def _ll_prepare_dispatch(self, x, topk_idx, M, E, cumulative_stats, wait_stats, use_fp8, round_scale, use_ue8m0, phases):
-        C = self._C
-        T, H = x.shape
-        K = topk_idx.shape[1]
-        ll = self._ll_setup(M, H, E, K)
-        R, El = self.num_ranks, E // self.num_ranks
-        dev = x.device
-        G = (H + 127) // 128
-        call = C.LLDispatchCall()
-        call.x, call.topk_idx = x.contiguous(), topk_idx.contiguous()
-        call.num_experts, call.num_max_tokens = E, M
-        call.use_fp8, call.round_scale, call.use_ue8m0 = use_fp8, round_scale or use_ue8m0, use_ue8m0
-        call.phases = phases
-        call.off_slab0, call.off_slab1 = ll['dispatch'][0], ll['dispatch'][1]
-        call.msg_bytes = ll['msg']
-        call.packed_x = torch.empty((El, R * M, H), dtype=torch.float8_e4m3fn if use_fp8 else torch.bfloat16, device=dev)
-        sf_view = None
-        if use_fp8:
-            if use_ue8m0:
-                store = torch.zeros((El, (G + 3) // 4, R * M), dtype=torch.int32, device=dev)
-            else:
-                store = torch.empty((El, G, R * M), dtype=torch.float32, device=dev)
-            call.packed_sf = store
-            sf_view = store.transpose(1, 2)      # [E_local, R*M, G(/4)], column-major in the last two dims
-        call.packed_src_info = torch.empty((El, R * M), dtype=torch.int32, device=dev)
-        call.layout_range = torch.empty((El, R), dtype=torch.int64, device=dev)
-        call.packed_count = torch.empty((El,), dtype=torch.int32, device=dev)
-        if cumulative_stats is not None:
-            call.stats = cumulative_stats
-        if wait_stats is not None:
-            call.wait_stats = wait_stats
-        if self.profile is not None:
-            call.prof = self.profile['ll_dispatch']
-        call.mask = ll['mask']
-        call.shrink = self.low_latency_shrink
-        return call, sf_view
+    def _ll_prepare_dispatch(self, x, topk_idx, M, E, cumulative_stats, wait_stats, use_fp8, round_scale, use_ue8m0, phases, stream_id=None):
+        ll = self._ll_setup(M, x.shape[1], E, topk_idx.shape[1])
+        call = self._C.make_ll_dispatch_call(
+            self.core, x, topk_idx, E, M, use_fp8, round_scale, use_ue8m0, phases, ll['dispatch_regions'], cumulative_stats, wait_stats,
+            None if self.profile is None else self.profile['ll_dispatch'], ll['mask'], self.low_latency_shrink, stream_id)
+        # [E_local, R*M, G(/4)], column-major in the last two dims
+        return call, call.packed_sf.transpose(1, 2) if use_fp8 else None
 
     def low_latency_dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, num_max_dispatch_tokens_per_rank: int,
                              num_experts: int, cumulative_local_expert_recv_stats: Optional[torch.Tensor] = None,
@@ -115,50 +86,35 @@ class LowLatencyMixin:
                                                        use_ue8m0)
         C = self._C
         num_sms = self._ll_num_sms(num_sms)
-        cur = current_stream()
-        stream = cur if return_recv_hook else self.comm_stream
-        if not return_recv_hook:
-            stream.wait_stream(cur)
+        # with a hook both halves run on the caller's stream
+        stream = None if return_recv_hook else self.comm_stream
+        stream_id = None if stream is None else stream.stream_id
+        if stream is not None:
+            self.core.stream_waits_for_current(stream_id)
         phases = 1 if return_recv_hook else 3
-        with on_stream(stream):
-            call, sf_view = self._ll_prepare_dispatch(x, topk_idx, M, E, cumulative_local_expert_recv_stats,
-                                                      dispatch_wait_recv_cost_stats, use_fp8, round_scale, use_ue8m0, phases)
-            C.ll_dispatch_group([self.core], [call], num_sms)
+        call, sf_view = self._ll_prepare_dispatch(x, topk_idx, M, E, cumulative_local_expert_recv_stats, dispatch_wait_recv_cost_stats,
+                                                  use_fp8, round_scale, use_ue8m0, phases, stream_id)
+        C.ll_dispatch(self.core, call, num_sms, stream_id)
         handle = (call.packed_src_info, call.layout_range, M, x.shape[1], E)
         recv_x = (call.packed_x, sf_view) if use_fp8 else call.packed_x
         event, hook = EventOverlap(None), None
         if return_recv_hook:
             def hook():
                 call.phases = 2
-                C.ll_dispatch_group([self.core], [call], num_sms)
+                C.ll_dispatch(self.core, call, num_sms)
         elif async_finish:
             event = EventOverlap(EventHandle(stream, (call.packed_x,)))
         else:
-            cur.wait_stream(stream)
+            self.core.current_waits_for_stream(stream_id)
         return recv_x, call.packed_count, handle, event, hook
 
     # ------------------------------------------------------------------------------------------ combine
-    def _ll_prepare_combine(self, x, topk_idx, topk_weights, handle, out, wait_stats, phases, use_logfmt=False):
-        C = self._C
+    def _ll_prepare_combine(self, x, topk_idx, topk_weights, handle, out, wait_stats, phases, use_logfmt=False, stream_id=None):
         src_info, layout_range, M, H, E = handle
-        K = topk_idx.shape[1]
-        ll = self._ll_setup(M, H, E, K)
-        call = C.LLCombineCall()
-        call.x = x
-        call.topk_idx, call.topk_weights = topk_idx.contiguous(), topk_weights.contiguous()
-        call.src_info, call.layout_range = src_info, layout_range
-        call.out = out if out is not None else torch.empty((topk_idx.shape[0], H), dtype=torch.bfloat16, device=x.device)
-        call.num_experts, call.num_max_tokens = E, M
-        call.phases = phases
-        call.off_slab0, call.off_slab1 = ll['combine'][0], ll['combine'][1]
-        if wait_stats is not None:
-            call.wait_stats = wait_stats
-        if self.profile is not None:
-            call.prof = self.profile['ll_combine']
-        call.mask = ll['mask']
-        call.shrink = self.low_latency_shrink
-        call.use_logfmt = bool(use_logfmt)
-        return call
+        ll = self._ll_setup(M, H, E, topk_idx.shape[1])
+        return self._C.make_ll_combine_call(
+            self.core, x, topk_idx, topk_weights, src_info, layout_range, H, E, M, phases, ll['combine'], out, wait_stats,
+            None if self.profile is None else self.profile['ll_combine'], ll['mask'], self.low_latency_shrink, bool(use_logfmt), stream_id)
 
     def low_latency_combine(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor, handle: tuple,
                             use_logfmt: bool = False, zero_copy: bool = False, async_finish: bool = False,
@@ -177,24 +133,23 @@ class LowLatencyMixin:
             return self._cpu_coll.low_latency_combine(x, topk_idx, topk_weights, handle, use_logfmt, out)
         C = self._C
         num_sms = self._ll_num_sms(num_sms)
-        cur = current_stream()
-        stream = cur if return_recv_hook else self.comm_stream
-        if not return_recv_hook:
-            stream.wait_stream(cur)
-        with on_stream(stream):
-            call = self._ll_prepare_combine(x, topk_idx, topk_weights, handle, out, combine_wait_recv_cost_stats,
-                                            1 if return_recv_hook else 3, use_logfmt)
-            C.ll_combine_group([self.core], [call], num_sms)
+        stream = None if return_recv_hook else self.comm_stream
+        stream_id = None if stream is None else stream.stream_id
+        if stream is not None:
+            self.core.stream_waits_for_current(stream_id)
+        call = self._ll_prepare_combine(x, topk_idx, topk_weights, handle, out, combine_wait_recv_cost_stats,
+                                        1 if return_recv_hook else 3, use_logfmt, stream_id)
+        C.ll_combine(self.core, call, num_sms, stream_id)
         event, hook = EventOverlap(None), None
         if return_recv_hook:
             def hook():
                 call.phases = 2
-                C.ll_combine_group([self.core], [call], num_sms)
+                C.ll_combine(self.core, call, num_sms)
         elif async_finish:
             event = EventOverlap(EventHandle(stream, (call.out,)))
         else:
-            cur.wait_stream(stream)
-        return call.out, event, hook
+            self.core.current_waits_for_stream(stream_id)
+        return call.out if out is None else out, event, hook
 
     def get_next_low_latency_combine_buffer(self, handle: tuple) -> torch.Tensor:
         """The bf16 ``[E_local, ranks * max_tokens, H]`` tensor that the expert outputs of the next combine should be

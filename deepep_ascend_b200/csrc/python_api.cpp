@@ -720,16 +720,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("psum_rank", &DispatchCall::psum_rank)
         .def_readwrite("psum_expert", &DispatchCall::psum_expert)
         .def_readwrite("recv_per_expert", &DispatchCall::recv_per_expert)
-        .def("allocate_handle",
-             [](DispatchCall& c, int64_t T, int64_t K, int64_t R, int64_t El, const at::Device& device) {
-                 // the int32 tensors that a fresh dispatch writes and its handle keeps
-                 const auto i32 = at::TensorOptions().dtype(at::kInt).device(device);
-                 c.lane_src = at::empty({T, K}, i32);
-                 c.plan = at::empty({T, K}, i32);
-                 c.psum_rank = at::empty({R}, i32);
-                 c.psum_expert = at::empty({El}, i32);
-                 c.recv_per_expert = at::empty({El}, i32);
-             })
         .def_readwrite("num_experts", &DispatchCall::num_experts)
         .def_readwrite("expert_alignment", &DispatchCall::expert_alignment)
         .def_readwrite("num_max_tokens", &DispatchCall::num_max_tokens)
@@ -801,8 +791,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("read_status", &ElasticBufferCore::read_status)
         .def("check_status", &ElasticBufferCore::check_status)
         .def("wait_recv_counts", &ElasticBufferCore::wait_recv_counts)
-        .def("dispatch", &ElasticBufferCore::dispatch)
-        .def("combine", &ElasticBufferCore::combine)
+        .def("stream_waits_for_current", &ElasticBufferCore::stream_waits_for_current)
+        .def("current_waits_for_stream", &ElasticBufferCore::current_waits_for_stream)
+        .def("make_dispatch_call", &ElasticBufferCore::make_dispatch_call)
+        .def("finish_dispatch", &ElasticBufferCore::finish_dispatch)
+        .def("make_combine_call", &ElasticBufferCore::make_combine_call)
+        .def("dispatch", &ElasticBufferCore::dispatch, py::arg("call"), py::arg("num_sms"), py::arg("stream") = py::none())
+        .def("combine", &ElasticBufferCore::combine, py::arg("call"), py::arg("num_sms"), py::arg("stream") = py::none())
         .def("barrier", &ElasticBufferCore::barrier, py::arg("channel") = static_cast<int>(EP_CH_BARRIER))
         .def("peer_copy", &ElasticBufferCore::peer_copy)
         .def("signal_and_wait_memops", &ElasticBufferCore::signal_and_wait_memops)
@@ -854,6 +849,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("mask", &LLCombineCall::mask)
         .def_readwrite("shrink", &LLCombineCall::shrink)
         .def_readwrite("use_logfmt", &LLCombineCall::use_logfmt);
+    m.def("make_ll_dispatch_call", &make_ll_dispatch_call);
+    m.def("make_ll_combine_call", &make_ll_combine_call);
+    m.def("ll_dispatch", &ll_dispatch, py::arg("core"), py::arg("call"), py::arg("num_sms"), py::arg("stream") = py::none());
+    m.def("ll_combine", &ll_combine, py::arg("core"), py::arg("call"), py::arg("num_sms"), py::arg("stream") = py::none());
     m.def("ll_dispatch_group", &ll_dispatch_group);
     m.def("ll_combine_group", &ll_combine_group);
     m.def("ll_message_bytes", &ll_message_bytes);

@@ -8,9 +8,11 @@
 // Parity: csrc/elastic/buffer.hpp:19-1346 (deep_ep::elastic::ElasticBuffer).
 #pragma once
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <chrono>
 #include <memory>
 #include <optional>
@@ -25,6 +27,43 @@
 namespace ep_host {
 
 using OptTensor = std::optional<at::Tensor>;
+
+using StreamId = std::optional<int64_t>;      // `torch.cuda.Stream.stream_id` of a stream on the buffer's device; none: the current stream
+
+inline c10::cuda::CUDAStream cuda_stream(int64_t id, int device) {
+    return c10::cuda::CUDAStream(c10::cuda::CUDAStream::UNCHECKED,
+                                 c10::Stream(c10::Stream::UNSAFE, c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)), id));
+}
+// The stream made current for one native call.
+class OnStream {
+public:
+    OnStream(const StreamId& id, int device) {
+        if (id.has_value()) guard_.reset_stream(cuda_stream(*id, device).unwrap());
+    }
+
+private:
+    c10::cuda::OptionalCUDAStreamGuard guard_;
+};
+// `waiter` waits for the work `other` has been given so far (`torch.cuda.Stream.wait_stream`).  The event between the two lives as long as
+// the calling thread, one per device: recording it again does not move a wait that has been queued, and no other thread can come
+// between this thread's record and its wait.
+inline void stream_waits(const c10::cuda::CUDAStream& waiter, const c10::cuda::CUDAStream& other) {
+    struct Events {
+        cudaEvent_t of_device[64] = {};
+        ~Events() {
+            for (cudaEvent_t e : of_device)
+                if (e != nullptr) cudaEventDestroy(e);
+        }
+    };
+    thread_local Events events;
+    const int device = other.device_index();
+    TORCH_CHECK(device >= 0 && device < 64, "device index beyond 63");
+    cudaEvent_t& event = events.of_device[device];
+    const c10::cuda::CUDAGuard on_device(other.device_index());
+    if (event == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+    C10_CUDA_CHECK(cudaEventRecord(event, other.stream()));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(waiter.stream(), event, 0));
+}
 
 // the kernels read and write rows 16 bytes at a time and with bulk copies: anything else is a fault on the device
 inline bool vector_aligned(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
@@ -52,6 +91,7 @@ struct DispatchCall {
     int64_t tail_pitch = 0;       // 0 = tail_bytes
     bool do_zero_padding = false;
     int64_t tune_warps = 0, tune_stages = 0;
+    int64_t slot = 0;             // receive slot
 };
 
 struct CombineCall {
@@ -98,6 +138,7 @@ public:
 
     int rank() const { return mem_->rank(); }
     int num_ranks() const { return mem_->num_ranks(); }
+    int device() const { return mem_->device(); }
     int64_t num_bytes() const { return mem_->bytes(); }
     std::string state() const { return to_string(coord_.state()); }
     uint64_t generation() const { return coord_.generation(); }
@@ -170,9 +211,160 @@ public:
         return out;
     }
 
+    // ------------------------------------------------------------------ streams
+    void stream_waits_for_current(int64_t stream) const { stream_waits(cuda_stream(stream, mem_->device()), c10::cuda::getCurrentCUDAStream()); }
+    void current_waits_for_stream(int64_t stream) const { stream_waits(c10::cuda::getCurrentCUDAStream(), cuda_stream(stream, mem_->device())); }
+
+    // ------------------------------------------------------------------ a dispatch: make the call, launch it, present its results
+    // `handle`: {lane_src, plan, psum_rank, psum_expert, recv_per_expert} of a cached layout
+    DispatchCall make_dispatch_call(const RegionLayout& regions, const at::Tensor& x, const OptTensor& sf, const at::Tensor& idx,
+                                    const OptTensor& weights, const OptTensor& stats, const std::optional<std::vector<at::Tensor>>& handle,
+                                    const OptTensor& prof, int64_t num_experts, int64_t alignment, int64_t num_max_tokens, bool quantize,
+                                    bool do_expand, bool do_zero_padding, bool col_major_sf, bool side_aligned, int64_t tune_warps,
+                                    int64_t tune_stages, int64_t slot_idx) const {
+        TORCH_CHECK(x.dim() == 2 && idx.dim() == 2, "x must be [T, H] and topk_idx [T, K]");
+        TORCH_CHECK(slot_idx >= 0 && slot_idx < regions.num_recv_slots, "slot index out of range");
+        const int64_t H = x.size(1), T = x.size(0), K = idx.size(1), G = (H + 127) / 128, cap = regions.capacity_rows;
+        const bool fp8_out = quantize || x.scalar_type() == at::kFloat8_e4m3fn;
+        DispatchCall c;
+        c.x = x.contiguous();
+        if (sf.has_value()) c.sf = sf->to(at::kFloat).contiguous();
+        c.topk_idx = idx.contiguous();
+        if (weights.has_value()) c.topk_weights = weights->contiguous();
+        c.stats = stats;
+        c.prof = prof;
+        c.cached = handle.has_value();
+        if (c.cached) {
+            TORCH_CHECK(handle->size() == 5, "a cached layout has five tensors");
+            c.lane_src = (*handle)[0];
+            c.plan = (*handle)[1];
+            c.psum_rank = (*handle)[2];
+            c.psum_expert = (*handle)[3];
+            c.recv_per_expert = (*handle)[4];
+        } else {
+            const auto i32 = x.options().dtype(at::kInt).requires_grad(false);
+            const int64_t R = mem_->num_ranks(), El = num_experts / R;
+            c.lane_src = at::empty({T, K}, i32);
+            c.plan = at::empty({T, K}, i32);
+            c.psum_rank = at::empty({R}, i32);
+            c.psum_expert = at::empty({El}, i32);
+            c.recv_per_expert = at::empty({El}, i32);
+        }
+        c.num_experts = num_experts;
+        c.expert_alignment = alignment;
+        c.num_max_tokens = num_max_tokens;
+        c.quantize = quantize;
+        c.do_expand = do_expand;
+        c.do_zero_padding = do_zero_padding;
+        c.tune_warps = tune_warps;
+        c.tune_stages = tune_stages;
+        c.slot = slot_idx;
+        const RecvSlot& slot = regions.slots[slot_idx];
+        c.off_recv_x = slot.x;
+        c.off_recv_sf = slot.sf;
+        c.off_recv_idx = slot.idx;
+        c.off_recv_w = slot.w;
+        c.off_recv_meta = slot.meta;
+        c.sf_stride_row = col_major_sf ? 1 : G;
+        c.sf_stride_col = col_major_sf ? cap : 1;
+        c.recv_capacity_rows = cap;
+        if (!do_expand && !col_major_sf && (!fp8_out || (G * 4) % 16 == 0)) {
+            // scales travel as one bulk store per row; expert ids (already relative to the receiver), weights and
+            // source ids as one more: the tail record {ids | weights | metadata}
+            c.side_packed = true;
+            c.tail_off_w = K * idx.element_size();
+            c.tail_off_meta = align_up(c.tail_off_w + K * 4, 8);
+            c.tail_bytes = align_up(c.tail_off_meta + 8, 16);
+            c.tail_pitch = side_aligned ? align_up(c.tail_bytes, 128) : c.tail_bytes;
+            c.sf_stride_row = side_aligned ? align_up(G * 4, 128) / 4 : G;
+            TORCH_CHECK(c.tail_pitch <= regions.tail_bytes && c.sf_stride_row * 4 <= regions.sf_row_bytes,
+                        "side records larger than the buffer was sized for");
+            c.off_recv_tail = slot.tail;
+        }
+        return c;
+    }
+
+    // -> (rows received, rows expanded, rows per expert as a list or None, recv_x, recv_sf, recv_idx, recv_w, metadata, copy of the ids).
+    // `do_cpu_sync` waits for the counts; otherwise `num_recv` / `num_expanded` are known (cached layout) or -1 (worst case).
+    // The copy of the ids is made on `stream`.
+    py::tuple finish_dispatch(const DispatchCall& c, const RegionLayout& regions, int64_t num_recv, int64_t num_expanded, bool do_cpu_sync,
+                              bool copy_idx, const StreamId& stream) {
+        const int64_t R = mem_->num_ranks(), El = c.num_experts / R, K = c.plan.size(1), H = c.x.size(1), G = (H + 127) / 128;
+        const int64_t cap = c.recv_capacity_rows;
+        py::object per_expert = py::none();
+        if (do_cpu_sync) {
+            const std::vector<int64_t> counts = wait_recv_counts(El);
+            num_recv = counts[0];
+            num_expanded = counts[1];
+            py::list list(El);
+            const int64_t A = c.expert_alignment;
+            for (int64_t j = 0; j < El; ++j) list[j] = A == 1 ? counts[2 + j] : (counts[2 + j] + A - 1) / A * A;
+            per_expert = std::move(list);
+        } else if (num_recv < 0) {
+            num_recv = std::min(cap, R * c.num_max_tokens);
+            num_expanded = c.do_expand ? cap : 0;
+        }
+        const int64_t rows = c.do_expand ? num_expanded : num_recv;
+        const bool fp8_out = c.quantize || c.x.scalar_type() == at::kFloat8_e4m3fn;
+        const at::ScalarType id_type = c.topk_idx->scalar_type();
+        const RecvSlot& slot = regions.slots[c.slot];
+        OptTensor recv_sf, recv_idx, recv_w, idx_copy;
+        at::Tensor meta;
+        const at::Tensor recv_x = view(slot.x, {rows, H}, {H, 1}, fp8_out ? at::kFloat8_e4m3fn : at::kBFloat16);
+        if (fp8_out) recv_sf = view(slot.sf, {rows, G}, {c.sf_stride_row, c.sf_stride_col}, at::kFloat);
+        if (c.side_packed) {
+            // strided views over the tail records
+            const int64_t id_size = c.topk_idx->element_size();
+            recv_idx = view(slot.tail, {rows, K}, {c.tail_pitch / id_size, 1}, id_type);
+            if (c.topk_weights.has_value()) recv_w = view(slot.tail + c.tail_off_w, {rows, K}, {c.tail_pitch / 4, 1}, at::kFloat);
+            meta = view(slot.tail + c.tail_off_meta, {rows, 2}, {c.tail_pitch / 4, 1}, at::kInt);
+        } else {
+            if (!c.do_expand) recv_idx = view(slot.idx, {rows, K}, {K, 1}, id_type);
+            if (c.topk_weights.has_value())
+                recv_w = c.do_expand ? view(slot.w, {rows}, {1}, at::kFloat) : view(slot.w, {rows, K}, {K, 1}, at::kFloat);
+            meta = view(slot.meta, {rows, 2}, {2, 1}, at::kInt);
+        }
+        if (copy_idx) {
+            const OnStream on(stream, mem_->device());
+            idx_copy = c.topk_idx->clone();
+        }
+        return py::make_tuple(num_recv, num_expanded, per_expert, recv_x, recv_sf, recv_idx, recv_w, meta, idx_copy);
+    }
+
+    // `out`: where the result goes, or none for a new tensor; `carry_w`: [T, K] weights travel back from the region at off_w
+    CombineCall make_combine_call(int64_t off_x, const OptTensor& local_x, const at::Tensor& plan, const at::Tensor& lane_src, int64_t hidden,
+                                  bool expanded, const OptTensor& prof, const OptTensor& out, bool carry_w, int64_t off_w, int64_t w_cols,
+                                  const OptTensor& mul_weights, const OptTensor& bias0, const OptTensor& bias1) const {
+        CombineCall c;
+        c.off_x = off_x;
+        c.local_x = local_x;
+        c.plan = plan;
+        c.lane_src = lane_src;
+        c.hidden = hidden;
+        c.expanded = expanded;
+        c.prof = prof;
+        const auto options = plan.options();
+        c.out = out.has_value() ? *out : at::empty({plan.size(0), hidden}, options.dtype(at::kBFloat16));
+        if (carry_w) {
+            c.off_w = off_w;
+            c.w_cols = w_cols;
+            c.out_w = at::empty({plan.size(0), plan.size(1)}, options.dtype(at::kFloat));
+        }
+        if (mul_weights.has_value()) c.mul_weights = mul_weights->contiguous();
+        if (bias0.has_value()) c.bias0 = bias0->contiguous();
+        if (bias1.has_value()) c.bias1 = bias1->contiguous();
+        return c;
+    }
+
     // ------------------------------------------------------------------ operations
-    void dispatch(const DispatchCall& call, int num_sms) { dispatch_group({this}, {call}, num_sms); }
-    void combine(const CombineCall& call, int num_sms) { combine_group({this}, {call}, num_sms); }
+    void dispatch(const DispatchCall& call, int num_sms, const StreamId& stream) {
+        const OnStream on(stream, mem_->device());
+        dispatch_group({this}, {call}, num_sms);
+    }
+    void combine(const CombineCall& call, int num_sms, const StreamId& stream) {
+        const OnStream on(stream, mem_->device());
+        combine_group({this}, {call}, num_sms);
+    }
     void barrier(int channel) { barrier_group({this}, channel); }
     void wait_flag_test(int64_t expected) { wait_flag_test_group({this}, expected); }
 

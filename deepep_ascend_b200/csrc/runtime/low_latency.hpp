@@ -2,6 +2,8 @@
 // Parity: the low-latency methods of csrc/legacy/buffer.hpp:1431-1748 and the buffer layout of
 // csrc/legacy/config.hpp:122-188.
 #pragma once
+#include <array>
+
 #include "elastic_buffer.hpp"
 
 namespace ep_host {
@@ -151,6 +153,66 @@ inline LLCombineArgs make_ll_combine_args(ElasticBufferCore& core, const LLCombi
     return a;
 }
 
+// The call and its result tensors, allocated with `stream` current; `regions`: {slab 0, slab 1, message bytes}
+inline LLDispatchCall make_ll_dispatch_call(ElasticBufferCore& core, const at::Tensor& x, const at::Tensor& topk_idx, int64_t num_experts,
+                                            int64_t num_max_tokens, bool use_fp8, bool round_scale, bool use_ue8m0, int64_t phases,
+                                            const std::array<int64_t, 3>& regions, const OptTensor& stats, const OptTensor& wait_stats,
+                                            const OptTensor& prof, const OptTensor& mask, bool shrink, const StreamId& stream) {
+    TORCH_CHECK(x.dim() == 2, "x must be [T, H]");
+    const OnStream on(stream, core.device());
+    const int64_t R = core.num_ranks(), El = num_experts / R, rows = R * num_max_tokens, H = x.size(1), G = (H + 127) / 128;
+    const auto options = x.options().requires_grad(false);
+    LLDispatchCall c;
+    c.x = x.contiguous();
+    c.topk_idx = topk_idx.contiguous();
+    c.num_experts = num_experts;
+    c.num_max_tokens = num_max_tokens;
+    c.use_fp8 = use_fp8;
+    c.round_scale = round_scale || use_ue8m0;
+    c.use_ue8m0 = use_ue8m0;
+    c.phases = phases;
+    c.off_slab0 = regions[0];
+    c.off_slab1 = regions[1];
+    c.msg_bytes = regions[2];
+    c.packed_x = at::empty({El, rows, H}, options.dtype(use_fp8 ? at::kFloat8_e4m3fn : at::kBFloat16));
+    if (use_fp8) c.packed_sf = use_ue8m0 ? at::zeros({El, (G + 3) / 4, rows}, options.dtype(at::kInt)) : at::empty({El, G, rows}, options.dtype(at::kFloat));
+    c.packed_src_info = at::empty({El, rows}, options.dtype(at::kInt));
+    c.layout_range = at::empty({El, R}, options.dtype(at::kLong));
+    c.packed_count = at::empty({El}, options.dtype(at::kInt));
+    c.stats = stats;
+    c.wait_stats = wait_stats;
+    c.prof = prof;
+    c.mask = mask;
+    c.shrink = shrink;
+    return c;
+}
+
+inline LLCombineCall make_ll_combine_call(ElasticBufferCore& core, const at::Tensor& x, const at::Tensor& topk_idx, const at::Tensor& topk_weights,
+                                          const at::Tensor& src_info, const at::Tensor& layout_range, int64_t hidden, int64_t num_experts,
+                                          int64_t num_max_tokens, int64_t phases, const std::array<int64_t, 2>& regions, const OptTensor& out,
+                                          const OptTensor& wait_stats, const OptTensor& prof, const OptTensor& mask, bool shrink, bool use_logfmt,
+                                          const StreamId& stream) {
+    const OnStream on(stream, core.device());
+    LLCombineCall c;
+    c.x = x;
+    c.topk_idx = topk_idx.contiguous();
+    c.topk_weights = topk_weights.contiguous();
+    c.src_info = src_info;
+    c.layout_range = layout_range;
+    c.out = out.has_value() ? *out : at::empty({topk_idx.size(0), hidden}, x.options().dtype(at::kBFloat16).requires_grad(false));
+    c.num_experts = num_experts;
+    c.num_max_tokens = num_max_tokens;
+    c.phases = phases;
+    c.off_slab0 = regions[0];
+    c.off_slab1 = regions[1];
+    c.wait_stats = wait_stats;
+    c.prof = prof;
+    c.mask = mask;
+    c.shrink = shrink;
+    c.use_logfmt = use_logfmt;
+    return c;
+}
+
 inline void ll_dispatch_group(const std::vector<ElasticBufferCore*>& group, const std::vector<LLDispatchCall>& calls, int num_sms) {
     TORCH_CHECK(group.size() == calls.size() && !group.empty(), "one call per buffer is required");
     std::vector<std::unique_ptr<OperationScope>> scopes;
@@ -177,6 +239,15 @@ inline void ll_combine_group(const std::vector<ElasticBufferCore*>& group, const
     cuda_check(ep::launch_ll_combine(args.data(), static_cast<int>(args.size()), num_sms, at::cuda::getCurrentCUDAStream()),
                "low-latency combine launch");
     for (auto& s : scopes) s->commit();
+}
+
+inline void ll_dispatch(ElasticBufferCore& core, const LLDispatchCall& call, int num_sms, const StreamId& stream) {
+    const OnStream on(stream, core.device());
+    ll_dispatch_group({&core}, {call}, num_sms);
+}
+inline void ll_combine(ElasticBufferCore& core, const LLCombineCall& call, int num_sms, const StreamId& stream) {
+    const OnStream on(stream, core.device());
+    ll_combine_group({&core}, {call}, num_sms);
 }
 
 }  // namespace ep_host

@@ -94,3 +94,41 @@ def test_combine_of_one_rank_is_the_sum_of_one_row(T, H, sms):
             assert torch.equal(out_w[idx >= 0], w[idx >= 0])
     finally:
         buf.destroy()
+
+
+def test_threads_with_streams_of_their_own():
+    """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
+    import threading
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K, n = 64, 1024, 16, 4, 3
+    errors = []
+    gate = threading.Barrier(n)
+
+    def work(i):
+        try:
+            torch.cuda.set_device(0)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+                idx, w = _routing(T, E, K, i)
+                sent = (idx >= 0).any(1)
+                x = torch.zeros(T, H, dtype=torch.bfloat16, device='cuda')
+                torch.cuda.current_stream().synchronize()
+                gate.wait()
+                for step in range(40):
+                    x.fill_(100 * i + step)              # the dispatch has to wait for this, and this for the combine before it
+                    y, _, _, handle, _ = buf.dispatch(x, idx, w, num_experts=E)
+                    out, _, _ = buf.combine(y, handle)
+                    if not bool((out == torch.where(sent, 100 * i + step, 0)[:, None]).all()):
+                        errors.append((i, step))
+                torch.cuda.current_stream().synchronize()
+                buf.destroy()
+        except Exception as e:                           # noqa: BLE001 (reported by the main thread)
+            gate.abort()
+            errors.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:5]
