@@ -13,13 +13,14 @@
 //                    CTAs: every row is bulk-copied into the slot [source token][top-k lane] of the token's home
 //                    rank; the last CTA to finish raises one epoch-tagged flag per rank pair.
 //            RECV  - wait for all ranks' flags, then out[t] = sum_k w[t,k] * slot[t,k] in fp32 -> bf16.
-// With one rank (both halves in one launch) nothing has to travel: dispatch stores a message's payload, scales and source straight at
-// the packed position, which is the claimed slot, and combine leaves row numbers in the slots and reduces the rows where they lie.
+// With one rank (both halves in one launch) nothing has to travel, and kernels of their own place and reduce the rows directly.
 // No CTA waits for another CTA of its own rank (no grid barrier): phases end with an arrival counter whose last
 // arriver does the publishing.
 // SEND and RECV can be launched separately (phases argument) so that no SM is held while data is in flight.
 //
 // Parity: csrc/kernels/legacy/internode_ll.cu:128-554 (dispatch) and 714-1238 (combine) of the reference.
+#include <algorithm>
+
 #include "common.cuh"
 #include "logfmt.cuh"
 
@@ -117,19 +118,19 @@ __device__ __forceinline__ bool shrink_wait(const RankCtx& ctx, Workspace* ws, c
     return true;
 }
 
-// the G scales of one packed row (local expert j, row `at` of `rows` per expert), stored by one warp; get(group) -> fp32 scale
+// scales [g0, g1) of the G of one packed row (local expert j, row `at` of `rows` per expert), stored by one warp; get(group) -> fp32 scale
 template <typename Get>
-__device__ __forceinline__ void ll_store_scales(const LLDispatchArgs& a, int j, int G, int64_t rows, int64_t at, Get get) {
+__device__ __forceinline__ void ll_store_scales(const LLDispatchArgs& a, int j, int g0, int g1, int G, int64_t rows, int64_t at, Get get) {
     const int lane = threadIdx.x & 31;
     if (a.use_ue8m0) {
         // four exponents per int32, groups along the slow axis: [E_local, ceil(G/4), R*M]
         uint8_t* dst = reinterpret_cast<uint8_t*>(a.packed_sf);
         const int64_t G4 = (G + 3) / 4;
-        for (int gi = lane; gi < G; gi += 32)
+        for (int gi = g0 + lane; gi < g1; gi += 32)
             dst[((static_cast<int64_t>(j) * G4 + gi / 4) * rows + at) * 4 + (gi & 3)] = static_cast<uint8_t>(__float_as_uint(get(gi)) >> 23);
     } else {
         float* dst = reinterpret_cast<float*>(a.packed_sf);
-        for (int gi = lane; gi < G; gi += 32) dst[(static_cast<int64_t>(j) * G + gi) * rows + at] = get(gi);
+        for (int gi = g0 + lane; gi < g1; gi += 32) dst[(static_cast<int64_t>(j) * G + gi) * rows + at] = get(gi);
     }
 }
 
@@ -194,26 +195,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
             }
             ptx::fence_proxy_async_smem();
             __syncthreads();
-            if (a.direct_rows && warp < K) {
-                // one rank: the claimed slot IS the packed position, so payload, scales and source go there at once
-                const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
-                if (e >= 0 && e < E && !rank_masked(a.mask, 0)) {
-                    uint32_t slot = 0;
-                    if (lane == 0) slot = atomicAdd(&slot_counter[e], 1u);
-                    slot = __shfl_sync(0xffffffffu, slot, 0);
-                    if (slot < static_cast<uint32_t>(M)) {
-                        const int64_t pos = static_cast<int64_t>(e) * M + slot;
-                        if (lane == 0) {
-                            ptx::bulk_store(reinterpret_cast<uint8_t*>(a.packed_x) + pos * payload, msg + 16, payload);
-                            a.packed_src_info[pos] = (warp << 20) | t;
-                        }
-                        if (a.use_fp8) ll_store_scales(a, e, G, M, slot, [&](int gi) { return reinterpret_cast<const float*>(msg + 16 + H)[gi]; });
-                    } else if (lane == 0) {
-                        report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
-                    }
-                }
-                ptx::bulk_commit();
-            } else if (!a.direct_rows && warp < K && lane == 0) {
+            if (warp < K && lane == 0) {
                 const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
                 if (e >= 0 && e < E && !rank_masked(a.mask, e / El)) {
                     const uint32_t slot = atomicAdd(&slot_counter[e], 1u);
@@ -300,7 +282,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
                 }
             }
             const uint32_t pieces = (payload + 2047) / 2048;
-            const uint32_t items = a.direct_rows ? 0u : s_pref[P] * pieces;
+            const uint32_t items = s_pref[P] * pieces;
             for (uint32_t u = blockIdx.x * kLLWarps + warp; u < items; u += gridDim.x * kLLWarps) {
                 const uint32_t g = u / pieces, c = u - g * pieces;
                 const int p = find_segment(s_pref, P, g);
@@ -325,7 +307,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
                 }
                 if (a.use_fp8 && c == pieces - 1) {
                     const float* sf = reinterpret_cast<const float*>(m + 16 + H);
-                    ll_store_scales(a, j, G, rows_per_expert, begin + i, [&](int gi) { return __ldcg(sf + gi); });
+                    ll_store_scales(a, j, 0, G, G, rows_per_expert, begin + i, [&](int gi) { return __ldcg(sf + gi); });
                 }
             }
         }
@@ -400,20 +382,9 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
             }
             return pos;
         };
-        bool indexed = false;
-        if (a.direct_rows) {
-            // one rank: the slot of a (token, lane) gets the row's number instead of the row, one thread each
-            for (uint32_t r = blockIdx.x * blockDim.x + tid; r < total && alive; r += gridDim.x * blockDim.x) {
-                const int p = find_segment(s_pref, P, r);
-                const int64_t at = static_cast<int64_t>(p) * M + s_begin[p] + (r - s_pref[p]);
-                const int info = a.src_info[at];
-                *reinterpret_cast<int*>(s_peer[me] + a.off_slab[set] + (static_cast<int64_t>(info & 0xfffff) * K + (info >> 20)) * row_bytes) = static_cast<int>(at);
-                indexed = true;
-            }
-        }
         uint32_t g = blockIdx.x * send_warps + warp;
         int64_t pos = 0;
-        const bool stage_rows = warp < send_warps && !a.direct_rows;
+        const bool stage_rows = warp < send_warps;
         if (stage_rows && g < total && alive) pos = issue_load(g, 0);
         for (; stage_rows && g < total && alive; g += g_stride) {
             const int s = next_src;
@@ -447,7 +418,7 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
         stamp(1);
         ptx::bulk_wait<0>();
         // only lanes that have stored to a peer have something to make visible
-        if ((n_loaded > 0 && lane == 0) || indexed) __threadfence_system();
+        if (n_loaded > 0 && lane == 0) __threadfence_system();
         stamp(2);
         // the last CTA of this rank to finish its stores raises this rank's flag at every peer (no grid barrier)
         if (arrive_is_last(&ws->arrive[EP_CH_LL_COMBINE][0]) && !is_aborted(ws)) {
@@ -561,19 +532,11 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
                 }
                 const uint32_t srcs = __ballot_sync(0xffffffffu, e_k >= 0 && e_k < E);
                 const uint8_t* rows = slab + static_cast<int64_t>(t) * K * row_bytes + off;
-                // direct rows: the slots hold row numbers (of this call; anything else is kept inside x)
-                int my_row = 0;
-                if (a.direct_rows && lane < K && ((srcs >> lane) & 1u)) {
-                    my_row = __ldcg(reinterpret_cast<const int*>(slab + (static_cast<int64_t>(t) * K + lane) * row_bytes));
-                    if (static_cast<uint32_t>(my_row) >= static_cast<uint32_t>(E) * M) my_row = 0;
-                }
                 int4 raw[EP_MAX_TOPK];
 #pragma unroll
                 for (int k = 0; k < EP_MAX_TOPK; ++k)
                     if (k < K && ((srcs >> k) & 1u)) {
-                        const int64_t at = __shfl_sync(0xffffffffu, my_row, k);
-                        const uint8_t* src = a.direct_rows ? reinterpret_cast<const uint8_t*>(a.x) + at * row_bytes + off : rows + static_cast<int64_t>(k) * row_bytes;
-                        if (in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(src));
+                        if (in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(rows + static_cast<int64_t>(k) * row_bytes));
                     }
                 float acc[8];
 #pragma unroll
@@ -608,6 +571,197 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
             if (a.prof != nullptr) a.prof[6] = globaltimer_ns();
         }
     }
+}
+
+// ------------------------------------------------------------------------------------------------ one rank
+// With one rank and both halves in one launch a row's packed position can be computed, so no CTA has to hear from another one: no
+// slot claims, counts, flags or arrivals, and a plain launch.  Both kernels are chains of a few dependent memory accesses; the
+// protocol they replace added two arrivals of all CTAs and a flag to each.  40 tokens x 7168, top-8 of 256, bf16: 17 -> 4.3 us and
+// 15 -> 4.8 us; 128 tokens, top-8 of 32: 20 (with the cast) -> 6.5 us and 27 -> 8.9 us.
+
+// Dispatch: the row of (token, lane) in its expert's segment is the number of selections of that expert before it, counted in a copy of
+// all ids in shared memory, so rows are in token order, the same on every run.  A unit is a column part of a token (several parts
+// when there are more CTAs than tokens).
+constexpr int kLLDirectIds = 8192;
+__device__ __forceinline__ int count_ids(const int16_t* ids, int end, int e) {      // ids[0, end) equal to e, by one warp
+    int n = 0;
+#pragma unroll 8
+    for (int i = threadIdx.x & 31; i < end; i += 32) n += ids[i] == e ? 1 : 0;
+    return __reduce_add_sync(0xffffffffu, n);
+}
+__global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const __grid_constant__ LLDispatchArgs a, const int parts) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const RankCtx& ctx = a.ctx;
+    Workspace* ws = local_ws(ctx);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int E = a.num_experts, K = a.num_topk, H = a.hidden, M = a.num_max_tokens, T = a.num_tokens, G = (H + 127) / 128;
+    const int payload = a.use_fp8 ? H : 2 * H, units = T * parts;
+    const int part_channels = ((H + 255) / 256 + parts - 1) / parts * 256;
+    const uint8_t* xb = reinterpret_cast<const uint8_t*>(a.x);
+    int16_t* s_ids = reinterpret_cast<int16_t*>(smem);
+    float* s_sf = reinterpret_cast<float*>(smem + (T * K * 2 + 15) / 16 * 16);
+    uint8_t* s_row = reinterpret_cast<uint8_t*>(s_sf) + (G * 4 + 15) / 16 * 16;
+    if (is_aborted(ws)) return;
+    auto stamp = [&](int i) {
+        if (a.prof != nullptr && blockIdx.x == 0 && tid == 0) a.prof[i] = globaltimer_ns();
+    };
+    stamp(0);
+    if (tid == 0 && static_cast<int>(blockIdx.x) < units) {
+        // the first unit's channels start on their way beside the ids
+        const int t = blockIdx.x / parts, c0 = (blockIdx.x - t * parts) * part_channels;
+        if (c0 < H) ptx::bulk_prefetch_l2(xb + (static_cast<int64_t>(t) * H + c0) * 2, min(part_channels, H - c0) * 2);
+    }
+    const bool masked = rank_masked(a.mask, 0);
+    for (int i = tid; i < T * K; i += kLLThreads) {
+        const int e = masked ? -1 : ll_load_idx(a.topk_idx, a.idx_is_64, i);
+        s_ids[i] = static_cast<int16_t>(e >= 0 && e < E ? e : -1);
+    }
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const int t = u / parts, part = u - t * parts, c0 = part * part_channels, c1 = min(H, c0 + part_channels);
+        if (c0 >= H) continue;                            // uniform: a row of fewer parts
+        ptx::bulk_wait_read<0>();                         // the row in shared memory was the source of the stores of the unit before
+        __syncthreads();
+        const uint8_t* src = xb + static_cast<int64_t>(t) * H * 2;
+        if (a.use_fp8) {
+            for (int ch0 = c0 + warp * 256; ch0 < c1; ch0 += kLLWarps * 256) {
+                const int ch = ch0 + lane * 8;
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = 0.f;
+                if (ch < c1) {
+                    const int4 raw = ptx::ld_nc_v4(src + ch * 2);
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = __bfloat1622float2(h[j]);
+                        v[2 * j] = f.x;
+                        v[2 * j + 1] = f.y;
+                    }
+                }
+                float sf;
+                const uint2 q = cast_8(v, a.round_scale | a.use_ue8m0, sf);
+                if (ch < c1) {
+                    *reinterpret_cast<uint2*>(s_row + ch - c0) = q;
+                    if ((lane & 15) == 0) s_sf[ch / 128] = sf;
+                }
+            }
+        } else {
+            for (int off = tid * 16; off < (c1 - c0) * 2; off += kLLThreads * 16)
+                *reinterpret_cast<int4*>(s_row + off) = ptx::ld_nc_v4(src + c0 * 2 + off);
+        }
+        ptx::fence_proxy_async_smem();
+        __syncthreads();
+        for (int k = warp; k < K; k += kLLWarps) {
+            const int e = s_ids[t * K + k];
+            if (e < 0) continue;
+            const int slot = count_ids(s_ids, t * K + k, e);
+            if (slot >= M) {
+                if (lane == 0) report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
+                continue;
+            }
+            const int64_t pos = static_cast<int64_t>(e) * M + slot;
+            if (lane == 0) {
+                const int bytes_per = a.use_fp8 ? 1 : 2;
+                ptx::bulk_store(reinterpret_cast<uint8_t*>(a.packed_x) + pos * payload + c0 * bytes_per, s_row, (c1 - c0) * bytes_per);
+                if (part == 0) a.packed_src_info[pos] = (k << 20) | t;
+            }
+            if (a.use_fp8) ll_store_scales(a, e, c0 / 128, (c1 + 127) / 128, G, M, slot, [&](int gi) { return s_sf[gi]; });
+        }
+        ptx::bulk_commit();
+    }
+    __syncthreads();                                      // the ids, also in a CTA without a unit
+    stamp(1);
+    for (int e = blockIdx.x + warp * gridDim.x; e < E; e += gridDim.x * kLLWarps) {
+        const int n = min(count_ids(s_ids, T * K, e), M);
+        if (lane == 0) {
+            a.packed_count[e] = n;
+            a.layout_range[e] = n;
+            if (a.stats != nullptr) a.stats[e] += n;
+        }
+    }
+    ptx::bulk_wait<0>();
+    for (int i = 2; i < 7; ++i) stamp(i);
+}
+
+// Combine: the rows of a token are found by their source marks among the rows of the experts it selected, then summed in top-k lane
+// order as everywhere.  A unit is a column part of a token.
+__global__ void __launch_bounds__(kLLThreads, 1) ll_combine_direct_kernel(const __grid_constant__ LLCombineArgs a, const int parts) {
+    __shared__ int s_row[EP_MAX_TOPK];
+    __shared__ float s_w[EP_MAX_TOPK];
+    const RankCtx& ctx = a.ctx;
+    Workspace* ws = local_ws(ctx);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int E = a.num_experts, K = a.num_topk, M = a.num_max_tokens, T = a.num_tokens, row_bytes = 2 * a.hidden;
+    constexpr int kChunk = 32 * 16;
+    const int part_bytes = ((row_bytes + kChunk - 1) / kChunk + parts - 1) / parts * kChunk;
+    if (is_aborted(ws)) return;
+    auto stamp = [&](int i) {
+        if (a.prof != nullptr && blockIdx.x == 0 && tid == 0) a.prof[i] = globaltimer_ns();
+    };
+    stamp(0);
+    const bool masked = rank_masked(a.mask, 0);
+    for (int u = blockIdx.x; u < T * parts; u += gridDim.x) {
+        const int t = u / parts, c0 = (u - t * parts) * part_bytes, c1 = min(row_bytes, c0 + part_bytes);
+        if (c0 >= row_bytes) continue;                    // uniform: a row of fewer parts
+        __syncthreads();                                  // the row numbers of the unit before have been used
+        for (int k = warp; k < K; k += kLLWarps) {
+            const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + k);
+            int found = -1;
+            if (!masked && e >= 0 && e < E) {
+                const int n = min(static_cast<int>(__ldg(a.layout_range + e) & 0xffffffffll), M);
+                const int32_t* info = a.src_info + static_cast<int64_t>(e) * M;
+                const int mark = (k << 20) | t;
+                for (int i0 = 0; i0 < n && found < 0; i0 += 128) {
+                    int at = -1;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int i = i0 + j * 32 + lane;
+                        if (i < n && __ldg(info + i) == mark) at = i;
+                    }
+                    found = __reduce_max_sync(0xffffffffu, at);
+                }
+                if (found >= 0) found += e * M;
+            }
+            if (lane == 0) {
+                s_row[k] = found;
+                s_w[k] = __ldg(a.topk_weights + static_cast<int64_t>(t) * K + k);
+            }
+        }
+        __syncthreads();
+        for (int c = c0 + warp * kChunk; c < c1; c += kLLWarps * kChunk) {
+            const int off = c + lane * 16;
+            if (off >= c1) continue;
+            int4 raw[EP_MAX_TOPK];
+#pragma unroll
+            for (int k = 0; k < EP_MAX_TOPK; ++k)
+                if (k < K && s_row[k] >= 0) raw[k] = __ldcg(reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.x) + static_cast<int64_t>(s_row[k]) * row_bytes + off));
+            float acc[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll
+            for (int k = 0; k < EP_MAX_TOPK; ++k)
+                if (k < K && s_row[k] >= 0) {
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 f = __bfloat1622float2(h[q]);
+                        acc[2 * q] = fmaf(s_w[k], f.x, acc[2 * q]);
+                        acc[2 * q + 1] = fmaf(s_w[k], f.y, acc[2 * q + 1]);
+                    }
+                }
+            int4 outv;
+            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&outv);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
+            *reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(t) * row_bytes + off) = outv;
+        }
+    }
+    for (int i = 1; i < 7; ++i) stamp(i);
+}
+
+// column parts of a token's row: as many as give every CTA work, each of `steps_per_part` steps at least
+inline int ll_direct_parts(int ctas, int tokens, int steps, int steps_per_part) {
+    return std::max(1, std::min(ctas / std::max(1, tokens), steps / steps_per_part));
 }
 
 __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_kernel(const __grid_constant__ LLDispatchArgs a) { ll_dispatch_body(a); }
@@ -651,10 +805,19 @@ cudaError_t launch_ll(const void* single, const void* multi, const Args* args, i
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* args, int n, int num_sms, cudaStream_t stream) {
     const int smem = 2 * args[0].msg_bytes;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (n == 1) {
-        LLDispatchArgs one = args[0];
-        one.direct_rows = one.ctx.num_ranks == 1 && one.phases == (EP_LL_SEND | EP_LL_RECV);
-        return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, &one, n, num_sms, smem, stream);
+    const LLDispatchArgs& a = args[0];
+    const int64_t ids = static_cast<int64_t>(a.num_tokens) * a.num_topk;
+    // Counting the ids costs every CTA a pass over them per selection; with more than 8192 of them the slot claims are cheaper.
+    if (n == 1 && a.ctx.num_ranks == 1 && a.phases == (EP_LL_SEND | EP_LL_RECV) && ids <= kLLDirectIds) {
+        const int ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
+        int parts = ll_direct_parts(ctas, a.num_tokens, (a.hidden + 255) / 256, 4);
+        const int bytes = static_cast<int>((ids * 2 + 15) / 16 * 16) + ((a.hidden + 127) / 128 * 4 + 15) / 16 * 16 + (a.use_fp8 ? a.hidden : 2 * a.hidden);
+        if (bytes <= 200 * 1024) {
+            cudaError_t err = cudaFuncSetAttribute((const void*)ll_dispatch_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (err != cudaSuccess) return err;
+            void* params[] = {const_cast<LLDispatchArgs*>(&a), &parts};
+            return cudaLaunchKernel((const void*)ll_dispatch_direct_kernel, dim3(ctas, 1, 1), dim3(kLLThreads, 1, 1), params, bytes, stream);
+        }
     }
     return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, args, n, num_sms, smem, stream);
 }
@@ -666,11 +829,16 @@ cudaError_t launch_ll_combine(const LLCombineArgs* args, int n, int num_sms, cud
     if (n == 1) {
         // Rows are reduced where they lie if nobody else needs them (one rank), no one may change them in between (both phases in one
         // launch), they are not re-coded, and the output does not overlap them.
-        LLCombineArgs one = args[0];
-        const uint64_t row = static_cast<uint64_t>(one.hidden) * 2, x0 = reinterpret_cast<uint64_t>(one.x), o0 = reinterpret_cast<uint64_t>(one.out);
-        const uint64_t x1 = x0 + row * one.num_experts * one.num_max_tokens, o1 = o0 + row * one.num_tokens;
-        one.direct_rows = one.ctx.num_ranks == 1 && one.phases == (EP_LL_SEND | EP_LL_RECV) && !one.use_logfmt && (x1 <= o0 || o1 <= x0) && x0 % 16 == 0;
-        return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, &one, n, num_sms, smem, stream);
+        const LLCombineArgs& a = args[0];
+        const uint64_t row = static_cast<uint64_t>(a.hidden) * 2, x0 = reinterpret_cast<uint64_t>(a.x), o0 = reinterpret_cast<uint64_t>(a.out);
+        const uint64_t x1 = x0 + row * a.num_experts * a.num_max_tokens, o1 = o0 + row * a.num_tokens;
+        if (a.ctx.num_ranks == 1 && a.phases == (EP_LL_SEND | EP_LL_RECV) && !a.use_logfmt && (x1 <= o0 || o1 <= x0) && x0 % 16 == 0 && row % 16 == 0 &&
+            static_cast<int64_t>(a.num_experts) * a.num_max_tokens < (1ll << 31)) {
+            const int ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
+            int parts = ll_direct_parts(ctas, a.num_tokens, (a.hidden * 2 + 511) / 512, 4);
+            void* params[] = {const_cast<LLCombineArgs*>(&a), &parts};
+            return cudaLaunchKernel((const void*)ll_combine_direct_kernel, dim3(ctas, 1, 1), dim3(kLLThreads, 1, 1), params, 0, stream);
+        }
     }
     return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, args, n, num_sms, smem, stream);
 }

@@ -96,6 +96,57 @@ def test_combine_of_one_rank_is_the_sum_of_one_row(T, H, sms):
         buf.destroy()
 
 
+@pytest.mark.parametrize('T,H,E,K,sms', [(0, 256, 8, 2, 4), (1, 128, 4, 1, 148), (7, 1040, 8, 3, 148), (40, 7168, 256, 8, 0), (128, 2176, 1024, 16, 0),
+                                         (300, 512, 24, 6, 5), (1024, 256, 16, 8, 0), (1100, 256, 16, 8, 0)])
+@pytest.mark.parametrize('use_fp8', [False, True])
+def test_low_latency_rows_of_one_rank(T, H, E, K, sms, use_fp8):
+    """Rows cut into column parts (few tokens), several tokens per CTA, the most ids that are counted (8192) and more (slot claims).  Counted
+    rows are in token order.  The combine in one launch has the bits of the two halves, which go through the slabs."""
+    from deepep_ascend_b200 import ElasticBuffer
+    from deepep_ascend_b200.ops import gemm as G
+    M = T + 2
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=M, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(M, H, 1, E, K) + (1 << 20))
+    try:
+        x = torch.randn(T, H, device='cuda').bfloat16()
+        idx, w = _routing(T, E, K, T) if T else (torch.zeros(0, K, dtype=torch.int64, device='cuda'), torch.zeros(0, K, device='cuda'))
+        stats = torch.zeros(E, dtype=torch.int32, device='cuda')
+        recv, count, handle, _, _ = buf.low_latency_dispatch(x, idx, M, E, stats, use_fp8=use_fp8, num_sms=sms)
+        torch.cuda.synchronize()
+        buf.core.check_status()
+        t, k = (idx >= 0).nonzero(as_tuple=True)
+        e = idx[t, k]
+        want = torch.bincount(e, minlength=E)
+        assert torch.equal(count.long(), want) and torch.equal(stats.long(), want)
+        order = torch.sort(e * (T * K + 1) + t * K + k).indices                      # by expert, then in token order
+        slot = torch.cat([torch.arange(int(n), device='cuda') for n in want]) if e.numel() else e
+        rows, (t, k) = e[order] * M + slot, (t[order], k[order])
+        info = handle[0].view(-1)[rows]
+        if T * K > 8192:                                                              # claimed: any order inside an expert
+            assert torch.equal(torch.sort(info).values, torch.sort((k << 20 | t).int()).values)
+            t, k = info & 0xfffff, info >> 20
+        assert torch.equal(info, (k << 20 | t).int())
+        if use_fp8:
+            q, sf = G.per_token_cast_to_fp8(x) if T else (x.to(torch.float8_e4m3fn), torch.zeros(0, H // 128, device='cuda'))
+            assert torch.equal(recv[0].view(E * M, H)[rows].view(torch.uint8), q[t.long()].view(torch.uint8))
+            assert torch.equal(recv[1].reshape(E * M, -1)[rows], sf[t.long()])
+        else:
+            assert torch.equal(recv.view(E * M, H)[rows], x[t.long()])
+        y = torch.randn(E, M, H, device='cuda').bfloat16()
+        out, _, _ = buf.low_latency_combine(y, idx, w, handle, num_sms=sms)
+        split, _, hook = buf.low_latency_combine(y, idx, w, handle, return_recv_hook=True)
+        hook()
+        torch.cuda.synchronize()
+        buf.core.check_status()
+        assert torch.equal(out, split)
+        exact = torch.zeros(T, H, dtype=torch.float64, device='cuda')
+        exact.index_add_(0, t.long(), w[t.long(), k.long()].double()[:, None] * y.view(E * M, H)[rows].double())
+        # one rounding to bf16 (2^-9 of the result) and up to 16 fp32 sums of terms below 1 * 6
+        assert bool(((out.double() - exact).abs() <= exact.abs() * 2.0**-8 + 16 * 6 * 2.0**-23).all())
+    finally:
+        buf.destroy()
+
+
 def test_threads_with_streams_of_their_own():
     """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
     import threading
