@@ -379,17 +379,29 @@ template <int kUnroll, bool kFull>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32, 1) combine_kernel_multi(const CombineArgs* args) {
     combine_body<kUnroll, kFull>(args[blockIdx.y]);
 }
-template <int kUnroll, bool kFull>
-const void* combine_fn(int n) {
-    return n == 1 ? (const void*)combine_kernel<kUnroll, kFull> : (const void*)combine_kernel_multi<kUnroll, kFull>;
+template <int kUnroll>
+const void* combine_fn(bool full, int n) {
+    if (full) return n == 1 ? (const void*)combine_kernel<kUnroll, true> : (const void*)combine_kernel_multi<kUnroll, true>;
+    return n == 1 ? (const void*)combine_kernel<kUnroll, false> : (const void*)combine_kernel_multi<kUnroll, false>;
+}
+const void* combine_fn(int unroll, bool full, int n) {
+    switch (unroll) {
+        case 8: return combine_fn<8>(full, n);
+        case 7: return combine_fn<7>(full, n);
+        case 6: return combine_fn<6>(full, n);
+        case 5: return combine_fn<5>(full, n);
+        case 4: return combine_fn<4>(full, n);
+        case 2: return combine_fn<2>(full, n);
+        default: return combine_fn<1>(full, n);
+    }
 }
 
-// column chunk = 512 B x unroll: larger chunks amortise the per-chunk bookkeeping: 3584 B when the row divides evenly
-// (hidden 7168), else 2048 B
+// Column chunk = 512 B x unroll.  A warp's chain per chunk (about 1.5 us whatever the chunk's size) is what bounds the kernel, so a row is
+// cut into as few chunks of at most 4 KB as it takes, all alike: 3001 tokens x 4096, six rows each, 64 SMs: 47 us in chunks of 2 KB,
+// 31 us in chunks of 4 KB (the sums of a 4 KB chunk take 64 of the 128 registers).
 inline int pick_unroll(const CombineArgs& a) {
-    const int row_bytes = a.hidden * 2;
-    if (row_bytes % 3584 == 0) return 7;
-    return row_bytes % 2048 == 0 ? 4 : (row_bytes % 1024 == 0 ? 2 : (row_bytes >= 2048 ? 4 : 1));
+    const int steps = (a.hidden * 2 + 511) / 512, chunks = (steps + 7) / 8, unroll = (steps + chunks - 1) / chunks;
+    return unroll == 3 ? 4 : unroll;
 }
 
 }  // namespace
@@ -417,10 +429,7 @@ cudaError_t launch_combine(const CombineArgs* args, int n, int num_sms, cudaStre
     if (shape.smem_bytes > 227 * 1024) return cudaErrorInvalidValue;
     const int unroll = pick_unroll(a0);
     const bool full = a0.hidden * 2 % (512 * unroll) == 0;
-    const void* fn = unroll == 7   ? combine_fn<7, true>(n)
-                     : unroll == 4 ? (full ? combine_fn<4, true>(n) : combine_fn<4, false>(n))
-                     : unroll == 2 ? combine_fn<2, true>(n)
-                                   : (full ? combine_fn<1, true>(n) : combine_fn<1, false>(n));
+    const void* fn = combine_fn(unroll, full, n);
     cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, shape.smem_bytes);
     if (err != cudaSuccess) return err;
     dim3 grid(shape.num_ctas, n, 1), block(shape.num_warps * 32, 1, 1);

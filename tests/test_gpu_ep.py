@@ -58,6 +58,13 @@ def test_dispatch_combine_line_aligned_side_records(R, T, H, E, K, mode):
     _run_dispatch_combine(R, T, H, E, K, mode, False, aligned=True)
 
 
+@pytest.mark.parametrize('H', [240, 256, 272, 768, 1040, 1280, 1536, 1792, 2048, 2064, 2304, 2432, 2560, 3584, 4096, 4112, 5120, 6144, 8192])
+@pytest.mark.parametrize('do_expand', [False, True])
+def test_combine_in_chunks_of_every_width(H, do_expand):
+    """Rows of one to four chunks of 512 to 4096 bytes, whole and with a short last one."""
+    _run_dispatch_combine(2, 37, H, 8, 3, 'bf16', do_expand)
+
+
 def _run_dispatch_combine(R, T, H, E, K, mode, do_expand, aligned=False):
     from deepep_ascend_b200.backends.emulated import EmulatedWorld
     from deepep_ascend_b200.utils import refs
