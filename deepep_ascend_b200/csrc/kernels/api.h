@@ -259,6 +259,12 @@ cudaError_t launch_engram_fetch(const EngramFetchArgs* args, int n, int num_sms,
 cudaError_t launch_reduce_slots(const ReduceSlotsArgs& args, cudaStream_t stream);
 }  // namespace ep
 
+// ------------------------------------------------------------------------------------------------ dependent launches
+namespace ep {
+// Launch of a kernel that calls wait_for_previous_kernel() before it touches global memory: it is set up while the kernel before it drains.
+cudaError_t launch_dependent(const void* fn, dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t stream);
+}  // namespace ep
+
 // ------------------------------------------------------------------------------------------------ tcgen05 GEMM
 // C[M, N] (bf16) = A[M, K] * B[g][N, K]^T, both operands K-major.  bf16 inputs, or e4m3 inputs with fp32 block
 // scales (A: one per row and 128 channels; B: one per 128 x 128 block).  With `tile_group` the M dimension is

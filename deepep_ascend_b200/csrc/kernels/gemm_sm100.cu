@@ -168,11 +168,11 @@ __device__ __forceinline__ TileWork tile_work(const GemmArgs& g, int tile, int n
     w.n = tc.n;
     if (g.k_group_off != nullptr) {
         w.grp = 0;
-        w.kb0 = __ldg(g.k_group_off + e) / block_k;
-        w.kb1 = __ldg(g.k_group_off + e + 1) / block_k;
+        w.kb0 = *(g.k_group_off + e) / block_k;
+        w.kb1 = *(g.k_group_off + e + 1) / block_k;
         w.c_row0 = static_cast<int64_t>(e) * g.M;
     } else {
-        w.grp = g.tile_group != nullptr ? __ldg(g.tile_group + tc.m) : 0;
+        w.grp = g.tile_group != nullptr ? *(g.tile_group + tc.m) : 0;
         w.kb0 = 0;
         w.kb1 = num_k;
         w.c_row0 = 0;
@@ -216,6 +216,13 @@ struct PipeState {
         }
     }
 };
+
+// Products of few waves overlap their launch with the kernel before, and let the next one start early: barriers, tensor memory and the
+// launch itself, about 2 us per kernel, are ready when the inputs are.  A layer of 64 tokens (32 experts, 3.5 and 6 waves) takes 367 us
+// instead of 375, one of 128 tokens through the low-latency pair 343 instead of 347.  Above 8 waves the gain is gone, and with
+// CTAs of the next kernel waiting beside the last wave it is a loss: 8192 x 7168 x 7168 (14 waves) 692 us against 686, the layer of
+// 4096 tokens 2223 against 2190.  Launches that wait for peers (fused ones) never let another one start beside them.
+__host__ __device__ constexpr bool few_waves(int num_tiles, int ctas) { return num_tiles <= 8 * ctas; }
 
 // kMnOperands: how many operands are MN-major (bf16 only).  0: A [M, K], B [N, K].  1: B is [K, N] (data gradients read the forward
 // weights as they are).  2: A is [K, M] too (weight gradients read row-major activations and gradients as they are).
@@ -291,6 +298,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     __syncthreads();
     umma::fence_after_thread_sync();
     const uint32_t tmem_base = sm->tmem_base;
+    ptx::wait_for_previous_kernel();
+    if (g.fuse == EP_GEMM_FUSE_NONE && few_waves(num_tiles, gemm_ctas)) ptx::let_next_kernel_start();
 
     if (warp < kEpiWarp0) {
         // ---------------------------------------------------------------------- producer warps
@@ -335,7 +344,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     // A thin tile (few tokens of an expert) is loaded in boxes of 32 rows: the SM's loads in flight are what bounds a
                     // product that streams the weights, and a full box takes a third of them.  The other rows of the stage keep
                     // what they held; their products are not stored.
-                    const int a_boxes = kWide && g.tile_rows != nullptr ? min(4, max(1, (__ldg(g.tile_rows + m_blk) + 31) / 32)) : 4;
+                    const int a_boxes = kWide && g.tile_rows != nullptr ? min(4, max(1, (*(g.tile_rows + m_blk) + 31) / 32)) : 4;
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
                         ok = wait_bar<kWide>(&sm->empty[p.stage], p.phase ^ 1, sm, g, 1);
                         if (!ok) break;
@@ -545,15 +554,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     const uint32_t taddr0 = tmem_base + lane_addr + col_half * kCols;
                     // The scales of the next block are requested a whole block ahead and multiplied only when they are used: a product formed
                     // at the load waits for it, and with 230 KB of shared memory taken, L1 keeps few of the scale lines.
-                    float sa = __ldg(sfa), sb = __ldg(sfb);
+                    float sa = *sfa, sb = *sfb;
 #pragma unroll 1
                     for (int kb = 0; kb < num_k; ++kb) {
                         const float scale = sa * sb;
                         const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale), __float_as_uint(scale));
                         if (kb + 1 < num_k) {
                             sfa += g.sfa_stride_kb;
-                            sa = __ldg(sfa);
-                            sb = __ldg(++sfb);
+                            sa = *sfa;
+                            sb = *++sfb;
                         }
                         ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                         ok = __all_sync(0xffffffffu, ok);
@@ -585,7 +594,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     }
                     if (ok) {
                         const TileWork out = item_work(tile);
-                        const int rows_end = g.tile_rows != nullptr ? min(g.M, out.m * kBlockM + __ldg(g.tile_rows + out.m)) : g.M;
+                        const int rows_end = g.tile_rows != nullptr ? min(g.M, out.m * kBlockM + *(g.tile_rows + out.m)) : g.M;
 #pragma unroll
                         for (int c = 0; c < kCols / 64; ++c) {
                             uint32_t w[32];
@@ -610,11 +619,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     // the B scale block of this warp's columns (a half tile never straddles two 128-column blocks)
                     const int nb_sf = min((n0 + col_half * kCols) / 128, num_nb_sf - 1);
                     const float* sfb = g.sfb + (static_cast<int64_t>(grp) * num_nb_sf + nb_sf) * num_kb_sf;
-                    float scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row) : 0.f) * __ldg(sfb);
+                    float scale_next = (row < g.M ? *(g.sfa + row * g.sfa_stride_row) : 0.f) * *sfb;
                     for (int kb = 0; kb < num_k && ok; ++kb) {
                         const uint64_t scale2 = umma::pack_f32x2(__float_as_uint(scale_next), __float_as_uint(scale_next));
                         if (kb + 1 < num_k)
-                            scale_next = (row < g.M ? __ldg(g.sfa + row * g.sfa_stride_row + (kb + 1) * g.sfa_stride_kb) : 0.f) * __ldg(sfb + kb + 1);
+                            scale_next = (row < g.M ? *(g.sfa + row * g.sfa_stride_row + (kb + 1) * g.sfa_stride_kb) : 0.f) * *(sfb + kb + 1);
                         ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
@@ -910,7 +919,9 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     }
     // whole tiles, or halves where all of them fit into one wave (the kernel cuts its last wave by the same rule)
     if (ctas > num_tiles) ctas = g.is_fp8 && block_n == 256 && 2 * num_tiles <= ctas ? 2 * num_tiles : num_tiles;
-    return cudaLaunchKernel(fn, dim3(ctas, 1, 1), dim3(gemm_threads(g.is_fp8 != 0, block_n), 1, 1), params, kGemmSmemBytes, stream);
+    const dim3 block(gemm_threads(g.is_fp8 != 0, block_n), 1, 1);
+    if (few_waves(num_tiles, ctas)) return launch_dependent(fn, dim3(ctas, 1, 1), block, params, kGemmSmemBytes, stream);
+    return cudaLaunchKernel(fn, dim3(ctas, 1, 1), block, params, kGemmSmemBytes, stream);
 }
 
 }  // namespace ep

@@ -6,6 +6,22 @@
 
 namespace ep {
 
+cudaError_t launch_dependent(const void* fn, dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t stream) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    const cudaError_t err = cudaLaunchKernelExC(&config, fn, params);
+    if (err != cudaSuccess) cudaGetLastError();   // the caller reports it
+    return err;
+}
+
 namespace {
 
 __device__ __forceinline__ void barrier_body(const RankCtx& ctx, int channel) {

@@ -29,8 +29,8 @@ struct SwigluStep {
 __device__ __forceinline__ SwigluStep swiglu_load(const uint8_t* gate, const uint8_t* up, int elem, int I) {
     SwigluStep s;
     if (elem < I) {
-        s.gate = ptx::ld_nc_v4(gate + elem * 2);
-        s.up = ptx::ld_nc_v4(up + elem * 2);
+        s.gate = ptx::ld_na_v4(gate + elem * 2);
+        s.up = ptx::ld_na_v4(up + elem * 2);
     } else {
         s.gate = s.up = make_int4(0, 0, 0, 0);
     }
@@ -38,6 +38,8 @@ __device__ __forceinline__ SwigluStep swiglu_load(const uint8_t* gate, const uin
 }
 
 __global__ void swiglu_quant_kernel(const SwigluQuantArgs a) {
+    ptx::wait_for_previous_kernel();
+    ptx::let_next_kernel_start();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= a.rows || (a.valid != nullptr && a.valid[row] == 0)) return;
@@ -677,15 +679,18 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_layout_kernel(co
 }
 
 // COPY: one warp per received row (or part of it); every 512-byte piece is read once and written to each expert row of the row.
+// This kernel, the reduction and the forward activation stand between products, so all start early (see few_waves).
 constexpr int kExpandWarps = 8, kMaxExpandTopk = 32;
 __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(const LocalExpandCopyArgs a) {
+    ptx::wait_for_previous_kernel();
+    ptx::let_next_kernel_start();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kExpandWarps + (threadIdx.x >> 5);
     if (row >= a.num_rows) return;
-    const int my_pos = lane < a.num_topk ? __ldg(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
+    const int my_pos = lane < a.num_topk ? *(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
     uint32_t dests = __ballot_sync(0xffffffffu, my_pos >= 0);
     if (dests == 0) return;
-    if (a.w_src != nullptr && my_pos >= 0 && blockIdx.y == 0) a.w_dst[my_pos] = __ldg(a.w_src + static_cast<int64_t>(row) * a.w_pitch + lane);
+    if (a.w_src != nullptr && my_pos >= 0 && blockIdx.y == 0) a.w_dst[my_pos] = *(a.w_src + static_cast<int64_t>(row) * a.w_pitch + lane);
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src) + static_cast<int64_t>(row) * a.src_pitch;
     uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst);
     const int pieces = a.row_bytes / 16;
@@ -694,7 +699,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int p = p0 + j * 32 + lane;
-            v[j] = p < pieces ? ptx::ld_nc_v4(src + p * 16) : make_int4(0, 0, 0, 0);
+            v[j] = p < pieces ? ptx::ld_na_v4(src + p * 16) : make_int4(0, 0, 0, 0);
         }
         for (uint32_t m = dests; m != 0; m &= m - 1) {
             const int64_t to = __shfl_sync(0xffffffffu, my_pos, __ffs(m) - 1);
@@ -710,7 +715,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
         // every lane takes part in the shuffles, also where the last columns leave some without work
         for (int c0 = 0; c0 < a.sf_cols; c0 += 32) {
             const int c = c0 + lane;
-            const float f = c < a.sf_cols ? __ldg(a.sf_src + static_cast<int64_t>(row) * a.sf_stride_row + c * a.sf_stride_col) : 0.f;
+            const float f = c < a.sf_cols ? *(a.sf_src + static_cast<int64_t>(row) * a.sf_stride_row + c * a.sf_stride_col) : 0.f;
             for (uint32_t m = dests; m != 0; m &= m - 1) {
                 const int64_t to = __shfl_sync(0xffffffffu, my_pos, __ffs(m) - 1);
                 if (c < a.sf_cols) a.sf_dst[to * a.sf_cols + c] = f;
@@ -725,11 +730,13 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
 // one, with whole rows, otherwise: it leaves registers for more warps (4096 rows, 530 MB: 96 us against 109 us).
 template <int kAhead>
 __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const LocalReduceArgs a) {
+    ptx::wait_for_previous_kernel();
+    ptx::let_next_kernel_start();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kExpandWarps + (threadIdx.x >> 5);
     if (row >= a.num_rows) return;
-    const int my_pos = lane < a.num_topk ? __ldg(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
-    const float my_w = (a.w != nullptr && my_pos >= 0) ? __ldg(a.w + my_pos) : 1.f;
+    const int my_pos = lane < a.num_topk ? *(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
+    const float my_w = (a.w != nullptr && my_pos >= 0) ? *(a.w + my_pos) : 1.f;
     const uint32_t srcs = __ballot_sync(0xffffffffu, my_pos >= 0);
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src);
     uint8_t* out = reinterpret_cast<uint8_t*>(a.dst) + static_cast<int64_t>(row) * a.cols * 2;
@@ -746,7 +753,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const L
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 const int p = p0 + j * 32 + lane;
-                v[j] = p < pieces ? ptx::ld_nc_v4(src + from * a.cols * 2 + p * 16) : make_int4(0, 0, 0, 0);
+                v[j] = p < pieces ? ptx::ld_na_v4(src + from * a.cols * 2 + p * 16) : make_int4(0, 0, 0, 0);
             }
         };
         auto add = [&](const int4 (&v)[kPer], float w) {
@@ -850,8 +857,9 @@ cudaError_t launch_local_expand_copy(const LocalExpandCopyArgs& a, cudaStream_t 
         reinterpret_cast<uintptr_t>(a.src) % 16 != 0 || reinterpret_cast<uintptr_t>(a.dst) % 16 != 0)
         return cudaErrorInvalidValue;
     const int ctas = (a.num_rows + kExpandWarps - 1) / kExpandWarps;
-    local_expand_copy_kernel<<<dim3(ctas, column_splits(ctas, (a.row_bytes + 2047) / 2048)), kExpandWarps * 32, 0, stream>>>(a);
-    return cudaGetLastError();
+    void* params[] = {const_cast<LocalExpandCopyArgs*>(&a)};
+    return launch_dependent((const void*)local_expand_copy_kernel, dim3(ctas, column_splits(ctas, (a.row_bytes + 2047) / 2048)),
+                            dim3(kExpandWarps * 32), params, 0, stream);
 }
 
 cudaError_t launch_local_reduce(const LocalReduceArgs& a, cudaStream_t stream) {
@@ -861,9 +869,9 @@ cudaError_t launch_local_reduce(const LocalReduceArgs& a, cudaStream_t stream) {
         return cudaErrorInvalidValue;
     const int ctas = (a.num_rows + kExpandWarps - 1) / kExpandWarps;
     const dim3 grid(ctas, column_splits(ctas, (a.cols + 1023) / 1024));
-    if (ctas < kWantedCtas) local_reduce_kernel<2><<<grid, kExpandWarps * 32, 0, stream>>>(a);
-    else local_reduce_kernel<1><<<grid, kExpandWarps * 32, 0, stream>>>(a);
-    return cudaGetLastError();
+    void* params[] = {const_cast<LocalReduceArgs*>(&a)};
+    const void* fn = ctas < kWantedCtas ? (const void*)local_reduce_kernel<2> : (const void*)local_reduce_kernel<1>;
+    return launch_dependent(fn, grid, dim3(kExpandWarps * 32), params, 0, stream);
 }
 
 cudaError_t launch_expert_segments(const ExpertSegmentsArgs& a, cudaStream_t stream) {
@@ -890,8 +898,8 @@ cudaError_t launch_swiglu_quant(const SwigluQuantArgs& a, cudaStream_t stream) {
     SwigluQuantArgs args = a;
     const int per = (steps + column_splits(ctas, steps) - 1) / column_splits(ctas, steps);
     args.col_chunk = per * 256;
-    swiglu_quant_kernel<<<dim3(ctas, (steps + per - 1) / per), warps * 32, 0, stream>>>(args);
-    return cudaGetLastError();
+    void* params[] = {&args};
+    return launch_dependent((const void*)swiglu_quant_kernel, dim3(ctas, (steps + per - 1) / per), dim3(warps * 32), params, 0, stream);
 }
 
 }  // namespace ep

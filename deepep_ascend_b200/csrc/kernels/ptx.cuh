@@ -133,6 +133,14 @@ __device__ __forceinline__ int4 ld_nc_v4(const void* p) {
                  : "l"(p));
     return v;
 }
+__device__ __forceinline__ int4 ld_na_v4(const void* p) {
+    int4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.s32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
 __device__ __forceinline__ void st_na_v4(void* p, const int4& v) {
     asm volatile("st.global.L1::no_allocate.v4.s32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
                  "r"(v.w)
@@ -169,6 +177,13 @@ __device__ __forceinline__ uint32_t max_magnitude2(uint32_t a, uint32_t b) {
     asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(b));
     return out;
 }
+
+// ---------------------------------------------------------------- dependent launches
+// A kernel that launch_dependent() started may begin while the kernel before it in the stream still runs: it must call this before it touches
+// anything an earlier kernel wrote or still reads, and reads it without .nc (__ldg, ld_nc_v4): the memory is written in its own lifetime.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel may be started as soon as SMs are free (it waits by itself)
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- warp helpers
 __device__ __forceinline__ float warp_max_16(float v) {   // max over each aligned group of 16 lanes

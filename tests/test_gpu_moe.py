@@ -481,6 +481,52 @@ def test_thin_tiles_are_read_and_stored_by_rows(counts):
     assert torch.equal(a1.view(torch.uint8)[valid], a.view(torch.uint8)[valid]) and torch.equal(s1[valid], s[valid])
 
 
+@pytest.mark.parametrize('rows,H,I', [(128, 128, 128), (384, 7168, 384), (2048, 1024, 2048)])
+@pytest.mark.parametrize('captured', [False, True])
+def test_kernels_that_start_before_the_one_before_has_ended(rows, H, I, captured):
+    """The same buffers written and read again and again by launches that may overlap (one tile up to several waves, in a stream and
+    in a CUDA graph): every pass gives the bytes that it gives when the host waits after each kernel."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows + I)
+    passes = 12
+    q0, s0 = ops.per_token_cast_to_fp8(torch.randn(passes * rows, H, device='cuda').bfloat16())
+    w1, sw1 = ops.quantize_weight_blocks(torch.randn(1, 2 * I, H, device='cuda').bfloat16() * 0.1)
+    w2, sw2 = ops.quantize_weight_blocks(torch.randn(1, H, I, device='cuda').bfloat16() * 0.1)
+    group = torch.zeros(rows // 128, dtype=torch.int32, device='cuda')
+    pos = torch.randperm(rows, device='cuda').view(rows // 2, 2).to(torch.int32)
+    x = torch.empty(rows, H, dtype=q0.dtype, device='cuda')
+    sf = torch.empty(rows, s0.shape[1], device='cuda')
+    h, y = (torch.empty(rows, n, dtype=torch.bfloat16, device='cuda') for n in (2 * I, H))
+
+    def run(pause):
+        outs = []
+        for i in range(passes):
+            x.view(torch.uint8).copy_(q0[i * rows:(i + 1) * rows].view(torch.uint8))
+            sf.copy_(s0[i * rows:(i + 1) * rows])
+            ops.grouped_gemm_nt(x, w1, group, out=h, sfa=sf, sfb=sw1)
+            pause()
+            a, sa = ops.swiglu_quant(h)
+            pause()
+            ops.grouped_gemm_nt(a, w2, group, out=y, sfa=sa, sfb=sw2)
+            pause()
+            outs.append(ops.local_reduce(pos, y))
+            pause()
+            outs.append(ops.local_expand_copy(pos, outs[-1], rows)[0])
+            pause()
+        return outs
+    want = run(torch.cuda.synchronize)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = run(lambda: None)
+        graph.replay()
+        torch.cuda.synchronize()
+    else:
+        got = run(lambda: None)
+    for g, w in zip(got, want):
+        assert torch.equal(g.view(torch.int16), w.view(torch.int16))
+
+
 @pytest.mark.parametrize('rows,I', [(0, 128), (4, 0), (0, 0)])
 @pytest.mark.parametrize('masked', [False, True])
 def test_swiglu_of_nothing(rows, I, masked):
