@@ -349,7 +349,8 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
     def set_dispatch_tuning(self, num_warps: int = 0, num_stages: int = 0, line_aligned_side: Optional[bool] = None) -> None:
         """Shape of the dispatch kernel: warps per CTA (1..12, each with its own staging ring) and, for the fused
         FP8 cast, staging buffers per warp (2..4; more buffers keep more tokens' stores in flight per warp but
-        leave room for fewer warps).  0 selects the default (12 warps, 2 buffers).  ``line_aligned_side``: place every
+        leave room for fewer warps).  0 selects the default (12 warps, 2 buffers; 20 warps on one rank, whose rows
+        need no staging buffers).  ``line_aligned_side``: place every
         row's scales and tail record on 128-byte boundaries at the receiver (``recv_sf`` and ``recv_topk_idx`` /
         ``recv_topk_weights`` become row-strided views), so that each of these small stores is whole lines on the wire."""
         assert 0 <= num_warps <= 12 and num_stages in (0, 2, 3, 4)
