@@ -601,7 +601,6 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
     int16_t* s_ids = reinterpret_cast<int16_t*>(smem);
     float* s_sf = reinterpret_cast<float*>(smem + (T * K * 2 + 15) / 16 * 16);
     uint8_t* s_row = reinterpret_cast<uint8_t*>(s_sf) + (G * 4 + 15) / 16 * 16;
-    if (is_aborted(ws)) return;
     auto stamp = [&](int i) {
         if (a.prof != nullptr && blockIdx.x == 0 && tid == 0) a.prof[i] = globaltimer_ns();
     };
@@ -616,6 +615,8 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
         const int e = masked ? -1 : ll_load_idx(a.topk_idx, a.idx_is_64, i);
         s_ids[i] = static_cast<int16_t>(e >= 0 && e < E ? e : -1);
     }
+    // The flag can rise at any time, also in this launch, so the CTA leaves as a whole: warps that went alone would leave ids unfilled.
+    if (__syncthreads_or(is_aborted(ws))) return;
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
         const int t = u / parts, part = u - t * parts, c0 = part * part_channels, c1 = min(H, c0 + part_channels);
         if (c0 >= H) continue;                            // uniform: a row of fewer parts
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
         __syncthreads();
         for (int k = warp; k < K; k += kLLWarps) {
             const int e = s_ids[t * K + k];
-            if (e < 0) continue;
+            if (e < 0 || e >= E) continue;
             const int slot = count_ids(s_ids, t * K + k, e);
             if (slot >= M) {
                 if (lane == 0) report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
@@ -694,7 +695,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_combine_direct_kernel(const 
     const int E = a.num_experts, K = a.num_topk, M = a.num_max_tokens, T = a.num_tokens, row_bytes = 2 * a.hidden;
     constexpr int kChunk = 32 * 16;
     const int part_bytes = ((row_bytes + kChunk - 1) / kChunk + parts - 1) / parts * kChunk;
-    if (is_aborted(ws)) return;
+    if (__syncthreads_or(is_aborted(ws))) return;          // all warps or none: they fill the row numbers together
     auto stamp = [&](int i) {
         if (a.prof != nullptr && blockIdx.x == 0 && tid == 0) a.prof[i] = globaltimer_ns();
     };

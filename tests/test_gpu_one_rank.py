@@ -147,6 +147,36 @@ def test_low_latency_rows_of_one_rank(T, H, E, K, sms, use_fp8):
         buf.destroy()
 
 
+@pytest.mark.parametrize('sms', [1, 7, 148])
+@pytest.mark.parametrize('use_fp8', [False, True])
+def test_low_latency_expert_with_too_many_selections(sms, use_fp8):
+    """Tokens that name an expert twice give it more selections than the rows it has.  The failure is reported while other CTAs start and
+    end; whatever each of them sees of it, nothing is written outside the call's tensors."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 96, 1024, 8, 4
+    guards = [torch.full((1 << 22,), 0x5A, dtype=torch.uint8, device='cuda') for _ in range(4)]
+    for attempt in range(4):
+        buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K,
+                            extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+        try:
+            idx = torch.arange(T * K, device='cuda').view(T, K) % E
+            idx[:, 1] = idx[:, 0]                            # 0, 0, 2, 3 / 4, 4, 6, 7: experts 0 and 4 get T selections, T rows each: fits
+            x = torch.randn(T, H, device='cuda').bfloat16()
+            buf.low_latency_dispatch(x, idx, T, E, use_fp8=use_fp8, num_sms=sms)
+            torch.cuda.synchronize()
+            buf.core.check_status()
+            idx[attempt, 2] = idx[attempt, 0]                # one more: does not fit
+            buf.low_latency_dispatch(x, idx, T, E, use_fp8=use_fp8, num_sms=sms)
+            torch.cuda.synchronize()
+            code, _, peer, expected, observed, rank = buf.core.read_status()
+            assert (code, peer, expected, rank) == (2, 0, T, 0) and observed >= T
+            with pytest.raises(RuntimeError):
+                buf.core.check_status()
+            assert all(bool((g == 0x5A).all()) for g in guards)
+        finally:
+            buf.destroy()
+
+
 def test_threads_with_streams_of_their_own():
     """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
     import threading
