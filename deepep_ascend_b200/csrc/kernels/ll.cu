@@ -581,7 +581,8 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
 
 // Dispatch: the row of (token, lane) in its expert's segment is the number of selections of that expert before it, counted in a copy of
 // all ids in shared memory, so rows are in token order, the same on every run.  A unit is a column part of a token (several parts
-// when there are more CTAs than tokens).
+// when there are more CTAs than tokens).  Every CTA knows all counts before it places a row (0.2 us), so a call that cannot be served
+// places none and counts none.
 constexpr int kLLDirectIds = 8192;
 __device__ __forceinline__ int count_ids(const int16_t* ids, int end, int e) {      // ids[0, end) equal to e, by one warp
     int n = 0;
@@ -591,6 +592,7 @@ __device__ __forceinline__ int count_ids(const int16_t* ids, int end, int e) {  
 }
 __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const __grid_constant__ LLDispatchArgs a, const int parts) {
     extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ int s_count[EP_MAX_EXPERTS];               // selections of every expert
     const RankCtx& ctx = a.ctx;
     Workspace* ws = local_ws(ctx);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -610,13 +612,26 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
         const int t = blockIdx.x / parts, c0 = (blockIdx.x - t * parts) * part_channels;
         if (c0 < H) ptx::bulk_prefetch_l2(xb + (static_cast<int64_t>(t) * H + c0) * 2, min(part_channels, H - c0) * 2);
     }
+    int gives_up = is_aborted(ws);
     const bool masked = rank_masked(a.mask, 0);
+    auto load_id = [&](int i) { return i < T * K ? ll_load_idx(a.topk_idx, a.idx_is_64, i) : -1; };
+    int id = load_id(tid);                                // on its way beside the flags and while the counts are cleared
+    for (int e = tid; e < E; e += kLLThreads) s_count[e] = 0;
+    __syncthreads();
     for (int i = tid; i < T * K; i += kLLThreads) {
-        const int e = masked ? -1 : ll_load_idx(a.topk_idx, a.idx_is_64, i);
-        s_ids[i] = static_cast<int16_t>(e >= 0 && e < E ? e : -1);
+        const int e = id >= 0 && id < E && !masked ? id : -1;
+        s_ids[i] = static_cast<int16_t>(e);
+        if (e >= 0) atomicAdd(&s_count[e], 1);
+        id = load_id(i + kLLThreads);
     }
-    // The flag can rise at any time, also in this launch, so the CTA leaves as a whole: warps that went alone would leave ids unfilled.
-    if (__syncthreads_or(is_aborted(ws))) return;
+    __syncthreads();
+    // A call gives up as a whole, with counts of zero: if an expert has more selections than rows, which every CTA sees for itself, and
+    // if a failure was reported before.  That flag can rise at any time, so the warps of a CTA take one decision, at the next barrier.
+    for (int e = tid; e < E; e += kLLThreads)
+        if (s_count[e] > M) {
+            gives_up = 1;
+            if (blockIdx.x == 0) report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, s_count[e]);
+        }
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
         const int t = u / parts, part = u - t * parts, c0 = part * part_channels, c1 = min(H, c0 + part_channels);
         if (c0 >= H) continue;                            // uniform: a row of fewer parts
@@ -651,15 +666,12 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
                 *reinterpret_cast<int4*>(s_row + off) = ptx::ld_nc_v4(src + c0 * 2 + off);
         }
         ptx::fence_proxy_async_smem();
-        __syncthreads();
+        gives_up = __syncthreads_or(gives_up);
+        if (gives_up) break;
         for (int k = warp; k < K; k += kLLWarps) {
             const int e = s_ids[t * K + k];
             if (e < 0 || e >= E) continue;
             const int slot = count_ids(s_ids, t * K + k, e);
-            if (slot >= M) {
-                if (lane == 0) report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
-                continue;
-            }
             const int64_t pos = static_cast<int64_t>(e) * M + slot;
             if (lane == 0) {
                 const int bytes_per = a.use_fp8 ? 1 : 2;
@@ -670,15 +682,13 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
         }
         ptx::bulk_commit();
     }
-    __syncthreads();                                      // the ids, also in a CTA without a unit
+    gives_up = __syncthreads_or(gives_up);                // also in a CTA without a unit
     stamp(1);
-    for (int e = blockIdx.x + warp * gridDim.x; e < E; e += gridDim.x * kLLWarps) {
-        const int n = min(count_ids(s_ids, T * K, e), M);
-        if (lane == 0) {
-            a.packed_count[e] = n;
-            a.layout_range[e] = n;
-            if (a.stats != nullptr) a.stats[e] += n;
-        }
+    for (int e = blockIdx.x + tid * gridDim.x; e < E; e += gridDim.x * kLLThreads) {
+        const int n = gives_up ? 0 : s_count[e];
+        a.packed_count[e] = n;
+        a.layout_range[e] = n;
+        if (a.stats != nullptr) a.stats[e] += n;
     }
     ptx::bulk_wait<0>();
     for (int i = 2; i < 7; ++i) stamp(i);

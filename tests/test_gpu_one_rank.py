@@ -177,6 +177,34 @@ def test_low_latency_expert_with_too_many_selections(sms, use_fp8):
             buf.destroy()
 
 
+@pytest.mark.parametrize('why', ['too_many_selections', 'failed_before'])
+def test_low_latency_dispatch_that_gives_up_counts_nothing(why):
+    """Work that is queued behind a call takes the counts before the host can look at the status: they are zero if the call gave up."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 64, 512, 16, 4
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=0.2,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+    try:
+        idx = torch.arange(T * K, device='cuda').view(T, K) % E
+        if why == 'too_many_selections':
+            idx[:, 1] = 5
+            idx[3] = 5
+        x = torch.randn(T, H, device='cuda').bfloat16()
+        stats = torch.full((E,), 3, dtype=torch.int32, device='cuda')
+        with torch.cuda.stream(buf.comm_stream):             # what the call's small tensors will be made of
+            old = [torch.full((n,), 77, dtype=torch.int32, device='cuda') for n in (E, E, 2 * E, E * T) for _ in range(4)]
+        torch.cuda.synchronize()
+        del old
+        if why == 'failed_before':
+            buf.core.wait_flag_test(7)                       # ends after 0.2 s with a failure; the call is queued behind it
+        _, count, handle, _, _ = buf.low_latency_dispatch(x, idx, T, E, stats, num_sms=7)
+        torch.cuda.synchronize()
+        assert buf.core.read_status()[0] != 0
+        assert not count.any() and not handle[1].any() and bool((stats == 3).all())
+    finally:
+        buf.destroy()
+
+
 def test_threads_with_streams_of_their_own():
     """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
     import threading
