@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_combine_direct_kernel(const 
     const int E = a.num_experts, K = a.num_topk, M = a.num_max_tokens, T = a.num_tokens, row_bytes = 2 * a.hidden;
     constexpr int kChunk = 32 * 16;
     const int part_bytes = ((row_bytes + kChunk - 1) / kChunk + parts - 1) / parts * kChunk;
-    if (__syncthreads_or(is_aborted(ws))) return;          // all warps or none: they fill the row numbers together
+    const int gives_up = is_aborted(ws);
     auto stamp = [&](int i) {
         if (a.prof != nullptr && blockIdx.x == 0 && tid == 0) a.prof[i] = globaltimer_ns();
     };
@@ -714,7 +714,8 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_combine_direct_kernel(const 
     for (int u = blockIdx.x; u < T * parts; u += gridDim.x) {
         const int t = u / parts, c0 = (u - t * parts) * part_bytes, c1 = min(row_bytes, c0 + part_bytes);
         if (c0 >= row_bytes) continue;                    // uniform: a row of fewer parts
-        __syncthreads();                                  // the row numbers of the unit before have been used
+        // the row numbers of the unit before have been used; a CTA gives up as a whole, because its warps fill the row numbers together
+        if (__syncthreads_or(gives_up)) break;
         for (int k = warp; k < K; k += kLLWarps) {
             const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + k);
             int found = -1;
