@@ -200,6 +200,7 @@ struct LLDispatchArgs {
     int shrink;                  // a source that never arrives is masked instead of poisoning the buffer
     uint64_t* prof;              // [8] phase timestamps (ns) or null: start, sends issued, sends complete, counts published
                                  //     (by the last CTA), first counts received, packed, end
+    int direct_rows;             // one rank, both phases: rows go straight to their packed places (set by the launcher)
 };
 
 struct LLCombineArgs {
@@ -220,6 +221,7 @@ struct LLCombineArgs {
     int use_logfmt;              // rows cross the wire as 10-bit logarithmic codes with one range per 128 channels (logfmt.cuh)
     uint64_t* prof;              // [8] phase timestamps (ns) or null: start, stores issued, stores complete, flags published
                                  //     (by the last CTA), flags received, reduced
+    int direct_rows;             // one rank, both phases, bf16: rows are reduced where they lie (set by the launcher)
 };
 
 namespace ep {

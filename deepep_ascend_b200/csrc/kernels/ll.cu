@@ -13,7 +13,9 @@
 //                    CTAs: every row is bulk-copied into the slot [source token][top-k lane] of the token's home
 //                    rank; the last CTA to finish raises one epoch-tagged flag per rank pair.
 //            RECV  - wait for all ranks' flags, then out[t] = sum_k w[t,k] * slot[t,k] in fp32 -> bf16.
-// With one rank (both halves in one launch) nothing has to travel, and kernels of their own place and reduce the rows directly.
+// With one rank (both halves in one launch) nothing has to travel.  Small batches have kernels of their own, which place and reduce the
+// rows directly.  With larger ones dispatch stores a message's payload, scales and source straight at the packed position, which is the
+// claimed slot, and combine leaves row numbers in the slots and reduces the rows where they lie.
 // No CTA waits for another CTA of its own rank (no grid barrier): phases end with an arrival counter whose last
 // arriver does the publishing.
 // SEND and RECV can be launched separately (phases argument) so that no SM is held while data is in flight.
@@ -195,7 +197,26 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
             }
             ptx::fence_proxy_async_smem();
             __syncthreads();
-            if (warp < K && lane == 0) {
+            if (a.direct_rows && warp < K) {
+                // one rank: the claimed slot IS the packed position, so payload, scales and source go there at once
+                const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
+                if (e >= 0 && e < E && !rank_masked(a.mask, 0)) {
+                    uint32_t slot = 0;
+                    if (lane == 0) slot = atomicAdd(&slot_counter[e], 1u);
+                    slot = __shfl_sync(0xffffffffu, slot, 0);
+                    if (slot < static_cast<uint32_t>(M)) {
+                        const int64_t pos = static_cast<int64_t>(e) * M + slot;
+                        if (lane == 0) {
+                            ptx::bulk_store(reinterpret_cast<uint8_t*>(a.packed_x) + pos * payload, msg + 16, payload);
+                            a.packed_src_info[pos] = (warp << 20) | t;
+                        }
+                        if (a.use_fp8) ll_store_scales(a, e, 0, G, G, M, slot, [&](int gi) { return reinterpret_cast<const float*>(msg + 16 + H)[gi]; });
+                    } else if (lane == 0) {
+                        report_failure(ctx, ws, EP_ERR_BOUNDS, EP_PH_LL_RECV_COUNT, 0, M, slot);
+                    }
+                }
+                ptx::bulk_commit();
+            } else if (!a.direct_rows && warp < K && lane == 0) {
                 const int e = ll_load_idx(a.topk_idx, a.idx_is_64, static_cast<int64_t>(t) * K + warp);
                 if (e >= 0 && e < E && !rank_masked(a.mask, e / El)) {
                     const uint32_t slot = atomicAdd(&slot_counter[e], 1u);
@@ -282,7 +303,7 @@ __device__ __forceinline__ void ll_dispatch_body(const LLDispatchArgs& a) {
                 }
             }
             const uint32_t pieces = (payload + 2047) / 2048;
-            const uint32_t items = s_pref[P] * pieces;
+            const uint32_t items = a.direct_rows ? 0u : s_pref[P] * pieces;
             for (uint32_t u = blockIdx.x * kLLWarps + warp; u < items; u += gridDim.x * kLLWarps) {
                 const uint32_t g = u / pieces, c = u - g * pieces;
                 const int p = find_segment(s_pref, P, g);
@@ -382,9 +403,20 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
             }
             return pos;
         };
+        bool indexed = false;
+        if (a.direct_rows) {
+            // one rank: the slot of a (token, lane) gets the row's number instead of the row, one thread each
+            for (uint32_t r = blockIdx.x * blockDim.x + tid; r < total && alive; r += gridDim.x * blockDim.x) {
+                const int p = find_segment(s_pref, P, r);
+                const int64_t at = static_cast<int64_t>(p) * M + s_begin[p] + (r - s_pref[p]);
+                const int info = a.src_info[at];
+                *reinterpret_cast<int*>(s_peer[me] + a.off_slab[set] + (static_cast<int64_t>(info & 0xfffff) * K + (info >> 20)) * row_bytes) = static_cast<int>(at);
+                indexed = true;
+            }
+        }
         uint32_t g = blockIdx.x * send_warps + warp;
         int64_t pos = 0;
-        const bool stage_rows = warp < send_warps;
+        const bool stage_rows = warp < send_warps && !a.direct_rows;
         if (stage_rows && g < total && alive) pos = issue_load(g, 0);
         for (; stage_rows && g < total && alive; g += g_stride) {
             const int s = next_src;
@@ -418,7 +450,7 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
         stamp(1);
         ptx::bulk_wait<0>();
         // only lanes that have stored to a peer have something to make visible
-        if (n_loaded > 0 && lane == 0) __threadfence_system();
+        if ((n_loaded > 0 && lane == 0) || indexed) __threadfence_system();
         stamp(2);
         // the last CTA of this rank to finish its stores raises this rank's flag at every peer (no grid barrier)
         if (arrive_is_last(&ws->arrive[EP_CH_LL_COMBINE][0]) && !is_aborted(ws)) {
@@ -532,11 +564,19 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
                 }
                 const uint32_t srcs = __ballot_sync(0xffffffffu, e_k >= 0 && e_k < E);
                 const uint8_t* rows = slab + static_cast<int64_t>(t) * K * row_bytes + off;
+                // direct rows: the slots hold row numbers (of this call; anything else is kept inside x)
+                int my_row = 0;
+                if (a.direct_rows && lane < K && ((srcs >> lane) & 1u)) {
+                    my_row = __ldcg(reinterpret_cast<const int*>(slab + (static_cast<int64_t>(t) * K + lane) * row_bytes));
+                    if (static_cast<uint32_t>(my_row) >= static_cast<uint32_t>(E) * M) my_row = 0;
+                }
                 int4 raw[EP_MAX_TOPK];
 #pragma unroll
                 for (int k = 0; k < EP_MAX_TOPK; ++k)
                     if (k < K && ((srcs >> k) & 1u)) {
-                        if (in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(rows + static_cast<int64_t>(k) * row_bytes));
+                        const int64_t at = __shfl_sync(0xffffffffu, my_row, k);
+                        const uint8_t* src = a.direct_rows ? reinterpret_cast<const uint8_t*>(a.x) + at * row_bytes + off : rows + static_cast<int64_t>(k) * row_bytes;
+                        if (in_row) raw[k] = __ldcg(reinterpret_cast<const int4*>(src));
                     }
                 float acc[8];
 #pragma unroll
@@ -583,7 +623,13 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
 // all ids in shared memory, so rows are in token order, the same on every run.  A unit is a column part of a token (several parts
 // when there are more CTAs than tokens).  Every CTA knows all counts before it places a row (0.2 us), so a call that cannot be served
 // places none and counts none.
+// Counting costs every CTA a pass over the ids per selection, and a token's steps are not overlapped with the next token's as they are in
+// the kernel that claims slots; that one takes 12 us for its arrivals and counts.  us, this kernel / claimed slots, bf16 rows of 2048:
+// 512 tokens, top-8 14 / 20; 768 23 / 24; 1024 29 / 27; 1536 49 / 35; top-4 1536 tokens 31 / 32, 2048 43 / 38; top-2 2048 tokens
+// 30 / 32, 4096 72 / 59; top-16 512 tokens 24 / 27.  Rows of 7168, top-8: 768 tokens 35 / 36, 1024 45 / 43 (e4m3 41 / 44).
 constexpr int kLLDirectIds = 8192;
+constexpr int64_t kLLDirectWork = 9 << 20;               // ids x tokens
+inline bool ll_dispatch_is_small(int64_t tokens, int64_t ids) { return ids <= kLLDirectIds && ids * tokens <= kLLDirectWork; }
 __device__ __forceinline__ int count_ids(const int16_t* ids, int end, int e) {      // ids[0, end) equal to e, by one warp
     int n = 0;
 #pragma unroll 8
@@ -696,6 +742,11 @@ __global__ void __launch_bounds__(kLLThreads, 1) ll_dispatch_direct_kernel(const
 
 // Combine: the rows of a token are found by their source marks among the rows of the experts it selected, then summed in top-k lane
 // order as everywhere.  A unit is a column part of a token.
+// An expert has a row for every token at most, so the search grows with the tokens and weighs less beside wide rows; the kernel that
+// leaves row numbers in the slots pays 12 us for its arrivals instead.  us, this kernel / that one, top-8, even routing (all
+// tokens on the same experts): rows of 512, 1024 tokens 17 (19) / 18; 2048 32 (39) / 23; rows of 2048, 1536 tokens 28 (32) / 34, 2048
+// 40 (42) / 40; rows of 4096, 2048 tokens 57 (64) / 71, 3072 92 (103) / 98; rows of 7168, 3072 tokens 129 (139) / 150, 4096 195 (193) / 193.
+inline int ll_combine_direct_tokens(int hidden) { return std::max(1024, std::min(3072, hidden * 3 / 4)); }
 __global__ void __launch_bounds__(kLLThreads, 1) ll_combine_direct_kernel(const __grid_constant__ LLCombineArgs a, const int parts) {
     __shared__ int s_row[EP_MAX_TOPK];
     __shared__ float s_w[EP_MAX_TOPK];
@@ -819,17 +870,19 @@ cudaError_t launch_ll_dispatch(const LLDispatchArgs* args, int n, int num_sms, c
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     const LLDispatchArgs& a = args[0];
     const int64_t ids = static_cast<int64_t>(a.num_tokens) * a.num_topk;
-    // Counting the ids costs every CTA a pass over them per selection; with more than 8192 of them the slot claims are cheaper.
-    if (n == 1 && a.ctx.num_ranks == 1 && a.phases == (EP_LL_SEND | EP_LL_RECV) && ids <= kLLDirectIds) {
+    if (n == 1 && a.ctx.num_ranks == 1 && a.phases == (EP_LL_SEND | EP_LL_RECV)) {
         const int ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
         int parts = ll_direct_parts(ctas, a.num_tokens, (a.hidden + 255) / 256, 4);
         const int bytes = static_cast<int>((ids * 2 + 15) / 16 * 16) + ((a.hidden + 127) / 128 * 4 + 15) / 16 * 16 + (a.use_fp8 ? a.hidden : 2 * a.hidden);
-        if (bytes <= 200 * 1024) {
+        if (ll_dispatch_is_small(a.num_tokens, ids) && bytes <= 200 * 1024) {
             cudaError_t err = cudaFuncSetAttribute((const void*)ll_dispatch_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             if (err != cudaSuccess) return err;
             void* params[] = {const_cast<LLDispatchArgs*>(&a), &parts};
             return cudaLaunchKernel((const void*)ll_dispatch_direct_kernel, dim3(ctas, 1, 1), dim3(kLLThreads, 1, 1), params, bytes, stream);
         }
+        LLDispatchArgs claimed = a;
+        claimed.direct_rows = 1;
+        return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, &claimed, n, num_sms, smem, stream);
     }
     return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, args, n, num_sms, smem, stream);
 }
@@ -846,6 +899,11 @@ cudaError_t launch_ll_combine(const LLCombineArgs* args, int n, int num_sms, cud
         const uint64_t x1 = x0 + row * a.num_experts * a.num_max_tokens, o1 = o0 + row * a.num_tokens;
         if (a.ctx.num_ranks == 1 && a.phases == (EP_LL_SEND | EP_LL_RECV) && !a.use_logfmt && (x1 <= o0 || o1 <= x0) && x0 % 16 == 0 && row % 16 == 0 &&
             static_cast<int64_t>(a.num_experts) * a.num_max_tokens < (1ll << 31)) {
+            if (a.num_tokens > ll_combine_direct_tokens(a.hidden)) {
+                LLCombineArgs indexed = a;
+                indexed.direct_rows = 1;
+                return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, &indexed, n, num_sms, smem, stream);
+            }
             const int ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
             int parts = ll_direct_parts(ctas, a.num_tokens, (a.hidden * 2 + 511) / 512, 4);
             void* params[] = {const_cast<LLCombineArgs*>(&a), &parts};

@@ -205,6 +205,48 @@ def test_low_latency_dispatch_that_gives_up_counts_nothing(why):
         buf.destroy()
 
 
+@pytest.mark.parametrize('T,H,E,K', [(1536, 128, 16, 4), (1537, 128, 16, 4), (2048, 256, 8, 4), (1024, 128, 8, 9), (1025, 512, 32, 2), (1536, 2048, 4, 1),
+                                     (1537, 2048, 4, 1)])
+@pytest.mark.parametrize('use_fp8', [False, True])
+def test_low_latency_batches_on_both_sides_of_the_rules(T, H, E, K, use_fp8):
+    """One launch (counted or claimed positions, searched or indexed rows) against the two halves, which go through the slabs."""
+    from deepep_ascend_b200 import ElasticBuffer
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=2 * T, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(2 * T, H, 1, E, K) + (1 << 20))
+    try:
+        x = torch.randn(T, H, device='cuda').bfloat16()
+        g = torch.Generator().manual_seed(T)
+        idx = torch.randint(-1, E, (T, K), generator=g).cuda()             # an expert may be named twice
+        idx[:, 0] = torch.where(torch.arange(T, device='cuda') % 3 == 0, 0, idx[:, 0])
+        w = torch.rand(T, K, generator=g).cuda()
+        packed = []
+        for halves in (False, True):
+            stats = torch.zeros(E, dtype=torch.int32, device='cuda')
+            recv, count, handle, _, hook = buf.low_latency_dispatch(x, idx, 2 * T, E, stats, use_fp8=use_fp8, return_recv_hook=halves)
+            if halves:
+                hook()
+            torch.cuda.synchronize()
+            buf.core.check_status()
+            assert torch.equal(count, stats) and torch.equal(handle[1].view(-1), count.long())
+            rows = torch.arange(2 * T, device='cuda')[None] < count[:, None]
+            info = torch.where(rows, handle[0], 1 << 30)
+            order = info.sort(1).indices                                   # every expert's rows by (lane, token)
+            data = [t.view(torch.uint8) if t.dtype == torch.float8_e4m3fn else t for t in (recv if use_fp8 else (recv,))]
+            packed.append([count, info.gather(1, order)] + [d[torch.arange(E, device='cuda')[:, None], order][rows] for d in data])
+            last = handle
+        for a, b in zip(*packed):
+            assert torch.equal(a, b)
+        y = torch.randn(E, 2 * T, H, device='cuda').bfloat16()
+        out, _, _ = buf.low_latency_combine(y, idx, w, last)
+        split, _, hook = buf.low_latency_combine(y, idx, w, last, return_recv_hook=True)
+        hook()
+        torch.cuda.synchronize()
+        buf.core.check_status()
+        assert torch.equal(out, split)
+    finally:
+        buf.destroy()
+
+
 def test_threads_with_streams_of_their_own():
     """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
     import threading
