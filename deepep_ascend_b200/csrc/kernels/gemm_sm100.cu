@@ -221,7 +221,8 @@ struct PipeState {
 // launch itself, about 2 us per kernel, are ready when the inputs are.  A layer of 64 tokens (32 experts, 3.5 and 6 waves) takes 367 us
 // instead of 375, one of 128 tokens through the low-latency pair 343 instead of 347.  Above 8 waves the gain is gone, and with
 // CTAs of the next kernel waiting beside the last wave it is a loss: 8192 x 7168 x 7168 (14 waves) 692 us against 686, the layer of
-// 4096 tokens 2223 against 2190.  Launches that wait for peers (fused ones) never let another one start beside them.
+// 4096 tokens 2223 against 2190.  Launches that wait for others (fused ones, products whose rows are announced by flags) never let another
+// one start beside them: it could hold the SMs that they are waiting for.
 __host__ __device__ constexpr bool few_waves(int num_tiles, int ctas) { return num_tiles <= 8 * ctas; }
 
 // kMnOperands: how many operands are MN-major (bf16 only).  0: A [M, K], B [N, K].  1: B is [K, N] (data gradients read the forward
@@ -299,7 +300,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     umma::fence_after_thread_sync();
     const uint32_t tmem_base = sm->tmem_base;
     ptx::wait_for_previous_kernel();
-    if (g.fuse == EP_GEMM_FUSE_NONE && few_waves(num_tiles, gemm_ctas)) ptx::let_next_kernel_start();
+    if (g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && few_waves(num_tiles, gemm_ctas)) ptx::let_next_kernel_start();
 
     if (warp < kEpiWarp0) {
         // ---------------------------------------------------------------------- producer warps

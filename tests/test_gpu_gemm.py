@@ -170,3 +170,28 @@ def test_output_rows_leave_through_shared_memory(M, N, K, num_sms, fp8):
     bound = ref.abs() * 2.0 ** -8 + (a.abs() @ b_t.abs()) * K * 2.0 ** -24 + 1e-6
     assert bool(((out.double() - ref).abs() <= bound).all())
     assert bool((full[M:] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize('M,N,K', [(128, 128, 128), (512, 768, 1024), (1300, 512, 512)])
+@pytest.mark.parametrize('named', [False, True])
+def test_rows_announced_by_flags(M, N, K, named):
+    """A product whose row tiles are announced by flags, all of them set before the launch, with other kernels of the library in front of and behind it."""
+    from deepep_ascend_b200 import _native
+    from deepep_ascend_b200.ops import gemm as G
+    C = _native.load()
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device='cuda').bfloat16(), torch.randn(N, K, device='cuda').bfloat16()
+    tiles = (M + 127) // 128
+    flags = torch.full((2 * tiles,), 4, dtype=torch.int64, device='cuda')
+    of_tile = torch.arange(2 * tiles - 1, tiles - 1, -1, dtype=torch.int32, device='cuda') if named else None
+    flags[(of_tile if named else torch.arange(tiles, device='cuda')).long()] = 5
+    pos = torch.randperm(M, device='cuda')[:M // 2 * 2].view(-1, 2).to(torch.int32)
+    want = G.gemm_nt(a, b)
+    torch.cuda.synchronize()
+    reduced = G.local_reduce(pos, want)
+    for _ in range(3):
+        copy = G.local_expand_copy(torch.arange(M, device='cuda', dtype=torch.int32)[:, None], a, M)[0]
+        out = C.gemm_nt(copy, b, None, None, None, None, 0, flags, 5, of_tile, None, None)
+        again = G.local_reduce(pos, out)
+        assert torch.equal(out, want) and torch.equal(again, reduced)
+    assert C.gemm_error(0) == 0
