@@ -217,12 +217,14 @@ struct PipeState {
     }
 };
 
-// Products of few waves overlap their launch with the kernel before, and let the next one start early: barriers, tensor memory and the
-// launch itself, about 2 us per kernel, are ready when the inputs are.  A layer of 64 tokens (32 experts, 3.5 and 6 waves) takes 367 us
-// instead of 375, one of 128 tokens through the low-latency pair 343 instead of 347.  Above 8 waves the gain is gone, and with
-// CTAs of the next kernel waiting beside the last wave it is a loss: 8192 x 7168 x 7168 (14 waves) 692 us against 686, the layer of
-// 4096 tokens 2223 against 2190.  Launches that wait for others (fused ones, products whose rows are announced by flags) never let another
-// one start beside them: it could hold the SMs that they are waiting for.
+// Products of few waves overlap their launch with the kernel before, and let the next one start when their last operands have been
+// requested: barriers, tensor memory and the launch itself, about 2 us per kernel, are ready when the inputs are.  Not earlier: CTAs of
+// the next kernel would wait on SMs that a product of fewer CTAs leaves to an exchange beside it, until the product ends.
+// Where the line lies: product -> SwiGLU -> product -> reduction (e4m3, 7168 x 2 x 2048), in turn / overlapped, by waves of the
+// products: 0.9 and 1.5: 95.0 / 91.0 us, 3.5 and 6.1: 320 / 315; 5 to 9 waves: the same within 1 %; (2048 x 2 x 1024) 10.4: 280 / 288.
+// Layer of 64 tokens 370 / 364, of 4096 tokens (29 and 51 waves) 2187 / 2232; 8192 x 7168 x 7168 in bf16 (14 waves) 683 / 695.
+// Launches that wait for others (fused ones, products whose rows are announced by flags) never let another one start beside them: it
+// could hold the SMs that they are waiting for.
 __host__ __device__ constexpr bool few_waves(int num_tiles, int ctas) { return num_tiles <= 8 * ctas; }
 
 // kMnOperands: how many operands are MN-major (bf16 only).  0: A [M, K], B [N, K].  1: B is [K, N] (data gradients read the forward
@@ -300,7 +302,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     umma::fence_after_thread_sync();
     const uint32_t tmem_base = sm->tmem_base;
     ptx::wait_for_previous_kernel();
-    if (g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && few_waves(num_tiles, gemm_ctas)) ptx::let_next_kernel_start();
+    const bool lets_next_start = g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && few_waves(num_tiles, gemm_ctas);
 
     if (warp < kEpiWarp0) {
         // ---------------------------------------------------------------------- producer warps
@@ -380,6 +382,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         p.advance();
                     }
                 }
+                if (lets_next_start) ptx::let_next_kernel_start();
             }
         } else if (warp == 1) {
             // ------------------------------------------------------------------ MMA issuer

@@ -679,7 +679,8 @@ __global__ void __launch_bounds__(kPlanWarps * 32) local_expand_layout_kernel(co
 }
 
 // COPY: one warp per received row (or part of it); every 512-byte piece is read once and written to each expert row of the row.
-// This kernel, the reduction and the forward activation stand between products, so all start early (see few_waves).
+// This kernel, the reduction and the forward activation stand between products, so all start early (see few_waves); they let the next
+// one start when their own last CTAs have started.
 constexpr int kExpandWarps = 8, kMaxExpandTopk = 32;
 __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(const LocalExpandCopyArgs a) {
     ptx::wait_for_previous_kernel();

@@ -29,8 +29,8 @@ class _MoEFunction(torch.autograd.Function):
     pipeline: while the tensor cores work on the experts of chunk c, the communication stream combines chunk c - 1 and
     dispatches chunk c + 1, each through one of the buffer's two receive slots / two combine input regions.  Every rank
     issues its communication kernels in the same order on ONE stream (d0, d1, c0, d2, c1, ...), and the GEMMs leave the
-    communication kernels their SMs (``num_sms`` of them), so the kernels of different ranks can never wait for SMs that
-    a kernel waiting for them holds."""
+    communication kernels their SMs (``num_sms`` of them; the kernel behind a GEMM is let in beside it only when the GEMM has
+    requested its last operands), so the kernels of different ranks can never wait for SMs that a kernel waiting for them holds."""
 
     @staticmethod
     def forward(ctx, x, topk_weights, w13, w2, layer, topk_idx):

@@ -527,6 +527,37 @@ def test_kernels_that_start_before_the_one_before_has_ended(rows, H, I, captured
         assert torch.equal(g.view(torch.int16), w.view(torch.int16))
 
 
+def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
+    """The kernel behind a product is launched early, but not so early that its waiting CTAs take the SMs that the product leaves free: a dispatch
+    that is issued meanwhile ends long before the product does."""
+    from deepep_ascend_b200 import ElasticBuffer
+    from deepep_ascend_b200.ops import gemm as ops
+    T, H, E, K = 256, 1024, 16, 4
+    a, b = (torch.randn(2048, 32768, device='cuda').bfloat16() for _ in range(2))           # 128 tiles: eight waves of 16 CTAs, over a millisecond
+    out = torch.empty(2048, 2048, dtype=torch.bfloat16, device='cuda')
+    y = torch.randn(1 << 17, 256, device='cuda').bfloat16()
+    pos = torch.randperm(1 << 17, device='cuda').view(-1, 1).to(torch.int32)
+    x, idx = torch.randn(T, H, device='cuda').bfloat16(), torch.rand(T, E, device='cuda').topk(K, dim=-1).indices
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    side = torch.cuda.Stream()
+    try:
+        for attempt in range(3):
+            start, sent, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+            torch.cuda.synchronize()
+            start.record()
+            ops.gemm_nt(a, b, out=out, num_sms=16)
+            ops.local_reduce(pos, y)
+            end.record()
+            with torch.cuda.stream(side):
+                buf.dispatch(x, idx, num_experts=E, num_sms=24, do_cpu_sync=False)
+                sent.record()
+            torch.cuda.synchronize()
+            times = start.elapsed_time(sent), start.elapsed_time(end)
+            assert attempt == 0 or times[0] < 0.6 * times[1], times                         # the first pass may load code
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize('rows,I', [(0, 128), (4, 0), (0, 0)])
 @pytest.mark.parametrize('masked', [False, True])
 def test_swiglu_of_nothing(rows, I, masked):
