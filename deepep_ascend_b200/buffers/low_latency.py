@@ -79,6 +79,8 @@ class LowLatencyMixin:
         ``ops.gemm.grouped_gemm_nt(tile_rows=...)`` loads and stores only the rows of a tile that count (with one 128-row tile per
         expert the argument is ``recv_count`` itself), ``ops.gemm.swiglu_quant(valid_row=...)`` skips the others.
         ``handle = (src_info, layout_range, max_tokens, hidden, num_experts)``.
+        The time spent waiting for every source rank, in ns, is added to ``dispatch_wait_recv_cost_stats`` (int64 ``[ranks]``).  A
+        small batch on one rank, both halves in one launch, waits for nobody: nothing is added.
         """
         M, E = num_max_dispatch_tokens_per_rank, num_experts
         if self.is_cpu:
@@ -128,6 +130,7 @@ class LowLatencyMixin:
         logarithmic codes with one range per 128 channels (36 % fewer bytes; ``H`` must be a multiple of 128), coded by
         the sender and decoded inside the weighted reduction
         (csrc/kernels/legacy/internode_ll.cu:556-712 of the reference; ``utils.math.logfmt10_roundtrip`` states the code).
+        ``combine_wait_recv_cost_stats`` as in :meth:`low_latency_dispatch`.
         """
         if self.is_cpu:
             return self._cpu_coll.low_latency_combine(x, topk_idx, topk_weights, handle, use_logfmt, out)

@@ -247,6 +247,31 @@ def test_low_latency_batches_on_both_sides_of_the_rules(T, H, E, K, use_fp8):
         buf.destroy()
 
 
+@pytest.mark.parametrize('how', ['one_launch', 'halves'])
+def test_low_latency_wait_statistics(how):
+    """Waiting is added up where there is any: never in the one launch of a small batch, whose kernels wait for nobody."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 16, 256, 8, 2
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+    try:
+        idx, w = _routing(T, E, K, 4)
+        sent, back = (torch.full((1,), 1000, dtype=torch.int64, device='cuda') for _ in range(2))
+        x, halves = torch.randn(T, H, device='cuda').bfloat16(), how == 'halves'
+        recv, _, handle, _, hook = buf.low_latency_dispatch(x, idx, T, E, dispatch_wait_recv_cost_stats=sent, use_fp8=False, return_recv_hook=halves)
+        if halves:
+            hook()
+        _, _, hook = buf.low_latency_combine(recv, idx, w, handle, combine_wait_recv_cost_stats=back, return_recv_hook=halves)
+        if halves:
+            hook()
+        torch.cuda.synchronize()
+        buf.core.check_status()
+        for stat in (sent, back):
+            assert 1000 <= int(stat) < 10**9 if halves else int(stat) == 1000
+    finally:
+        buf.destroy()
+
+
 def test_threads_with_streams_of_their_own():
     """Every thread has a buffer and a current stream; all share the communication stream and the code that orders streams against it."""
     import threading
