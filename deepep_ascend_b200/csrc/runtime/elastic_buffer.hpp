@@ -277,8 +277,11 @@ public:
             c.tail_bytes = align_up(c.tail_off_meta + 8, 16);
             c.tail_pitch = side_aligned ? align_up(c.tail_bytes, 128) : c.tail_bytes;
             c.sf_stride_row = side_aligned ? align_up(G * 4, 128) / 4 : G;
-            TORCH_CHECK(c.tail_pitch <= regions.tail_bytes && c.sf_stride_row * 4 <= regions.sf_row_bytes,
-                        "side records larger than the buffer was sized for");
+            if (c.tail_pitch > regions.tail_bytes || c.sf_stride_row * 4 > regions.sf_row_bytes) {
+                // the other shape checks of a dispatch are assertions in Python
+                PyErr_SetString(PyExc_AssertionError, "side records larger than the buffer was sized for");
+                throw py::error_already_set();
+            }
             c.off_recv_tail = slot.tail;
         }
         return c;

@@ -402,6 +402,21 @@ def test_buffers_allocated_with_cuda_virtual_memory():
     assert results['ipc'] == results['vmm'] and len(results['vmm']) == 1
 
 
+def test_more_selections_per_token_than_the_buffer_was_made_for():
+    """Refused as an assertion, like the other shape checks of a dispatch, and the buffer stays usable."""
+    from deepep_ascend_b200 import ElasticBuffer
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=32, hidden=256, num_topk=2)
+    try:
+        x, idx = torch.randn(32, 256, device='cuda').bfloat16(), torch.rand(32, 32, device='cuda').topk(16, dim=-1).indices
+        with pytest.raises(AssertionError, match='side records larger'):
+            buf.dispatch(x, idx, torch.rand(32, 16, device='cuda'), num_experts=32)
+        buf.dispatch(x, idx[:, :2].contiguous(), num_experts=32)
+        torch.cuda.synchronize()
+        buf.check_status()
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize('kind', ['plain', 'taller', 'strided', 'misaligned', 'region', 'into_input', 'no_rows'])
 def test_combine_input_of_one_rank_wherever_it_lies(kind):
     """One rank reads a plain tensor in place; inputs that the kernel cannot read there (pitch, alignment, an output over the input)
