@@ -347,13 +347,13 @@ class ElasticBuffer(LowLatencyMixin, CollectivesMixin):
         return 0
 
     def set_dispatch_tuning(self, num_warps: int = 0, num_stages: int = 0, line_aligned_side: Optional[bool] = None) -> None:
-        """Shape of the dispatch kernel: warps per CTA (1..12, each with its own staging ring) and, for the fused
-        FP8 cast, staging buffers per warp (2..4; more buffers keep more tokens' stores in flight per warp but
-        leave room for fewer warps).  0 selects the default (12 warps, 2 buffers; 20 warps on one rank, whose rows
-        need no staging buffers).  ``line_aligned_side``: place every
+        """Shape of the dispatch kernel: warps per CTA (1..12, each with its own staging ring; 1..20 on one rank) and, for the
+        fused FP8 cast, staging buffers per warp (2..4; more buffers keep more tokens' stores in flight per warp but
+        leave room for fewer warps; one rank, whose rows are not staged on their way out, ignores the number).  0 selects the
+        default (12 warps, 2 buffers; 20 warps on one rank).  ``line_aligned_side``: place every
         row's scales and tail record on 128-byte boundaries at the receiver (``recv_sf`` and ``recv_topk_idx`` /
         ``recv_topk_weights`` become row-strided views), so that each of these small stores is whole lines on the wire."""
-        assert 0 <= num_warps <= 12 and num_stages in (0, 2, 3, 4)
+        assert 0 <= num_warps <= (20 if self.num_ranks == 1 else 12) and num_stages in (0, 2, 3, 4)
         self._tune = (num_warps, num_stages)
         if line_aligned_side is not None:
             self._side_aligned = bool(line_aligned_side)

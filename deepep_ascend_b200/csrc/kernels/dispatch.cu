@@ -1040,7 +1040,8 @@ LaunchShape dispatch_launch_shape(const DispatchArgs& a, int num_sms, bool local
     // staging buffers per warp of the fused-cast path (two unless the caller asks for more), then as many warps (each
     // with its own staging ring) as fit in shared memory; the token-per-step layout needs at least one warp
     s.num_stages = a.tune_stages >= 2 && a.tune_stages <= kDispatchMaxStages ? a.tune_stages : 2;
-    s.num_warps = a.tune_warps >= 1 && a.tune_warps <= kDispatchMaxWarps ? a.tune_warps : (local ? kLocalWarps : kDispatchMaxWarps);
+    const int max_warps = local ? kLocalWarps : kDispatchMaxWarps;
+    s.num_warps = a.tune_warps >= 1 && a.tune_warps <= max_warps ? a.tune_warps : max_warps;
     while (s.num_warps > 1 && make_smem_plan(a, s.num_warps, s.num_stages, local).total > kDispatchSmemBudget) --s.num_warps;
     s.smem_bytes = make_smem_plan(a, s.num_warps, s.num_stages, local).total;
     return s;

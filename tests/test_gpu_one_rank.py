@@ -67,6 +67,38 @@ def test_dispatch_rows_at_the_edges_of_a_batch(R, T, H, sms, mode, do_expand):
         world.destroy()
 
 
+@pytest.mark.parametrize('fp8', [False, True])
+def test_dispatch_with_every_number_of_warps(fp8):
+    """1 to 20 warps on one rank, where 20 is the default; more are refused, and more than 12 with several ranks."""
+    from deepep_ascend_b200 import ElasticBuffer
+    from deepep_ascend_b200.backends.emulated import EmulatedWorld
+    T, H, E, K = 45, 2176, 8, 3
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K, use_fp8_dispatch=fp8)
+    try:
+        x = _rows(T, H, 3)
+        idx, w = _routing(T, E, K, 3)
+        results = []
+        for warps in (0, 20, 19, 13, 12, 7, 1):
+            buf.set_dispatch_tuning(warps, 4 if warps == 7 else 0)
+            rx, ri, rw, handle, _ = buf.dispatch(x, idx, w, num_experts=E, num_sms=3)
+            results.append([t.clone().view(torch.uint8) for t in (*(rx if fp8 else (rx,)), ri.contiguous(), rw.contiguous(), handle.plan)])
+        torch.cuda.synchronize()
+        buf.check_status()
+        for r in results[1:]:
+            assert all(torch.equal(a, b) for a, b in zip(r, results[0]))
+        with pytest.raises(AssertionError):
+            buf.set_dispatch_tuning(21)
+    finally:
+        buf.destroy()
+    world = EmulatedWorld(2, num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    try:
+        world.buffers[0].set_dispatch_tuning(12)
+        with pytest.raises(AssertionError):
+            world.buffers[0].set_dispatch_tuning(13)
+    finally:
+        world.destroy()
+
+
 @pytest.mark.parametrize('T,H,sms', [(1, 128, 3), (5, 256, 2), (37, 1168, 1), (64, 2048, 3), (90, 4112, 7), (41, 7168, 64), (300, 7168, 4)])
 def test_combine_of_one_rank_is_the_sum_of_one_row(T, H, sms):
     """Non-expand layout on one rank: every token has its row or none; the result has the bits of an fp32 sum that starts at zero
