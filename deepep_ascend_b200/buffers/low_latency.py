@@ -11,7 +11,7 @@ from typing import Optional
 
 import torch
 
-from ..utils.event import EventHandle, EventOverlap
+from ..utils.event import EventOverlap
 from ..utils.math import align
 
 
@@ -105,7 +105,8 @@ class LowLatencyMixin:
                 call.phases = 2
                 C.ll_dispatch(self.core, call, num_sms)
         elif async_finish:
-            event = EventOverlap(EventHandle(stream, (call.packed_x,)))
+            event = self._async_event((recv_x, call.packed_count, *handle[:2]),
+                                      (x, topk_idx, call.x, call.topk_idx, cumulative_local_expert_recv_stats, dispatch_wait_recv_cost_stats), stream)
         else:
             self.core.current_waits_for_stream(stream_id)
         return recv_x, call.packed_count, handle, event, hook
@@ -149,7 +150,8 @@ class LowLatencyMixin:
                 call.phases = 2
                 C.ll_combine(self.core, call, num_sms)
         elif async_finish:
-            event = EventOverlap(EventHandle(stream, (call.out,)))
+            event = self._async_event((call.out, out), (x, topk_idx, topk_weights, call.topk_idx, call.topk_weights, *handle[:2],
+                                                        combine_wait_recv_cost_stats), stream)
         else:
             self.core.current_waits_for_stream(stream_id)
         return call.out if out is None else out, event, hook

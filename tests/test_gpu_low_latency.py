@@ -153,3 +153,40 @@ def test_one_rank_moves_rows_once(T, H, E, K, mode, split):
         assert torch.equal(got, want)
     finally:
         buf.destroy()
+
+
+def test_tensors_of_an_asynchronous_call_live_until_it_has_run():
+    """With ``async_finish`` the kernels may still be waiting for the communication stream when the caller drops its inputs and allocates again."""
+    from deepep_ascend_b200 import ElasticBuffer
+    T, H, E, K = 32, 1024, 8, 2
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+    try:
+        x0, idx0, w0 = torch.randn(T, H, device='cuda').bfloat16(), torch.rand(T, E, device='cuda').topk(K, dim=-1).indices, torch.rand(T, K, device='cuda')
+
+        def run(late):
+            tensors = [t.clone() for t in (x0, idx0, w0)]
+            torch.cuda.synchronize()
+            if late:
+                with torch.cuda.stream(buf.comm_stream):
+                    torch.cuda._sleep(20_000_000)                          # about 10 ms
+            recv, count, handle, event, _ = buf.low_latency_dispatch(tensors[0], tensors[1], T, E, use_fp8=False, async_finish=late)
+            del event
+            tensors[0] = None
+            later = [torch.full_like(x0, 7)]                               # where the rows lay, if their memory is free
+            if late:
+                with torch.cuda.stream(buf.comm_stream):
+                    torch.cuda._sleep(20_000_000)
+            out, event, _ = buf.low_latency_combine(recv, tensors[1], tensors[2], handle, async_finish=late)
+            shapes = [(t.shape, t.dtype) for t in (recv, tensors[1], tensors[2], *handle[:2])]
+            del event, recv, handle
+            tensors.clear()
+            later += [torch.full(shape, 1, dtype=dtype, device='cuda') for shape, dtype in shapes]
+            torch.cuda.synchronize()
+            buf.core.check_status()
+            return out.clone(), count.clone()
+        want = run(False)
+        for _ in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(run(True), want))
+    finally:
+        buf.destroy()
