@@ -484,8 +484,8 @@ def test_thin_tiles_are_read_and_stored_by_rows(counts):
 @pytest.mark.parametrize('rows,H,I', [(128, 128, 128), (384, 7168, 384), (2048, 1024, 2048)])
 @pytest.mark.parametrize('captured', [False, True])
 def test_kernels_that_start_before_the_one_before_has_ended(rows, H, I, captured):
-    """The same buffers written and read again and again by launches that may overlap (one tile up to several waves, in a stream and
-    in a CUDA graph): every pass gives the bytes that it gives when the host waits after each kernel."""
+    """A chain of launches that may overlap, each reading what the one before it writes (one tile up to several waves, in a stream and in a
+    CUDA graph): every pass gives the bytes that it gives when the host waits after each kernel.  Copies part the passes."""
     from deepep_ascend_b200.ops import gemm as ops
     torch.manual_seed(rows + I)
     passes = 12
@@ -525,6 +525,42 @@ def test_kernels_that_start_before_the_one_before_has_ended(rows, H, I, captured
         got = run(lambda: None)
     for g, w in zip(got, want):
         assert torch.equal(g.view(torch.int16), w.view(torch.int16))
+
+
+@pytest.mark.parametrize('M,N,sms', [(128, 256, (0,)), (512, 1024, (0, 3)), (1024, 512, (2, 1)), (1024, 512, (1, 2, 0)), (2048, 2048, (148, 8))])
+@pytest.mark.parametrize('captured', [False, True])
+def test_launches_that_overwrite_what_the_one_before_reads(M, N, sms, captured):
+    """Products and reductions write each other's operands in turn, so every launch overwrites what the one before it reads, without anything between
+    them.  The numbers of SMs give products on both sides of the eight waves up to which launches overlap."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(M + N)
+    passes = 24
+    x0 = torch.randn(M, N, device='cuda').bfloat16()
+    w = (torch.randn(N, N, device='cuda') * N**-0.5).bfloat16()
+    pos = torch.randperm(M, device='cuda').view(-1, 1).to(torch.int32)
+    x, y = torch.empty_like(x0), torch.empty_like(x0)
+
+    def run(pause):
+        x.copy_(x0)
+        for i in range(passes):
+            ops.gemm_nt(x, w, out=y, num_sms=sms[i % len(sms)])
+            pause()
+            if i % 3 == 2:
+                ops.gemm_nt(y, w, out=x, num_sms=sms[i % len(sms)])
+            else:
+                ops.local_reduce(pos, y, out=x)
+            pause()
+    run(torch.cuda.synchronize)
+    want = x.clone()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run(lambda: None)
+        graph.replay()
+    else:
+        run(lambda: None)
+    torch.cuda.synchronize()
+    assert bool(want.any()) and torch.equal(x.view(torch.int16), want.view(torch.int16))
 
 
 def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
