@@ -1,7 +1,8 @@
 // Expert-parallel combine for one NVLink domain, as ONE kernel per call: the token's home rank PULLS the rows
 // that its experts produced straight out of the expert ranks' symmetric buffers (TMA bulk loads through the
 // peer mappings, no multicast) and reduces them in fp32 registers, so the reduction is fused into the gather
-// and no intermediate slab is written or re-read.
+// and no intermediate slab is written or re-read.  With one rank and at most one row per token a kernel without barrier, claims and
+// staging moves the rows instead (combine_local_kernel).
 //
 // A row is pulled in column chunks of 32 lanes x 16 B x kUnroll; units of work are claimed dynamically by the warps of all CTAs,
 // whole tokens first and single chunks at the end (see the body).  Each warp owns a ring of chunk buffers with one mbarrier
@@ -10,8 +11,8 @@
 //
 // What bounds it: a warp's own chain per chunk (wait, read, convert, store, refill), so SM count and warps matter until HBM or the
 // link does.  With divisions, queue and claim work per chunk taken off that chain, the claims and plan entries requested ahead,
-// and 16 instead of 12 warps, 8192 rows x 7168 (235 MB moved, one rank) take 378 / 104 / 56 / 47 us on 8 / 32 / 64 / 148 SMs
-// (before: 717 / 190 / 101 / 53); 24 warps with 2 KB chunks are slower (403 / 111 / 63 / 47).
+// and 16 instead of 12 warps, 8192 rows x 7168 (235 MB moved by one rank, before it had the other kernel) took 378 / 104 / 56 / 47 us on
+// 8 / 32 / 64 / 148 SMs (before: 717 / 190 / 101 / 53); 24 warps with 2 KB chunks were slower (403 / 111 / 63 / 47).
 //
 // There is no grid-wide barrier and no exit barrier.  Entry: CTA 0 signals every peer, every CTA watches the peers'
 // signals itself (all ranks' input rows are in place once all ranks have entered the call).  Exit: the caller

@@ -13,9 +13,10 @@
 //                 owns the token); per token: optional fused bf16 -> e4m3 cast with 1x128 scales (register batches
 //                 straight from global memory) or a TMA bulk load, then per destination rank one bulk store of the row
 //                 straight into that rank's recv_x through its peer mapping, one of the scales and one of a tail record
-//                 (expert ids already relative to the receiver, weights, source token and sending lane);
+//                 (expert ids already relative to the receiver, weights, source token and sending lane).  With one rank every
+//                 CTA moves the tokens of its own slice through registers (scatter_local);
 //   5. finish   - every CTA drains its bulk stores and arrives; the last one tells every peer "my rows have arrived",
-//                 waits for the peers' words and closes the call.  All other CTAs leave as soon as they are drained.
+//                 waits for the peers' words (several ranks) and closes the call.  All other CTAs leave as soon as they are drained.
 //
 // Parity: does the work of dispatch_impl + dispatch_copy_epilogue_impl
 // (deep_ep/include/deep_ep/impls/dispatch.cuh:17-409, dispatch_copy_epilogue.cuh:11-323, zero padding :231-322) and of
@@ -52,7 +53,7 @@ struct DispatchSmemPlan {
 
 __host__ __device__ inline int align_int(int x, int a) { return (x + a - 1) / a * a; }
 
-// local (one rank): rows go straight from registers to their place, so nothing is staged
+// local (one rank): rows go straight from registers to their place; only rows to be cast are staged, on their way in
 __host__ __device__ inline DispatchSmemPlan make_smem_plan(const DispatchArgs& a, int num_warps, int num_stages, bool local) {
     DispatchSmemPlan p;
     const int E = a.num_experts, R = a.ctx.num_ranks;
@@ -188,9 +189,10 @@ __device__ __forceinline__ void layout_pass(const DispatchArgs& a, Slice sl, uin
 
 __device__ __forceinline__ uint32_t count_of(uint64_t word) { return static_cast<uint32_t>(word & 0xffffffffull); }
 
-// Fused cast: a row is processed in register batches of two blocks of 1024 channels.  All 16-byte loads of a batch are issued back
-// to back straight from global memory and the next batch is requested before the current one is converted, so the memory latency
-// is not exposed.  q = x * (448 / max(amax, 1e-4)) rounded to nearest even, scale = max(amax, 1e-4) / 448.
+// Fused cast: a row is processed in register batches of two blocks of 1024 channels.  All 16-byte loads of a batch are issued back to
+// back, and the memory latency is not exposed: with several ranks they come straight from global memory, the next batch requested
+// before the current one is converted; with one rank from two buffers per warp in shared memory that are filled two batches ahead.
+// q = x * (448 / max(amax, 1e-4)) rounded to nearest even, scale = max(amax, 1e-4) / 448.
 // The correctly rounded division amax / 448 costs ~20 instructions that only eight lanes of a block would use, so the blocks
 // leave the clamped amax in the staging row and scales_from_amax divides all groups of the row at once, one group per lane.
 constexpr int kCastChannels = 1024, kCastBlocks = 2;      // per block, blocks per batch
@@ -208,7 +210,7 @@ __device__ __forceinline__ int cast_lane(int odd) {
 }
 __device__ __forceinline__ int cast_piece(int k, int i) { return k * kCastChannels + (i >> 1) * 64; }
 
-// the pieces of `batch` from a row of bf16 in global memory; channels beyond the row are zero
+// the pieces of a batch whose first channel is at `row`, wherever `load` reads it; channels beyond the row are zero
 template <typename Load>
 __device__ __forceinline__ void load_pieces(RowBatch& b, const uint8_t* row, int channels, Load load) {
     const uint8_t* p[2] = {row + cast_lane(0) * 2, row + cast_lane(1) * 2};
@@ -324,7 +326,8 @@ __device__ __forceinline__ void bulk_wait_read_n(int pending) {
 // of all tokens come first, and with them the small pieces.  A warp has the plan entries and small pieces of its next unit on their
 // way; rows to be cast come through two buffers per warp that are filled two units ahead, others are requested as a whole unit.
 // An SM moves at most 97 GB/s in and out together (plain copies, any number of warps): 5003 pre-quantised tokens on 24 SMs take 58 us
-// against 74 in the staging kernel (31 at that rate), 4096 bf16 tokens on 64 SMs 40 against 53 (19).  The cast is bound by
+// against 74 in the staging kernel (31 at that rate: count, exchange and assignment are 10 of the 58, rows 35 to 41, drain and launch the
+// rest), 4096 bf16 tokens on 64 SMs 40 against 53 (19; 7 before the rows, 23 to 29 for them).  The cast is bound by
 // instruction issue: 8192 tokens on 64 SMs 73 us against 92.  20 warps: with 24 the kernel spills (+ 8 us), 16 are slower (+ 6 us).
 // The small pieces of a token: lane k has its id and weight of top-k lane k, every lane two scales of a pre-quantised token.
 struct SidePieces {
