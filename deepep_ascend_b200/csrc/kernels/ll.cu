@@ -616,8 +616,9 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
 // ------------------------------------------------------------------------------------------------ one rank
 // With one rank and both halves in one launch a row's packed position can be computed, so no CTA has to hear from another one: no
 // slot claims, counts, flags or arrivals, and a plain launch.  Both kernels are chains of a few dependent memory accesses; the
-// protocol they replace added two arrivals of all CTAs and a flag to each.  Nobody waits, so the wait statistics stay as they are.  40 tokens x 7168, top-8 of 256, bf16: 17 -> 4.3 us and
-// 15 -> 4.8 us; 128 tokens, top-8 of 32: 20 (with the cast) -> 6.5 us and 27 -> 8.9 us.
+// protocol they replace added two arrivals of all CTAs and a flag to each.  40 tokens x 7168, top-8 of 256, bf16: 17 -> 4.6 us and
+// 15 -> 4.7 us; 128 tokens, top-8 of 32: 20 (with the cast) -> 6.9 us and 27 -> 9.2 us.  Nobody waits, so the wait statistics stay as
+// they are.
 
 // Dispatch: the row of (token, lane) in its expert's segment is the number of selections of that expert before it, counted in a copy of
 // all ids in shared memory, so rows are in token order, the same on every run.  A unit is a column part of a token (several parts
@@ -626,7 +627,8 @@ __device__ __forceinline__ void ll_combine_body(const LLCombineArgs& a) {
 // Counting costs every CTA a pass over the ids per selection, and a token's steps are not overlapped with the next token's as they are in
 // the kernel that claims slots; that one takes 12 us for its arrivals and counts.  us, this kernel / claimed slots, bf16 rows of 2048:
 // 512 tokens, top-8 14 / 20; 768 23 / 24; 1024 29 / 27; 1536 49 / 35; top-4 1536 tokens 31 / 32, 2048 43 / 38; top-2 2048 tokens
-// 30 / 32, 4096 72 / 59; top-16 512 tokens 24 / 27.  Rows of 7168, top-8: 768 tokens 35 / 36, 1024 45 / 43 (e4m3 41 / 44).
+// 30 / 32, 4096 72 / 59; top-16 512 tokens 24 / 27.  Rows of 7168, top-8: 768 tokens 35 / 36, 1024 45 / 43 (e4m3 41 / 44).  Up to 1024
+// top-8 tokens, where the two are close, rows are in token order.
 constexpr int kLLDirectIds = 8192;
 constexpr int64_t kLLDirectWork = 9 << 20;               // ids x tokens
 inline bool ll_dispatch_is_small(int64_t tokens, int64_t ids) { return ids <= kLLDirectIds && ids * tokens <= kLLDirectWork; }
