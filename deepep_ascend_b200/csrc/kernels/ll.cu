@@ -867,6 +867,13 @@ cudaError_t launch_ll(const void* single, const void* multi, const Args* args, i
 
 }  // namespace
 
+// The small-batch kernels take more CTAs than the GPU has SMs; their cooperative counterparts for large batches would be refused.
+static int resident_ctas(int num_sms) {
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return num_sms;
+    return std::min(num_sms, sms);
+}
+
 cudaError_t launch_ll_dispatch(const LLDispatchArgs* args, int n, int num_sms, cudaStream_t stream) {
     const int smem = 2 * args[0].msg_bytes;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
@@ -884,7 +891,7 @@ cudaError_t launch_ll_dispatch(const LLDispatchArgs* args, int n, int num_sms, c
         }
         LLDispatchArgs claimed = a;
         claimed.direct_rows = 1;
-        return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, &claimed, n, num_sms, smem, stream);
+        return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, &claimed, n, resident_ctas(num_sms), smem, stream);
     }
     return launch_ll<LLDispatchArgs>((const void*)ll_dispatch_kernel, (const void*)ll_dispatch_kernel_multi, args, n, num_sms, smem, stream);
 }
@@ -904,7 +911,7 @@ cudaError_t launch_ll_combine(const LLCombineArgs* args, int n, int num_sms, cud
             if (a.num_tokens > ll_combine_direct_tokens(a.hidden)) {
                 LLCombineArgs indexed = a;
                 indexed.direct_rows = 1;
-                return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, &indexed, n, num_sms, smem, stream);
+                return launch_ll<LLCombineArgs>((const void*)ll_combine_kernel, (const void*)ll_combine_kernel_multi, &indexed, n, resident_ctas(num_sms), smem, stream);
             }
             const int ctas = num_sms < 1 ? 1 : (num_sms > EP_MAX_CTAS ? EP_MAX_CTAS : num_sms);
             int parts = ll_direct_parts(ctas, a.num_tokens, (a.hidden * 2 + 511) / 512, 4);

@@ -279,6 +279,26 @@ def test_low_latency_batches_on_both_sides_of_the_rules(T, H, E, K, use_fp8):
         buf.destroy()
 
 
+@pytest.mark.parametrize('T,H,E,K', [(40, 256, 8, 4), (3000, 1024, 4, 2), (3000, 2048, 4, 4)])
+def test_low_latency_on_more_sms_than_there_are(T, H, E, K):
+    """160 SMs may be asked for with any batch; the kernels of large batches take what the GPU has."""
+    from deepep_ascend_b200 import ElasticBuffer
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=T, hidden=H, num_topk=K,
+                        extra_bytes=ElasticBuffer.get_low_latency_size_hint(T, H, 1, E, K) + (1 << 20))
+    try:
+        idx, w = _routing(T, E, K, T)
+        x = torch.randn(T, H, device='cuda').bfloat16()
+        outs = []
+        for sms in (0, 160):
+            recv, count, handle, _, _ = buf.low_latency_dispatch(x, idx, T, E, use_fp8=False, num_sms=sms)
+            outs.append((count, buf.low_latency_combine(recv, idx, w, handle, num_sms=sms)[0]))
+        torch.cuda.synchronize()
+        buf.core.check_status()
+        assert all(torch.equal(a, b) for a, b in zip(*outs))
+    finally:
+        buf.destroy()
+
+
 @pytest.mark.parametrize('how', ['one_launch', 'halves'])
 def test_low_latency_wait_statistics(how):
     """Waiting is added up where there is any: never in the one launch of a small batch, whose kernels wait for nobody."""
