@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kLocalWarps * 32, 1) combine_local_kernel(cons
     int t = first / parts, part = first - t * parts;
     auto load_plan = [&](int token) -> int { return token < T && lane < K ? __ldg(a.plan + static_cast<int64_t>(token) * K + lane) : -1; };
     int next_plan = load_plan(t);
-    const bool alive = !is_aborted(ws);
+    const bool alive = __all_sync(0xffffffffu, !is_aborted(ws));      // the flag can rise at any time: one decision per warp
     while (alive && t < T) {
         const int token = t, col0 = part * part_bytes, end = min(row_bytes, col0 + part_bytes);
         const uint32_t srcs = __ballot_sync(0xffffffffu, next_plan >= 0);

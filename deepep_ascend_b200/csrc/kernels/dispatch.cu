@@ -527,7 +527,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs& a) {
 
     const Slice cta_tokens = cta_slice<kLocal>(T), sl = warp_slice(cta_tokens, K, num_warps, warp);
     const int own_chunk = max(1, (T + num_ctas - 1) / num_ctas);
-    bool alive = !is_aborted(ws);
+    bool alive = __all_sync(0xffffffffu, !is_aborted(ws));            // the flag can rise at any time: one decision per warp
     auto stamp = [&](int i) {
         if (a.prof != nullptr && cta == 0 && tid == 0) a.prof[i] = globaltimer_ns();
     };
