@@ -12,6 +12,10 @@
 // 128-channel block is accumulated into its own TMEM buffer and promoted into fp32 registers with its scale by
 // EIGHT epilogue warps, two per TMEM lane quadrant: 64 columns each of 128-column tiles, with four TMEM buffers, so that the MMAs
 // run up to three blocks ahead of the promotion; 128 columns each of 256-column tiles, with two.
+// In the 256-column kernel the loop of a K block (MMAs, commit, promotion, hand-over) is what takes the time: 783 cycles for 512 of
+// MMAs at 36864 rows x 4096 x 7168 (65 % of the tensor cycles), at 1.3 to 1.45 GHz under the power cap: 1020 us in short runs, 1204 in
+// long ones (1097 / 1275 before its producer and MMA threads were elected ones, the stage was awaited before the accumulator and
+// the accumulator committed before the stage); 36864 x 7168 x 2048: 577 / 684 us (608 / 721).
 // MN-major bf16 operands (`mn_operands`): the backward pass of a layer reads weights, activations and gradients row-major as the
 // forward pass left them (64 x 64 TMA boxes, transposing descriptors), at the rate of the K-major kernel: 2.3 ms for the two data
 // gradients and 2.6 ms for the two weight gradients of 34816 rows x (7168, 2 x 2048) bf16.  Transposed copies of the weights
@@ -310,7 +314,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (kWide) reg_dealloc<40>();
         if (warp == 0) {
             // ------------------------------------------------------------------ TMA producer
-            if (lane == 0) {
+            // One elected thread, here and in the MMA warp: with `lane == 0` the compiler does not know that a single thread runs the loop,
+            // and a stage of three boxes took the producer 336 ns instead of 260 (six boxes 480 / 280), more than its MMAs.
+            if (ptx::elect_one()) {
                 PipeState<kStages> p;
                 bool ok = true;
                 for (int tile = blockIdx.x; !is_copier && tile < num_items && ok; tile += gemm_ctas) {
@@ -386,7 +392,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             }
         } else if (warp == 1) {
             // ------------------------------------------------------------------ MMA issuer
-            if (lane == 0) {
+            if (ptx::elect_one()) {
                 PipeState<kStages> p;
                 int acc = 0;
                 uint32_t acc_phase = 0;
@@ -400,29 +406,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         umma::fence_after_thread_sync();
                     }
                     for (int kb = tw.kb0; kb < tw.kb1 && ok; ++kb) {
-                        if (kFp8) {
-                            ok = wait_bar<kWide>(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
-                            if (!ok) break;
-                        }
                         ok = wait_bar<kWide>(&sm->full[p.stage], p.phase, sm, g, 4);
                         if (!ok) break;
-                        umma::fence_after_thread_sync();
                         const uint64_t desc_a = kMnOperands >= 2 ? umma::make_smem_desc_mn_sw128(s_a + p.stage * kTileBytes)
                                                                  : umma::make_smem_desc_sw128(s_a + p.stage * kTileBytes);
                         const uint64_t desc_b = kMnOperands >= 1 ? umma::make_smem_desc_mn_sw128(s_b + p.stage * kTileBytesB)
                                                                  : umma::make_smem_desc_sw128(s_b + p.stage * kTileBytesB);
                         // 16 (bf16) / 32 (e4m3) elements of K: 32 bytes along a K-major row, 16 K rows of 128 bytes otherwise
                         constexpr int kStepA = kMnOperands >= 2 ? kUmmaK * 128 : 32, kStepB = kMnOperands >= 1 ? kUmmaK * 128 : 32;
+                        if (kFp8) {
+                            // e4m3: the accumulator is what everyone waits for, so nothing stands between its hand-over and the MMAs
+                            ok = wait_bar<kWide>(&sm->tmem_empty[acc], acc_phase ^ 1, sm, g, 2);
+                            if (!ok) break;
+                        }
+                        umma::fence_after_thread_sync();
 #pragma unroll
                         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
                             const uint32_t accumulate = kFp8 ? (k != 0) : (kb != tw.kb0 || k != 0);
                             umma::mma_ss<kFp8>(tmem_base + acc * kBlockN, umma::advance_desc_k(desc_a, k * kStepA),
                                                umma::advance_desc_k(desc_b, k * kStepB), kWide && tw.half >= 0 ? kIdescHalf : kIdesc, accumulate);
                         }
+                        if (kFp8) umma::mma_commit(&sm->tmem_full[acc]);   // one 128-channel block is ready for promotion
                         umma::mma_commit(&sm->empty[p.stage]);       // the stage may be refilled once these MMAs are done
                         p.advance();
                         if (kFp8) {
-                            umma::mma_commit(&sm->tmem_full[acc]);   // one 128-channel block is ready for promotion
                             if (++acc == kAccBufs) {
                                 acc = 0;
                                 acc_phase ^= 1;
@@ -530,8 +537,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
             } else {
                 if constexpr (kWide) {
-                    // this warp promotes 128 of the 256 columns for its 32 rows; little is kept alive across the K blocks (128 sums and 64
-                    // loaded values per thread leave about 40 registers)
+                    // this warp promotes 128 of the 256 columns for its 32 rows; little is kept alive across the K blocks (128 sums and 32
+                    // loaded values per thread: with 64, or with the scales of four blocks held ahead, the loop spills)
                     constexpr int kCols = 128;
                     const int col_half = (warp - kEpiWarp0) >> 2;
                     if (tw.half >= 0 && col_half == 1) {
@@ -568,28 +575,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             sa = *sfa;
                             sb = *++sfb;
                         }
-                        ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
+                        if (!__all_sync(0xffffffffu, ptx::mbar_try_wait(&sm->tmem_full[acc], acc_phase))) {
+                            ok = wait_bar<kWide>(&sm->tmem_full[acc], acc_phase, sm, g, 5);
+                            ok = __all_sync(0xffffffffu, ok);
+                            if (!ok) break;
+                        }
                         umma::fence_after_thread_sync();
                         const uint32_t taddr = taddr0 + acc * kBlockN;
-                        // 128 columns in two steps of two loads each (64 loaded values live at a time)
 #pragma unroll
-                        for (int c = 0; c < kCols / 64; ++c) {
-                            uint32_t r0[32], r1[32];
-                            umma::tmem_ld_32x32(taddr + c * 64, r0);
-                            umma::tmem_ld_32x32(taddr + c * 64 + 32, r1);
+                        for (int c = 0; c < kCols / 32; ++c) {
+                            uint32_t r[32];
+                            umma::tmem_ld_32x32(taddr + c * 32, r);
                             umma::tmem_ld_wait();
-                            if (c == kCols / 64 - 1) {
+                            if (c == kCols / 32 - 1) {   // the values are in registers: hand the accumulator back before the arithmetic
                                 umma::fence_before_thread_sync();
                                 __syncwarp();
                                 if (lane == 0) ptx::mbar_arrive(&sm->tmem_empty[acc]);
                             }
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                umma::fma_f32x2(sum2[c * 32 + i], umma::pack_f32x2(r0[2 * i], r0[2 * i + 1]), scale2);
-                                umma::fma_f32x2(sum2[c * 32 + 16 + i], umma::pack_f32x2(r1[2 * i], r1[2 * i + 1]), scale2);
-                            }
+                            for (int i = 0; i < 16; ++i) umma::fma_f32x2(sum2[c * 16 + i], umma::pack_f32x2(r[2 * i], r[2 * i + 1]), scale2);
                         }
                         if (++acc == kAccBufs) {
                             acc = 0;
