@@ -284,7 +284,8 @@ struct GemmArgs {
     const float* sfb;                 // fp8: [num_groups, ceil(N/128), ceil(K/128)] contiguous
     const int32_t* tile_group;        // [ceil(M/128)] or null (single group 0)
     const int32_t* tile_rows;         // optional [ceil(M/128)]: leading rows of every tile that count; the others need not be read and
-                                      // their results are not needed (used by the wide e4m3 kernel, ignored elsewhere)
+                                      // their results are not needed (used by the e4m3 kernels for N >= 256, ignored elsewhere)
+    int64_t total_rows;               // upper bound of the sum of tile_rows, 0: not known (chooses between kernels, nothing else)
     int* error;                       // device int set to non-zero if a pipeline wait ran out
     uint64_t* status;                 // status block of a communication buffer that should hear about such a failure, or null
     int status_rank;

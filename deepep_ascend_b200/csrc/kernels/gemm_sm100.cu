@@ -113,15 +113,15 @@ __device__ __noinline__ void gemm_fail_by_value(int* error, uint64_t* status, in
 __device__ __noinline__ void gemm_fail_by_reference(const GemmArgs& g, int* failed, int code) {
     gemm_fail_values(g.error, g.status, g.status_rank, failed, code);
 }
-template <bool kByReference>
-__device__ __forceinline__ void gemm_fail(const GemmArgs& g, GemmSmem* sm, int code) {
+template <bool kByReference, class Smem>
+__device__ __forceinline__ void gemm_fail(const GemmArgs& g, Smem* sm, int code) {
     if constexpr (kByReference) gemm_fail_by_reference(g, &sm->failed, code);
     else gemm_fail_by_value(g.error, g.status, g.status_rank, &sm->failed, code);
 }
 
 // bounded mbarrier wait; returns false (and raises the failure flags) when the limit runs out
-template <bool kByReference>
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, GemmSmem* sm, const GemmArgs& g, int code) {
+template <bool kByReference, class Smem>
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, Smem* sm, const GemmArgs& g, int code) {
     if (ptx::mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = gemm_timer();
     uint32_t spins = 0;
@@ -824,6 +824,380 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
 }
 
+// ------------------------------------------------------------------------------------------------ products that stream the weights
+// e4m3 products with at most one M tile per group (decode layers, short prompts): every weight is read once and the tokens decide
+// nothing, so this kernel is built around how the weights arrive.
+//   * A stage is 128 weight rows x 256 bytes, two TMA boxes side by side.  What streams 32 x 4096 x 7168 and 32 x 7168 x 2048 bytes from
+//     HBM, boxes alone (148 SMs): 256 rows x 128 bytes 154 / 82 us, 128 x 256 141 / 77, 64 x 512 138 / 74, boxes of 32 rows 173 / 95
+//     (a box costs its issuer 35 to 60 ns whatever its size).
+//   * Operands change places: the 128 weight rows are the M of the MMA and the tokens, as many as the tile has (in steps of 16), its
+//     N, so nothing is multiplied, read from tensor memory or promoted for rows that do not exist.  Same sums, same bits.  Tiles of more
+//     than 64 token rows keep the usual places: with one scale per value instead of one per thread, 128 rows of 7168 x 2048 take
+//     137 us instead of 110.
+//   * Tokens come from L2 through a ring and a producer of their own; scales are multiplied and put into shared memory by a
+//     fourth warp (reading them four K blocks ahead changes nothing).  Two accumulators of a stage (two K blocks of 128 columns each).
+//   * The tiles of a last wave that would use at most half (a quarter) of the CTAs are cut into pieces of 64 (32) weight rows.
+// warp 0: weights, 1: MMA, 2: tokens, 3: scales, 4-11: epilogue (32 weight rows each; two warps share the tokens, 16 by 16).
+// Bound by HBM where the weights do not fit L2: 32 experts of 16 token rows, 4096 x 7168 at 6.7 TB/s (5.6 in the 256-column kernel), 7168 x
+// 2048 at 5.9 (5.0); a plain copy moves 6.5.  The second is short of it by its epilogues: one per 16 K blocks.
+constexpr int kStreamStagesW = 4, kStreamStagesA = 3, kStreamKb = 2, kStreamAccs = 2, kStreamScaleSlots = 2;
+constexpr int kStreamThreads = 384, kStreamEpiWarps = 8;
+constexpr int kStreamStageBytes = kStreamKb * kTileBytes;
+struct StreamSmem {
+    uint64_t w_full[kStreamStagesW], w_empty[kStreamStagesW], a_full[kStreamStagesA], a_empty[kStreamStagesA];
+    uint64_t acc_full[kStreamAccs], acc_empty[kStreamAccs], sc_full[kStreamScaleSlots], sc_empty[kStreamScaleSlots];
+    uint32_t tmem_base;
+    int failed;
+};
+static_assert(sizeof(StreamSmem) <= 512, "barrier block");
+constexpr int kStreamSwapRows = 64;      // token rows up to which the operands change places
+constexpr int kStreamScaleBytes = kStreamScaleSlots * kStreamKb * kBlockM * 4;
+constexpr int kStreamSmemBytes = (kStreamStagesW + kStreamStagesA) * kStreamStageBytes + 512 + kStreamScaleBytes;
+static_assert(kStreamSmemBytes <= 232448, "shared memory of a CTA");
+
+// pieces that a tile of the last wave is cut into
+__host__ __device__ constexpr int stream_cut(int num_tiles, int ctas) {
+    const int rem = num_tiles % ctas;
+    return rem == 0 ? 1 : rem * 4 <= ctas ? 4 : rem * 2 <= ctas ? 2 : 1;
+}
+struct StreamItem {
+    int m, col0, out_rows;    // M tile, first weight row of the group, weight rows of this piece
+    int grp, rows;            // group (-1: none), token rows
+};
+
+__global__ void __launch_bounds__(kStreamThreads, 1)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a32, const __grid_constant__ CUtensorMap map_w,
+                   const __grid_constant__ CUtensorMap map_w32, const GemmArgs g) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* s_w = smem;
+    uint8_t* s_a = smem + kStreamStagesW * kStreamStageBytes;
+    StreamSmem* sm = reinterpret_cast<StreamSmem*>(s_a + kStreamStagesA * kStreamStageBytes);
+    float* s_scale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sm) + 512);      // [slot][K block][token]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_m = (g.M + kBlockM - 1) / kBlockM, num_n = (g.N + 127) / 128, num_k = (g.K + 127) / 128;
+    const int num_tiles = num_m * num_n, ctas = static_cast<int>(gridDim.x);
+    const int cut = stream_cut(num_tiles, ctas), whole = cut > 1 ? num_tiles - num_tiles % ctas : num_tiles;
+    const int num_items = whole + (num_tiles - whole) * cut;
+    // item -> piece.  Every role looks an item up before it works on the one in front of it, and looks at what was loaded only
+    // afterwards (`busy`): the two loads take a microsecond.
+    auto get_item = [&](int item) {
+        StreamItem it;
+        item = min(item, num_items - 1);
+        const int tile = item < whole ? item : whole + (item - whole) / cut, piece = item < whole ? 0 : (item - whole) % cut;
+        it.out_rows = item < whole ? 128 : 128 / cut;
+        it.m = tile / num_n;
+        it.col0 = (tile - it.m * num_n) * 128 + piece * it.out_rows;
+        it.rows = g.tile_rows != nullptr ? *(g.tile_rows + it.m) : kBlockM;
+        it.grp = g.tile_group != nullptr ? *(g.tile_group + it.m) : 0;
+        return it;
+    };
+    auto weights_as_m = [](const StreamItem& it) { return it.rows <= kStreamSwapRows; };
+    auto busy = [&](StreamItem& it) {
+        it.rows = min(it.rows, min(kBlockM, g.M - it.m * kBlockM));
+        return it.grp >= 0 && it.rows > 0 && it.col0 < g.N;
+    };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStreamStagesW; ++i) {
+            ptx::mbar_init(&sm->w_full[i], 1);
+            ptx::mbar_init(&sm->w_empty[i], 1);
+        }
+        for (int i = 0; i < kStreamStagesA; ++i) {
+            ptx::mbar_init(&sm->a_full[i], 1);
+            ptx::mbar_init(&sm->a_empty[i], 1);
+        }
+        for (int i = 0; i < kStreamAccs; ++i) {
+            ptx::mbar_init(&sm->acc_full[i], 1);
+            ptx::mbar_init(&sm->acc_empty[i], kStreamEpiWarps);
+        }
+        for (int i = 0; i < kStreamScaleSlots; ++i) {
+            ptx::mbar_init(&sm->sc_full[i], 1);
+            ptx::mbar_init(&sm->sc_empty[i], kStreamEpiWarps);
+        }
+        sm->failed = 0;
+        ptx::mbar_fence_init();
+        umma::prefetch_tensormap(&map_a);
+        umma::prefetch_tensormap(&map_w);
+    }
+    if (warp == 1) {
+        umma::tmem_alloc(&sm->tmem_base, 512);
+        umma::tmem_relinquish();
+    }
+    umma::fence_before_thread_sync();
+    __syncthreads();
+    umma::fence_after_thread_sync();
+    const uint32_t tmem_base = sm->tmem_base;
+    ptx::wait_for_previous_kernel();
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------------- weights
+        if (ptx::elect_one()) {
+            PipeState<kStreamStagesW> p;
+            bool ok = true;
+            StreamItem next = get_item(blockIdx.x);
+            for (int item = blockIdx.x; item < num_items && ok; item += ctas) {
+                StreamItem it = next;
+                next = get_item(item + ctas);
+                if (!busy(it)) continue;
+                const int row = it.grp * g.N + it.col0;
+                for (int kb = 0; kb < num_k; kb += kStreamKb) {
+                    ok = wait_bar<false>(&sm->w_empty[p.stage], p.phase ^ 1, sm, g, 1);
+                    if (!ok) break;
+                    uint8_t* dst = s_w + p.stage * kStreamStageBytes;
+                    const int blocks = min(kStreamKb, num_k - kb);
+                    ptx::mbar_arrive_expect_tx(&sm->w_full[p.stage], blocks * it.out_rows * 128);
+                    if (it.out_rows == 128) {
+                        umma::tma_load_2d(dst, &map_w, kb * 128, row, &sm->w_full[p.stage]);
+                        if (blocks > 1) umma::tma_load_2d(dst + kTileBytes, &map_w, (kb + 1) * 128, row, &sm->w_full[p.stage]);
+                    } else {
+                        for (int j = 0; j < blocks; ++j)
+                            for (int r = 0; r < it.out_rows; r += 32)
+                                umma::tma_load_2d(dst + j * kTileBytes + r * 128, &map_w32, (kb + j) * 128, row + r, &sm->w_full[p.stage]);
+                    }
+                    p.advance();
+                }
+            }
+        }
+        if (few_waves(num_tiles, ctas)) ptx::let_next_kernel_start();
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------------- MMA issuer
+        if (ptx::elect_one()) {
+            PipeState<kStreamStagesW> pw;
+            PipeState<kStreamStagesA> pa;
+            PipeState<kStreamAccs> acc;
+            bool ok = true;
+            StreamItem next = get_item(blockIdx.x);
+            for (int item = blockIdx.x; item < num_items && ok; item += ctas) {
+                StreamItem it = next;
+                next = get_item(item + ctas);
+                if (!busy(it)) continue;
+                const bool swap = weights_as_m(it);
+                const uint32_t idesc = umma::make_instr_desc(128, swap ? (it.rows + 15) / 16 * 16 : it.out_rows, umma::kFormatE4M3);
+                for (int kb = 0; kb < num_k && ok; kb += kStreamKb) {
+                    ok = wait_bar<false>(&sm->a_full[pa.stage], pa.phase, sm, g, 4) && wait_bar<false>(&sm->w_full[pw.stage], pw.phase, sm, g, 4) &&
+                         wait_bar<false>(&sm->acc_empty[acc.stage], acc.phase ^ 1, sm, g, 2);
+                    if (!ok) break;
+                    umma::fence_after_thread_sync();
+                    const uint64_t desc_w = umma::make_smem_desc_sw128(s_w + pw.stage * kStreamStageBytes);
+                    const uint64_t desc_a = umma::make_smem_desc_sw128(s_a + pa.stage * kStreamStageBytes);
+                    const uint64_t desc_m = swap ? desc_w : desc_a, desc_n = swap ? desc_a : desc_w;
+#pragma unroll
+                    for (int j = 0; j < kStreamKb; ++j) {
+                        if (kb + j >= num_k) break;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            umma::mma_ss<true>(tmem_base + (acc.stage * kStreamKb + j) * 128, umma::advance_desc_k(desc_m, j * kTileBytes + k * 32),
+                                               umma::advance_desc_k(desc_n, j * kTileBytes + k * 32), idesc, k != 0);
+                    }
+                    umma::mma_commit(&sm->acc_full[acc.stage]);
+                    acc.advance();
+                    umma::mma_commit(&sm->w_empty[pw.stage]);
+                    umma::mma_commit(&sm->a_empty[pa.stage]);
+                    pw.advance();
+                    pa.advance();
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ---------------------------------------------------------------------- tokens
+        if (ptx::elect_one()) {
+            PipeState<kStreamStagesA> p;
+            bool ok = true;
+            StreamItem next = get_item(blockIdx.x);
+            for (int item = blockIdx.x; item < num_items && ok; item += ctas) {
+                StreamItem it = next;
+                next = get_item(item + ctas);
+                if (!busy(it)) continue;
+                const int boxes = (it.rows + 31) / 32, row = it.m * kBlockM;
+                for (int kb = 0; kb < num_k; kb += kStreamKb) {
+                    ok = wait_bar<false>(&sm->a_empty[p.stage], p.phase ^ 1, sm, g, 1);
+                    if (!ok) break;
+                    const int blocks = min(kStreamKb, num_k - kb);
+                    ptx::mbar_arrive_expect_tx(&sm->a_full[p.stage], blocks * boxes * (kTileBytes / 4));
+                    for (int j = 0; j < blocks; ++j) {
+                        uint8_t* dst = s_a + p.stage * kStreamStageBytes + j * kTileBytes;
+                        if (boxes == 4) umma::tma_load_2d(dst, &map_a, (kb + j) * 128, row, &sm->a_full[p.stage]);
+                        else
+                            for (int i = 0; i < boxes; ++i) umma::tma_load_2d(dst + i * (kTileBytes / 4), &map_a32, (kb + j) * 128, row + i * 32, &sm->a_full[p.stage]);
+                    }
+                    p.advance();
+                }
+            }
+        }
+    } else if (warp == 3) {
+        // ---------------------------------------------------------------------- scales: (token's x weight block's) of a stage's K blocks
+        PipeState<kStreamScaleSlots> p;
+        bool ok = true;
+        StreamItem next = get_item(blockIdx.x);
+        for (int item = blockIdx.x; item < num_items && ok; item += ctas) {
+            StreamItem it = next;
+            next = get_item(item + ctas);
+            if (!busy(it)) continue;
+            const float* sfb = g.sfb + (static_cast<int64_t>(it.grp) * num_n + it.col0 / 128) * num_k;
+            const float* sfa = g.sfa + (static_cast<int64_t>(it.m) * kBlockM + lane) * g.sfa_stride_row;
+            for (int kb = 0; kb < num_k; kb += kStreamKb) {
+                float v[kStreamKb][kBlockM / 32];
+#pragma unroll
+                for (int j = 0; j < kStreamKb; ++j) {
+                    const int k = min(kb + j, num_k - 1);
+                    const float b = sfb[k];
+#pragma unroll
+                    for (int i = 0; i < kBlockM / 32; ++i) v[j][i] = i * 32 + lane < it.rows ? sfa[i * 32 * g.sfa_stride_row + k * g.sfa_stride_kb] * b : 0.f;
+                }
+                ok = __all_sync(0xffffffffu, wait_bar<false>(&sm->sc_empty[p.stage], p.phase ^ 1, sm, g, 6));
+                if (!ok) break;
+#pragma unroll
+                for (int j = 0; j < kStreamKb; ++j)
+#pragma unroll
+                    for (int i = 0; i < kBlockM / 32; ++i) s_scale[(p.stage * kStreamKb + j) * kBlockM + i * 32 + lane] = v[j][i];
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&sm->sc_full[p.stage]);
+                p.advance();
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------------- epilogue: thread = one weight row, tokens 16 by 16
+        const int quad = warp & 3, half = (warp - 4) >> 2;
+        const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * 16;
+        constexpr int kChunks = 4;          // of 16 tokens per warp: tokens (2 i + half) * 16 ...
+        PipeState<kStreamAccs> acc;
+        PipeState<kStreamScaleSlots> sc;
+        bool ok = true;
+        StreamItem next = get_item(blockIdx.x);
+        for (int item = blockIdx.x; item < num_items && ok; item += ctas) {
+            StreamItem it = next;
+            next = get_item(item + ctas);
+            if (!busy(it)) continue;
+            if (!weights_as_m(it)) {
+                // thread = one token, this warp's 64 of the weight rows: one scale per K block instead of one per value
+                const int pieces = max(0, min(2, (it.out_rows - half * 64 + 31) / 32));      // of 32 weight rows
+                uint64_t sum2[2][16];
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum2[c][i] = 0ull;
+#pragma unroll 1
+                for (int kb = 0; kb < num_k; kb += kStreamKb) {
+                    ok = __all_sync(0xffffffffu, wait_bar<false>(&sm->sc_full[sc.stage], sc.phase, sm, g, 6));
+                    if (!ok) break;
+                    ok = __all_sync(0xffffffffu, wait_bar<false>(&sm->acc_full[acc.stage], acc.phase, sm, g, 5));
+                    if (!ok) break;
+                    umma::fence_after_thread_sync();
+#pragma unroll
+                    for (int j = 0; j < kStreamKb; ++j) {
+                        if (kb + j >= num_k) break;
+                        const uint32_t scale = __float_as_uint(s_scale[(sc.stage * kStreamKb + j) * kBlockM + quad * 32 + lane]);
+                        const uint64_t scale2 = umma::pack_f32x2(scale, scale);
+                        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (acc.stage * kStreamKb + j) * 128 + half * 64;
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            if (c >= pieces) break;
+                            uint32_t r[32];
+                            umma::tmem_ld_32x32(taddr + c * 32, r);
+                            umma::tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) umma::fma_f32x2(sum2[c][i], umma::pack_f32x2(r[2 * i], r[2 * i + 1]), scale2);
+                        }
+                    }
+                    umma::fence_before_thread_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        ptx::mbar_arrive(&sm->acc_empty[acc.stage]);
+                        ptx::mbar_arrive(&sm->sc_empty[sc.stage]);
+                    }
+                    acc.advance();
+                    sc.advance();
+                }
+                if (!ok) break;
+                if (quad * 32 + lane < it.rows) {
+                    uint8_t* c_row = reinterpret_cast<uint8_t*>(g.c) + ((static_cast<int64_t>(it.m) * kBlockM + quad * 32 + lane) * g.ldc + it.col0 + half * 64) * 2;
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) {
+                            int4 out;
+                            uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                float lo, hi;
+                                umma::unpack_f32x2(sum2[c][4 * v + i], lo, hi);
+                                o[i] = pack_bf16(lo, hi);
+                            }
+                            if (c < pieces && it.col0 + half * 64 + c * 32 + v * 8 < g.N) *reinterpret_cast<int4*>(c_row + (c * 32 + v * 8) * 2) = out;
+                        }
+                }
+                continue;
+            }
+            const int chunks = max(0, (it.rows - half * 16 + 31) / 32);      // of this warp that hold tokens
+            float sum[kChunks][16];
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i)
+#pragma unroll
+                for (int t = 0; t < 16; ++t) sum[i][t] = 0.f;
+#pragma unroll 1
+            for (int kb = 0; kb < num_k; kb += kStreamKb) {
+                ok = __all_sync(0xffffffffu, wait_bar<false>(&sm->sc_full[sc.stage], sc.phase, sm, g, 6));
+                if (!ok) break;
+                ok = __all_sync(0xffffffffu, wait_bar<false>(&sm->acc_full[acc.stage], acc.phase, sm, g, 5));
+                if (!ok) break;
+                umma::fence_after_thread_sync();
+#pragma unroll
+                for (int j = 0; j < kStreamKb; ++j) {
+                    if (kb + j >= num_k) break;
+                    const float4* scale = reinterpret_cast<const float4*>(s_scale + (sc.stage * kStreamKb + j) * kBlockM + half * 16);
+                    const uint32_t taddr = taddr0 + (acc.stage * kStreamKb + j) * 128;
+#pragma unroll
+                    for (int i0 = 0; i0 < kChunks; i0 += 2) {        // 32 values in registers at a time
+                        if (i0 >= chunks) break;
+                        uint32_t r[2][16];
+                        umma::tmem_ld_32x16(taddr + i0 * 32, r[0]);
+                        if (i0 + 1 < chunks) umma::tmem_ld_32x16(taddr + (i0 + 1) * 32, r[1]);
+                        umma::tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            if (i0 + i < chunks)
+#pragma unroll
+                                for (int v = 0; v < 4; ++v) {
+                                    const float4 f = scale[(i0 + i) * 8 + v];
+                                    float* d = &sum[i0 + i][4 * v];
+                                    d[0] = fmaf(__uint_as_float(r[i][4 * v]), f.x, d[0]);
+                                    d[1] = fmaf(__uint_as_float(r[i][4 * v + 1]), f.y, d[1]);
+                                    d[2] = fmaf(__uint_as_float(r[i][4 * v + 2]), f.z, d[2]);
+                                    d[3] = fmaf(__uint_as_float(r[i][4 * v + 3]), f.w, d[3]);
+                                }
+                    }
+                }
+                umma::fence_before_thread_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    ptx::mbar_arrive(&sm->acc_empty[acc.stage]);
+                    ptx::mbar_arrive(&sm->sc_empty[sc.stage]);
+                }
+                acc.advance();
+                sc.advance();
+            }
+            if (!ok) break;
+            // Two lanes trade values so that each has two neighbouring columns of every other token: half the stores, 4 bytes each.
+            const int odd = lane & 1, row = quad * 32 + lane, col = it.col0 + row - odd;
+            const bool stored = row < it.out_rows && col < g.N;
+            uint8_t* c = reinterpret_cast<uint8_t*>(g.c) + ((static_cast<int64_t>(it.m) * kBlockM + half * 16 + odd) * g.ldc + col) * 2;
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i) {
+                if (i >= chunks) break;
+#pragma unroll
+                for (int t = 0; t < 16; t += 2) {
+                    const float got = __shfl_xor_sync(0xffffffffu, odd ? sum[i][t] : sum[i][t + 1], 1);
+                    const uint32_t two = odd ? pack_bf16(got, sum[i][t + 1]) : pack_bf16(sum[i][t], got);
+                    if (stored && i * 32 + half * 16 + t + odd < it.rows) *reinterpret_cast<uint32_t*>(c + (i * 32 + t) * g.ldc * 2) = two;
+                }
+            }
+        }
+    }
+    umma::fence_before_thread_sync();
+    __syncthreads();
+    if (warp == 1) umma::tmem_dealloc(tmem_base, 512);
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -866,6 +1240,21 @@ bool make_mn_operand_map(CUtensorMap* map, const void* base, int64_t groups, int
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// e4m3 products of thin tiles that read every weight once.  Where the lines lie (32 experts, us in long runs, 256-column kernel / this
+// one, by token rows of an expert):
+//     rows            16          32          48          64          96
+//     4096 x 7168     168 / 141   170 / 144   180 / 152   180 / 160   187 / 194
+//     7168 x 2048      95 / 79     94 / 82     97 / 87     99 / 91    104 / 115
+//     512 x 2048                 10.9 / 8.3              11.0 / 9.5              (weights in L2)
+//   * at most one M tile per group: a second one reads its weights from L2, and the operand traffic of 128-column tiles bounds the product
+//   * at most 56 token rows per tile on average, where the caller knows a bound; one who gives `tile_rows` without has thin tiles
+constexpr int kStreamMaxRows = 56;
+bool streams_weights(const GemmArgs& g) {
+    const int64_t num_m = (g.M + kBlockM - 1) / kBlockM;
+    return g.is_fp8 && g.N >= 256 && g.tile_rows != nullptr && g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && g.k_group_off == nullptr &&
+           g.mn_operands == 0 && num_m <= g.num_groups && (g.total_rows == 0 || g.total_rows <= kStreamMaxRows * num_m);
+}
+
 }  // namespace
 
 cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
@@ -889,6 +1278,24 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
             return (tiles + workers - 1) / workers * (bn + 16);     // waves x (columns + per-tile overhead)
         };
         if (cost(224) < cost(256)) block_n = 224;
+    }
+    if (streams_weights(g)) {
+        CUtensorMap map_a, map_a32, map_w, map_w32;
+        const int64_t w_rows = static_cast<int64_t>(g.num_groups) * g.N;
+        if (!make_operand_map(&map_a, g.a, g.M, g.K, g.lda, true, 128) || !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32) ||
+            !make_operand_map(&map_w, g.b, w_rows, g.K, g.ldb, true, 128) || !make_operand_map(&map_w32, g.b, w_rows, g.K, g.ldb, true, 32))
+            return cudaErrorInvalidValue;
+        const void* fn = (const void*)gemm_stream_kernel;
+        const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmemBytes);
+        if (err != cudaSuccess) return err;
+        const int num_tiles = ((g.M + kBlockM - 1) / kBlockM) * ((g.N + 127) / 128);
+        // with fewer tiles than SMs: the pieces that they are cut into (the kernel cuts by the same rule)
+        int ctas = num_sms < 1 ? 1 : num_sms;
+        if (num_tiles < ctas) ctas = num_tiles * stream_cut(num_tiles, ctas);
+        void* params[] = {&map_a, &map_a32, &map_w, &map_w32, const_cast<GemmArgs*>(&g)};
+        const dim3 block(kStreamThreads, 1, 1);
+        if (few_waves(num_tiles, ctas)) return launch_dependent(fn, dim3(ctas, 1, 1), block, params, kStreamSmemBytes, stream);
+        return cudaLaunchKernel(fn, dim3(ctas, 1, 1), block, params, kStreamSmemBytes, stream);
     }
     if (g.mn_operands < 0 || g.mn_operands > 2 || (g.mn_operands != 0 && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE))) return cudaErrorInvalidValue;
     if ((g.mn_operands == 2) != (g.k_group_off != nullptr && g.mn_operands != 0)) return cudaErrorInvalidValue;

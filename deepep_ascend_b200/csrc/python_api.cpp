@@ -71,7 +71,7 @@ at::Tensor& gemm_error_flag(int device) {
 at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional<at::Tensor>& sfa, const std::optional<at::Tensor>& sfb,
                    const std::optional<at::Tensor>& tile_group, const std::optional<at::Tensor>& out, int64_t num_sms,
                    const std::optional<at::Tensor>& a_ready_flags, int64_t a_ready_value, const std::optional<at::Tensor>& a_flag_of_tile,
-                   ElasticBufferCore* report_to, const std::optional<at::Tensor>& tile_rows) {
+                   ElasticBufferCore* report_to, const std::optional<at::Tensor>& tile_rows, int64_t total_rows) {
     TORCH_CHECK(a.is_cuda() && a.dim() == 2 && a.stride(1) == 1, "A must be [M, K] with contiguous rows");
     TORCH_CHECK(b.is_cuda() && (b.dim() == 2 || b.dim() == 3) && b.is_contiguous(), "B must be contiguous [N, K] or [G, N, K]");
     const bool fp8 = a.scalar_type() == at::kFloat8_e4m3fn;
@@ -112,6 +112,7 @@ at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional
         TORCH_CHECK(tile_rows->is_cuda() && tile_rows->scalar_type() == at::kInt && tile_rows->is_contiguous() && tile_rows->numel() >= (M + 127) / 128,
                     "bad tile_rows");
         g.tile_rows = tile_rows->data_ptr<int32_t>();
+        g.total_rows = std::max<int64_t>(0, total_rows);
     }
     if (a_ready_flags.has_value()) {
         TORCH_CHECK(a_ready_flags->scalar_type() == at::kLong, "flags must be int64");
@@ -877,7 +878,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.attr("CH_ENGRAM") = static_cast<int>(EP_CH_ENGRAM);
     m.def("gemm_nt", &gemm_nt, py::arg("a"), py::arg("b"), py::arg("sfa") = py::none(), py::arg("sfb") = py::none(),
           py::arg("tile_group") = py::none(), py::arg("out") = py::none(), py::arg("num_sms") = 0, py::arg("a_ready_flags") = py::none(),
-          py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr, py::arg("tile_rows") = py::none());
+          py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr, py::arg("tile_rows") = py::none(), py::arg("total_rows") = 0);
     m.def("ag_gemm", &ag_gemm);
     m.def("gemm_rs", &gemm_rs);
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));

@@ -66,6 +66,7 @@ class _MoEFunction(torch.autograd.Function):
             lo, hi = bounds[c], bounds[c + 1]
             (rx, rsf), recv_idx, recv_w, handle, ev = disp.pop(c)
             ev.current_stream_wait()
+            total_rows = recv_idx.numel() if local else 0       # (row, lane) pairs: an upper bound of the expert rows
             if local:
                 # One row per (token, rank) came over NVLink; every local expert the token selected gets its copy here, in the
                 # expert's 128-aligned segment (rows in received order).  The copies are private to this call.
@@ -75,7 +76,7 @@ class _MoEFunction(torch.autograd.Function):
             else:
                 rows, pos = handle.num_rows, no_pos
                 tile_group, valid_row, seg_off, tile_rows = G.expert_tiles(handle.psum_num_recv_tokens_per_expert, rows)
-            h = G.grouped_gemm_nt(rx, q13, tile_group, sfa=rsf, sfb=s13, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows)    # [rows, 2I]
+            h = G.grouped_gemm_nt(rx, q13, tile_group, sfa=rsf, sfb=s13, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)    # [rows, 2I]
             if keep_copy and not local:
                 # the received rows live in a receive slot of the buffer that later dispatches will reuse
                 rx, rsf, recv_w = rx.clone(), rsf.clone(), recv_w.clone()
@@ -90,11 +91,11 @@ class _MoEFunction(torch.autograd.Function):
                 comb_done[c - 1].current_stream_wait()
             if local:
                 # the weighted sum over a token's local experts happens here, so one row per (token, rank) travels home
-                y_exp = G.grouped_gemm_nt(a2, q2, tile_group, sfa=sf2, sfb=s2, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows)      # [rows, H]
+                y_exp = G.grouped_gemm_nt(a2, q2, tile_group, sfa=sf2, sfb=s2, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)      # [rows, H]
                 y = G.local_reduce(pos, y_exp, w=recv_w, out=buf.get_combine_buffer(handle))
             else:
                 y = buf.get_combine_buffer(handle)
-                G.grouped_gemm_nt(a2, q2, tile_group, out=y, sfa=sf2, sfb=s2, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows)    # [rows, H] in the combine region
+                G.grouped_gemm_nt(a2, q2, tile_group, out=y, sfa=sf2, sfb=s2, num_sms=gemm_sms, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)    # [rows, H] in the combine region
             kw = dict(previous_event=buf.capture(), allocate_on_comm_stream=True, async_with_compute_stream=True) if pipelined else {}
             _, _, cev = buf.combine(y, handle, weighted=not local, num_sms=comm_sms, out=out[lo:hi], **kw)
             comb_done.append(cev)
@@ -117,6 +118,7 @@ class _MoEFunction(torch.autograd.Function):
             rx, rsf, recv_w, h, tile_group, valid_row, seg_off, pos, tile_rows = ctx.saved_tensors[9 * c:9 * c + 9]
             rw = recv_w.contiguous()
             local, rows = layer.local_expand, h.shape[0]
+            total_rows = pos.numel()                            # as in the forward pass (0 without local expansion)
 
             def send_home(d_rows_exp, d_w_rows):
                 """Backward of dispatch: the gradient rows (and the gradient of every routing weight) travel to the tokens' ranks."""
@@ -133,11 +135,11 @@ class _MoEFunction(torch.autograd.Function):
                 (g_q, g_sf), _, _, _, _ = buf.dispatch(d_out[bounds[c]:bounds[c + 1]], handle=handle, fused_fp8_cast=True, num_sms=layer.num_sms)
                 if local:
                     g_q, g_sf = G.local_expand_copy(pos, g_q, rows, sf=g_sf)
-                d_act_u = G.grouped_gemm_nt(g_q, q2_t, tile_group, sfa=g_sf, sfb=s2_t, buffer=buf, tile_rows=tile_rows)     # [rows, I]
+                d_act_u = G.grouped_gemm_nt(g_q, q2_t, tile_group, sfa=g_sf, sfb=s2_t, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)     # [rows, I]
                 dh, act, d_w_rows = G.swiglu_bwd_rows(d_act_u, h, valid_row, rw)
                 dh_q, dh_sf = G.per_token_cast_to_fp8(dh)
                 d_recv = None if local else buf.get_combine_buffer(handle)
-                d_recv = G.grouped_gemm_nt(dh_q, q13_t, tile_group, out=d_recv, sfa=dh_sf, sfb=s13_t, buffer=buf, tile_rows=tile_rows)
+                d_recv = G.grouped_gemm_nt(dh_q, q13_t, tile_group, out=d_recv, sfa=dh_sf, sfb=s13_t, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)
                 dx, d_topk_w = send_home(d_recv, d_w_rows)
                 # g * w for the weight gradient: the routing weight rides on the scales of the dequantisation
                 dy = G.dequant_rows(g_q, g_sf, valid_row, row_weight=rw)

@@ -25,12 +25,13 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
 
 def grouped_gemm_nt(a: torch.Tensor, b: torch.Tensor, tile_group: torch.Tensor, out: Optional[torch.Tensor] = None,
                     sfa: Optional[torch.Tensor] = None, sfb: Optional[torch.Tensor] = None, num_sms: int = 0, buffer=None,
-                    tile_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
+                    tile_rows: Optional[torch.Tensor] = None, total_rows: int = 0) -> torch.Tensor:
     """Every 128-row tile ``t`` of ``a`` is multiplied by ``b[tile_group[t]]`` (``-1`` skips the tile).  bf16 operands,
     or e4m3 operands with ``sfa [M, K/128]`` and ``sfb [G, N/128, K/128]`` fp32 block scales.  ``buffer``: see
     :func:`gemm_nt`.  ``tile_rows`` int32 (of :func:`expert_tiles`): how many leading rows of every tile count; the kernel may leave
-    the others unread and their results unwritten, which it does for e4m3 with ``N >= 256``."""
-    return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer), tile_rows)
+    the others unread and their results unwritten, which it does for e4m3 with ``N >= 256``.  ``total_rows``: how many token rows all
+    tiles have together at most, for a caller that knows it on the host (0: not known); it helps to choose the kernel."""
+    return _native.load().gemm_nt(a, b, sfa, sfb, tile_group, out, num_sms, None, 0, None, _core_of(buffer), tile_rows, total_rows)
 
 
 def _plain(t: torch.Tensor) -> bool:

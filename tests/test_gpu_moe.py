@@ -481,6 +481,48 @@ def test_thin_tiles_are_read_and_stored_by_rows(counts):
     assert torch.equal(a1.view(torch.uint8)[valid], a.view(torch.uint8)[valid]) and torch.equal(s1[valid], s[valid])
 
 
+@pytest.mark.parametrize('G,N,K,num_sms', [(64, 264, 1168, 0), (64, 264, 1168, 37), (8, 2056, 640, 0), (3, 1000, 6912, 5), (13, 2048, 16, 0), (16, 256, 128, 148)])
+def test_products_that_stream_the_weights(G, N, K, num_sms):
+    """Thin tiles, at most one per expert: the bits of the 256-column kernel (which takes the product when no tile_rows are given), with every
+    number of token rows at which the kernel changes its way, idle tiles, two tiles of one group, a ragged last tile, odd K blocks,
+    columns that end inside a tile, last waves that are cut and whole, and scales in either order; a bound on the rows that rules the
+    kernel out changes nothing."""
+    from deepep_ascend_b200.ops import gemm as ops
+    gen = torch.Generator(device='cuda').manual_seed(N)
+    edges = [1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 127, 128, 0, 40]
+    tiles = G if G < 16 else 48
+    rows = torch.tensor([edges[(5 * t + G) % len(edges)] for t in range(tiles)], dtype=torch.int32, device='cuda')
+    M = tiles * 128 - 72                                          # the last tile has 56 rows in the tensor
+    rows[-1] = 128
+    group = torch.arange(tiles, dtype=torch.int32, device='cuda') * G // tiles
+    group[1] = group[0]
+    group[2] = -1
+
+    def e4m3(*shape):
+        b = torch.randint(0, 256, shape, dtype=torch.uint8, device='cuda', generator=gen)
+        return torch.where((b & 0x7f) == 0x7f, 0, b).to(torch.uint8).view(torch.float8_e4m3fn)
+    a, w = e4m3(M, K), e4m3(G, N, K)
+    sa = torch.rand(M, (K + 127) // 128, device='cuda', generator=gen) + 0.5
+    sb = torch.rand(G, (N + 127) // 128, (K + 127) // 128, device='cuda', generator=gen) + 0.5
+    want = ops.grouped_gemm_nt(a, w, group, sfa=sa, sfb=sb, num_sms=num_sms)
+    at = torch.arange(M, device='cuda')
+    valid = (at % 128 < rows[at // 128]) & (group[at // 128] >= 0)
+    a.view(torch.uint8)[~valid] = 0x7f
+    for scales, bound in ((sa, 0), (sa.t().contiguous().t(), 1), (sa, M)):
+        out = torch.full((M, N + 8), 7.0, dtype=torch.bfloat16, device='cuda')
+        ops.grouped_gemm_nt(a, w, group, out=out[:, :N], sfa=scales, sfb=sb, num_sms=num_sms, tile_rows=rows, total_rows=bound)
+        assert torch.equal(out[valid, :N], want[valid]) and bool((out[~valid] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    # and the product itself, in 64 bits: sums of K products in 32 bits and one rounding to bf16 (2^-8)
+    t = 0
+    r = int(rows[t])
+    k_scale = lambda s: s.repeat_interleave(128, dim=-1)[..., :K]    # noqa: E731
+    x = a[:r].double() * k_scale(sa[:r]).double()
+    y = w[0].double() * k_scale(sb[0].repeat_interleave(128, dim=0)[:N]).double()
+    exact = x @ y.t()
+    bound = exact.abs() * 2.0**-8 + (x.abs() @ y.abs().t()) * K * 2.0**-24
+    assert bool(((out[:r, :N].double() - exact).abs() <= bound).all())
+
+
 @pytest.mark.parametrize('rows,H,I', [(128, 128, 128), (384, 7168, 384), (2048, 1024, 2048)])
 @pytest.mark.parametrize('captured', [False, True])
 def test_kernels_that_start_before_the_one_before_has_ended(rows, H, I, captured):
