@@ -236,7 +236,8 @@ __host__ __device__ constexpr bool few_waves(int num_tiles, int ctas) { return n
 template <bool kFp8, int kBlockN, int kMnOperands>
 __global__ void __launch_bounds__(gemm_threads(kFp8, kBlockN), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-            const __grid_constant__ std::conditional_t<kFp8 && kBlockN == 256, CUtensorMap, int> map_a32, const GemmArgs g) {
+            const __grid_constant__ std::conditional_t<kFp8 && kBlockN == 256, CUtensorMap, int> map_a32,
+            const __grid_constant__ std::conditional_t<kFp8 && kBlockN == 256, CUtensorMap, int> map_b128, const GemmArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kStages = num_stages(kBlockN, kFp8);
     constexpr int kTileBytesB = kBlockN * 128;
@@ -377,11 +378,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 umma::tma_load_3d(s_b + p.stage * kTileBytesB + i * umma::kMnChunkBytes, &map_b, n_blk * kBlockN + i * 64, kb * kBlockK, grp,
                                                   &sm->full[p.stage]);
                         } else if constexpr (kWide) {
-                            // boxes of 128 rows: both halves of the tile, or one
+                            // the whole tile in one box (128 rows x 4096 x 7168 x 32: 216 us, in two boxes 219), or one half of it
                             const int b_row = grp * g.N + n_blk * kBlockN + (tw.half > 0 ? 128 : 0);
-                            umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, b_row, &sm->full[p.stage]);
-                            if (tw.half < 0)
-                                umma::tma_load_2d(s_b + p.stage * kTileBytesB + kTileBytesB / 2, &map_b, kb * kBlockK, b_row + 128, &sm->full[p.stage]);
+                            umma::tma_load_2d(s_b + p.stage * kTileBytesB, tw.half < 0 ? &map_b : &map_b128, kb * kBlockK, b_row, &sm->full[p.stage]);
                         } else {
                             umma::tma_load_2d(s_b + p.stage * kTileBytesB, &map_b, kb * kBlockK, grp * g.N + n_blk * kBlockN, &sm->full[p.stage]);
                         }
@@ -1299,14 +1298,17 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     }
     if (g.mn_operands < 0 || g.mn_operands > 2 || (g.mn_operands != 0 && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE))) return cudaErrorInvalidValue;
     if ((g.mn_operands == 2) != (g.k_group_off != nullptr && g.mn_operands != 0)) return cudaErrorInvalidValue;
-    CUtensorMap map_a, map_b, map_a32;
+    CUtensorMap map_a, map_b, map_a32, map_b128;
     const int64_t b_groups = g.k_group_off != nullptr ? 1 : g.num_groups;
     const bool maps_ok = (g.mn_operands >= 2 ? make_mn_operand_map(&map_a, g.a, 1, g.K, g.M, g.lda)
                                              : make_operand_map(&map_a, g.a, g.M, g.K, g.lda, g.is_fp8, 128)) &&
                          (g.mn_operands >= 1 ? make_mn_operand_map(&map_b, g.b, b_groups, g.K, g.N, g.ldb)
-                                             : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, g.is_fp8 ? 128 : block_n));
+                                             : make_operand_map(&map_b, g.b, b_groups * g.N, g.K, g.ldb, g.is_fp8, block_n));
     if (!maps_ok) return cudaErrorInvalidValue;
     map_a32 = map_a;
+    map_b128 = map_b;
+    // halves of a thin last wave: only the wide e4m3 kernel reads them
+    if (g.is_fp8 && block_n == 256 && !make_operand_map(&map_b128, g.b, b_groups * g.N, g.K, g.ldb, true, 128)) return cudaErrorInvalidValue;
     // boxes of 32 rows for thin tiles: only the wide e4m3 kernel reads them
     if (g.is_fp8 && block_n == 256 && g.tile_rows != nullptr && !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32)) return cudaErrorInvalidValue;
     const void* fn;
@@ -1322,7 +1324,7 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     if (g.k_group_off != nullptr && (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE || g.tile_group != nullptr || g.num_groups < 1)) return cudaErrorInvalidValue;
     const int num_tiles = ((g.M + kBlockM - 1) / kBlockM) * ((g.N + block_n - 1) / block_n) * (g.k_group_off != nullptr ? g.num_groups : 1);
     int ctas = num_sms < 1 ? 1 : num_sms;
-    void* params[] = {&map_a, &map_b, &map_a32, const_cast<GemmArgs*>(&g)};
+    void* params[] = {&map_a, &map_b, &map_a32, &map_b128, const_cast<GemmArgs*>(&g)};
     if (g.fuse != EP_GEMM_FUSE_NONE) {
         // the CTAs of a fused launch wait on one another (grid barrier, copier -> producer flags): cooperative launch
         const int R = g.ctx.num_ranks;
