@@ -378,7 +378,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 umma::tma_load_3d(s_b + p.stage * kTileBytesB + i * umma::kMnChunkBytes, &map_b, n_blk * kBlockN + i * 64, kb * kBlockK, grp,
                                                   &sm->full[p.stage]);
                         } else if constexpr (kWide) {
-                            // the whole tile in one box (128 rows x 4096 x 7168 x 32: 216 us, in two boxes 219), or one half of it
+                            // the whole tile in one box (128 rows x 4096 x 7168 x 32: 212 us, in two boxes 216), or one half of it
                             const int b_row = grp * g.N + n_blk * kBlockN + (tw.half > 0 ? 128 : 0);
                             umma::tma_load_2d(s_b + p.stage * kTileBytesB, tw.half < 0 ? &map_b : &map_b128, kb * kBlockK, b_row, &sm->full[p.stage]);
                         } else {
