@@ -363,7 +363,7 @@ struct MoeBwdArgs {
     // DEQUANT_T: y = q [rows, H] e4m3, w = scales (row, 128-block) at w[row * sf_stride_row + blk * sf_stride_col]
     //       -> out_t = (q * scale)^T [H, rows] bf16
     // SWIGLU_ROWS: g, y, w as SWIGLU (w required) -> out = d_h [rows, 2I], out2 = silu(gate) * up [rows, I],
-    //       row_dot[row] = sum of d_act * activation
+    //       row_dot[row] = sum of d_act * activation; optional q [rows, 2I] and q_sf [rows, 2I / 128]: d_h in e4m3 (I % 128 == 0)
     // DEQUANT_ROWS: y, w as DEQUANT_T, optional row_w -> out = q * (scale * row_w[row]) [rows, H] bf16
     // WEIGHT_ROWS: g [rows, H], row_w -> out = g * row_w[row]
     const void* g;
@@ -376,6 +376,8 @@ struct MoeBwdArgs {
     void* out2_t;
     void* out2;
     float* row_dot;
+    void* q;
+    float* q_sf;
 };
 
 // Bookkeeping of the expand layout for a grouped GEMM (see expert_segments_kernel).  The start of a segment is a tile

@@ -398,6 +398,27 @@ __global__ void __launch_bounds__(kTileThreads) moe_bwd_dequant_t_kernel(const M
 // Row-major results only, for weight-gradient GEMMs that read MN-major operands (`gemm_kgrouped_tn`): one warp per row, no shared
 // memory, every byte read and written once, so the kernels are bound by HBM (0.15 ms each for 34816 rows of 7168 / 2 x 2048).
 constexpr int kRowWarps = 8;
+
+// e4m3 of eight channels of a lane whose 16 neighbours hold the rest of a 128-channel group: the arithmetic of the stand-alone cast
+__device__ __forceinline__ uint2 cast_group(const float (&v)[8], float& amax) {
+    amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+    amax = fmaxf(ptx::warp_max_16(amax), 1e-4f);
+    const float scale = __fmul_rn(448.f, __frcp_rn(amax));
+    uint32_t packed[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] * scale, v[4 * j + 1] * scale), __NV_SATFINITE, __NV_E4M3);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j + 2] * scale, v[4 * j + 3] * scale), __NV_SATFINITE, __NV_E4M3);
+        packed[j] = lo | (hi << 16);
+    }
+    return make_uint2(packed[0], packed[1]);
+}
+
+// kQuant: d_h also leaves as e4m3 with 1 x 128 scales, for the data gradient on the e4m3 tensor cores (cols % 128 == 0).  A cast of its own
+// reads d_h once more: 14336 rows x 2 x 1024 33 + 17 us apart, 41 together (196 MB, 4.8 TB/s), 34816 x 2 x 2048 144 + 83 / 177.
+template <bool kQuant>
 __global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_swiglu_rows_kernel(const MoeBwdArgs a) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
@@ -407,8 +428,14 @@ __global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_swiglu_rows_kernel(con
     const uint8_t* hb = reinterpret_cast<const uint8_t*>(a.y) + static_cast<int64_t>(row) * I * 4;
     uint8_t* ob = reinterpret_cast<uint8_t*>(a.out) + static_cast<int64_t>(row) * I * 4;
     uint8_t* ab = reinterpret_cast<uint8_t*>(a.out2) + static_cast<int64_t>(row) * I * 2;
+    uint8_t* qb = kQuant ? reinterpret_cast<uint8_t*>(a.q) + static_cast<int64_t>(row) * 2 * I : nullptr;
+    float* sf = kQuant ? a.q_sf + static_cast<int64_t>(row) * (2 * I / 128) : nullptr;
     if (a.valid[row] == 0) {
         const int4 zero = make_int4(0, 0, 0, 0);
+        if constexpr (kQuant) {
+            for (int col = lane * 16; col < 2 * I; col += 512) *reinterpret_cast<int4*>(qb + col) = zero;
+            for (int grp = lane; grp < 2 * I / 128; grp += 32) sf[grp] = __fdiv_rn(1e-4f, 448.f);
+        }
         for (int col = lane * 8; col < I; col += 256) {
             *reinterpret_cast<int4*>(ob + col * 2) = zero;
             *reinterpret_cast<int4*>(ob + (I + col) * 2) = zero;
@@ -418,13 +445,17 @@ __global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_swiglu_rows_kernel(con
         return;
     }
     const float wr = __ldg(a.w + row);
-    float dot = 0.f;
+    float dot = 0.f, kept_g = 0.f, kept_u = 0.f;
 #pragma unroll 2
-    for (int col = lane * 8; col < I; col += 256) {
+    for (int col0 = 0; col0 < I; col0 += 256) {
+        const int col = col0 + lane * 8;
+        if (!kQuant && col >= I) break;
+        const bool in_range = !kQuant || col < I;        // the cast needs whole warps for its shuffles
         float d[8], gate[8], up[8], dg[8], du[8], act[8];
-        unpack8(ptx::ld_nc_v4(db + col * 2), d);
-        unpack8(ptx::ld_nc_v4(hb + col * 2), gate);
-        unpack8(ptx::ld_nc_v4(hb + (I + col) * 2), up);
+        const int4 none = make_int4(0, 0, 0, 0);
+        unpack8(in_range ? ptx::ld_nc_v4(db + col * 2) : none, d);
+        unpack8(in_range ? ptx::ld_nc_v4(hb + col * 2) : none, gate);
+        unpack8(in_range ? ptx::ld_nc_v4(hb + (I + col) * 2) : none, up);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float sig = 1.f / (1.f + __expf(-gate[j]));
@@ -434,9 +465,36 @@ __global__ void __launch_bounds__(kRowWarps * 32) moe_bwd_swiglu_rows_kernel(con
             du[j] = dj * gate[j] * sig;
             dg[j] = dj * up[j] * sig * (1.f + gate[j] * (1.f - sig));
         }
-        *reinterpret_cast<int4*>(ob + col * 2) = pack8(dg);
-        *reinterpret_cast<int4*>(ob + (I + col) * 2) = pack8(du);
-        *reinterpret_cast<int4*>(ab + col * 2) = pack8(act);
+        const int4 dg_raw = pack8(dg), du_raw = pack8(du);
+        if (in_range) {
+            *reinterpret_cast<int4*>(ob + col * 2) = dg_raw;
+            *reinterpret_cast<int4*>(ob + (I + col) * 2) = du_raw;
+            *reinterpret_cast<int4*>(ab + col * 2) = pack8(act);
+        }
+        if constexpr (kQuant) {
+            // the cast sees the values that were rounded to bf16
+            unpack8(dg_raw, dg);
+            unpack8(du_raw, du);
+            float amax_g, amax_u;
+            const uint2 qg = cast_group(dg, amax_g), qu = cast_group(du, amax_u);
+            if (in_range) {
+                *reinterpret_cast<uint2*>(qb + col) = qg;
+                *reinterpret_cast<uint2*>(qb + I + col) = qu;
+            }
+            // the divisions of 16 steps together, one group of each half per lane
+            const int step = col0 / 256;
+            if ((lane & 15) == (step & 15)) {
+                kept_g = amax_g;
+                kept_u = amax_u;
+            }
+            if ((step & 15) == 15 || col0 + 256 >= I) {
+                const int grp = ((step & ~15) + (lane & 15)) * 2 + (lane >> 4);
+                if ((lane & 15) <= (step & 15) && grp < I / 128) {
+                    sf[grp] = __fdiv_rn(kept_g, 448.f);
+                    sf[I / 128 + grp] = __fdiv_rn(kept_u, 448.f);
+                }
+            }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
@@ -811,7 +869,10 @@ cudaError_t launch_moe_bwd(const MoeBwdArgs& a, cudaStream_t stream) {
     if (a.op == EP_MOE_BWD_SWIGLU_ROWS || a.op == EP_MOE_BWD_DEQUANT_ROWS || a.op == EP_MOE_BWD_WEIGHT_ROWS) {
         const int blocks = (a.rows + kRowWarps - 1) / kRowWarps;
         if (a.cols % (a.op == EP_MOE_BWD_DEQUANT_ROWS ? 16 : 8) != 0) return cudaErrorInvalidValue;
-        if (a.op == EP_MOE_BWD_SWIGLU_ROWS) moe_bwd_swiglu_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
+        if (a.op == EP_MOE_BWD_SWIGLU_ROWS && a.q != nullptr) {
+            if (a.cols % 128 != 0 || !aligned(a.q, 16) || a.q_sf == nullptr) return cudaErrorInvalidValue;
+            moe_bwd_swiglu_rows_kernel<true><<<blocks, kRowWarps * 32, 0, stream>>>(a);
+        } else if (a.op == EP_MOE_BWD_SWIGLU_ROWS) moe_bwd_swiglu_rows_kernel<false><<<blocks, kRowWarps * 32, 0, stream>>>(a);
         else if (a.op == EP_MOE_BWD_DEQUANT_ROWS) moe_bwd_dequant_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
         else moe_bwd_weight_rows_kernel<<<blocks, kRowWarps * 32, 0, stream>>>(a);
         return cudaGetLastError();

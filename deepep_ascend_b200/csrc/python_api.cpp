@@ -458,7 +458,7 @@ at::Tensor gemm_kgrouped_tn(const at::Tensor& a, const at::Tensor& b, const at::
 }
 
 // Backward of SwiGLU with row-major results: (d_h [rows, 2I], activation [rows, I], d loss / d row_weight [rows])
-std::vector<at::Tensor> swiglu_bwd_rows(const at::Tensor& d_act, const at::Tensor& h, const at::Tensor& valid, const at::Tensor& row_weight) {
+std::vector<at::Tensor> swiglu_bwd_rows(const at::Tensor& d_act, const at::Tensor& h, const at::Tensor& valid, const at::Tensor& row_weight, bool quantize) {
     TORCH_CHECK(d_act.is_cuda() && d_act.dim() == 2 && d_act.is_contiguous() && d_act.scalar_type() == at::kBFloat16, "d_act must be contiguous bf16 [rows, I]");
     const int64_t rows = d_act.size(0), I = d_act.size(1);
     TORCH_CHECK(h.is_cuda() && h.is_contiguous() && h.scalar_type() == at::kBFloat16 && h.dim() == 2 && h.size(0) == rows && h.size(1) == 2 * I,
@@ -478,8 +478,16 @@ std::vector<at::Tensor> swiglu_bwd_rows(const at::Tensor& d_act, const at::Tenso
     a.out = out.data_ptr();
     a.out2 = act.data_ptr();
     a.row_dot = dot.data_ptr<float>();
+    std::vector<at::Tensor> results{out, act, dot};
+    if (quantize) {
+        TORCH_CHECK(I % 128 == 0, "the e4m3 gradient needs whole 128-channel groups");
+        results.push_back(at::empty({rows, 2 * I}, h.options().dtype(at::kFloat8_e4m3fn)));
+        results.push_back(at::empty({rows, 2 * I / 128}, h.options().dtype(at::kFloat)));
+        a.q = results[3].data_ptr();
+        a.q_sf = results[4].data_ptr<float>();
+    }
     cuda_check(ep::launch_moe_bwd(a, at::cuda::getCurrentCUDAStream()), "SwiGLU backward launch");
-    return {out, act, dot};
+    return results;
 }
 
 // g * w[:, None] in bf16 [rows, H]; padding rows give zeros
@@ -893,7 +901,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("grouped_gemm_nn", &grouped_gemm_nn, py::arg("a"), py::arg("b"), py::arg("tile_group"), py::arg("out") = py::none(), py::arg("num_sms") = 0,
           py::arg("report_to") = nullptr);
     m.def("gemm_kgrouped_tn", &gemm_kgrouped_tn, py::arg("a"), py::arg("b"), py::arg("k_off"), py::arg("num_sms") = 0);
-    m.def("swiglu_bwd_rows", &swiglu_bwd_rows);
+    m.def("swiglu_bwd_rows", &swiglu_bwd_rows, py::arg("d_act"), py::arg("h"), py::arg("valid"), py::arg("row_weight"), py::arg("quantize") = false);
     m.def("weighted_rows", &weighted_rows);
     m.def("dequant_rows", &dequant_rows, py::arg("q"), py::arg("sf"), py::arg("valid"), py::arg("row_weight") = py::none());
     m.def("moe_bwd_prep", &moe_bwd_prep);

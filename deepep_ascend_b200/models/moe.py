@@ -136,8 +136,7 @@ class _MoEFunction(torch.autograd.Function):
                 if local:
                     g_q, g_sf = G.local_expand_copy(pos, g_q, rows, sf=g_sf)
                 d_act_u = G.grouped_gemm_nt(g_q, q2_t, tile_group, sfa=g_sf, sfb=s2_t, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)     # [rows, I]
-                dh, act, d_w_rows = G.swiglu_bwd_rows(d_act_u, h, valid_row, rw)
-                dh_q, dh_sf = G.per_token_cast_to_fp8(dh)
+                dh, act, d_w_rows, dh_q, dh_sf = G.swiglu_bwd_rows_fp8(d_act_u, h, valid_row, rw)
                 d_recv = None if local else buf.get_combine_buffer(handle)
                 d_recv = G.grouped_gemm_nt(dh_q, q13_t, tile_group, out=d_recv, sfa=dh_sf, sfb=s13_t, buffer=buf, tile_rows=tile_rows, total_rows=total_rows)
                 dx, d_topk_w = send_home(d_recv, d_w_rows)

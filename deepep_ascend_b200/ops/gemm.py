@@ -216,6 +216,12 @@ def swiglu_bwd_rows(d_act: torch.Tensor, h: torch.Tensor, valid_row: torch.Tenso
     return _native.load().swiglu_bwd_rows(d_act, h, valid_row, row_weight)
 
 
+def swiglu_bwd_rows_fp8(d_act: torch.Tensor, h: torch.Tensor, valid_row: torch.Tensor, row_weight: torch.Tensor):
+    """:func:`swiglu_bwd_rows` with two more results, :func:`per_token_cast_to_fp8` of its ``d_h``: ``(d_h, activation,
+    d loss / d row_weight, e4m3 d_h [rows, 2I], scales [rows, 2I / 128])``; ``I % 128 == 0``."""
+    return _native.load().swiglu_bwd_rows(d_act, h, valid_row, row_weight, True)
+
+
 def weighted_rows(g_rows: torch.Tensor, w: torch.Tensor, valid_row: torch.Tensor) -> torch.Tensor:
     """``g * w[:, None]`` as bf16 ``[rows, H]``; padding rows give zeros whatever they hold."""
     return _native.load().weighted_rows(g_rows, w, valid_row)

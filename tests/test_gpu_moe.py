@@ -395,6 +395,23 @@ def test_row_major_backward_kernels(rows, I, H):
     assert torch.equal(ops.weighted_rows(x, w, valid), torch.where(vm, ref, torch.zeros_like(ref)))
 
 
+@pytest.mark.parametrize('rows,I', [(1, 128), (67, 384), (300, 1920), (256, 2048)])
+def test_swiglu_backward_with_cast(rows, I):
+    """The SwiGLU gradient that also leaves in e4m3: the bits of the kernel without and of the stand-alone cast of its result (whole and
+    half steps of 256 channels, masked rows with NaN payloads, a row of zeros)."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows + I)
+    valid = torch.rand(rows, device='cuda') > 0.2
+    d_act, h = torch.randn(rows, I, device='cuda').bfloat16(), torch.randn(rows, 2 * I, device='cuda').bfloat16()
+    w = torch.rand(rows, device='cuda')
+    w[0] = 0.0
+    d_act[~valid], h[~valid] = float('nan'), float('nan')
+    want = ops.swiglu_bwd_rows(d_act, h, valid, w)
+    want = (*want, *ops.per_token_cast_to_fp8(want[0]))
+    for got, ref in zip(ops.swiglu_bwd_rows_fp8(d_act, h, valid, w), want):
+        assert got.shape == ref.shape and got.dtype == ref.dtype and torch.equal(got.view(torch.uint8), ref.view(torch.uint8))
+
+
 @pytest.mark.parametrize('K', [1, 6, 8, 16])
 def test_expand_copy_of_few_scale_columns(K):
     """Scale rows whose last 32-column step has fewer columns than there are top-k lanes (hidden 512 .. 5120)."""
