@@ -440,6 +440,8 @@ int local_expand_pairs_per_cta();      // (row, k) pairs that one CTA of the pla
 cudaError_t launch_local_expand_layout(const LocalExpandPlanArgs& args, const ExpertSegmentsArgs& seg, cudaStream_t stream);
 cudaError_t launch_local_expand_copy(const LocalExpandCopyArgs& args, cudaStream_t stream);
 cudaError_t launch_local_reduce(const LocalReduceArgs& args, cudaStream_t stream);
+// out[i] = pos[i] >= 0 ? v[pos[i]] : 0
+cudaError_t launch_local_gather(const int32_t* pos, const float* v, float* out, int64_t total, cudaStream_t stream);
 cudaError_t launch_expert_segments(const ExpertSegmentsArgs& args, cudaStream_t stream);
 cudaError_t launch_weight_quant(const WeightQuantArgs& args, cudaStream_t stream);
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& args, cudaStream_t stream);

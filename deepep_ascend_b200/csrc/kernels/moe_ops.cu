@@ -5,6 +5,8 @@
 // ones; those that also write transposed results serve callers of the K-major weight-gradient product (`gemm_kgrouped`).
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace ep {
@@ -859,7 +861,22 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_reduce_kernel(const L
         }
     }
 }
+
+// One value per (row, k) pair from its expert row.  Bound by its launch: in PyTorch operations it was six of them.
+__global__ void __launch_bounds__(256) local_gather_kernel(const int32_t* pos, const float* v, float* out, int total) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+        const int at = __ldg(pos + i);
+        out[i] = at >= 0 ? __ldg(v + at) : 0.f;
+    }
+}
 }  // namespace
+
+cudaError_t launch_local_gather(const int32_t* pos, const float* v, float* out, int64_t total, cudaStream_t stream) {
+    if (total == 0) return cudaSuccess;
+    if (total < 0 || total > 0x7fffffff - 256 * 1024) return cudaErrorInvalidValue;
+    local_gather_kernel<<<static_cast<int>(std::min<int64_t>(1024, (total + 255) / 256)), 256, 0, stream>>>(pos, v, out, static_cast<int>(total));
+    return cudaGetLastError();
+}
 
 int moe_bwd_prep_col_blocks(int cols) { return (cols + kPrepCols - 1) / kPrepCols; }
 

@@ -386,6 +386,15 @@ at::Tensor local_reduce(const at::Tensor& pos, const at::Tensor& y, const std::o
     return res;
 }
 
+at::Tensor local_gather(const at::Tensor& pos, const at::Tensor& values) {
+    TORCH_CHECK(pos.is_cuda() && pos.is_contiguous() && pos.scalar_type() == at::kInt && pos.dim() == 2, "pos must be contiguous int32 [rows, K]");
+    TORCH_CHECK(values.is_cuda() && values.is_contiguous() && values.dim() == 1 && values.scalar_type() == at::kFloat, "values must be contiguous fp32 [expert rows]");
+    at::Tensor out = at::empty(pos.sizes(), values.options());
+    cuda_check(ep::launch_local_gather(pos.data_ptr<int32_t>(), values.data_ptr<float>(), out.data_ptr<float>(), pos.numel(), at::cuda::getCurrentCUDAStream()),
+               "local_gather launch");
+    return out;
+}
+
 const float* row_weight_ptr(const at::Tensor& w, int64_t rows) {
     TORCH_CHECK(w.is_cuda() && w.is_contiguous() && w.scalar_type() == at::kFloat && w.numel() == rows, "row weights must be fp32 [rows]");
     return w.data_ptr<float>();
@@ -893,6 +902,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("local_expand_layout", &local_expand_layout);
     m.def("local_expand_copy", &local_expand_copy, py::arg("pos"), py::arg("x"), py::arg("num_out"), py::arg("sf") = py::none(),
           py::arg("w") = py::none());
+    m.def("local_gather", &local_gather);
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("expert_segments", &expert_segments, py::arg("psum_ends"), py::arg("num_rows"), py::arg("alignment") = 128);
     m.def("quantize_weight_blocks", &quantize_weight_blocks);

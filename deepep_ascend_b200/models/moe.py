@@ -125,8 +125,7 @@ class _MoEFunction(torch.autograd.Function):
                 if not local:
                     return buf.combine(d_rows_exp, handle, topk_weights=d_w_rows, num_sms=layer.num_sms)[:2]
                 d_recv = G.local_reduce(pos, d_rows_exp, out=buf.get_combine_buffer(handle))
-                d_w = torch.where(pos >= 0, d_w_rows[pos.clamp(min=0).long()], torch.zeros((), device=pos.device))
-                return buf.combine(d_recv, handle, topk_weights=d_w, num_sms=layer.num_sms)[:2]
+                return buf.combine(d_recv, handle, topk_weights=G.local_gather(pos, d_w_rows), num_sms=layer.num_sms)[:2]
             if layer.fp8_backward:
                 # Data gradients on the e4m3 tensor cores, as the forward GEMMs: the gradient rows are cast (1 x 128 scales)
                 # inside the dispatch kernel, the weights are the forward e4m3 weights transposed (128 x 128 blocks stay

@@ -173,6 +173,11 @@ def local_reduce(pos: torch.Tensor, y: torch.Tensor, w: Optional[torch.Tensor] =
     return _native.load().local_reduce(pos, y, w, out)
 
 
+def local_gather(pos: torch.Tensor, values: torch.Tensor) -> torch.Tensor:
+    """``values[pos]`` for one fp32 value per expert row: fp32 ``[rows, K]``, zero where ``pos`` is -1."""
+    return _native.load().local_gather(pos, values)
+
+
 def per_token_cast_to_fp8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """bf16 ``[rows, H]`` -> (e4m3 ``[rows, H]``, fp32 scales ``[rows, ceil(H / 128)]``), one kernel."""
     q, sf = _native.load().per_token_cast_to_fp8(x.contiguous())

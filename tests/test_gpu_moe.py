@@ -466,6 +466,18 @@ def test_expand_plan_over_many_ctas(rows, K, El):
         assert torch.equal(got.cpu(), want)
 
 
+@pytest.mark.parametrize('rows,K', [(0, 3), (1, 1), (85, 3), (5000, 8), (40000, 7)])
+def test_local_gather(rows, K):
+    """Less than a block, ragged blocks, more than the grid covers at once; a NaN in a row nobody asks for stays out."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows)
+    v = torch.randn(max(1, rows * K), device='cuda')
+    v[0] = float('nan')
+    pos = torch.randint(-1, v.numel(), (rows, K), device='cuda', dtype=torch.int32)
+    pos[pos == 0] = -1
+    assert torch.equal(ops.local_gather(pos, v), torch.where(pos >= 0, v[pos.clamp(min=0).long()], torch.zeros((), device='cuda')))
+
+
 @pytest.mark.parametrize('counts', [[1, 31, 32, 33], [64, 0, 65, 96, 97], [127, 128, 129, 300, 0]])
 def test_thin_tiles_are_read_and_stored_by_rows(counts):
     """Tiles with few token rows: results of those rows are those of the whole-tile product, other rows of the output and of the
