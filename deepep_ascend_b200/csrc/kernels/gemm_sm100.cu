@@ -1277,6 +1277,10 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
             return (tiles + workers - 1) / workers * (bn + 16);     // waves x (columns + per-tile overhead)
         };
         if (cost(224) < cost(256)) block_n = 224;
+        // Few tiles: 128 columns, where that still makes one wave (a K block of half the columns takes about 0.65 of the time).  In a CUDA
+        // graph, 256 / 128 columns: 1000 x 2048 x 7168 (64 / 128 tiles) 36.0 / 26.9 us, 64 x 4096 x 4096 (16 / 32) 19.5 / 12.9, 1024^3 (32 / 64)
+        // 9.3 / 6.6; with more than a wave of them 1315 x 2536 x 3144 (110 / 220) 32.6 / 44.7.
+        if (g.fuse == EP_GEMM_FUSE_NONE && num_m_tiles * ((g.N + 127) / 128) * groups <= workers) block_n = 128;
     }
     if (streams_weights(g)) {
         CUtensorMap map_a, map_a32, map_w, map_w32;

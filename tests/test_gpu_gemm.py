@@ -11,7 +11,7 @@ def _C():
 
 
 @pytest.mark.parametrize('M,N,K', [(128, 128, 64), (128, 128, 256), (256, 384, 512), (1000, 520, 1096), (4096, 2048, 7168),
-                                   (1024, 896, 1024), (2048, 7168, 512)])
+                                   (1024, 896, 1024), (2048, 7168, 512), (18944, 896, 64), (130, 1000, 1096)])
 def test_bf16_gemm(M, N, K):
     """Shapes that take each of the three tile widths (128, 224 and 256 columns; the launcher picks by tile count)."""
     C = _C()
