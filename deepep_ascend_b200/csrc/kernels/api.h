@@ -311,11 +311,18 @@ struct GemmArgs {
     // bf16 operands stored MN-major (K rows of contiguous elements), read through the tensor core's transposing descriptors:
     // 0 none; 1 B is [num_groups][K, N] (row stride ldb); 2 (with k_group_off) A is [K, M] and B is [K, N]
     int mn_operands;
+    // the K blocks of every tile shared out over `k_splits` CTAs (gemm_k_splits; 0 or 1: not): their sums lie in partial [k_splits, M, N] on
+    // their way to a second kernel that adds them
+    int k_splits;
+    float* partial;
 };
+
 enum { EP_GEMM_FUSE_NONE = 0, EP_GEMM_FUSE_ALL_GATHER = 1, EP_GEMM_FUSE_REDUCE_SCATTER = 2 };
 
 namespace ep {
 cudaError_t launch_gemm(const GemmArgs& args, int num_sms, cudaStream_t stream);
+// into how many parts along K a product should be cut on this many SMs (GemmArgs::k_splits)
+int gemm_k_splits(const GemmArgs& args, int num_sms);
 }  // namespace ep
 
 // ------------------------------------------------------------------------------------------------ MoE helpers

@@ -233,7 +233,9 @@ __host__ __device__ constexpr bool few_waves(int num_tiles, int ctas) { return n
 
 // kMnOperands: how many operands are MN-major (bf16 only).  0: A [M, K], B [N, K].  1: B is [K, N] (data gradients read the forward
 // weights as they are).  2: A is [K, M] too (weight gradients read row-major activations and gradients as they are).
-template <bool kFp8, int kBlockN, int kMnOperands>
+// kSplits: a tile's K blocks are shared out over CTAs (g.k_splits), and the sums leave in 32 bits (an instance of its own: the
+// branches would cost small products 2 to 4 %)
+template <bool kFp8, int kBlockN, int kMnOperands, bool kSplits = false>
 __global__ void __launch_bounds__(gemm_threads(kFp8, kBlockN), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
             const __grid_constant__ std::conditional_t<kFp8 && kBlockN == 256, CUtensorMap, int> map_a32,
@@ -244,6 +246,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     constexpr int kAccBufs = (kFp8 && kBlockN == 128) ? 4 : 2;   // accumulator buffers of kBlockN fp32 columns in tensor memory
     constexpr int kEpiWarps = kFp8 ? 8 : 4;
     constexpr bool kWide = kFp8 && kBlockN == 256;   // register re-allocation between warpgroups
+    static_assert(!kSplits || (!kFp8 && kBlockN == 128 && kMnOperands == 0), "plain bf16 products of few tiles");
     constexpr int kEpiWarp0 = kWide ? 4 : 2;         // first epilogue warp
     constexpr int kTmemColumns = kAccBufs * kBlockN <= 256 ? 256 : 512;   // allocations are powers of two
     static_assert(kBlockN % 32 == 0 && kBlockN >= 32 && kBlockN <= 256 && kAccBufs * kBlockN <= 512, "tile width");
@@ -267,7 +270,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // thin last wave cannot pull the bandwidth that is free.
     const int rem = num_tiles % gemm_ctas;
     const bool cut_last = kWide && 2 * rem <= gemm_ctas;
-    const int whole_items = cut_last ? num_tiles - rem : num_tiles, num_items = cut_last ? num_tiles + rem : num_tiles;
+    const int whole_items = cut_last ? num_tiles - rem : num_tiles;
+    const int num_items = kSplits ? num_tiles * g.k_splits : cut_last ? num_tiles + rem : num_tiles;
     // output staging: of the 256-column variants, and of the reduce-scatter in the bf16 128-column one (narrow products, mostly of one
     // wave: 64 x 128 x 128 takes 5.0 us with direct stores, 5.3 us staged)
     uint8_t* s_epi = smem + kStages * (kTileBytes + kTileBytesB) + 1024;
@@ -278,6 +282,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int group_m = g.fuse == EP_GEMM_FUSE_ALL_GATHER ? min(8, tiles_per_shard) : 16;
 
     auto item_work = [&](int item) {
+        if constexpr (kSplits) {
+            // a part of the K blocks; its sums go to rows of their own in the workspace
+            const int part = item / num_tiles;
+            TileWork w = tile_work(g, item - part * num_tiles, num_m, num_n, num_k, group_m, kBlockK);
+            w.kb0 = num_k * part / g.k_splits;
+            w.kb1 = num_k * (part + 1) / g.k_splits;
+            w.c_row0 = static_cast<int64_t>(part) * g.M;
+            return w;
+        }
         if (!kWide || item < whole_items) return tile_work(g, item, num_m, num_n, num_k, group_m, kBlockK);
         TileWork w = tile_work(g, whole_items + (item - whole_items) / 2, num_m, num_n, num_k, group_m, kBlockK);
         w.half = (item - whole_items) & 1;
@@ -307,7 +320,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     umma::fence_after_thread_sync();
     const uint32_t tmem_base = sm->tmem_base;
     ptx::wait_for_previous_kernel();
-    const bool lets_next_start = g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && few_waves(num_tiles, gemm_ctas);
+    const bool lets_next_start = g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && few_waves(num_items, gemm_ctas);
 
     if (warp < kEpiWarp0) {
         // ---------------------------------------------------------------------- producer warps
@@ -498,7 +511,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         uint32_t r[32];
                         umma::tmem_ld_32x32(tmem_base + lane_addr + acc * kBlockN + c * 32, r);
                         umma::tmem_ld_wait();
-                        if (row < g.M) {
+                        if constexpr (kSplits) {
+                            if (row < g.M) {
+                                float* sums = g.partial + (tw.c_row0 + row) * g.N + n0 + c * 32;
+#pragma unroll
+                                for (int v = 0; v < 8; ++v)
+                                    if (n0 + c * 32 + v * 4 < g.N) *reinterpret_cast<uint4*>(sums + v * 4) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+                            }
+                        } else if (row < g.M) {
 #pragma unroll
                             for (int v = 0; v < 4; ++v) {
                                 const int col = n0 + c * 32 + v * 8;
@@ -1197,6 +1217,34 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (warp == 1) umma::tmem_dealloc(tmem_base, 512);
 }
 
+// Adds the parts of a product whose K blocks were shared out, in their order, and rounds once.  Eight columns per thread.
+__global__ void __launch_bounds__(256) gemm_reduce_kernel(const GemmArgs g) {
+    ptx::wait_for_previous_kernel();
+    ptx::let_next_kernel_start();
+    const int64_t vecs = static_cast<int64_t>(g.M) * (g.N / 8), part = static_cast<int64_t>(g.M) * g.N;
+    for (int64_t v = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; v < vecs; v += static_cast<int64_t>(gridDim.x) * 256) {
+        const float* p = g.partial + v * 8;
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll 4
+        for (int s = 0; s < g.k_splits; ++s) {
+            const float4 a = *reinterpret_cast<const float4*>(p + s * part), b = *reinterpret_cast<const float4*>(p + s * part + 4);
+            acc[0] += a.x;
+            acc[1] += a.y;
+            acc[2] += a.z;
+            acc[3] += a.w;
+            acc[4] += b.x;
+            acc[5] += b.y;
+            acc[6] += b.z;
+            acc[7] += b.w;
+        }
+        const int64_t row = v / (g.N / 8), col = (v - row * (g.N / 8)) * 8;
+        *reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(g.c) + (row * g.ldc + col) * 2) =
+            make_int4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
+    }
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1239,6 +1287,13 @@ bool make_mn_operand_map(CUtensorMap* map, const void* base, int64_t groups, int
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Plain bf16 products of so few tiles that a tile's K blocks can be shared out over several CTAs: bound by one CTA's chain of K blocks (0.15
+// to 0.4 us each) on a few SMs otherwise.  A second kernel adds the parts, in 32 bits and always in the same order.  The rule weighs the K
+// blocks that a CTA is spared against the second launch and the parts' way through L2, both in K blocks.  In a CUDA graph, whole / split:
+// 512 x 1024 x 5000 33.7 / 17.5 us, 74 x 832 x 5704 32.2 / 11.7, 64 x 4096 x 4096 13.0 / 10.3, 296 x 888 x 2184 16.9 / 11.2; not split by it: 128 x 7168 x
+// 2048 9.7 / 12.5, 1024^3 6.5 / 9.6, 96 x 2000 x 1600 7.4 / 8.5.
+constexpr int kMaxSplits = 16, kMinSplitBlocks = 4, kSplitCost = 16, kSplitBytesPerBlock = 512 * 1024;
+
 // e4m3 products of thin tiles that read every weight once.  Where the lines lie (32 experts, us in long runs, 256-column kernel / this
 // one, by token rows of an expert):
 //     rows            16          32          48          64          96
@@ -1255,6 +1310,20 @@ bool streams_weights(const GemmArgs& g) {
 }
 
 }  // namespace
+
+int gemm_k_splits(const GemmArgs& g, int num_sms) {
+    if (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE || g.mn_operands != 0 || g.k_group_off != nullptr || g.tile_group != nullptr || g.a_ready_flags != nullptr ||
+        g.M <= 0 || g.N <= 0 || g.K <= 0)
+        return 1;
+    const int64_t tiles = static_cast<int64_t>((g.M + kBlockM - 1) / kBlockM) * ((g.N + 127) / 128), num_k = (g.K + 63) / 64;
+    const int64_t most = std::min<int64_t>(std::min<int64_t>(num_sms / tiles, num_k / kMinSplitBlocks), kMaxSplits), part_bytes = static_cast<int64_t>(g.M) * g.N * 4;
+    int64_t best = 1, best_gain = 0;
+    for (int64_t s = 2; s <= most; ++s) {
+        const int64_t gain = num_k - (num_k + s - 1) / s - kSplitCost - s * part_bytes / kSplitBytesPerBlock;      // in K blocks
+        if (gain > best_gain) best = s, best_gain = gain;
+    }
+    return static_cast<int>(best);
+}
 
 cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
@@ -1339,6 +1408,21 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         return cudaLaunchCooperativeKernel(fn, dim3(ctas, 1, 1), dim3(kGemmThreads, 1, 1), params, kGemmSmemBytes, stream);
     }
     // whole tiles, or halves where all of them fit into one wave (the kernel cuts its last wave by the same rule)
+    if (g.k_splits > 1) {
+        // (one wave of 128-column tiles: gemm_k_splits)
+        if (fn != (const void*)gemm_kernel<false, 128, 0> || g.partial == nullptr || reinterpret_cast<uintptr_t>(g.partial) % 16 != 0 || g.tile_group != nullptr)
+            return cudaErrorInvalidValue;
+        fn = (const void*)gemm_kernel<false, 128, 0, true>;
+        err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
+        if (err != cudaSuccess) return err;
+        ctas = std::min(ctas, num_tiles * g.k_splits);
+        err = launch_dependent(fn, dim3(ctas, 1, 1), dim3(kGemmThreads, 1, 1), params, kGemmSmemBytes, stream);
+        if (err != cudaSuccess) return err;
+        void* reduce_params[] = {const_cast<GemmArgs*>(&g)};
+        const int64_t vecs = static_cast<int64_t>(g.M) * (g.N / 8);
+        return launch_dependent((const void*)gemm_reduce_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(1184, (vecs + 255) / 256)), 1, 1), dim3(256, 1, 1),
+                                reduce_params, 0, stream);
+    }
     if (ctas > num_tiles) ctas = g.is_fp8 && block_n == 256 && 2 * num_tiles <= ctas ? 2 * num_tiles : num_tiles;
     const dim3 block(gemm_threads(g.is_fp8 != 0, block_n), 1, 1);
     if (few_waves(num_tiles, ctas)) return launch_dependent(fn, dim3(ctas, 1, 1), block, params, kGemmSmemBytes, stream);

@@ -131,6 +131,12 @@ at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional
         g.timeout_ns = c0.timeout_ns;
     }
     const int sms = num_sms > 0 ? static_cast<int>(num_sms) : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    at::Tensor partial;
+    g.k_splits = ep::gemm_k_splits(g, sms);
+    if (g.k_splits > 1) {
+        partial = at::empty({g.k_splits, M, N}, a.options().dtype(at::kFloat));
+        g.partial = partial.data_ptr<float>();
+    }
     cuda_check(ep::launch_gemm(g, sms, at::cuda::getCurrentCUDAStream()), "tcgen05 GEMM launch");
     return c;
 }

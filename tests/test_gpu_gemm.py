@@ -140,6 +140,41 @@ def test_k_grouped_gemm_on_row_major_operands(M, N, segs):
         k0 += n
 
 
+@pytest.mark.parametrize('M,N,K,num_sms', [(64, 128, 8000, 0), (130, 264, 2056, 0), (74, 832, 5704, 0), (300, 256, 7168, 13), (512, 1024, 5000, 0), (1, 8, 1600, 0),
+                                           (129, 1032, 1992, 40)])
+@pytest.mark.parametrize('captured', [False, True])
+def test_products_whose_k_blocks_are_shared_out(M, N, K, num_sms, captured):
+    """Few tiles and a long K: parts of uneven length, a last K block that is not whole, ragged tiles, an output with a pitch; the same bits on
+    every pass, in a stream and from a CUDA graph, with the products following one another closely (their workspaces are reused)."""
+    from deepep_ascend_b200.ops import gemm as ops
+    gen = torch.Generator(device='cuda').manual_seed(M + N + K)
+    a, b = torch.randn(M, K, device='cuda', generator=gen).bfloat16(), torch.randn(N, K, device='cuda', generator=gen).bfloat16()
+    full = torch.full((M + 1, N + 8), 7.0, dtype=torch.bfloat16, device='cuda')
+    out = full[:M, :N]
+    ops.gemm_nt(a, b, out=out, num_sms=num_sms)
+    first = out.clone()
+    exact = a.double() @ b.double().t()
+    # fp32 sums rounded once to bf16: half an ulp (2^-9) of the value plus K fp32 roundings of the summed magnitudes
+    bound = exact.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24 + 1e-6
+    assert bool(((first.double() - exact).abs() <= bound).all())
+    assert bool((full[M] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
+
+    def passes():
+        return [ops.gemm_nt(a * s, b, num_sms=num_sms) for s in (1.0, 2.0, 4.0, 1.0)]
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        passes()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            results = passes()
+        for _ in range(3):
+            graph.replay()
+    else:
+        results = passes()
+    for got, s in zip(results, (1.0, 2.0, 4.0, 1.0)):        # powers of two: the same roundings
+        assert torch.equal(got, first * s)
+
+
 @pytest.mark.parametrize('M,N,K,num_sms', [(128, 256, 128, 0), (300, 264, 256, 0), (513, 520, 1152, 2), (200, 1032, 384, 1),
                                            (130, 256, 128, 1), (200, 1000, 384, 1), (513, 504, 1152, 2), (300, 1016, 256, 2)])
 @pytest.mark.parametrize('fp8', [False, True])
