@@ -430,6 +430,8 @@ struct LocalExpandCopyArgs {
     const float* w_src;               // optional weights [rows, K], row pitch w_pitch elements
     int64_t w_pitch;
     float* w_dst;                     // [expert rows]
+    const uint8_t* out_valid;         // optional, with w_dst: [num_out], rows without a token (0) get a weight of zero
+    int num_out;
 };
 struct LocalReduceArgs {
     const int32_t* pos;               // [rows, K]

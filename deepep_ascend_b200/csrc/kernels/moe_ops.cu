@@ -746,6 +746,12 @@ __global__ void __launch_bounds__(kExpandWarps * 32) local_expand_copy_kernel(co
     ptx::let_next_kernel_start();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kExpandWarps + (threadIdx.x >> 5);
+    if (a.out_valid != nullptr) {
+        // weights of alignment rows; those of token rows are written below
+        const int threads = gridDim.x * gridDim.y * kExpandWarps * 32;
+        for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * kExpandWarps * 32 + threadIdx.x; i < a.num_out; i += threads)
+            if (a.out_valid[i] == 0) a.w_dst[i] = 0.f;
+    }
     if (row >= a.num_rows) return;
     const int my_pos = lane < a.num_topk ? *(a.pos + static_cast<int64_t>(row) * a.num_topk + lane) : -1;
     uint32_t dests = __ballot_sync(0xffffffffu, my_pos >= 0);

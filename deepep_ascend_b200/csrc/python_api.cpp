@@ -330,7 +330,7 @@ std::vector<at::Tensor> local_expand_layout(const at::Tensor& recv_idx, const at
 
 // Copies every received row (and its scales / weights) to its expert rows -> (rows_out [num_out, width], sf_out or none, w_out or none).
 std::vector<at::Tensor> local_expand_copy(const at::Tensor& pos, const at::Tensor& x, int64_t num_out, const std::optional<at::Tensor>& sf,
-                                          const std::optional<at::Tensor>& w) {
+                                          const std::optional<at::Tensor>& w, const std::optional<at::Tensor>& valid_row) {
     TORCH_CHECK(pos.is_cuda() && pos.is_contiguous() && pos.scalar_type() == at::kInt && pos.dim() == 2, "pos must be contiguous int32 [rows, K]");
     TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && x.size(0) == pos.size(0), "x must be [rows, width] with contiguous rows");
     const int64_t row_bytes = x.size(1) * x.element_size();
@@ -356,7 +356,14 @@ std::vector<at::Tensor> local_expand_copy(const at::Tensor& pos, const at::Tenso
     if (w.has_value()) {
         TORCH_CHECK(w->is_cuda() && w->dim() == 2 && w->scalar_type() == at::kFloat && w->stride(1) == 1 && w->size(0) == x.size(0) &&
                         w->size(1) == pos.size(1), "w must be fp32 [rows, K] with contiguous rows");
-        w_out = at::zeros({num_out}, w->options());
+        // rows without a token get zeros: here, or by the kernel where it is told which they are (and is launched at all)
+        if (valid_row.has_value() && pos.size(0) > 0) {
+            w_out = at::empty({num_out}, w->options());
+            a.out_valid = valid_ptr(*valid_row, num_out);
+            a.num_out = static_cast<int>(num_out);
+        } else {
+            w_out = at::zeros({num_out}, w->options());
+        }
         a.w_src = w->data_ptr<float>();
         a.w_pitch = w->stride(0);
         a.w_dst = w_out.data_ptr<float>();
@@ -907,7 +914,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));
     m.def("local_expand_layout", &local_expand_layout);
     m.def("local_expand_copy", &local_expand_copy, py::arg("pos"), py::arg("x"), py::arg("num_out"), py::arg("sf") = py::none(),
-          py::arg("w") = py::none());
+          py::arg("w") = py::none(), py::arg("valid_row") = py::none());
     m.def("local_gather", &local_gather);
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("expert_segments", &expert_segments, py::arg("psum_ends"), py::arg("num_rows"), py::arg("alignment") = 128);

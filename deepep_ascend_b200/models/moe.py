@@ -72,7 +72,7 @@ class _MoEFunction(torch.autograd.Function):
                 # expert's 128-aligned segment (rows in received order).  The copies are private to this call.
                 rows = sum(handle.num_recv_tokens_per_expert_list)
                 pos, _, tile_group, valid_row, seg_off, tile_rows = G.local_expand_layout(recv_idx, handle.psum_num_recv_tokens_per_expert, rows)
-                rx, rsf, recv_w = G.local_expand_copy(pos, rx, rows, sf=rsf, w=recv_w)
+                rx, rsf, recv_w = G.local_expand_copy(pos, rx, rows, sf=rsf, w=recv_w, valid_row=valid_row)
             else:
                 rows, pos = handle.num_rows, no_pos
                 tile_group, valid_row, seg_off, tile_rows = G.expert_tiles(handle.psum_num_recv_tokens_per_expert, rows)

@@ -161,10 +161,11 @@ def local_expand_layout(recv_idx: torch.Tensor, psum_aligned: torch.Tensor, num_
 
 
 def local_expand_copy(pos: torch.Tensor, x: torch.Tensor, num_out: int, sf: Optional[torch.Tensor] = None,
-                      w: Optional[torch.Tensor] = None):
+                      w: Optional[torch.Tensor] = None, valid_row: Optional[torch.Tensor] = None):
     """Writes every received row of ``x`` (and its scales ``sf [rows, G]`` / weights ``w [rows, K]``) to its expert rows ->
-    ``[x_out [num_out, width], sf_out, w_out [num_out]]`` (only those asked for).  Alignment rows of the output are not written."""
-    return _native.load().local_expand_copy(pos, x, num_out, sf, w)
+    ``[x_out [num_out, width], sf_out, w_out [num_out]]`` (only those asked for).  Alignment rows of the rows and scales are not written; their weights
+    are zero (``valid_row`` of :func:`local_expand_layout`, if given, saves the launch that fills them)."""
+    return _native.load().local_expand_copy(pos, x, num_out, sf, w, valid_row)
 
 
 def local_reduce(pos: torch.Tensor, y: torch.Tensor, w: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:

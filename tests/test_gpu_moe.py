@@ -466,6 +466,25 @@ def test_expand_plan_over_many_ctas(rows, K, El):
         assert torch.equal(got.cpu(), want)
 
 
+@pytest.mark.parametrize('rows,K,El', [(0, 2, 3), (1, 1, 1), (5, 3, 2), (64, 8, 32), (700, 6, 5)])
+def test_weights_of_alignment_rows_are_zero(rows, K, El):
+    """With `valid_row` the copy itself fills them, for rows that are split by columns and whole ones, with fewer and with more
+    alignment rows than threads; without it, a launch in front does."""
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows)
+    idx = torch.stack([torch.randperm(max(K, El), device='cuda')[:K] for _ in range(rows)]) if rows else torch.empty(0, K, dtype=torch.int64, device='cuda')
+    counts = torch.bincount(idx[idx < El].flatten(), minlength=El)
+    psum = ((counts + 127) // 128 * 128).cumsum(0).to(torch.int32)
+    num = int(psum[-1])
+    pos, _, _, valid, _, _ = ops.local_expand_layout(idx, psum, num)
+    x, w = torch.randn(rows, 256, device='cuda').bfloat16(), torch.rand(rows, K, device='cuda') + 1
+    junk = torch.full((max(1, num),), float('nan'), device='cuda')         # what the allocator hands out next
+    del junk
+    x1, w1 = ops.local_expand_copy(pos, x, num, w=w, valid_row=valid)
+    x0, w0 = ops.local_expand_copy(pos, x, num, w=w)
+    assert torch.equal(w1, w0) and torch.equal(x1[valid], x0[valid]) and bool((w1[~valid] == 0).all()) and bool((w1[valid] >= 1).all())
+
+
 @pytest.mark.parametrize('rows,K', [(0, 3), (1, 1), (85, 3), (5000, 8), (40000, 7)])
 def test_local_gather(rows, K):
     """Less than a block, ragged blocks, more than the grid covers at once; a NaN in a row nobody asks for stays out."""
