@@ -323,6 +323,12 @@ namespace ep {
 cudaError_t launch_gemm(const GemmArgs& args, int num_sms, cudaStream_t stream);
 // into how many parts along K a product should be cut on this many SMs (GemmArgs::k_splits)
 int gemm_k_splits(const GemmArgs& args, int num_sms);
+// the launch that adds the parts
+struct GemmReduceShape {
+    int ctas, threads;
+    bool beside_product;              // launched while the product still runs
+};
+GemmReduceShape gemm_reduce_shape(const GemmArgs& args, int num_sms, int device_sms);
 }  // namespace ep
 
 // ------------------------------------------------------------------------------------------------ MoE helpers

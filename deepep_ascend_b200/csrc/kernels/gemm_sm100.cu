@@ -1217,12 +1217,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (warp == 1) umma::tmem_dealloc(tmem_base, 512);
 }
 
+constexpr int kReduceMaxThreads = 1024;
 // Adds the parts of a product whose K blocks were shared out, in their order, and rounds once.  Eight columns per thread.
-__global__ void __launch_bounds__(256) gemm_reduce_kernel(const GemmArgs g) {
+__global__ void __launch_bounds__(kReduceMaxThreads) gemm_reduce_kernel(const GemmArgs g) {
     ptx::wait_for_previous_kernel();
     ptx::let_next_kernel_start();
     const int64_t vecs = static_cast<int64_t>(g.M) * (g.N / 8), part = static_cast<int64_t>(g.M) * g.N;
-    for (int64_t v = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; v < vecs; v += static_cast<int64_t>(gridDim.x) * 256) {
+    for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < vecs; v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const float* p = g.partial + v * 8;
         float acc[8];
 #pragma unroll
@@ -1325,6 +1326,17 @@ int gemm_k_splits(const GemmArgs& g, int num_sms) {
     return static_cast<int>(best);
 }
 
+// The kernel that adds the parts stays on the product's SMs: with fewer than the device has, as many CTAs as SMs, and launched when the
+// product has ended, since CTAs that wait for its end would do so on the SMs that it leaves to others.
+GemmReduceShape gemm_reduce_shape(const GemmArgs& g, int num_sms, int device_sms) {
+    GemmReduceShape r;
+    const int64_t vecs = static_cast<int64_t>(g.M) * (g.N / 8);
+    r.beside_product = num_sms >= device_sms;
+    r.threads = r.beside_product ? 256 : kReduceMaxThreads;
+    r.ctas = static_cast<int>(std::min<int64_t>(r.beside_product ? 8 * static_cast<int64_t>(device_sms) : num_sms, (vecs + r.threads - 1) / r.threads));
+    return r;
+}
+
 cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
     const int elem = g.is_fp8 ? 1 : 2;
@@ -1418,10 +1430,14 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         ctas = std::min(ctas, num_tiles * g.k_splits);
         err = launch_dependent(fn, dim3(ctas, 1, 1), dim3(kGemmThreads, 1, 1), params, kGemmSmemBytes, stream);
         if (err != cudaSuccess) return err;
+        int device = 0, device_sms = 0;
+        if ((err = cudaGetDevice(&device)) != cudaSuccess || (err = cudaDeviceGetAttribute(&device_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
+            return err;
+        const GemmReduceShape r = gemm_reduce_shape(g, num_sms, device_sms);
         void* reduce_params[] = {const_cast<GemmArgs*>(&g)};
-        const int64_t vecs = static_cast<int64_t>(g.M) * (g.N / 8);
-        return launch_dependent((const void*)gemm_reduce_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(1184, (vecs + 255) / 256)), 1, 1), dim3(256, 1, 1),
-                                reduce_params, 0, stream);
+        const void* reduce = (const void*)gemm_reduce_kernel;
+        if (r.beside_product) return launch_dependent(reduce, dim3(r.ctas, 1, 1), dim3(r.threads, 1, 1), reduce_params, 0, stream);
+        return cudaLaunchKernel(reduce, dim3(r.ctas, 1, 1), dim3(r.threads, 1, 1), reduce_params, 0, stream);
     }
     if (ctas > num_tiles) ctas = g.is_fp8 && block_n == 256 && 2 * num_tiles <= ctas ? 2 * num_tiles : num_tiles;
     const dim3 block(gemm_threads(g.is_fp8 != 0, block_n), 1, 1);

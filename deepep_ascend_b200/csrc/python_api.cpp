@@ -65,6 +65,19 @@ at::Tensor& gemm_error_flag(int device) {
     return flags[device];
 }
 
+// What gemm_nt chooses for a bf16 product without tile_group, from its sizes alone (host code only): parts along K (1: one chain of K blocks), and CTAs,
+// threads and early launch of the kernel that adds them.
+py::tuple gemm_split_plan(int64_t M, int64_t N, int64_t K, int64_t num_sms, int64_t device_sms) {
+    GemmArgs g{};
+    g.M = static_cast<int>(M);
+    g.N = static_cast<int>(N);
+    g.K = static_cast<int>(K);
+    g.num_groups = 1;
+    g.k_splits = ep::gemm_k_splits(g, static_cast<int>(num_sms));
+    const ep::GemmReduceShape r = ep::gemm_reduce_shape(g, static_cast<int>(num_sms), static_cast<int>(device_sms));
+    return py::make_tuple(g.k_splits, r.ctas, r.threads, r.beside_product);
+}
+
 // C[M, N] (bf16) = A[M, K] @ B[g][N, K]^T on the tcgen05 tensor cores.  bf16 operands, or float8_e4m3fn operands
 // with fp32 block scales (sfa [M, ceil(K/128)] any strides, sfb [G, ceil(N/128), ceil(K/128)] contiguous).
 // `tile_group` int32 [ceil(M/128)]: weights group of every 128-row tile (-1 = skip the tile).
@@ -909,6 +922,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("gemm_nt", &gemm_nt, py::arg("a"), py::arg("b"), py::arg("sfa") = py::none(), py::arg("sfb") = py::none(),
           py::arg("tile_group") = py::none(), py::arg("out") = py::none(), py::arg("num_sms") = 0, py::arg("a_ready_flags") = py::none(),
           py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr, py::arg("tile_rows") = py::none(), py::arg("total_rows") = 0);
+    m.def("gemm_split_plan", &gemm_split_plan, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("num_sms"), py::arg("device_sms"));
     m.def("ag_gemm", &ag_gemm);
     m.def("gemm_rs", &gemm_rs);
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));

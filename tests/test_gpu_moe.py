@@ -653,14 +653,11 @@ def test_launches_that_overwrite_what_the_one_before_reads(M, N, sms, captured):
     assert bool(want.any()) and torch.equal(x.view(torch.int16), want.view(torch.int16))
 
 
-def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
-    """The kernel behind a product is launched early, but not so early that its waiting CTAs take the SMs that the product leaves free: a dispatch
-    that is issued meanwhile ends long before the product does."""
+def _assert_a_dispatch_fits_beside(product):
+    """`product` (about a millisecond on 16 SMs) with a kernel behind it, and a dispatch that is issued meanwhile: it ends long before they do."""
     from deepep_ascend_b200 import ElasticBuffer
     from deepep_ascend_b200.ops import gemm as ops
     T, H, E, K = 256, 1024, 16, 4
-    a, b = (torch.randn(2048, 32768, device='cuda').bfloat16() for _ in range(2))           # 128 tiles: eight waves of 16 CTAs, over a millisecond
-    out = torch.empty(2048, 2048, dtype=torch.bfloat16, device='cuda')
     y = torch.randn(1 << 17, 256, device='cuda').bfloat16()
     pos = torch.randperm(1 << 17, device='cuda').view(-1, 1).to(torch.int32)
     x, idx = torch.randn(T, H, device='cuda').bfloat16(), torch.rand(T, E, device='cuda').topk(K, dim=-1).indices
@@ -671,7 +668,7 @@ def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
             start, sent, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
             torch.cuda.synchronize()
             start.record()
-            ops.gemm_nt(a, b, out=out, num_sms=16)
+            product()
             ops.local_reduce(pos, y)
             end.record()
             with torch.cuda.stream(side):
@@ -682,6 +679,24 @@ def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
             assert attempt == 0 or times[0] < 0.6 * times[1], times                         # the first pass may load code
     finally:
         buf.destroy()
+
+
+def test_a_product_of_few_sms_leaves_the_others_to_an_exchange():
+    """The kernel behind a product is launched early, but not so early that its waiting CTAs take the SMs that the product leaves free."""
+    from deepep_ascend_b200.ops import gemm as ops
+    a, b = (torch.randn(2048, 32768, device='cuda').bfloat16() for _ in range(2))           # 128 tiles: eight waves of 16 CTAs, over a millisecond
+    out = torch.empty(2048, 2048, dtype=torch.bfloat16, device='cuda')
+    _assert_a_dispatch_fits_beside(lambda: ops.gemm_nt(a, b, out=out, num_sms=16))
+
+
+def test_a_product_of_few_sms_in_parts_leaves_the_others_to_an_exchange():
+    """The same for a product whose K blocks are shared out, with the kernel that adds the parts behind it."""
+    from deepep_ascend_b200 import _native
+    from deepep_ascend_b200.ops import gemm as ops
+    a, b = torch.randn(256, 1 << 20, device='cuda').bfloat16(), torch.randn(128, 1 << 20, device='cuda').bfloat16()     # 2 tiles in 8 parts
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _native.load().gemm_split_plan(256, 128, 1 << 20, num_sms=16, device_sms=sms)[0] == 8
+    _assert_a_dispatch_fits_beside(lambda: ops.gemm_nt(a, b, num_sms=16))
 
 
 @pytest.mark.parametrize('rows,I', [(0, 128), (4, 0), (0, 0)])
