@@ -460,6 +460,7 @@ cudaError_t launch_local_gather(const int32_t* pos, const float* v, float* out, 
 cudaError_t launch_expert_segments(const ExpertSegmentsArgs& args, cudaStream_t stream);
 cudaError_t launch_weight_quant(const WeightQuantArgs& args, cudaStream_t stream);
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& args, cudaStream_t stream);
+int swiglu_quant_col_chunk(int rows, int inter);   // columns of a row that one warp of it takes
 cudaError_t launch_moe_bwd(const MoeBwdArgs& args, cudaStream_t stream);
 int moe_bwd_prep_col_blocks(int cols);   // PREP writes row_dot as [col_blocks, rows] partial sums
 }  // namespace ep

@@ -975,18 +975,32 @@ cudaError_t launch_weight_quant(const WeightQuantArgs& a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+// A warp's steps of 256 columns are a chain (load, exponential, amax, store), and with a row mask many CTAs have next to nothing to do, so
+// rows are split further than in the other kernels.  Not into single steps in general: such a warp has nothing to load ahead.  us by the valid
+// ones of every 128 rows (16 / 64 / 128), split for 296 CTAs and by this:
+//     768 to 1152 CTAs of one step each      2048 x 1024    2.9 / 4.1 / 4.4    2.7 / 3.3 / 4.1      1024 x 2048    2.7 / 4.0 / 5.2    2.8 / 3.4 / 4.1
+//     up to 1536 CTAs of two steps or more   4096 x 2048    6.8 / 10.9 / 11.5  4.6 / 6.4 / 9.6      6016 x 1024    4.4 / 6.8 / 7.9    4.0 / 5.8 / 8.0
+//     chains of more than eight steps        8192 x 4096    15.8 / 23.0 / 30.9 10.8 / 18.9 / 30.6   9344 x 3072    12.8 / 17.9 / 26.8 9.2 / 16.4 / 26.9
+// Beyond these lines full rows get slower: one step each on 512 CTAs 512 x 2048 2.2 / 2.9 / 2.7 becomes 2.2 / 3.0 / 3.2, on 2048 CTAs 8192 x 512 3.6 / 4.5 / 5.7
+// becomes 3.7 / 5.0 / 6.8; two steps each on 2048 CTAs 8192 x 1024 5.3 / 7.0 / 9.0 becomes 4.6 / 7.0 / 9.9, on 384 CTAs 512 x 3072 2.6 / 3.7 / 3.3 becomes
+// 2.3 / 3.4 / 4.3.
+constexpr int kSwigluWarps = 8;
+int swiglu_quant_col_chunk(int rows, int inter) {
+    const int ctas = (rows + kSwigluWarps - 1) / kSwigluWarps, steps = (inter + 255) / 256;
+    int splits = column_splits(ctas, steps);
+    if (ctas >= 96 && ctas <= 1152 && ctas * steps >= 768 && ctas * steps <= 1152) splits = steps;
+    else if (ctas >= 128) splits = max(splits, max(min((steps + 1) / 2, 1536 / ctas), (steps + 7) / 8));
+    return (steps + splits - 1) / splits * 256;
+}
+
 cudaError_t launch_swiglu_quant(const SwigluQuantArgs& a, cudaStream_t stream) {
     if (a.rows == 0 || a.inter == 0) return cudaSuccess;
     if (!aligned(a.h, 16) || (a.rows > 1 && a.ldh % 8 != 0) || !aligned(a.q, 8) || !aligned(a.act_bf16, 16)) return cudaErrorInvalidValue;
-    const int warps = 8, ctas = (a.rows + warps - 1) / warps, steps = (a.inter + 255) / 256;
     SwigluQuantArgs args = a;
-    // A warp's steps are a chain (load, exponential, amax, store) and with a row mask many CTAs have next to nothing to do, so this kernel
-    // is split up to four times the CTAs of the others.  4096 rows x 2048, of every 128 rows 16 / 64 / 128 valid: 6.8 / 11.0 / 11.5 us
-    // without, 4.7 / 6.5 / 9.7 us with; from 9472 rows on nothing is split.
-    const int splits = column_splits((ctas + 3) / 4, steps), per = (steps + splits - 1) / splits;
-    args.col_chunk = per * 256;
+    args.col_chunk = swiglu_quant_col_chunk(a.rows, a.inter);
     void* params[] = {&args};
-    return launch_dependent((const void*)swiglu_quant_kernel, dim3(ctas, (steps + per - 1) / per), dim3(warps * 32), params, 0, stream);
+    return launch_dependent((const void*)swiglu_quant_kernel, dim3((a.rows + kSwigluWarps - 1) / kSwigluWarps, (a.inter + args.col_chunk - 1) / args.col_chunk),
+                            dim3(kSwigluWarps * 32), params, 0, stream);
 }
 
 }  // namespace ep

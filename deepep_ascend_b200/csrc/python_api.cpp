@@ -933,6 +933,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("local_reduce", &local_reduce, py::arg("pos"), py::arg("y"), py::arg("w") = py::none(), py::arg("out") = py::none());
     m.def("expert_segments", &expert_segments, py::arg("psum_ends"), py::arg("num_rows"), py::arg("alignment") = 128);
     m.def("quantize_weight_blocks", &quantize_weight_blocks);
+    m.def("swiglu_quant_col_chunk", &ep::swiglu_quant_col_chunk, py::arg("rows"), py::arg("inter"));
     m.def("swiglu_quant", &swiglu_quant, py::arg("h"), py::arg("keep_bf16") = false, py::arg("valid") = py::none());
     m.def("gemm_kgrouped", &gemm_kgrouped, py::arg("a_t"), py::arg("b_t"), py::arg("k_off"), py::arg("num_sms") = 0);
     m.def("grouped_gemm_nn", &grouped_gemm_nn, py::arg("a"), py::arg("b"), py::arg("tile_group"), py::arg("out") = py::none(), py::arg("num_sms") = 0,

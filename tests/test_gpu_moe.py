@@ -699,6 +699,25 @@ def test_a_product_of_few_sms_in_parts_leaves_the_others_to_an_exchange():
     _assert_a_dispatch_fits_beside(lambda: ops.gemm_nt(a, b, num_sms=16))
 
 
+@pytest.mark.parametrize('rows,I', [(768, 2032), (1024, 2048), (1029, 1040), (1152, 2064), (4090, 1808), (4099, 4096), (12300, 2320)])
+@pytest.mark.parametrize('masked', [False, True])
+def test_swiglu_of_rows_that_are_split(rows, I, masked):
+    """Single steps, two and more of them, chains that are halved, last pieces that are not whole: the bits of the same rows in small
+    launches that are cut differently."""
+    from deepep_ascend_b200 import _native
+    from deepep_ascend_b200.ops import gemm as ops
+    torch.manual_seed(rows + I)
+    h = torch.randn(rows, 2 * I, device='cuda').bfloat16()
+    valid = torch.rand(rows, device='cuda') > 0.5 if masked else None
+    chunk = _native.load().swiglu_quant_col_chunk
+    part = next(p for p in (40, 600) if chunk(p, I) != chunk(rows, I))
+    at = torch.arange(rows, device='cuda')[valid] if masked else slice(None)
+    got = ops.swiglu_quant(h, keep_bf16=True, valid_row=valid)
+    want = [ops.swiglu_quant(h[r:r + part], keep_bf16=True) for r in range(0, rows, part)]
+    for g, w in zip(got, (torch.cat(t) for t in zip(*[(q.view(torch.uint8), s, a) for q, s, a in want]))):
+        assert torch.equal((g.view(torch.uint8) if g.dtype == torch.float8_e4m3fn else g)[at], w[at])
+
+
 @pytest.mark.parametrize('rows,I', [(0, 128), (4, 0), (0, 0)])
 @pytest.mark.parametrize('masked', [False, True])
 def test_swiglu_of_nothing(rows, I, masked):
