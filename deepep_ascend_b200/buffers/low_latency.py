@@ -77,7 +77,8 @@ class LowLatencyMixin:
         [E_local, ranks * max_tokens, H / 128]`` fp32 (or ``H / 512`` int32 of packed UE8M0) column-major in the
         last two dims, ``recv_count [E_local]``; only the first ``recv_count[e]`` rows of expert ``e`` are valid.  Pass that on:
         ``ops.gemm.grouped_gemm_nt(tile_rows=...)`` loads and stores only the rows of a tile that count (with one 128-row tile per
-        expert the argument is ``recv_count`` itself), ``ops.gemm.swiglu_quant(valid_row=...)`` skips the others.
+        expert the argument is ``recv_count`` itself; with ``total_rows`` it also chooses the kernel for thin tiles),
+        ``ops.gemm.swiglu_quant(valid_row=...)`` skips the others.
         ``handle = (src_info, layout_range, max_tokens, hidden, num_experts)``.
         The time spent waiting for every source rank, in ns, is added to ``dispatch_wait_recv_cost_stats`` (int64 ``[ranks]``).  A
         small batch on one rank, both halves in one launch, waits for nobody: nothing is added.

@@ -285,7 +285,7 @@ struct GemmArgs {
     const int32_t* tile_group;        // [ceil(M/128)] or null (single group 0)
     const int32_t* tile_rows;         // optional [ceil(M/128)]: leading rows of every tile that count; the others need not be read and
                                       // their results are not needed (used by the e4m3 kernels for N >= 256, ignored elsewhere)
-    int64_t total_rows;               // upper bound of the sum of tile_rows, 0: not known (chooses between kernels, nothing else)
+    int64_t total_rows;               // about how much tile_rows add up to, 0: not known (chooses between kernels, nothing else)
     int* error;                       // device int set to non-zero if a pipeline wait ran out
     uint64_t* status;                 // status block of a communication buffer that should hear about such a failure, or null
     int status_rank;
@@ -321,6 +321,8 @@ enum { EP_GEMM_FUSE_NONE = 0, EP_GEMM_FUSE_ALL_GATHER = 1, EP_GEMM_FUSE_REDUCE_S
 
 namespace ep {
 cudaError_t launch_gemm(const GemmArgs& args, int num_sms, cudaStream_t stream);
+// whether a product takes the kernel for thin tiles that streams the weights
+bool gemm_streams_weights(const GemmArgs& args);
 // into how many parts along K a product should be cut on this many SMs (GemmArgs::k_splits)
 int gemm_k_splits(const GemmArgs& args, int num_sms);
 // the launch that adds the parts

@@ -1295,22 +1295,26 @@ bool make_mn_operand_map(CUtensorMap* map, const void* base, int64_t groups, int
 // 2048 9.7 / 12.5, 1024^3 6.5 / 9.6, 96 x 2000 x 1600 7.4 / 8.5.
 constexpr int kMaxSplits = 16, kMinSplitBlocks = 4, kSplitCost = 16, kSplitBytesPerBlock = 512 * 1024;
 
-// e4m3 products of thin tiles that read every weight once.  Where the lines lie (32 experts, us in long runs, 256-column kernel / this
-// one, by token rows of an expert):
-//     rows            16          32          48          64          96
-//     4096 x 7168     168 / 141   170 / 144   180 / 152   180 / 160   187 / 194
-//     7168 x 2048      95 / 79     94 / 82     97 / 87     99 / 91    104 / 115
-//     512 x 2048                 10.9 / 8.3              11.0 / 9.5              (weights in L2)
-//   * at most one M tile per group: a second one reads its weights from L2, and the operand traffic of 128-column tiles bounds the product
-//   * at most 56 token rows per tile on average, where the caller knows a bound; one who gives `tile_rows` without has thin tiles
+// e4m3 products of thin tiles that read every weight once.  Where the lines lie (32 experts, us in runs of half a second, 256-column kernel /
+// this one, by token rows of an expert; the first two in bursts of five: 166 / 147 and 92 / 82 at 16 rows, 182 / 183 and 103 / 109 at 128):
+//     rows            16          48          64          72          96          128
+//     4096 x 7168     197 / 149   205 / 175   205 / 187   210 / 224   210 / 228   219 / 238
+//     7168 x 2048     105 / 83    109 / 96    110 / 103   112 / 124   113 / 127   118 / 136
+//     2048 x 1024    15.5 / 13.2 16.7 / 15.8 17.2 / 16.7 17.8 / 17.8 18.4 / 18.6 20.0 / 20.4
+//     512 x 2048     10.7 / 7.8  11.1 / 9.0  11.0 / 9.5  11.1 / 9.9  11.2 / 10.1 11.1 / 10.3     (weights in L2)
+//   * no more M tiles than groups: a second tile of a group reads its weights from L2, and the operand traffic of 128-column tiles bounds the
+//     product (which tiles share a group is known on the device only)
+//   * at most 56 token rows per tile on average (with uneven routing some tiles have more than 64 then).  A caller who gives no count may have full
+//     tiles: the 256-column kernel
 constexpr int kStreamMaxRows = 56;
-bool streams_weights(const GemmArgs& g) {
-    const int64_t num_m = (g.M + kBlockM - 1) / kBlockM;
-    return g.is_fp8 && g.N >= 256 && g.tile_rows != nullptr && g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && g.k_group_off == nullptr &&
-           g.mn_operands == 0 && num_m <= g.num_groups && (g.total_rows == 0 || g.total_rows <= kStreamMaxRows * num_m);
-}
 
 }  // namespace
+
+bool gemm_streams_weights(const GemmArgs& g) {
+    const int64_t num_m = (g.M + kBlockM - 1) / kBlockM;
+    return g.is_fp8 && g.N >= 256 && g.tile_rows != nullptr && g.fuse == EP_GEMM_FUSE_NONE && g.a_ready_flags == nullptr && g.k_group_off == nullptr &&
+           g.mn_operands == 0 && num_m <= g.num_groups && g.total_rows > 0 && g.total_rows <= kStreamMaxRows * num_m;
+}
 
 int gemm_k_splits(const GemmArgs& g, int num_sms) {
     if (g.is_fp8 || g.fuse != EP_GEMM_FUSE_NONE || g.mn_operands != 0 || g.k_group_off != nullptr || g.tile_group != nullptr || g.a_ready_flags != nullptr ||
@@ -1363,7 +1367,7 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         // 9.3 / 6.6; with more than a wave of them 1315 x 2536 x 3144 (110 / 220) 32.6 / 44.7.
         if (g.fuse == EP_GEMM_FUSE_NONE && num_m_tiles * ((g.N + 127) / 128) * groups <= workers) block_n = 128;
     }
-    if (streams_weights(g)) {
+    if (gemm_streams_weights(g)) {
         CUtensorMap map_a, map_a32, map_w, map_w32;
         const int64_t w_rows = static_cast<int64_t>(g.num_groups) * g.N;
         if (!make_operand_map(&map_a, g.a, g.M, g.K, g.lda, true, 128) || !make_operand_map(&map_a32, g.a, g.M, g.K, g.lda, true, 32) ||

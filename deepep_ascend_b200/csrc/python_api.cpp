@@ -78,6 +78,19 @@ py::tuple gemm_split_plan(int64_t M, int64_t N, int64_t K, int64_t num_sms, int6
     return py::make_tuple(g.k_splits, r.ctas, r.threads, r.beside_product);
 }
 
+// Whether gemm_nt streams the weights of an e4m3 product with `tile_rows` (host code only)
+bool gemm_streams_weights(int64_t M, int64_t N, int64_t num_groups, int64_t total_rows) {
+    static const int32_t given = 0;
+    GemmArgs g{};
+    g.M = static_cast<int>(M);
+    g.N = static_cast<int>(N);
+    g.num_groups = static_cast<int>(num_groups);
+    g.is_fp8 = 1;
+    g.tile_rows = &given;
+    g.total_rows = total_rows;
+    return ep::gemm_streams_weights(g);
+}
+
 // C[M, N] (bf16) = A[M, K] @ B[g][N, K]^T on the tcgen05 tensor cores.  bf16 operands, or float8_e4m3fn operands
 // with fp32 block scales (sfa [M, ceil(K/128)] any strides, sfb [G, ceil(N/128), ceil(K/128)] contiguous).
 // `tile_group` int32 [ceil(M/128)]: weights group of every 128-row tile (-1 = skip the tile).
@@ -923,6 +936,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("tile_group") = py::none(), py::arg("out") = py::none(), py::arg("num_sms") = 0, py::arg("a_ready_flags") = py::none(),
           py::arg("a_ready_value") = 0, py::arg("a_flag_of_tile") = py::none(), py::arg("report_to") = nullptr, py::arg("tile_rows") = py::none(), py::arg("total_rows") = 0);
     m.def("gemm_split_plan", &gemm_split_plan, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("num_sms"), py::arg("device_sms"));
+    m.def("gemm_streams_weights", &gemm_streams_weights, py::arg("M"), py::arg("N"), py::arg("num_groups"), py::arg("total_rows"));
     m.def("ag_gemm", &ag_gemm);
     m.def("gemm_rs", &gemm_rs);
     m.def("local_expand_plan", &local_expand_plan, py::arg("recv_idx"), py::arg("seg_end_aligned"));

@@ -20,6 +20,15 @@ def test_the_parts_of_a_product_are_added_on_its_own_sms(M, N, K, num_sms):
     assert 1 <= ctas <= (M * N // 8 + threads - 1) // threads and ctas <= 8 * 148 and threads % 32 == 0 and threads <= 1024
 
 
+@pytest.mark.parametrize('tiles,N,groups,total_rows,streams', [
+    (32, 4096, 32, 0, False),                   # nothing known: the tiles may be full
+    (32, 4096, 32, 32 * 16, True), (32, 7168, 32, 32 * 56, True), (1, 256, 1, 1, True), (13, 512, 32, 13 * 56, True),
+    (32, 7168, 32, 32 * 56 + 1, False), (32, 4096, 32, 32 * 128, False), (33, 4096, 32, 33, False), (32, 248, 32, 32, False)])
+def test_thin_tiles_stream_the_weights_where_the_rows_are_known(tiles, N, groups, total_rows, streams):
+    for M in (128 * tiles, 128 * tiles - 127):
+        assert _C().gemm_streams_weights(M, N, num_groups=groups, total_rows=total_rows) == streams
+
+
 @pytest.mark.parametrize('inter', [8, 256, 264, 512, 768, 1024, 1408, 2048, 3072, 4096])
 @pytest.mark.parametrize('rows', [1, 128, 512, 767, 768, 1024, 1536, 2048, 4096, 6016, 8192, 9400, 12000, 1 << 20])
 def test_rows_of_swiglu_are_cut_where_that_pays(rows, inter):

@@ -533,8 +533,8 @@ def test_thin_tiles_are_read_and_stored_by_rows(counts):
 def test_products_that_stream_the_weights(G, N, K, num_sms):
     """Thin tiles, at most one per expert: the bits of the 256-column kernel (which takes the product when no tile_rows are given), with every
     number of token rows at which the kernel changes its way, idle tiles, two tiles of one group, a ragged last tile, odd K blocks,
-    columns that end inside a tile, last waves that are cut and whole, and scales in either order; a bound on the rows that rules the
-    kernel out changes nothing."""
+    columns that end inside a tile, last waves that are cut and whole, and scales in either order; a count of the rows that rules the
+    kernel out, or none, changes nothing."""
     from deepep_ascend_b200.ops import gemm as ops
     gen = torch.Generator(device='cuda').manual_seed(N)
     edges = [1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 127, 128, 0, 40]
@@ -556,7 +556,7 @@ def test_products_that_stream_the_weights(G, N, K, num_sms):
     at = torch.arange(M, device='cuda')
     valid = (at % 128 < rows[at // 128]) & (group[at // 128] >= 0)
     a.view(torch.uint8)[~valid] = 0x7f
-    for scales, bound in ((sa, 0), (sa.t().contiguous().t(), 1), (sa, M)):
+    for scales, bound in ((sa, 1), (sa.t().contiguous().t(), 1), (sa, 0), (sa, M)):
         out = torch.full((M, N + 8), 7.0, dtype=torch.bfloat16, device='cuda')
         ops.grouped_gemm_nt(a, w, group, out=out[:, :N], sfa=scales, sfb=sb, num_sms=num_sms, tile_rows=rows, total_rows=bound)
         assert torch.equal(out[valid, :N], want[valid]) and bool((out[~valid] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
@@ -569,6 +569,35 @@ def test_products_that_stream_the_weights(G, N, K, num_sms):
     exact = x @ y.t()
     bound = exact.abs() * 2.0**-8 + (x.abs() @ y.abs().t()) * K * 2.0**-24
     assert bool(((out[:r, :N].double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize('local_expand', [True, False])
+@pytest.mark.parametrize('tokens,K,streams', [(40, 2, True), (448, 1, True), (512, 2, False), (1024, 1, False)])
+def test_the_layer_streams_weights_for_thin_tiles_only(monkeypatch, tokens, K, streams, local_expand):
+    """Both layouts tell the products how many rows there are, forward and backward: 10 and 56 rows per expert are thin tiles, 128 are not."""
+    from deepep_ascend_b200 import ElasticBuffer, _native
+    from deepep_ascend_b200.models.moe import FusedMoE
+    from deepep_ascend_b200.ops import gemm as ops
+    E, H, I = 8, 512, 256
+    routes, product, choice = [], ops.grouped_gemm_nt, _native.load().gemm_streams_weights
+
+    def watched(a, b, tile_group, tile_rows=None, total_rows=0, **kw):
+        counted = int(tile_rows[tile_group >= 0].sum())
+        assert total_rows == counted == tokens * K                    # one rank, nothing dropped
+        routes.append(choice(a.shape[0], b.shape[1], num_groups=E, total_rows=total_rows))
+        return product(a, b, tile_group, tile_rows=tile_rows, total_rows=total_rows, **kw)
+    monkeypatch.setattr(ops, 'grouped_gemm_nt', watched)
+    buf = ElasticBuffer(None, num_max_tokens_per_rank=tokens, hidden=H, num_topk=K, enable_expand=not local_expand, num_experts=E,
+                        expert_alignment=1 if local_expand else 128)
+    try:
+        layer = FusedMoE(buf, E, H, I, fp8_backward=True, local_expand=local_expand)
+        x = torch.randn(tokens, H, device='cuda').bfloat16().requires_grad_(True)
+        at = torch.arange(tokens, device='cuda').unsqueeze(1)
+        idx = (at + torch.arange(K, device='cuda')) % E               # the same number of rows for every expert
+        layer(x, idx, torch.full((tokens, K), 1.0 / K, device='cuda')).sum().backward()
+    finally:
+        buf.destroy()
+    assert routes == [streams] * 4
 
 
 @pytest.mark.parametrize('rows,H,I', [(128, 128, 128), (384, 7168, 384), (2048, 1024, 2048)])
