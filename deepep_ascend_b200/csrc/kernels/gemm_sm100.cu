@@ -976,8 +976,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     p.advance();
                 }
             }
+            // by the thread that has requested the last weights: one thread speaks for its CTA, and the lanes that were not elected are here at once
+            if (few_waves(num_tiles, ctas)) ptx::let_next_kernel_start();
         }
-        if (few_waves(num_tiles, ctas)) ptx::let_next_kernel_start();
     } else if (warp == 1) {
         // ---------------------------------------------------------------------- MMA issuer
         if (ptx::elect_one()) {

@@ -728,6 +728,19 @@ def test_a_product_of_few_sms_in_parts_leaves_the_others_to_an_exchange():
     _assert_a_dispatch_fits_beside(lambda: ops.gemm_nt(a, b, num_sms=16))
 
 
+def test_a_product_of_few_sms_that_streams_weights_leaves_the_others_to_an_exchange():
+    """The same for thin tiles: 128 tiles of 16 token rows, eight waves of 16 CTAs, 268 MB of weights."""
+    from deepep_ascend_b200 import _native
+    from deepep_ascend_b200.ops import gemm as ops
+    G, N, K = 32, 512, 16384
+    assert _native.load().gemm_streams_weights(G * 128, N, num_groups=G, total_rows=G * 16)
+    a, w = torch.zeros(G * 128, K, dtype=torch.uint8, device='cuda'), torch.zeros(G, N, K, dtype=torch.uint8, device='cuda')
+    sa, sb = torch.ones(G * 128, K // 128, device='cuda'), torch.ones(G, N // 128, K // 128, device='cuda')
+    group, rows = torch.arange(G, dtype=torch.int32, device='cuda'), torch.full((G,), 16, dtype=torch.int32, device='cuda')
+    _assert_a_dispatch_fits_beside(lambda: ops.grouped_gemm_nt(a.view(torch.float8_e4m3fn), w.view(torch.float8_e4m3fn), group, sfa=sa, sfb=sb, num_sms=16,
+                                                               tile_rows=rows, total_rows=G * 16))
+
+
 @pytest.mark.parametrize('rows,I', [(768, 2032), (1024, 2048), (1029, 1040), (1152, 2064), (4090, 1808), (4099, 4096), (12300, 2320)])
 @pytest.mark.parametrize('masked', [False, True])
 def test_swiglu_of_rows_that_are_split(rows, I, masked):
