@@ -65,8 +65,8 @@ at::Tensor& gemm_error_flag(int device) {
     return flags[device];
 }
 
-// What gemm_nt chooses for a bf16 product without tile_group, from its sizes alone (host code only): parts along K (1: one chain of K blocks), and CTAs,
-// threads and early launch of the kernel that adds them.
+// What gemm_nt chooses for a bf16 product without tile_group and out, from its sizes alone (host code only): parts along K (1: one chain of K
+// blocks), and CTAs, threads and early launch of the kernel that adds them.
 py::tuple gemm_split_plan(int64_t M, int64_t N, int64_t K, int64_t num_sms, int64_t device_sms) {
     GemmArgs g{};
     g.M = static_cast<int>(M);
@@ -157,8 +157,9 @@ at::Tensor gemm_nt(const at::Tensor& a, const at::Tensor& b, const std::optional
         g.timeout_ns = c0.timeout_ns;
     }
     const int sms = num_sms > 0 ? static_cast<int>(num_sms) : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    // parts along K need a workspace; a caller who brings the result's memory gets a launch that allocates nothing
     at::Tensor partial;
-    g.k_splits = ep::gemm_k_splits(g, sms);
+    g.k_splits = out.has_value() ? 1 : ep::gemm_k_splits(g, sms);
     if (g.k_splits > 1) {
         partial = at::empty({g.k_splits, M, N}, a.options().dtype(at::kFloat));
         g.partial = partial.data_ptr<float>();

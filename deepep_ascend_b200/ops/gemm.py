@@ -19,7 +19,11 @@ def _core_of(buffer):
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, num_sms: int = 0, buffer=None) -> torch.Tensor:
     """``a [M, K] @ b [N, K]^T -> bf16 [M, N]`` (bf16 operands, fp32 accumulation in tensor memory).  With ``buffer``
     (an ``ElasticBuffer``) a pipeline wait that runs out inside the kernel is reported through that buffer's status
-    block and time limit, so ``buffer.check_status()`` raises and poisons it like any other failed device wait."""
+    block and time limit, so ``buffer.check_status()`` raises and poisons it like any other failed device wait.
+
+    Without ``out``, a product of few tiles and a long K is summed in up to 16 parts along K, in 32 bits and in an order that is fixed by M, N, K and
+    ``num_sms``: the bits of a row can change with the batch that it is in.  The parts take a workspace of at most ``num_sms`` x 64 KB from
+    PyTorch's allocator.  With ``out`` nothing is allocated and every sum is one chain along K: a row's bits depend on the row and the weights alone."""
     return _native.load().gemm_nt(a, b, None, None, None, out, num_sms, None, 0, None, _core_of(buffer))
 
 

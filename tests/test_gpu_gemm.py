@@ -144,20 +144,16 @@ def test_k_grouped_gemm_on_row_major_operands(M, N, segs):
                                            (129, 1032, 1992, 40)])
 @pytest.mark.parametrize('captured', [False, True])
 def test_products_whose_k_blocks_are_shared_out(M, N, K, num_sms, captured):
-    """Few tiles and a long K: parts of uneven length, a last K block that is not whole, ragged tiles, an output with a pitch; the same bits on
-    every pass, in a stream and from a CUDA graph, with the products following one another closely (their workspaces are reused)."""
+    """Few tiles and a long K: parts of uneven length, a last K block that is not whole, ragged tiles; the same bits on every pass, in a stream and
+    from a CUDA graph, with the products following one another closely (their workspaces are reused)."""
     from deepep_ascend_b200.ops import gemm as ops
     gen = torch.Generator(device='cuda').manual_seed(M + N + K)
     a, b = torch.randn(M, K, device='cuda', generator=gen).bfloat16(), torch.randn(N, K, device='cuda', generator=gen).bfloat16()
-    full = torch.full((M + 1, N + 8), 7.0, dtype=torch.bfloat16, device='cuda')
-    out = full[:M, :N]
-    ops.gemm_nt(a, b, out=out, num_sms=num_sms)
-    first = out.clone()
+    first = ops.gemm_nt(a, b, num_sms=num_sms)
     exact = a.double() @ b.double().t()
     # fp32 sums rounded once to bf16: half an ulp (2^-9) of the value plus K fp32 roundings of the summed magnitudes
     bound = exact.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24 + 1e-6
     assert bool(((first.double() - exact).abs() <= bound).all())
-    assert bool((full[M] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
 
     def passes():
         return [ops.gemm_nt(a * s, b, num_sms=num_sms) for s in (1.0, 2.0, 4.0, 1.0)]
@@ -173,6 +169,28 @@ def test_products_whose_k_blocks_are_shared_out(M, N, K, num_sms, captured):
         results = passes()
     for got, s in zip(results, (1.0, 2.0, 4.0, 1.0)):        # powers of two: the same roundings
         assert torch.equal(got, first * s)
+
+
+@pytest.mark.parametrize('M,N,K', [(64, 128, 8000), (130, 264, 2056), (512, 1024, 5000), (1, 8, 1600), (300, 256, 7168)])
+def test_products_into_given_memory_are_summed_in_one_chain(M, N, K):
+    """Shapes whose K blocks are shared out otherwise: with `out` nothing is allocated, and the bits of a row are those of the same row
+    among others, on any number of SMs and in a result with a pitch."""
+    from deepep_ascend_b200 import _native
+    from deepep_ascend_b200.ops import gemm as ops
+    assert _native.load().gemm_split_plan(M, N, K, num_sms=148, device_sms=148)[0] > 1
+    gen = torch.Generator(device='cuda').manual_seed(M + N + K)
+    b = torch.randn(N, K, device='cuda', generator=gen).bfloat16()
+    a = torch.randn(20000, K, device='cuda', generator=gen).bfloat16()
+    many = torch.empty(20000, N, dtype=torch.bfloat16, device='cuda')
+    ops.gemm_nt(a, b, out=many)
+    full = torch.empty(M + 1, N + 8, dtype=torch.bfloat16, device='cuda')
+    for num_sms in (0, 24, 100, 1):
+        full.fill_(7.0)
+        out, rows = full[:M, :N], a[:M]
+        before = torch.cuda.memory_stats()['allocation.all.allocated']
+        ops.gemm_nt(rows, b, out=out, num_sms=num_sms)
+        assert torch.cuda.memory_stats()['allocation.all.allocated'] == before
+        assert torch.equal(out, many[:M]) and bool((full[M] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
 
 
 @pytest.mark.parametrize('M,N,K,num_sms', [(128, 256, 128, 0), (300, 264, 256, 0), (513, 520, 1152, 2), (200, 1032, 384, 1),
