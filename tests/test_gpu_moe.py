@@ -535,10 +535,11 @@ def test_products_that_stream_the_weights(G, N, K, num_sms):
     number of token rows at which the kernel changes its way, idle tiles, two tiles of one group, a ragged last tile, odd K blocks,
     columns that end inside a tile, last waves that are cut and whole, and scales in either order; a count of the rows that rules the
     kernel out, or none, changes nothing."""
+    from deepep_ascend_b200 import _native
     from deepep_ascend_b200.ops import gemm as ops
     gen = torch.Generator(device='cuda').manual_seed(N)
     edges = [1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 127, 128, 0, 40]
-    tiles = G if G < 16 else 48
+    tiles = min(G, 48)
     rows = torch.tensor([edges[(5 * t + G) % len(edges)] for t in range(tiles)], dtype=torch.int32, device='cuda')
     M = tiles * 128 - 72                                          # the last tile has 56 rows in the tensor
     rows[-1] = 128
@@ -556,19 +557,24 @@ def test_products_that_stream_the_weights(G, N, K, num_sms):
     at = torch.arange(M, device='cuda')
     valid = (at % 128 < rows[at // 128]) & (group[at // 128] >= 0)
     a.view(torch.uint8)[~valid] = 0x7f
-    for scales, bound in ((sa, 1), (sa.t().contiguous().t(), 1), (sa, 0), (sa, M)):
+    streams = _native.load().gemm_streams_weights
+    for scales, bound in ((sa, 0), (sa, M), (sa.t().contiguous().t(), 1), (sa, 1)):
+        assert streams(M, N, num_groups=G, total_rows=bound) == (bound == 1)
         out = torch.full((M, N + 8), 7.0, dtype=torch.bfloat16, device='cuda')
         ops.grouped_gemm_nt(a, w, group, out=out[:, :N], sfa=scales, sfb=sb, num_sms=num_sms, tile_rows=rows, total_rows=bound)
         assert torch.equal(out[valid, :N], want[valid]) and bool((out[~valid] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
-    # and the product itself, in 64 bits: sums of K products in 32 bits and one rounding to bf16 (2^-8)
-    t = 0
-    r = int(rows[t])
+    # and the product itself (the streaming kernel's, of the last pass), in 64 bits: sums of K products in 32 bits and one rounding to bf16 (2^-8)
     k_scale = lambda s: s.repeat_interleave(128, dim=-1)[..., :K]    # noqa: E731
-    x = a[:r].double() * k_scale(sa[:r]).double()
-    y = w[0].double() * k_scale(sb[0].repeat_interleave(128, dim=0)[:N]).double()
-    exact = x @ y.t()
-    bound = exact.abs() * 2.0**-8 + (x.abs() @ y.abs().t()) * K * 2.0**-24
-    assert bool(((out[:r, :N].double() - exact).abs() <= bound).all())
+    for t in range(tiles):
+        e, r = int(group[t]), min(int(rows[t]), M - t * 128)
+        if e < 0 or r == 0:
+            continue
+        at = slice(t * 128, t * 128 + r)
+        x = a[at].double() * k_scale(sa[at]).double()
+        y = w[e].double() * k_scale(sb[e].repeat_interleave(128, dim=0)[:N]).double()
+        exact = x @ y.t()
+        bound = exact.abs() * 2.0**-8 + (x.abs() @ y.abs().t()) * K * 2.0**-24
+        assert bool(((out[at, :N].double() - exact).abs() <= bound).all()), t
 
 
 @pytest.mark.parametrize('local_expand', [True, False])
