@@ -397,9 +397,9 @@ const void* combine_fn(int unroll, bool full, int n) {
     }
 }
 
-// Column chunk = 512 B x unroll.  A warp's chain per chunk (about 1.5 us whatever the chunk's size) is what bounds the kernel, so a row is
-// cut into as few chunks of at most 4 KB as it takes, all alike: 3001 tokens x 4096, six rows each, 64 SMs: 47 us in chunks of 2 KB,
-// 31 us in chunks of 4 KB (the sums of a 4 KB chunk take 64 of the 128 registers).
+// Column chunk = 512 B x unroll.  A warp's chain per chunk, which hardly grows with the chunk, is what bounds the kernel, so a row is cut into
+// as few chunks of at most 4 KB as it takes, all alike: 3001 tokens x 4096, six rows each, 64 SMs: 60 us in chunks of 2 KB, 43 us in
+// chunks of 4 KB, weighted or not (the sums of a 4 KB chunk take 64 of the 128 registers).
 inline int pick_unroll(const CombineArgs& a) {
     const int steps = (a.hidden * 2 + 511) / 512, chunks = (steps + 7) / 8, unroll = (steps + chunks - 1) / chunks;
     return unroll == 3 ? 4 : unroll;

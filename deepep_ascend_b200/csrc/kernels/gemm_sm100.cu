@@ -89,7 +89,7 @@ __device__ __forceinline__ uint64_t wait_limit_ns(const GemmArgs& g) { return g.
 // A pipeline wait ran out: stop this CTA's loops, raise the per-device flag and, when the caller gave the status block of
 // a communication buffer, record the failure there too, so that the buffer's check_status() reports it and poisons the
 // buffer like any other failed device wait.  `code`: 1 = empty stage, 2 = free accumulator, 3 = rows-ready flag,
-// 4 = full stage, 5 = finished accumulator, 7 = all-gather copy.
+// 4 = full stage, 5 = finished accumulator, 6 = scales of the streaming kernel (a slot, or its values), 7 = all-gather copy.
 __device__ __forceinline__ void gemm_fail_values(int* error, uint64_t* status, int status_rank, int* failed, int code) {
     *failed = code;
     if (error != nullptr && atomicCAS(error, 0, code) == 0 && status != nullptr) {
@@ -906,7 +906,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         it.out_rows = item < whole ? 128 : 128 / cut;
         it.m = tile / num_n;
         it.col0 = (tile - it.m * num_n) * 128 + piece * it.out_rows;
-        it.rows = g.tile_rows != nullptr ? *(g.tile_rows + it.m) : kBlockM;
+        it.rows = *(g.tile_rows + it.m);
         it.grp = g.tile_group != nullptr ? *(g.tile_group + it.m) : 0;
         return it;
     };
@@ -1424,7 +1424,6 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         if (g.M / kBlockM >= EP_MAX_TILE_FLAGS - 1) return cudaErrorInvalidValue;
         return cudaLaunchCooperativeKernel(fn, dim3(ctas, 1, 1), dim3(kGemmThreads, 1, 1), params, kGemmSmemBytes, stream);
     }
-    // whole tiles, or halves where all of them fit into one wave (the kernel cuts its last wave by the same rule)
     if (g.k_splits > 1) {
         // (one wave of 128-column tiles: gemm_k_splits)
         if (fn != (const void*)gemm_kernel<false, 128, 0> || g.partial == nullptr || reinterpret_cast<uintptr_t>(g.partial) % 16 != 0 || g.tile_group != nullptr)
@@ -1444,6 +1443,7 @@ cudaError_t launch_gemm(const GemmArgs& g, int num_sms, cudaStream_t stream) {
         if (r.beside_product) return launch_dependent(reduce, dim3(r.ctas, 1, 1), dim3(r.threads, 1, 1), reduce_params, 0, stream);
         return cudaLaunchKernel(reduce, dim3(r.ctas, 1, 1), dim3(r.threads, 1, 1), reduce_params, 0, stream);
     }
+    // whole tiles, or halves where all of them fit into one wave (the kernel cuts its last wave by the same rule)
     if (ctas > num_tiles) ctas = g.is_fp8 && block_n == 256 && 2 * num_tiles <= ctas ? 2 * num_tiles : num_tiles;
     const dim3 block(gemm_threads(g.is_fp8 != 0, block_n), 1, 1);
     if (few_waves(num_tiles, ctas)) return launch_dependent(fn, dim3(ctas, 1, 1), block, params, kGemmSmemBytes, stream);

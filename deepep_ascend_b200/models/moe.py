@@ -66,7 +66,7 @@ class _MoEFunction(torch.autograd.Function):
             lo, hi = bounds[c], bounds[c + 1]
             (rx, rsf), recv_idx, recv_w, handle, ev = disp.pop(c)
             ev.current_stream_wait()
-            total_rows = handle.num_recv_tokens * topk_idx.shape[1]       # (token, lane) pairs: an upper bound of the expert rows
+            total_rows = handle.num_recv_tokens * handle.num_topk       # (token, lane) pairs: an upper bound of the expert rows
             if local:
                 # One row per (token, rank) came over NVLink; every local expert the token selected gets its copy here, in the
                 # expert's 128-aligned segment (rows in received order).  The copies are private to this call.
@@ -118,7 +118,7 @@ class _MoEFunction(torch.autograd.Function):
             rx, rsf, recv_w, h, tile_group, valid_row, seg_off, pos, tile_rows = ctx.saved_tensors[9 * c:9 * c + 9]
             rw = recv_w.contiguous()
             local, rows = layer.local_expand, h.shape[0]
-            total_rows = handle.num_recv_tokens * handle.topk_idx.shape[1]          # as in the forward pass
+            total_rows = handle.num_recv_tokens * handle.num_topk          # as in the forward pass
 
             def send_home(d_rows_exp, d_w_rows):
                 """Backward of dispatch: the gradient rows (and the gradient of every routing weight) travel to the tokens' ranks."""
